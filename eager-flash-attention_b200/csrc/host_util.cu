@@ -145,34 +145,45 @@ int* work_counter_slot()
     return ring[dev] + (next[dev]++ % kSlots);
 }
 
-int make_tmap_f16(CUtensorMap* out, const void* base, int rank,
-                  const unsigned long long* dims, const unsigned long long* strides_bytes,
-                  const unsigned* box)
+static int make_tmap(CUtensorMap* out, CUtensorMapDataType type, unsigned elem_bytes, const void* base, int rank,
+                     const unsigned long long* dims, const unsigned long long* strides_bytes, const unsigned* box)
 {
     const DriverApi* api = driver_api();
     if (!api) return 1;
-    if (rank < 2 || rank > 3) { set_error("make_tmap_f16: rank %d unsupported", rank); return 1; }
-    if (((uintptr_t)base & 15) != 0) { set_error("make_tmap_f16: base address not 16-byte aligned"); return 1; }
-    const unsigned inner_bytes = box[0] * 2u;
+    if (rank < 2 || rank > 3) { set_error("make_tmap: rank %d unsupported", rank); return 1; }
+    if (((uintptr_t)base & 15) != 0) { set_error("make_tmap: base address not 16-byte aligned"); return 1; }
+    const unsigned inner_bytes = box[0] * elem_bytes;
     CUtensorMapSwizzle swz;
     switch (inner_bytes) {
         case 128: swz = CU_TENSOR_MAP_SWIZZLE_128B; break;
         case 64:  swz = CU_TENSOR_MAP_SWIZZLE_64B;  break;
         case 32:  swz = CU_TENSOR_MAP_SWIZZLE_32B;  break;
-        default: set_error("make_tmap_f16: inner box of %u bytes has no swizzle mode", inner_bytes); return 1;
+        default: set_error("make_tmap: inner box of %u bytes has no swizzle mode", inner_bytes); return 1;
     }
     cuuint64_t gdim[3]; cuuint64_t gstr[2]; cuuint32_t bdim[3]; cuuint32_t estr[3];
     for (int i = 0; i < rank; i++) { gdim[i] = dims[i]; bdim[i] = box[i]; estr[i] = 1; }
     for (int i = 0; i + 1 < rank; i++) {
-        if (strides_bytes[i] % 16 != 0) { set_error("make_tmap_f16: stride %d (%llu B) not a multiple of 16", i, strides_bytes[i]); return 1; }
+        if (strides_bytes[i] % 16 != 0) { set_error("make_tmap: stride %d (%llu B) not a multiple of 16", i, strides_bytes[i]); return 1; }
         gstr[i] = strides_bytes[i];
     }
-    CUresult r = api->cuTensorMapEncodeTiled(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank,
+    CUresult r = api->cuTensorMapEncodeTiled(out, type, (cuuint32_t)rank,
                                              const_cast<void*>(base), gdim, gstr, bdim, estr,
                                              CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
                                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return check_cu(r, "cuTensorMapEncodeTiled", __FILE__, __LINE__);
+}
+
+int make_tmap_f16(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
+                  const unsigned long long* strides_bytes, const unsigned* box)
+{
+    return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2u, base, rank, dims, strides_bytes, box);
+}
+
+int make_tmap_f32(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
+                  const unsigned long long* strides_bytes, const unsigned* box)
+{
+    return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4u, base, rank, dims, strides_bytes, box);
 }
 
 }  // namespace efa

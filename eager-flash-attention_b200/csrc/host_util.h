@@ -64,5 +64,8 @@ int* work_counter_slot();
 int make_tmap_f16(CUtensorMap* out, const void* base, int rank,
                   const unsigned long long* dims, const unsigned long long* strides_bytes /* rank-1 */,
                   const unsigned* box);
+// The same over fp32 data.
+int make_tmap_f32(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
+                  const unsigned long long* strides_bytes, const unsigned* box);
 
 }  // namespace efa

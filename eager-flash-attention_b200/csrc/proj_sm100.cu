@@ -4,8 +4,17 @@
 // Stands in for project() of eager-flash-attention (attn_main.cu:262-273), which calls cublasSgemm on
 // fp32 data. Warp-specialised: warp 0 streams A (K-major, [128 rows][64 k]) and W (MN-major,
 // [64 k][BN columns] as 64-column boxes) through a ring of shared-memory stages with TMA; warp 1
-// issues tcgen05.mma (128 x BN x 16) into a BN-column fp32 accumulator in tensor memory and frees each
-// stage with tcgen05.commit; warps 2-5 read the accumulator (tcgen05.ld), round to fp16 and store.
+// issues tcgen05.mma (128 x BN x 16) into one of two BN-column fp32 accumulators in tensor memory and frees each
+// stage with tcgen05.commit; warps 2-5 read the accumulator (tcgen05.ld), round to fp16, stage 32 rows x 128 bytes
+// per warp in shared memory and store them with TMA (which clips ragged edges).
+//
+// A CTA keeps taking tiles for as long as blocks of its grid are waiting: clusterlaunchcontrol.try_cancel hands it
+// the coordinates of a block that has not started. The copies and MMAs of the next tile then run while this tile is
+// written, and barriers and tensor memory are set up once per SM, which is most of the time where d_local is small
+// (a 128 x 256 tile of d_local = 512 is 4k cycles of MMA). Unlike a grid of one CTA per SM with a fixed share of the
+// tiles, it also suits the launch that starts beside the attention kernel: SMs that come free late find only the
+// tiles that nobody has taken. Measured, 4160 x 512 x 4096 (17.4 GFLOP): 30.7 us with a block per tile and row-wise
+// stores from registers, 24.2 us like this.
 #include "fa_fwd_sm100.cuh"
 #include "host_util.h"
 #include "sm100_ptx.cuh"
@@ -16,6 +25,7 @@ namespace {
 
 constexpr int PJ_BM = 128;
 constexpr int PJ_BK = 64;
+constexpr int PJ_EPI_WARPS = 4;
 
 template <int BN>
 struct PjCfg {
@@ -24,18 +34,20 @@ struct PjCfg {
     static constexpr int B_BYTES    = B_BOX * (BN / 64);
     static constexpr int STAGE      = A_BYTES + B_BYTES;
     static constexpr int NSTAGE     = BN == 256 ? 4 : 6;
-    static constexpr int SMEM_BYTES = STAGE * NSTAGE + 1024;
+    static constexpr int OUT_BOX    = 32 * 128;                   // 32 rows of 128 bytes: one TMA store of one warp
+    static constexpr int OUT_BYTES  = PJ_EPI_WARPS * 2 * OUT_BOX; // two per warp
+    static constexpr int SMEM_BYTES = STAGE * NSTAGE + OUT_BYTES + 1024;
 };
 
 struct PjArgs {
-    void* out;          // fp16 or fp32 [M][N]
     int M, N, K;
     int* status;
 };
 
 template <int BN, bool OUT_F32>
-__global__ void __launch_bounds__(192)
-proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const PjArgs a)
+__global__ void __launch_bounds__(192, 1)
+proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
+                 const __grid_constant__ CUtensorMap tmOut, const PjArgs a)
 {
     using C = PjCfg<BN>;
     constexpr uint32_t IDESC = idesc_f16_f32(PJ_BM, BN, 0, 1);
@@ -43,106 +55,174 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sOut = smem + C::NSTAGE * C::STAGE;
 
     __shared__ __align__(8) uint64_t bar_full[C::NSTAGE];
     __shared__ __align__(8) uint64_t bar_empty[C::NSTAGE];
-    __shared__ __align__(8) uint64_t bar_acc;
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t next_full[2], next_empty[2];
+    __shared__ __align__(16) uint4 next_tile[2];                  // answers of try_cancel
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_word;
 
     const int tid  = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    const int n0 = blockIdx.x * BN;
-    const int m0 = blockIdx.y * PJ_BM;
     const int num_k = (a.K + PJ_BK - 1) / PJ_BK;
 
     if (tid == 0) {
         abort_word = 0;
         for (int s = 0; s < C::NSTAGE; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
-        mbar_init(&bar_acc, 1);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], PJ_EPI_WARPS);
+            mbar_init(&next_full[s], 1);
+            mbar_init(&next_empty[s], 1 + PJ_EPI_WARPS);          // everyone but the thread that asks
+        }
         mbar_fence_init();
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmW);
+        tma_prefetch_desc(&tmOut);
     }
     __syncwarp();
-    if (warp == 1) tmem_alloc(&tmem_base_smem, BN);
+    if (warp == 1) tmem_alloc(&tmem_base_smem, 2 * BN);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_acc = tmem_base_smem;
+    const uint32_t tmem_base = tmem_base_smem;
+
+    // Tile of round `it`: the CTA's own block first, then the answer to request it - 1. false: no more (or gave up).
+    auto next = [&](int it, int& bx, int& by) -> bool {
+        const int s = it & 1;
+        if (!mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
+        return clc_query(&next_tile[s], bx, by);
+    };
 
     if (warp == 0) {
-        // ---- TMA producer
+        // ---- TMA producer; also asks for the next tile at the start of every tile
         if (lane == 0) {
-            for (int kb = 0; kb < num_k; kb++) {
-                const int s = kb % C::NSTAGE;
-                const int use = kb / C::NSTAGE;
-                if (use > 0 && !mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), &abort_word, 11)) break;
-                uint8_t* sa = smem + s * C::STAGE;
-                uint8_t* sb = sa + C::A_BYTES;
-                mbar_expect_tx(&bar_full[s], C::STAGE);
-                tma_load_2d(sa, &tmA, &bar_full[s], kb * PJ_BK, m0);
-                #pragma unroll
-                for (int nb = 0; nb < BN / 64; nb++)
-                    tma_load_2d(sb + nb * C::B_BOX, &tmW, &bar_full[s], n0 + nb * 64, kb * PJ_BK);
+            int bx = blockIdx.x, by = blockIdx.y;
+            int g = 0;                                            // stages filled so far, over all tiles
+            bool ok = true;
+            for (int it = 0; ok; it++) {
+                const int ns = it & 1;
+                if (it >= 2 && !mbar_wait(&next_empty[ns], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 15)) break;
+                mbar_expect_tx(&next_full[ns], 16);
+                clc_try_cancel(&next_tile[ns], &next_full[ns]);
+                const int n0 = bx * BN, m0 = by * PJ_BM;
+                const int nbox = min(BN / 64, (a.N - n0) / 64);   // N is a multiple of 64
+                for (int kb = 0; kb < num_k; kb++, g++) {
+                    const int s = g % C::NSTAGE;
+                    const int use = g / C::NSTAGE;
+                    if (use > 0 && !mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), &abort_word, 11)) { ok = false; break; }
+                    uint8_t* sa = smem + s * C::STAGE;
+                    uint8_t* sb = sa + C::A_BYTES;
+                    mbar_expect_tx(&bar_full[s], C::A_BYTES + nbox * C::B_BOX);
+                    tma_load_2d(sa, &tmA, &bar_full[s], kb * PJ_BK, m0);
+                    for (int nb = 0; nb < nbox; nb++)
+                        tma_load_2d(sb + nb * C::B_BOX, &tmW, &bar_full[s], n0 + nb * 64, kb * PJ_BK);
+                }
+                if (!ok || !next(it, bx, by)) break;
+                fence_proxy_async_smem();
             }
         }
     } else if (warp == 1) {
         // ---- MMA issuer
         if (lane == 0) {
+            int bx = 0, by = 0, g = 0;
             bool ok = true;
-            for (int kb = 0; kb < num_k && ok; kb++) {
-                const int s = kb % C::NSTAGE;
-                ok = mbar_wait(&bar_full[s], (uint32_t)((kb / C::NSTAGE) & 1), &abort_word, 12);
-                if (!ok) break;
-                tc_fence_after_sync();
-                const uint32_t sa = smem_u32(smem + s * C::STAGE);
-                const uint32_t sb = sa + C::A_BYTES;
-                #pragma unroll
-                for (int ks = 0; ks < PJ_BK / 16; ks++) {
-                    tc_mma_ss(tmem_acc,
-                              smem_desc(sa + ks * 32, 16, 1024, SWZ),                    // K-major: 32 B per 16 k
-                              smem_desc(sb + ks * 16 * 128, C::B_BOX, 1024, SWZ),        // MN-major: 16 k rows of 128 B
-                              IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+            for (int it = 0; ok; it++) {
+                const int acc = it & 1;
+                if (it >= 2) {
+                    ok = mbar_wait(&acc_empty[acc], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 16);
+                    if (!ok) break;
+                    tc_fence_after_sync();
                 }
-                tc_commit(&bar_empty[s]);
+                const uint32_t tmem_acc = tmem_base + acc * BN;
+                for (int kb = 0; kb < num_k && ok; kb++, g++) {
+                    const int s = g % C::NSTAGE;
+                    ok = mbar_wait(&bar_full[s], (uint32_t)((g / C::NSTAGE) & 1), &abort_word, 12);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const uint32_t sa = smem_u32(smem + s * C::STAGE);
+                    const uint32_t sb = sa + C::A_BYTES;
+                    #pragma unroll
+                    for (int ks = 0; ks < PJ_BK / 16; ks++) {
+                        tc_mma_ss(tmem_acc,
+                                  smem_desc(sa + ks * 32, 16, 1024, SWZ),                    // K-major: 32 B per 16 k
+                                  smem_desc(sb + ks * 16 * 128, C::B_BOX, 1024, SWZ),        // MN-major: 16 k rows of 128 B
+                                  IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+                    }
+                    tc_commit(&bar_empty[s]);
+                }
+                if (!ok) break;
+                tc_commit(&acc_full[acc]);
+                const bool more = next(it, bx, by);
+                fence_proxy_async_smem();
+                mbar_arrive(&next_empty[it & 1]);
+                if (!more) break;
             }
-            if (ok) tc_commit(&bar_acc);
         }
     } else {
         // ---- epilogue: warps 2..5 own TMEM lanes 32*(warp % 4) .. +31
+        constexpr int COLS = OUT_F32 ? 32 : 64;                   // columns in 128 bytes
         const int lane_grp = warp & 3;
-        const int row = m0 + lane_grp * 32 + lane;
-        if (mbar_wait(&bar_acc, 0, &abort_word, 13)) {
+        uint8_t* box0 = sOut + lane_grp * 2 * C::OUT_BOX;
+        int bx = blockIdx.x, by = blockIdx.y;
+        int stores = 0;
+        for (int it = 0; ; it++) {
+            const int acc = it & 1;
+            const int row0 = by * PJ_BM + lane_grp * 32, n0 = bx * BN;
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (uint32_t)((it >> 1) & 1), &abort_word, 13))) break;
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_acc + ((uint32_t)(lane_grp * 32) << 16);
+            const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(lane_grp * 32) << 16);
             #pragma unroll 1
-            for (int c = 0; c < BN / 32; c++) {
-                uint32_t r[32];
-                tmem_ld32(taddr + c * 32, r);
-                tmem_wait_ld();
-                const int col = n0 + c * 32;
-                if (OUT_F32) {
-                    if (row < a.M && col < a.N) {
-                        uint4* dst = reinterpret_cast<uint4*>(static_cast<float*>(a.out) + (size_t)row * a.N + col);
-                        #pragma unroll
-                        for (int q = 0; q < 8; q++) dst[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                    }
-                } else if (row < a.M && col < a.N) {   // N is a multiple of 64, so a 32-column chunk is all in or all out
-                    uint4* dst = reinterpret_cast<uint4*>(static_cast<__half*>(a.out) + (size_t)row * a.N + col);
+            for (int c = 0; c < BN / COLS; c++, stores++) {
+                if (n0 + c * COLS >= a.N) break;
+                uint4 v[8];                                       // this lane's row: eight 16-byte chunks
+                if constexpr (OUT_F32) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + c * 32, r);
+                    tmem_wait_ld();
                     #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        uint4 v;
-                        v.x = pack_f16x2(__uint_as_float(r[8 * q + 0]), __uint_as_float(r[8 * q + 1]));
-                        v.y = pack_f16x2(__uint_as_float(r[8 * q + 2]), __uint_as_float(r[8 * q + 3]));
-                        v.z = pack_f16x2(__uint_as_float(r[8 * q + 4]), __uint_as_float(r[8 * q + 5]));
-                        v.w = pack_f16x2(__uint_as_float(r[8 * q + 6]), __uint_as_float(r[8 * q + 7]));
-                        dst[q] = v;
+                    for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                } else {
+                    uint32_t r[2][32];
+                    tmem_ld32(taddr + c * 64, r[0]);
+                    tmem_ld32(taddr + c * 64 + 32, r[1]);
+                    tmem_wait_ld();
+                    #pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const uint32_t* x = &r[q >> 2][8 * (q & 3)];
+                        v[q].x = pack_f16x2(__uint_as_float(x[0]), __uint_as_float(x[1]));
+                        v[q].y = pack_f16x2(__uint_as_float(x[2]), __uint_as_float(x[3]));
+                        v[q].z = pack_f16x2(__uint_as_float(x[4]), __uint_as_float(x[5]));
+                        v[q].w = pack_f16x2(__uint_as_float(x[6]), __uint_as_float(x[7]));
                     }
                 }
+                uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
+                if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
+                __syncwarp();
+                #pragma unroll
+                for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
+                    *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (row0 < a.M) tma_store_2d(&tmOut, box, n0 + c * COLS, row0);
+                    tma_store_commit();                           // also without a store: the waits above count groups
+                }
             }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            const bool more = __all_sync(0xffffffffu, next(it, bx, by));
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&next_empty[it & 1]);
+            if (!more) break;
         }
+        if (lane == 0) tma_store_wait_all();
     }
 
     __syncwarp();
@@ -158,11 +238,11 @@ proj_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         __syncthreads();
     }
-    if (warp == 1) tmem_dealloc(tmem_acc, BN);
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
 }
 
 template <int BN, bool OUT_F32>
-int launch_proj(const CUtensorMap& ta, const CUtensorMap& tw, const PjArgs& args, cudaStream_t stream)
+int launch_proj(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& to, const PjArgs& args, cudaStream_t stream)
 {
     using C = PjCfg<BN>;
     static bool configured[64] = {};
@@ -173,7 +253,7 @@ int launch_proj(const CUtensorMap& ta, const CUtensorMap& tw, const PjArgs& args
         configured[dev] = true;
     }
     dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
-    proj_gemm_kernel<BN, OUT_F32><<<grid, 192, C::SMEM_BYTES, stream>>>(ta, tw, args);
+    proj_gemm_kernel<BN, OUT_F32><<<grid, 192, C::SMEM_BYTES, stream>>>(ta, tw, to, args);
     EFA_CUDA(cudaGetLastError());
     return 0;
 }
@@ -188,7 +268,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     if (d <= 0 || d % 64 != 0) { set_error("project: d (%d) must be a positive multiple of 64", d); return 2; }
     if (!A || !W || !out) { set_error("project: null pointer"); return 2; }
 
-    CUtensorMap ta, tw;
+    CUtensorMap ta, tw, to;
     {
         unsigned long long dims[2] = {(unsigned long long)d_local, (unsigned long long)rows};
         unsigned long long strides[1] = {(unsigned long long)d_local * 2ull};
@@ -201,11 +281,21 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
         unsigned box[2] = {64u, 64u};
         if (make_tmap_f16(&tw, W, 2, dims, strides, box)) return 1;
     }
-    PjArgs a{out, rows, d, d_local, kernel_status_word()};
-    const long tiles256 = (long)((rows + 127) / 128) * (d / 256);
-    const bool wide = d % 256 == 0 && tiles256 >= 148;
-    if (out_dtype == EFA_F32) return wide ? launch_proj<256, true>(ta, tw, a, stream) : launch_proj<128, true>(ta, tw, a, stream);
-    return wide ? launch_proj<256, false>(ta, tw, a, stream) : launch_proj<128, false>(ta, tw, a, stream);
+    {
+        const bool f32 = out_dtype == EFA_F32;
+        unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)rows};
+        unsigned long long strides[1] = {(unsigned long long)d * (f32 ? 4ull : 2ull)};
+        unsigned box[2] = {f32 ? 32u : 64u, 32u};
+        if (f32 ? make_tmap_f32(&to, out, 2, dims, strides, box) : make_tmap_f16(&to, out, 2, dims, strides, box)) return 1;
+    }
+    PjArgs a{rows, d, d_local, kernel_status_word()};
+    // Tile width: the one that leaves the busiest SM fewer columns to compute; the wide one (each A tile read half as
+    // often) where both are equal.
+    const long row_tiles = (rows + PJ_BM - 1) / PJ_BM;
+    auto busiest = [&](int bn) { return (row_tiles * ((d + bn - 1) / bn) + 147) / 148 * bn; };
+    const bool wide = busiest(256) <= busiest(128);
+    if (out_dtype == EFA_F32) return wide ? launch_proj<256, true>(ta, tw, to, a, stream) : launch_proj<128, true>(ta, tw, to, a, stream);
+    return wide ? launch_proj<256, false>(ta, tw, to, a, stream) : launch_proj<128, false>(ta, tw, to, a, stream);
 }
 
 

@@ -145,8 +145,41 @@ __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
+__device__ __forceinline__ void tma_store_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+
 // Generic-proxy writes to shared memory must be fenced before the async proxy (TMA store, tcgen05.mma) reads them.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
+// Cluster launch control: take over a block of this grid that has not started
+// ---------------------------------------------------------------------------------------------
+// The answer (16 bytes) arrives at `answer` and counts as 16 transaction bytes on `bar`. Not to be called again
+// after an answer that said no.
+__device__ __forceinline__ void clc_try_cancel(uint4* answer, uint64_t* bar)
+{
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 :: "r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
+}
+
+// true: the block (x, y) is now the caller's and will not be launched.
+__device__ __forceinline__ bool clc_query(const uint4* answer, int& x, int& y)
+{
+    uint32_t got, cx, cy;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b32 z;\n"
+        ".reg .b128 h;\n"
+        "ld.shared.b128 h, [%3];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "mov.u32 %1, 0;\n"
+        "mov.u32 %2, 0;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, z, _}, h;\n"
+        "}\n" : "=&r"(got), "=&r"(cx), "=&r"(cy) : "r"(smem_u32(answer)) : "memory");
+    if (got) { x = (int)cx; y = (int)cy; }
+    return got != 0;
+}
 
 // ---------------------------------------------------------------------------------------------
 // TMEM + tcgen05

@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("rows,d_local,d", [(64, 16, 64), (128, 64, 64), (128, 128, 1024), (64, 512, 1024),
                                              (256, 1024, 1024), (192, 32, 256), (2048, 512, 512), (4096, 256, 4096),
-                                             (128, 4096, 4096), (19072, 128, 1024)])
+                                             (128, 4096, 4096), (19072, 128, 1024),
+                                             # several tiles per SM, with ragged last rows and columns, one k-block and many
+                                             (19136, 48, 320), (9536, 16, 704), (4160, 512, 4096), (64, 80, 448)])
 def test_projection_matches_float64(pkg, torch_cuda, rows, d_local, d):
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(rows + d_local + d)

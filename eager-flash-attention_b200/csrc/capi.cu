@@ -71,13 +71,9 @@ extern "C" int efa_compute_qkv_f16(const void* X, const void* W_q, const void* W
     if (!X || !W_q || !W_k || !W_v || !Qh || !Kh || !Vh) { set_error("efa_compute_qkv_f16: null argument"); return 2; }
     if (d_h != 64 && d_h != 128) { set_error("efa_compute_qkv_f16: d_h must be 64 or 128 (got %d)", d_h); return 2; }
     if (H_local < 1) { set_error("efa_compute_qkv_f16: H_local must be positive"); return 2; }
-    const __half* W[3] = {static_cast<const __half*>(W_q), static_cast<const __half*>(W_k), static_cast<const __half*>(W_v)};
-    __half* out[3] = {static_cast<__half*>(Qh), static_cast<__half*>(Kh), static_cast<__half*>(Vh)};
-    for (int h = 0; h < H_local; h++)
-        for (int t = 0; t < 3; t++)
-            if (int rc = project_f16(X, W[t] + (size_t)h * d * d_h, out[t] + (size_t)h * S * d_h, S, d, d_h, (cudaStream_t)stream))
-                return rc;
-    return 0;
+    const void* W[3] = {W_q, W_k, W_v};
+    void* out[3] = {Qh, Kh, Vh};
+    return project_heads_f16(X, W, out, S, d, H_local, d_h, (cudaStream_t)stream);
 }
 
 extern "C" int efa_kernel_status(int* out4)

@@ -41,7 +41,9 @@ def test_projection_rejects_bad_shapes(pkg, torch_cuda):
         pkg.project(A, W, out, 128, 64, 96)
 
 
-@pytest.mark.parametrize("S,d,H_local,d_h", [(512, 512, 4, 128), (1024, 1024, 2, 64), (2048, 256, 4, 64)])
+@pytest.mark.parametrize("S,d,H_local,d_h", [(512, 512, 4, 128), (1024, 1024, 2, 64), (2048, 256, 4, 64),
+                                            # tiles that span heads and tensors, ragged rows, columns and k; several tiles per SM
+                                            (192, 80, 3, 64), (64, 16, 1, 64), (320, 144, 1, 128), (8256, 208, 5, 64), (4160, 96, 3, 128)])
 def test_compute_qkv_matches_float64(pkg, torch_cuda, S, d, H_local, d_h):
     """The step before the block (compute_qkv, attn_main.cu:127-153) on fp16 data, head-major output."""
     torch = torch_cuda

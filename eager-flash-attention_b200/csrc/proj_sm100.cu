@@ -292,13 +292,14 @@ int launch_proj(const PjMaps& maps, const PjArgs& args, cudaStream_t stream)
     return 0;
 }
 
-// Tile width: the one that leaves the busiest SM fewer columns to compute; the wide one (each A tile read half as
-// often) where both are equal.
+// Tile width: the one that leaves the busiest SM less to fetch. What bounds the kernel is the rate at which tiles come
+// from L2 (48 KB per 64 k for a wide tile, 32 KB for a narrow one, 512 and 256 cycles of MMA), so wide tiles count 3, narrow
+// ones 2: 4096 x 4096 x 4096 keeps wide tiles although narrow ones would leave the busiest SM fewer columns.
 bool wide_tiles(int rows, int cols)
 {
     const long row_tiles = (rows + PJ_BM - 1) / PJ_BM;
-    auto busiest = [&](int bn) { return (row_tiles * ((cols + bn - 1) / bn) + 147) / 148 * bn; };
-    return busiest(256) <= busiest(128);
+    auto waves = [&](int bn) { return (row_tiles * ((cols + bn - 1) / bn) + 147) / 148; };
+    return waves(256) * 3 <= waves(128) * 2;
 }
 
 int check_shape(int rows, int d_local, int d)

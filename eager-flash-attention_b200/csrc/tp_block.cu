@@ -89,6 +89,25 @@ struct Run {
     size_t send_row_bytes() const { return (size_t)p.d * (wire_f32() ? sizeof(float) : sizeof(__half)); }
     char* send_base() const { return static_cast<char*>(pull() ? nvls_pull_send_buf(c) : nvls() ? nvls_send_buf(c) : c->send_buf); }
 
+    // One rank: its partial sum is the result, so the projection writes `output` itself and nothing is reduced. A
+    // one-rank AllReduce is a copy (0.5 GB read and written at 32k rows of d = 4096) and, tile by tile, a launch and several
+    // microseconds of host time per group. Not where the kernel's TMA stores could not go (an output that is
+    // not this GPU's own memory or not 16-byte aligned) or where writing early would disturb W_O.
+    bool direct = false;
+    void choose_direct(const void* output)
+    {
+        if (p.R != 1 || p.skip_comm || p.skip_proj || p.reduce == EFA_REDUCE_P2P || ((uintptr_t)output & 15) != 0) return;
+        int dev = -1;
+        if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return; }
+        cudaPointerAttributes attr;
+        if (cudaPointerGetAttributes(&attr, output) != cudaSuccess) { (void)cudaGetLastError(); return; }
+        if (attr.type != cudaMemoryTypeDevice || attr.device != dev) return;
+        const char* o = static_cast<const char*>(output);
+        const char* wo = static_cast<const char*>(static_cast<const void*>(w.W_O));
+        if (o < wo + (size_t)p.d_local * p.d * sizeof(__half) && wo < o + (size_t)p.S * row_bytes()) return;
+        direct = true;
+    }
+
     efa_flash_partials ws(int rows) const
     {
         efa_flash_partials q{c->ws_O, c->ws_m, c->ws_l, rows};
@@ -137,7 +156,9 @@ struct Run {
     {
         if (p.skip_comm) return 0;
         cudaStream_t cs = c->comm_streams[slot];
-        if (nvls()) {
+        if (direct) {
+            // the projection has written `recv`
+        } else if (nvls()) {
             // the switch sums the ranks' send buffers into every rank's result buffer; one local copy to `output`
             const bool f32 = wire_f32();
             const size_t first = (size_t)(static_cast<char*>(send) - send_base()) / (f32 ? sizeof(float) : sizeof(__half));
@@ -240,7 +261,7 @@ int scratch(efa_ctx* c, const Run& r, size_t o_rows, size_t send_rows, size_t nc
     const efa_params& p = r.p;
     if (o_rows && ensure_bytes(&c->O_all, &c->O_all_bytes, o_rows * p.d_local * sizeof(__half))) return 1;
     if (r.nvls()) { if (nvls_prepare(c, p)) return 1; }
-    else if (send_rows && ensure_bytes(&c->send_buf, &c->send_bytes, send_rows * r.send_row_bytes())) return 1;
+    else if (send_rows && !r.direct && ensure_bytes(&c->send_buf, &c->send_bytes, send_rows * r.send_row_bytes())) return 1;
     if (ncounters) {
         size_t have = c->counters_n * sizeof(int);
         if (ensure_bytes((void**)&c->counters, &have, ncounters * sizeof(int))) return 1;
@@ -288,7 +309,7 @@ int run_megatron(Run& r, char* output, efa_run_stats* st)
     efa_ctx* c = r.c; const efa_params& p = r.p;
     if (scratch(c, r, p.S, p.S, 0, p.S, 2)) return 1;
     __half* O_all = static_cast<__half*>(c->O_all);
-    char* send_buf = r.send_base();
+    char* send_buf = r.direct ? output : r.send_base();
     cudaEvent_t attn_done = c->events[0], proj_done = c->events[1];
 
     if (world_barrier(c->world)) return 1;
@@ -322,9 +343,11 @@ int run_sync(Run& r, char* output, efa_run_stats* st)
     for (int t = 0; t < p.num_tiles; t++) {
         if (r.attention(O_tile, p.tile, t * p.tile, p.tile, c->compute_stream)) return 1;
         if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
-        if (r.project(O_tile, send_buf, p.tile)) return 1;
+        char* out_t = output + (size_t)t * p.tile * r.row_bytes();
+        char* send = r.direct ? out_t : send_buf;
+        if (r.project(O_tile, send, p.tile)) return 1;
         if (sync_stream(c, c->proj_stream, nullptr, 0)) return 1;
-        if (r.allreduce(0, send_buf, output + (size_t)t * p.tile * r.row_bytes(), (size_t)p.tile * p.d)) return 1;
+        if (r.allreduce(0, send, out_t, (size_t)p.tile * p.d)) return 1;
         if (sync_stream(c, c->comm_streams[0], nullptr, 0)) return 1;
     }
     return finish_timing(c, t0, st, false, false, r.launches);
@@ -350,7 +373,8 @@ int run_overlap(Run& r, char* output, efa_run_stats* st)
     for (int t = 0; t < p.num_tiles; t++) {
         const int b = t % nbuf;
         __half* O_t = O_buf + (size_t)b * p.tile * p.d_local;
-        char* S_t = S_buf + (size_t)b * p.tile * r.send_row_bytes();
+        char* out_t = output + (size_t)t * p.tile * r.row_bytes();
+        char* S_t = r.direct ? out_t : S_buf + (size_t)b * p.tile * r.send_row_bytes();
         if (t >= nbuf) EFA_CUDA(cudaStreamWaitEvent(c->compute_stream, proj_done(b), 0));
         if (r.attention(O_t, p.tile, t * p.tile, p.tile, c->compute_stream)) return 1;
         EFA_CUDA(cudaEventRecord(attn_done(b), c->compute_stream));
@@ -362,7 +386,7 @@ int run_overlap(Run& r, char* output, efa_run_stats* st)
 
         const int slot = t % c->ncomm;
         EFA_CUDA(cudaStreamWaitEvent(c->comm_streams[slot], proj_done(b), 0));
-        if (r.allreduce(slot, S_t, output + (size_t)t * p.tile * r.row_bytes(), (size_t)p.tile * p.d)) return 1;
+        if (r.allreduce(slot, S_t, out_t, (size_t)p.tile * p.d)) return 1;
         EFA_CUDA(cudaEventRecord(comm_done(b), c->comm_streams[slot]));
     }
     if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
@@ -382,7 +406,7 @@ int run_stream(Run& r, char* output, efa_run_stats* st)
     if (!api) return 1;
     if (scratch(c, r, p.S, p.S, p.num_tiles, p.S, (size_t)p.num_tiles + 1)) return 1;
     __half* O_all = static_cast<__half*>(c->O_all);
-    char* send_buf = r.send_base();
+    char* send_buf = r.direct ? output : r.send_base();
     int* counters = c->counters;
     const int target = efa_blocks_per_tile(&p) + p.debug_target_bias;
     const bool fused = (p.reduce == EFA_REDUCE_P2P) && !p.skip_comm && !p.skip_proj;
@@ -478,6 +502,7 @@ int run_stream(Run& r, char* output, efa_run_stats* st)
         if (trace) cudaEventRecord(c->trace_events[3 * gidx], c->proj_stream);
         if (r.combine(O_t, p.S, t0g * p.tile, rows, c->proj_stream)) return fail();
         if (r.project(O_t, S_t, rows)) return fail();
+        if (r.direct && !r.residual && !trace) continue;          // nothing follows on the communication streams
         if (cudaEventRecord(c->events[gidx], c->proj_stream) != cudaSuccess) return fail();
         if (trace) cudaEventRecord(c->trace_events[3 * gidx + 1], c->proj_stream);
         const int slot = gidx % c->ncomm;
@@ -555,10 +580,11 @@ int run_stream_host_pipelined(efa_ctx* c, const uint16_t* Qh, const uint16_t* Kh
     }
     const int nchunk = (int)chunk_first.size();
     Run r{c, dev, p};
+    r.choose_direct(dev_out);
     if (scratch(c, r, p.S, p.S, p.num_tiles, p.S, (size_t)3 * nchunk + 2)) return 1;
     __half* O_all = static_cast<__half*>(c->O_all);
-    char* send_buf = r.send_base();
     char* output = static_cast<char*>(dev_out);
+    char* send_buf = r.direct ? output : r.send_base();
     char* host_bytes = reinterpret_cast<char*>(host_out);
     const size_t rb = r.row_bytes(), sb = r.send_row_bytes();
     int* counters = c->counters;
@@ -658,6 +684,7 @@ int run_mode_impl(efa_ctx* c, int mode, const efa_weights& w, void* output, cons
     char* out = static_cast<char*>(output);
     r.residual = static_cast<const __half*>(residual);
     r.out_base = out;
+    if (mode == EFA_MODE_MEGATRON || mode == EFA_MODE_SYNC || mode == EFA_MODE_OVERLAP || mode == EFA_MODE_STREAM) r.choose_direct(out);
     switch (mode) {
         case EFA_MODE_ATTN:       return run_attn_only(r, stats, false);
         case EFA_MODE_ATTN_TILED: return run_attn_only(r, stats, true);

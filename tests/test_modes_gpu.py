@@ -271,3 +271,27 @@ def test_fp32_partial_sums_and_output(pkg, oracle, torch_cuda, ctx, case):
     p.reduce = pkg.REDUCE_P2P
     with pytest.raises(pkg.EfaError, match="NCCL reduction"):
         pkg.run_mode(ctx, pkg.MODE_STREAM, w, out, p)
+
+
+@pytest.mark.parametrize("f32", [0, 1])
+@pytest.mark.parametrize("mode", CHECKED_MODES)
+def test_outputs_that_the_projection_cannot_write_itself(pkg, torch_cuda, ctx, mode, f32):
+    """One rank writes an aligned device output straight from the projection; an output at an address that its
+    TMA stores could not take is still filled, with the same values."""
+    torch = torch_cuda
+    S, d, H, tile = 1024, 512, 8, 128
+    p = pkg.make_params(S, d, H, tile, causal=1)
+    p.proj_f32 = f32
+    odt = torch.float32 if f32 else torch.float16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    dev = [torch.randn(H, S, d // H, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev.append(torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5)
+    w = pkg.Weights(*(t.data_ptr() for t in dev))
+    results = []
+    for out in (torch.zeros(S * d, dtype=odt, device="cuda"), torch.zeros(S * d + 1, dtype=odt, device="cuda")[1:]):
+        torch.cuda.synchronize()
+        pkg.run_mode(ctx, pkg.parse_mode(mode), w, out, p)
+        torch.cuda.synchronize()
+        results.append(out.cpu())
+    assert bool(results[0].any()) and torch.isfinite(results[0]).all()
+    assert torch.equal(results[0], results[1])

@@ -59,7 +59,7 @@ const DriverApi* driver_api()
     if (state == 1) return &api;
     if (state == -1) return nullptr;
     if (resolve("cuTensorMapEncodeTiled", (void**)&api.cuTensorMapEncodeTiled) ||
-        resolve("cuStreamWaitValue32", (void**)&api.cuStreamWaitValue32) ||
+        resolve("cuStreamBatchMemOp", (void**)&api.cuStreamBatchMemOp) ||
         resolve("cuStreamWriteValue32", (void**)&api.cuStreamWriteValue32) ||
         resolve("cuGetErrorString", (void**)&api.cuGetErrorString) ||
         resolve("cuMemGetAddressRange", (void**)&api.cuMemGetAddressRange) ||

@@ -26,7 +26,7 @@ struct DriverApi {
                                        const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                        const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                        CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    CUresult (*cuStreamWaitValue32)(CUstream, CUdeviceptr, cuuint32_t, unsigned int);
+    CUresult (*cuStreamBatchMemOp)(CUstream, unsigned int, CUstreamBatchMemOpParams*, unsigned int);
     CUresult (*cuStreamWriteValue32)(CUstream, CUdeviceptr, cuuint32_t, unsigned int);
     CUresult (*cuGetErrorString)(CUresult, const char**);
     CUresult (*cuMemGetAddressRange)(CUdeviceptr*, size_t*, CUdeviceptr);

@@ -61,6 +61,25 @@ int add_residual(__half* out, const __half* residual, size_t n, cudaStream_t str
     return 0;
 }
 
+// Front-end waits until each of n counters has reached `target`: one call for up to 128 of them (the driver takes
+// fewer than 256), since a call of its own for every tile costs the host more than the launches it guards.
+int wait_tiles(const DriverApi* api, cudaStream_t s, int* counters, int n, int target)
+{
+    CUstreamBatchMemOpParams ops[128];
+    for (int i = 0; i < n; i += 128) {
+        const int m = std::min(128, n - i);
+        std::memset(ops, 0, sizeof(ops[0]) * m);
+        for (int k = 0; k < m; k++) {
+            ops[k].waitValue.operation = CU_STREAM_MEM_OP_WAIT_VALUE_32;
+            ops[k].waitValue.address = (CUdeviceptr)(counters + i + k);
+            ops[k].waitValue.value = (cuuint32_t)target;
+            ops[k].waitValue.flags = CU_STREAM_WAIT_VALUE_GEQ;
+        }
+        EFA_CU(api->cuStreamBatchMemOp((CUstream)s, (unsigned)m, ops, 0));
+    }
+    return 0;
+}
+
 struct Run {
     efa_ctx* c;
     const efa_weights& w;
@@ -202,7 +221,7 @@ void release_counter_waits(efa_ctx* c, int* counters, size_t ncounters)
 }
 
 // Wait for a stream with a deadline. When the deadline passes (a tile counter that never reaches its target would
-// block cuStreamWaitValue32 forever), the counters are overwritten so that every pending wait is released, the
+// block a front-end wait forever), the counters are overwritten so that every pending wait is released, the
 // stream is given the same time again to drain, and an error is returned either way.
 int sync_stream(efa_ctx* c, cudaStream_t s, int* counters, size_t ncounters)
 {
@@ -397,7 +416,7 @@ int run_overlap(Run& r, char* output, efa_run_stats* st)
 
 // run_stream (run_drivers.cu:201-255): one attention launch over all rows; the kernel counts finished
 // 64-row blocks per tile; the projection stream holds, for every tile, a front-end wait on that
-// tile's counter (cuStreamWaitValue32, no SM involved), the split combine, the projection and an
+// tile's counter (cuStreamBatchMemOp, no SM involved), the split combine, the projection and an
 // event; the tile's AllReduce follows on communicator t % ncomm.
 int run_stream(Run& r, char* output, efa_run_stats* st)
 {
@@ -493,9 +512,7 @@ int run_stream(Run& r, char* output, efa_run_stats* st)
     };
     for (int gidx = 0; gidx < ngroups; gidx++) {
         const int t0g = groups[gidx].first_tile, nt = groups[gidx].ntiles;
-        for (int t = t0g; t < t0g + nt; t++)
-            if (check_cu(api->cuStreamWaitValue32((CUstream)c->proj_stream, (CUdeviceptr)(counters + t), (cuuint32_t)target,
-                                                  CU_STREAM_WAIT_VALUE_GEQ), "cuStreamWaitValue32", __FILE__, __LINE__)) return fail();
+        if (wait_tiles(api, c->proj_stream, counters + t0g, nt, target)) return fail();
         const int rows = nt * p.tile;
         __half* O_t = O_all + (size_t)t0g * p.tile * p.d_local;
         char* S_t = send_buf + (size_t)t0g * p.tile * r.send_row_bytes();
@@ -620,8 +637,7 @@ int run_stream_host_pipelined(efa_ctx* c, const uint16_t* Qh, const uint16_t* Kh
         if (r.attention_raw(O_all + (size_t)row0 * p.d_local, p.S, row0, rows, c->compute_stream, counters + t0c, p.tile, 0,
                             /* the chunk is consumed as a whole: */ rows >= 512 ? (rows > 2048 ? 2048 : (rows / 256) * 256) : 0,
                             row0)) return 1;
-        for (int t = t0c; t < t0c + nt; t++)
-            EFA_CU(api->cuStreamWaitValue32((CUstream)c->proj_stream, (CUdeviceptr)(counters + t), (cuuint32_t)target, CU_STREAM_WAIT_VALUE_GEQ));
+        if (wait_tiles(api, c->proj_stream, counters + t0c, nt, target)) return 1;
         if (r.combine(O_all + (size_t)row0 * p.d_local, p.S, row0, rows, c->proj_stream)) return 1;
         if (r.project(O_all + (size_t)row0 * p.d_local, send_buf + (size_t)row0 * sb, rows)) return 1;
         EFA_CUDA(cudaEventRecord(ev_proj(i), c->proj_stream));

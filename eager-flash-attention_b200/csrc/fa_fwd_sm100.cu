@@ -1,16 +1,6 @@
-// FlashAttention forward for sm_100a: fp16 Q/K/V, fp32 accumulate in tensor memory, fp32 or fp16 O.
-//
-// Stands in for flash_attn_tc_kernel / flash_attn_tc_forward of eager-flash-attention
-// (flash_attn_tc.cu:73-312, 363-399) behind the same launch interface: same tensor layouts, same
-// split-KV partial format (row max in the log2 domain), same per-tile completion counters.
-//
-// One CTA = 128 query rows of one (head, split). K and V stream through shared memory in 128-key
-// stages filled by TMA (128/64/32-byte swizzle chosen from d_h). S = Q K^T is a tcgen05.mma with both
-// operands in shared memory and the 128x128 fp32 result in tensor memory; each of the 128 threads owns
-// one row of S (tcgen05.ld 32x32b), does the online softmax for that row without any shuffle,
-// and writes P as fp16 back into tensor memory over S. O += P V is a tcgen05.mma with A = P from tensor
-// memory and B = V from shared memory in MN-major form; O stays in tensor memory for the whole
-// key sweep and is rescaled there only when a row maximum moved.
+// The attention launch interface (flash_attn_tc_forward of eager-flash-attention, flash_attn_tc.cu:363-399): argument
+// checks, tensor maps, the merge of split-KV partials and the entry that allocates nothing. The kernel is in
+// fa_fwd_ws_sm100.cu.
 #include "fa_fwd_sm100.cuh"
 #include "fa_args.cuh"
 #include "host_util.h"
@@ -26,311 +16,6 @@
 namespace efa {
 
 namespace {
-
-constexpr int FA_BM = 128;      // query rows per CTA
-constexpr int FA_BN = 128;      // keys per stage
-constexpr float kNegInf = -INFINITY;
-
-template <int D>
-struct FaCfg {
-    static constexpr int SWB        = D >= 64 ? 128 : D * 2;     // swizzle width = TMA box row, bytes
-    static constexpr int BOXC       = SWB / 2;                   // fp16 columns per box
-    static constexpr int NBOX       = D / BOXC;                  // boxes per 128-row tile (2 when D = 128)
-    static constexpr int BOX_BYTES  = 128 * SWB;
-    static constexpr int TILE_BYTES = 128 * D * 2;
-    static constexpr int NSTAGE     = D == 128 ? 1 : 2;
-    static constexpr int SMEM_BYTES = TILE_BYTES * (1 + 2 * NSTAGE) + 1024;   // + alignment slack
-    static constexpr int TMEM_COLS  = 256;                       // S/P: 128 columns, O: D columns
-    static constexpr int OCH        = D >= 32 ? 32 : 16;         // O columns per tcgen05.ld
-};
-
-template <int D, bool OUT_F16>
-__global__ void __launch_bounds__(128)
-fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
-              const __grid_constant__ CUtensorMap tmK,
-              const __grid_constant__ CUtensorMap tmV,
-              const FaArgs a)
-{
-    using C = FaCfg<D>;
-    constexpr uint32_t SWZ = swizzle_code(C::SWB);
-    constexpr uint32_t IDESC_QK = idesc_f16_f32(FA_BM, FA_BN, 0, 0);
-    constexpr uint32_t IDESC_PV = idesc_f16_f32(FA_BM, D, 0, 1);
-
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* sQ = smem;
-    uint8_t* sK = sQ + C::TILE_BYTES;
-    uint8_t* sV = sK + C::NSTAGE * C::TILE_BYTES;
-
-    __shared__ __align__(8) uint64_t bar_q;
-    __shared__ __align__(8) uint64_t bar_k[C::NSTAGE];
-    __shared__ __align__(8) uint64_t bar_v[C::NSTAGE];
-    __shared__ __align__(8) uint64_t bar_s;
-    __shared__ uint32_t tmem_base_smem;
-    __shared__ int abort_word;
-
-    const int tid  = threadIdx.x;
-    const int warp = tid >> 5;
-
-    // x enumerates (head, split) pairs, y the 128-row blocks: blocks are dispatched in query-row order.
-    const int head  = blockIdx.x % a.H_local;
-    const int split = blockIdx.x / a.H_local;
-    const int block_row0 = blockIdx.y * FA_BM;                     // first row of this block within the launch
-    const int rows_valid = min(FA_BM, a.q_rows - block_row0);      // 64 or 128
-    const int q_abs0 = a.q_start + block_row0;                     // absolute index of the block's first row
-    const int kv_lo = split * a.kv_len;
-    const int kv_hi = kv_lo + a.kv_len;
-    const int kv_end = a.causal ? min(kv_hi, q_abs0 + rows_valid) : kv_hi;
-    const int nblk = kv_end > kv_lo ? (kv_end - kv_lo + FA_BN - 1) / FA_BN : 0;
-
-    if (tid == 0) {
-        abort_word = 0;
-        mbar_init(&bar_q, 1);
-        for (int s = 0; s < C::NSTAGE; s++) { mbar_init(&bar_k[s], 1); mbar_init(&bar_v[s], 1); }
-        mbar_init(&bar_s, 1);
-        mbar_fence_init();
-        tma_prefetch_desc(&tmQ);
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
-    }
-    __syncwarp();
-    if (warp == 0) tmem_alloc(&tmem_base_smem, C::TMEM_COLS);
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-
-    const uint32_t tmem_base = tmem_base_smem;
-    const uint32_t tmem_S = tmem_base;            // fp32 S, 128 columns; P (fp16 pairs) reuses columns 0..63
-    const uint32_t tmem_O = tmem_base + 128;      // fp32 O, D columns
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;   // this warp's 32 TMEM lanes
-
-    auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int row) {
-        mbar_expect_tx(bar, C::TILE_BYTES);
-        #pragma unroll
-        for (int b = 0; b < C::NBOX; b++)
-            tma_load_3d(dst + b * C::BOX_BYTES, tm, bar, b * C::BOXC, row, head);
-    };
-    auto issue_qk = [&](int stage) {
-        const uint32_t qa = smem_u32(sQ);
-        const uint32_t ka = smem_u32(sK + stage * C::TILE_BYTES);
-        #pragma unroll
-        for (int ks = 0; ks < D / 16; ks++) {
-            const uint32_t off = (uint32_t)((ks * 16) / C::BOXC) * C::BOX_BYTES + (uint32_t)((ks * 16) % C::BOXC) * 2u;
-            tc_mma_ss(tmem_S, smem_desc(qa + off, 16, 8 * C::SWB, SWZ), smem_desc(ka + off, 16, 8 * C::SWB, SWZ),
-                      IDESC_QK, ks > 0 ? 1u : 0u);
-        }
-    };
-    auto issue_pv = [&](int stage, bool first) {
-        const uint32_t va = smem_u32(sV + stage * C::TILE_BYTES);
-        #pragma unroll
-        for (int ks = 0; ks < FA_BN / 16; ks++) {
-            // 16 keys = two 8-row groups of the MN-major layout; column blocks (D = 128) are BOX_BYTES apart.
-            tc_mma_ts(tmem_O, tmem_S + ks * 8, smem_desc(va + ks * 16 * C::SWB, C::BOX_BYTES, 8 * C::SWB, SWZ),
-                      IDESC_PV, (!first || ks > 0) ? 1u : 0u);
-        }
-    };
-
-    float m_run = kNegInf;     // running row max, already multiplied by scale*log2(e)
-    float l_run = 0.f;         // running row denominator
-    bool  failed = false;
-
-    if (nblk > 0) {
-        if (tid == 0) {
-            load_tile(sQ, &tmQ, &bar_q, q_abs0);
-            for (int s = 0; s < C::NSTAGE && s < nblk; s++)
-                load_tile(sK + s * C::TILE_BYTES, &tmK, &bar_k[s], kv_lo + s * FA_BN);
-            for (int s = 0; s + 1 < C::NSTAGE && s < nblk; s++)
-                load_tile(sV + s * C::TILE_BYTES, &tmV, &bar_v[s], kv_lo + s * FA_BN);
-            if (mbar_wait(&bar_q, 0, &abort_word, 1) && mbar_wait(&bar_k[0], 0, &abort_word, 2)) {
-                tc_fence_after_sync();
-                issue_qk(0);
-                tc_commit(&bar_s);
-            }
-        }
-
-        for (int j = 0; j < nblk; j++) {
-            const int stage = j % C::NSTAGE;
-            const int kb = kv_lo + j * FA_BN;                       // first key of this stage
-
-            bool ok = mbar_wait(&bar_s, (uint32_t)(j & 1), &abort_word, 3);
-            if (__syncthreads_or((!ok) || abort_word != 0)) { failed = true; break; }
-            tc_fence_after_sync();
-
-            // S(j) is complete, hence so are QK(j) and PV(j-1): K stage `stage` and the V stage
-            // used by block j-1 are free again.
-            if (tid == 0) {
-                if (j + C::NSTAGE < nblk)
-                    load_tile(sK + stage * C::TILE_BYTES, &tmK, &bar_k[stage], kv_lo + (j + C::NSTAGE) * FA_BN);
-                const int vb = j + C::NSTAGE - 1;
-                if (vb < nblk && vb >= C::NSTAGE - 1)
-                    load_tile(sV + (vb % C::NSTAGE) * C::TILE_BYTES, &tmV, &bar_v[vb % C::NSTAGE], kv_lo + vb * FA_BN);
-            }
-
-            // ---- this thread's row of S -> registers
-            uint32_t su[4][32];
-            #pragma unroll
-            for (int c = 0; c < 4; c++) tmem_ld32(tmem_S + lane_base + c * 32, su[c]);
-            tmem_wait_ld();
-
-            const bool need_mask = (kb + FA_BN > kv_hi) || (a.causal && kb + FA_BN - 1 > q_abs0);
-            if (need_mask) {
-                int lim = kv_hi - 1 - kb;                            // last admissible column of this stage
-                if (a.causal) lim = min(lim, q_abs0 + tid - kb);
-                #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    #pragma unroll
-                    for (int i = 0; i < 32; i++)
-                        if (c * 32 + i > lim) su[c][i] = 0xff800000u;   // -inf
-            }
-
-            float mx = kNegInf;
-            #pragma unroll
-            for (int c = 0; c < 4; c++)
-                #pragma unroll
-                for (int i = 0; i < 32; i++) mx = fmaxf(mx, __uint_as_float(su[c][i]));
-
-            const float m_new = fmaxf(m_run, mx * a.scale_log2e);
-            const float m_use = (m_new == kNegInf) ? 0.f : m_new;    // rows with no admissible key yet
-            const float alpha = ex2(m_run - m_use);                  // 0 on the first stage
-            float psum = 0.f;
-            #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t pk[16];
-                #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float p0 = ex2(fmaf(__uint_as_float(su[c][2 * i]),     a.scale_log2e, -m_use));
-                    const float p1 = ex2(fmaf(__uint_as_float(su[c][2 * i + 1]), a.scale_log2e, -m_use));
-                    psum += p0 + p1;
-                    pk[i] = pack_f16x2(p0, p1);
-                }
-                tmem_st16(tmem_S + lane_base + c * 16, pk);
-            }
-            l_run = l_run * alpha + psum;
-            m_run = m_new;
-
-            // ---- rescale the O accumulator when some row of this warp moved its maximum
-            if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                #pragma unroll
-                for (int c = 0; c < D / C::OCH; c++) {
-                    if constexpr (C::OCH == 32) {
-                        uint32_t o[32];
-                        tmem_ld32(tmem_O + lane_base + c * 32, o);
-                        tmem_wait_ld();
-                        #pragma unroll
-                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st32(tmem_O + lane_base + c * 32, o);
-                    } else {
-                        uint32_t o[16];
-                        tmem_ld16(tmem_O + lane_base + c * 16, o);
-                        tmem_wait_ld();
-                        #pragma unroll
-                        for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st16(tmem_O + lane_base + c * 16, o);
-                    }
-                }
-            }
-            tmem_wait_st();
-            tc_fence_before_sync();
-            __syncthreads();
-
-            if (tid == 0) {
-                tc_fence_after_sync();
-                if (mbar_wait(&bar_v[stage], (uint32_t)((j / C::NSTAGE) & 1), &abort_word, 4)) {
-                    issue_pv(stage, j == 0);
-                    bool issue_ok = true;
-                    if (j + 1 < nblk) {
-                        const int ns = (j + 1) % C::NSTAGE;
-                        issue_ok = mbar_wait(&bar_k[ns], (uint32_t)(((j + 1) / C::NSTAGE) & 1), &abort_word, 5);
-                        if (issue_ok) issue_qk(ns);
-                    }
-                    if (issue_ok) tc_commit(&bar_s);
-                }
-            }
-        }
-
-        if (!failed) {
-            bool ok = mbar_wait(&bar_s, (uint32_t)(nblk & 1), &abort_word, 6);
-            if (__syncthreads_or((!ok) || abort_word != 0)) failed = true;
-            tc_fence_after_sync();
-        }
-    }
-
-    // ---- epilogue: this thread's row of O
-    if (!failed && tid < rows_valid) {
-        const size_t ld_o = (size_t)a.H_local * D;
-        const size_t row = (size_t)block_row0 + tid;
-        const float inv = (a.nsplit == 1) ? 1.f / l_run : 1.f;
-        float*  dst32 = nullptr;
-        __half* dst16 = nullptr;
-        if (a.nsplit == 1) {
-            if constexpr (OUT_F16) dst16 = a.O16 + row * ld_o + (size_t)head * D;
-            else                   dst32 = a.O32 + row * ld_o + (size_t)head * D;
-        } else {
-            dst32 = a.O_part + ((size_t)split * a.part_rows + row) * ld_o + (size_t)head * D;
-            const size_t s0 = ((size_t)split * a.part_rows + row) * a.H_local + head;
-            a.m_part[s0] = m_run;
-            a.l_part[s0] = l_run;
-        }
-        #pragma unroll
-        for (int c = 0; c < D / 16; c++) {
-            uint32_t o[16];
-            if (nblk > 0) {
-                tmem_ld16(tmem_O + lane_base + c * 16, o);
-                tmem_wait_ld();
-            } else {
-                #pragma unroll
-                for (int i = 0; i < 16; i++) o[i] = 0u;
-            }
-            if (dst16) {
-                uint4 v0, v1;
-                v0.x = pack_f16x2(__uint_as_float(o[0]) * inv,  __uint_as_float(o[1]) * inv);
-                v0.y = pack_f16x2(__uint_as_float(o[2]) * inv,  __uint_as_float(o[3]) * inv);
-                v0.z = pack_f16x2(__uint_as_float(o[4]) * inv,  __uint_as_float(o[5]) * inv);
-                v0.w = pack_f16x2(__uint_as_float(o[6]) * inv,  __uint_as_float(o[7]) * inv);
-                v1.x = pack_f16x2(__uint_as_float(o[8]) * inv,  __uint_as_float(o[9]) * inv);
-                v1.y = pack_f16x2(__uint_as_float(o[10]) * inv, __uint_as_float(o[11]) * inv);
-                v1.z = pack_f16x2(__uint_as_float(o[12]) * inv, __uint_as_float(o[13]) * inv);
-                v1.w = pack_f16x2(__uint_as_float(o[14]) * inv, __uint_as_float(o[15]) * inv);
-                uint4* d = reinterpret_cast<uint4*>(dst16 + c * 16);
-                d[0] = v0;
-                d[1] = v1;
-            } else {
-                float4* d = reinterpret_cast<float4*>(dst32 + c * 16);
-                #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    d[q] = make_float4(__uint_as_float(o[4 * q]) * inv, __uint_as_float(o[4 * q + 1]) * inv,
-                                       __uint_as_float(o[4 * q + 2]) * inv, __uint_as_float(o[4 * q + 3]) * inv);
-            }
-        }
-    }
-    // rows_valid is 64 or 128, so a warp takes the branch above as a whole and every tcgen05.ld in it
-    // is executed by a full warp.
-
-    // ---- signal tile completion: one count per finished 64-row block, after the rows are visible
-    if (!failed && a.tile_counters != nullptr) {
-        if (a.counters_sys) __threadfence_system(); else __threadfence();
-        __syncthreads();
-        if (tid == 0) {
-            for (int sb = 0; sb < rows_valid; sb += 64)
-                atomicAdd(a.tile_counters + (block_row0 + sb) / a.tile_rows, 1);
-        }
-    }
-
-    // ---- teardown
-    if (failed) {
-        // Give copies that may still be in flight time to land before the shared memory is released.
-        for (int i = 0; i < 64; i++) __nanosleep(100000);
-        if (tid == 0 && a.status != nullptr) {
-            if (atomicCAS(a.status, 0, (int)KS_WAIT_TIMEOUT) == 0) {
-                a.status[1] = (int)(blockIdx.y * gridDim.x + blockIdx.x);
-                a.status[2] = abort_word;
-            }
-        }
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
-}
 
 // Merge of the split-KV partials (the job of combine_kernel, flash_attn_tc.cu:319-349):
 //     O = sum_i w_i O_i / sum_i w_i l_i,   w_i = 2^(m_i - max_k m_k).
@@ -405,8 +90,7 @@ struct TmapKey {
     bool operator<(const TmapKey& o) const { return std::tie(ptr, S, H, D, rows) < std::tie(o.ptr, o.S, o.H, o.D, o.rows); }
 };
 
-// box_rows: rows of the tensor per TMA box (128 for Q tiles and for the one-tile kernel's K/V stages, the
-// two-tile kernel's stage length for its K and V).
+// box_rows: rows of the tensor per TMA box (128 for Q tiles, the stage length for K and V).
 int get_qkv_tmap(const void* ptr, int S, int H_local, int D, int box_rows, CUtensorMap* out)
 {
     static std::map<TmapKey, CUtensorMap> cache;
@@ -424,23 +108,6 @@ int get_qkv_tmap(const void* ptr, int S, int H_local, int D, int box_rows, CUten
     if (cache.size() > 256) cache.clear();
     cache[key] = tm;
     *out = tm;
-    return 0;
-}
-
-template <int D, bool OUT_F16>
-int launch_fa(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args,
-              dim3 grid, cudaStream_t stream)
-{
-    using C = FaCfg<D>;
-    static bool configured[64] = {};
-    int dev = 0;
-    EFA_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_kernel<D, OUT_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-        configured[dev] = true;
-    }
-    fa_fwd_kernel<D, OUT_F16><<<grid, 128, C::SMEM_BYTES, stream>>>(tq, tk, tv, args);
-    EFA_CUDA(cudaGetLastError());
     return 0;
 }
 
@@ -482,12 +149,9 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
         return 2;
     }
 
-    // d_h = 64 / 128 run on the warp-specialised two-tile kernel, 16 / 32 on the one-tile kernel below.
-    const bool two_tile = (p.d_h == 64 || p.d_h == 128);
-    const int kv_rows = two_tile ? fa_ws_kv_box_rows() : 128;
     CUtensorMap tq, tk, tv;
-    if (get_qkv_tmap(Q, p.S, p.H_local, p.d_h, 128, &tq) || get_qkv_tmap(K, p.S, p.H_local, p.d_h, kv_rows, &tk) ||
-        get_qkv_tmap(V, p.S, p.H_local, p.d_h, kv_rows, &tv))
+    if (get_qkv_tmap(Q, p.S, p.H_local, p.d_h, 128, &tq) || get_qkv_tmap(K, p.S, p.H_local, p.d_h, fa_ws_kv_box_rows(), &tk) ||
+        get_qkv_tmap(V, p.S, p.H_local, p.d_h, fa_ws_kv_box_rows(), &tv))
         return 1;
 
     FaArgs a;
@@ -517,16 +181,7 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
     a.heavy_first = heavy_first >= 0 ? (heavy_first ? 1 : 0) : ((tile_counters == nullptr && p.causal) ? 1 : 0);
 
     const bool f16 = (o_dtype == EFA_F16);
-    if (two_tile) return fa_forward_ws(tq, tk, tv, a, p.d_h, f16, reserve_sms, stream);
-    dim3 grid(p.H_local * p.split, (q_rows + FA_BM - 1) / FA_BM);
-    switch (p.d_h) {
-        case 16:  return f16 ? launch_fa<16, true>(tq, tk, tv, a, grid, stream)  : launch_fa<16, false>(tq, tk, tv, a, grid, stream);
-        case 32:  return f16 ? launch_fa<32, true>(tq, tk, tv, a, grid, stream)  : launch_fa<32, false>(tq, tk, tv, a, grid, stream);
-        case 64:  return f16 ? launch_fa<64, true>(tq, tk, tv, a, grid, stream)  : launch_fa<64, false>(tq, tk, tv, a, grid, stream);
-        case 128: return f16 ? launch_fa<128, true>(tq, tk, tv, a, grid, stream) : launch_fa<128, false>(tq, tk, tv, a, grid, stream);
-    }
-    set_error("flash_attn_tc_forward: unsupported d_h=%d", p.d_h);
-    return 2;
+    return fa_forward_ws(tq, tk, tv, a, p.d_h, f16, reserve_sms, stream);
 }
 
 int fa_combine(const efa_flash_partials& part, void* O, int o_dtype, int row0, int rows,
@@ -655,19 +310,11 @@ int fa_forward_noalloc(const void* Q, const void* K, const void* V, void* O, int
     a.tile_counters = nullptr; a.tile_rows = 0;
     a.counters_sys = 0;
     a.status = status;                       // a word of the module, see noalloc_status()
-    a.band_blocks = 0;
+    a.band_blocks = (q_rows + 255) / 256;
     a.order_tab = nullptr;
-    a.heavy_first = 0;
+    a.heavy_first = p.causal ? 1 : 0;
 
-    dim3 grid(p.H_local * p.split, (q_rows + FA_BM - 1) / FA_BM);
-    const bool f16 = (o_dtype == EFA_F16);
-    int rc = 2;
-    switch (p.d_h) {
-        case 16:  rc = f16 ? launch_fa<16, true>(tq, tk, tv, a, grid, stream)  : launch_fa<16, false>(tq, tk, tv, a, grid, stream); break;
-        case 32:  rc = f16 ? launch_fa<32, true>(tq, tk, tv, a, grid, stream)  : launch_fa<32, false>(tq, tk, tv, a, grid, stream); break;
-        case 64:  rc = f16 ? launch_fa<64, true>(tq, tk, tv, a, grid, stream)  : launch_fa<64, false>(tq, tk, tv, a, grid, stream); break;
-        case 128: rc = f16 ? launch_fa<128, true>(tq, tk, tv, a, grid, stream) : launch_fa<128, false>(tq, tk, tv, a, grid, stream); break;
-    }
+    const int rc = fa_forward_ws(tq, tk, tv, a, p.d_h, o_dtype == EFA_F16, 0, stream);
     if (rc) return rc;
     return fa_combine(part, O, o_dtype, 0, q_rows, p, stream);
 }
@@ -696,11 +343,7 @@ template <class K> int touch_kernel(K kernel)
 
 int fa_preload()
 {
-    return touch_kernel(fa_fwd_kernel<16, true>) || touch_kernel(fa_fwd_kernel<16, false>) ||
-           touch_kernel(fa_fwd_kernel<32, true>) || touch_kernel(fa_fwd_kernel<32, false>) ||
-           touch_kernel(fa_fwd_kernel<64, true>) || touch_kernel(fa_fwd_kernel<64, false>) ||
-           touch_kernel(fa_fwd_kernel<128, true>) || touch_kernel(fa_fwd_kernel<128, false>) ||
-           touch_kernel(combine_splits_kernel<true>) || touch_kernel(combine_splits_kernel<false>) ||
+    return touch_kernel(combine_splits_kernel<true>) || touch_kernel(combine_splits_kernel<false>) ||
            touch_kernel(f32_to_f16_kernel) || fa_ws_preload();
 }
 

@@ -1,13 +1,17 @@
-// Warp-specialised FlashAttention forward for sm_100a, d_h = 64 or 128: the fast path behind
-// flash_attn_tc_forward (flash_attn_tc.cu:73-312 of eager-flash-attention), same interface and
-// semantics as the one-tile kernel in fa_fwd_sm100.cu.
+// Warp-specialised FlashAttention forward for sm_100a: fp16 Q/K/V, fp32 accumulate in tensor memory, fp32 or fp16 O.
+// Stands in for flash_attn_tc_kernel (flash_attn_tc.cu:73-312 of eager-flash-attention) behind the same launch
+// interface: same tensor layouts, split-KV partial format (row max in the log2 domain) and completion counters.
+//
+// Described for two tiles of d_h = 64 or 128. Small heads (AHEAD) and few rows (KSPLIT) use it with the differences
+// stated at those two constants; they had a kernel of one tile per block before: 4032 rows of eight heads of 32,
+// 71.5 -> 63 us; 128 rows against 16384 keys in eight splits (16 heads of 64), 55 -> 41.5 us.
 //
 // One CTA = 256 query rows (two 128-row Q tiles) of one (head, split), 384 threads:
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
 //   warps 4-7   softmax of Q tile 1
 //   warp  8     TMA producer: Q tiles once, then K and V 128-key stages through two rings
 //   warp  9     tcgen05.mma issuer; owns the tensor-memory allocation
-//   warps 10-11 idle (they give their registers to the softmax warps)
+//   warp  10    the second issuer where there is one, else idle; warp 11 idle (they give their registers to the softmax)
 // Both Q tiles share each K/V stage, which halves the L2 -> shared-memory traffic per FLOP. Each tile is a
 // chain  S(j) -> softmax -> P(j) -> P(j)*V(j) -> Q*K^T(j+1) -> S(j+1)  (P overwrites S in tensor memory, and the
 // tensor pipe executes in issue order), and the two chains run half a period apart: the one issuing thread
@@ -24,7 +28,10 @@
 // (it shares its scheduler with two softmax warps); a V ring one slot deeper than the K ring (V(j) is wanted
 // right at the start of stage j, K(j+1) a whole stage after its slot is freed); packed fp32 pairs in the softmax.
 // Computing a share of the exponentials with a polynomial on the FMA pipes lengthens the softmax and with it the
-// chain; it was measured slower at every share.
+// chain; it was measured slower at every share (d_h = 64 with Q*K^T a stage ahead, a quarter of them: 3.36 against 3.14 ms
+// at S = 65536, two heads). So was Q*K^T in two 64-key halves, the upper one issued as soon as its columns of S are in
+// registers, with its exponentials under the offset in use while the maximum is still being found: the halves'
+// MMAs fetch Q twice (d_h = 128, S = 32768, four heads, causal: 1.27 ms against 1.02).
 // Tensor memory (512 columns): S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+D) O1 [384,384+D).
 // O is rescaled in tensor memory by the softmax warps themselves, and only when a row maximum grew
 // by more than 2^8 since the value last used as the exponent offset (P then stays below 256, well
@@ -58,10 +65,10 @@ constexpr float kRescaleThreshold = 8.0f;   // log2 units
 
 template <int D>
 struct WsCfg {
-    static constexpr int SWB        = 128;
-    static constexpr int BOXC       = 64;
-    static constexpr int NBOX       = D / 64;
-    static constexpr int BOX_BYTES  = 128 * SWB;                 // 16 KB
+    static constexpr int SWB        = D >= 64 ? 128 : D * 2;      // swizzle width = TMA box row, bytes
+    static constexpr int BOXC       = SWB / 2;
+    static constexpr int NBOX       = D / BOXC;
+    static constexpr int BOX_BYTES  = 128 * SWB;
     static constexpr int TILE_BYTES = 128 * D * 2;
     static constexpr int NSTAGE_K   = D == 128 ? 2 : 4;           // K(j+1) is wanted a whole stage after its slot is freed,
     static constexpr int NSTAGE_V   = D == 128 ? 3 : 4;           // V(j) right at the start of the stage: the deeper ring
@@ -112,7 +119,10 @@ __device__ __forceinline__ void setmaxnreg_inc_224() { asm volatile("setmaxnreg.
 // PERSIST = true: a 1-D grid of fewer CTAs than SMs; each CTA takes work items from a global counter in
 // the same row-major order. The SMs left without a CTA stay free for the projection and the AllReduce
 // of finished tiles, which otherwise can only start when an attention CTA retires.
-template <int D, bool OUT_F16, bool PERSIST>
+// KSPLIT: a work item is 128 rows, and both softmax warpgroups take its one Q tile, warpgroup q the key stages
+// q, q + 2, ...: an item is half as long for half as many rows, which fills the GPU where 256-row items do not. The
+// two running results are merged at the end, straight from tensor memory (both warpgroups see the same lanes).
+template <int D, bool OUT_F16, bool PERSIST, bool KSPLIT>
 __global__ void __launch_bounds__(WS_THREADS, 1)
 fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                  const __grid_constant__ CUtensorMap tmK,
@@ -120,10 +130,18 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                  const FaArgs a, int* work_counter, int items_x, int items_total)
 {
     using C = WsCfg<D>;
-    constexpr uint32_t SWZ = swizzle_code(128);
+    constexpr uint32_t SWZ = swizzle_code(C::SWB);
     constexpr uint32_t IDESC_QK = idesc_f16_f32(WS_BM, WS_BN, 0, 0);
     constexpr uint32_t IDESC_PV = idesc_f16_f32(WS_BM, D, 0, 1);
     constexpr int NSK = C::NSTAGE_K, NSV = C::NSTAGE_V;
+    // P in tensor-memory columns of its own (they fit beside S and O up to D = 64), so that Q*K^T runs a stage ahead of
+    // the softmax. Taken where there is one chain per tile and nothing alternates with it. With two tiles of D = 64 it is
+    // no faster (S = 65536, two heads: 3.14 ms either way; S = 16384, four splits: 274 us against 268): the
+    // special-function unit is busy 82 % of a working SM's time, and tiles that end together store together.
+    constexpr bool AHEAD = D < 64 || (KSPLIT && D == 64);
+    constexpr int ISSUERS = AHEAD || KSPLIT ? 2 : 1;    // issuing threads: one per tile where the tiles need not alternate
+    constexpr int SLOT_USERS = AHEAD && !KSPLIT ? 2 : 1; // issuers that read one K/V slot
+    constexpr int ITEM_ROWS = KSPLIT ? WS_BM : 2 * WS_BM;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -133,7 +151,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
 
     __shared__ __align__(8) uint64_t q_full[2];
     __shared__ __align__(8) uint64_t k_full[NSK], k_empty[NSK], v_full[NSV], v_empty[NSV];
-    __shared__ __align__(8) uint64_t s_full[2], p_full[2][2], o_done[2];
+    __shared__ __align__(8) uint64_t s_full[2], s_read[2], p_full[2][2], o_done[2];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_word;
     __shared__ int half_done[2][2];                       // [tile][64-row half]: warps that finished their stores
@@ -166,19 +184,20 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             s_item = PERSIST ? atomicAdd(work_counter, 1) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
             half_done[0][0] = half_done[0][1] = half_done[1][0] = half_done[1][1] = 0;
             if (round > 0) {
-                for (int q = 0; q < 2; q++) { mbar_inval(&q_full[q]); mbar_inval(&s_full[q]); mbar_inval(&p_full[q][0]); mbar_inval(&p_full[q][1]); mbar_inval(&o_done[q]); }
+                for (int q = 0; q < 2; q++) { mbar_inval(&q_full[q]); mbar_inval(&s_full[q]); mbar_inval(&s_read[q]); mbar_inval(&p_full[q][0]); mbar_inval(&p_full[q][1]); mbar_inval(&o_done[q]); }
                 for (int s = 0; s < NSK; s++) { mbar_inval(&k_full[s]); mbar_inval(&k_empty[s]); }
                 for (int s = 0; s < NSV; s++) { mbar_inval(&v_full[s]); mbar_inval(&v_empty[s]); }
             }
             for (int q = 0; q < 2; q++) {
                 mbar_init(&q_full[q], 1);
                 mbar_init(&s_full[q], 1);
-                mbar_init(&p_full[q][0], WS_BM);
-                mbar_init(&p_full[q][1], WS_BM);
+                mbar_init(&s_read[q], WS_BM / 32);
+                mbar_init(&p_full[q][0], WS_BM / 32);
+                mbar_init(&p_full[q][1], WS_BM / 32);
                 mbar_init(&o_done[q], 1);
             }
-            for (int s = 0; s < NSK; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-            for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+            for (int s = 0; s < NSK; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], SLOT_USERS); }
+            for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], SLOT_USERS); }
             mbar_fence_init();
         }
         __syncthreads();
@@ -191,12 +210,15 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
         // groups of tiles needs.
         int item_x, item_y;
         {
-            const int items_y = items_total / items_x;
-            const int band = a.band_blocks > 1 ? min(a.band_blocks, items_y) : 1;
+            const bool tail = KSPLIT && a.tail_first >= 0;         // halves of the 256-row items from tail_first on
+            const int units = tail ? a.tail_total : items_total, unit = tail ? a.tail_first + item / 2 : item;
+            const int items_y = units / items_x;
+            const int band_items = a.band_blocks * (KSPLIT && !tail ? 2 : 1);
+            const int band = band_items > 1 ? min(band_items, items_y) : 1;
             const int per_band = items_x * band;
             const int full = items_y / band;
-            int b = item / per_band, rem = item - b * per_band, nb = band;
-            if (b >= full) { b = full; rem = item - full * per_band; nb = items_y - full * band; }
+            int b = unit / per_band, rem = unit - b * per_band, nb = band;
+            if (b >= full) { b = full; rem = unit - full * per_band; nb = items_y - full * band; }
             item_x = rem / nb;
             item_y = b * band + rem % nb;
             // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
@@ -206,16 +228,17 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
         }
         it.head  = item_x % a.H_local;
         it.split = item_x / a.H_local;
-        it.block_row0 = item_y * (2 * WS_BM);
-        const int rows_valid = min(2 * WS_BM, a.q_rows - it.block_row0);      // 64, 128, 192 or 256
+        it.block_row0 = KSPLIT && a.tail_first >= 0 ? item_y * 2 * WS_BM + (item & 1) * WS_BM : item_y * ITEM_ROWS;
+        const int rows_valid = min(ITEM_ROWS, a.q_rows - it.block_row0);      // 64, 128, 192 or 256 (in a tail also none)
         it.kv_lo = it.split * kv_len;
         it.kv_hi = it.kv_lo + kv_len;
 
         // Per Q tile: first absolute row, valid rows, number of key stages.
         #pragma unroll
         for (int q = 0; q < 2; q++) {
-            it.q_abs0[q] = a.q_start + it.block_row0 + q * WS_BM;
-            it.rows_q[q] = max(0, min(WS_BM, rows_valid - q * WS_BM));
+            const int tile0 = KSPLIT ? 0 : q * WS_BM;
+            it.q_abs0[q] = a.q_start + it.block_row0 + tile0;
+            it.rows_q[q] = max(0, min(WS_BM, rows_valid - tile0));
             const int kv_end = a.causal ? min(it.kv_hi, it.q_abs0[q] + it.rows_q[q]) : it.kv_hi;
             it.nblk[q] = (it.rows_q[q] > 0 && kv_end > it.kv_lo) ? (kv_end - it.kv_lo + WS_BN - 1) / WS_BN : 0;
         }
@@ -250,7 +273,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     for (int b = 0; b < C::NBOX; b++)
                         tma_load_3d(dst + b * C::BOX_BYTES, tm, bar, b * C::BOXC, row, head);
                 };
-                for (int q = 0; q < 2; q++)
+                for (int q = 0; q < (KSPLIT ? 1 : 2); q++)
                     if (nblk[q] > 0) load_tile(sQ + q * C::TILE_BYTES, &tmQ, &q_full[q], q_abs0[q]);
                 for (int j = 0; j < nblk_max; j++) {
                     const int sk = j % NSK, uk = j / NSK, sv = j % NSV, uv = j / NSV;
@@ -259,17 +282,17 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     if (uv > 0 && !mbar_wait(&v_empty[sv], (uint32_t)((uv - 1) & 1), &abort_word, 22)) break;
                     load_tile(sV + sv * C::TILE_BYTES, &tmV, &v_full[sv], kv_lo + j * WS_BN);
                 }
-            } else if (warp == 9 && lane == 0) {
+            } else if (warp >= 9 && warp < 9 + ISSUERS && lane == 0) {
                 // ---- MMA issuer. Descriptors as (low, high) words; a k-step or a ring slot only moves the address
                 // field of the low word.
-                const uint64_t dq0 = smem_desc(smem_u32(sQ), 16, 1024, SWZ);
-                const uint64_t dk0 = smem_desc(smem_u32(sK), 16, 1024, SWZ);
-                const uint64_t dv0 = smem_desc(smem_u32(sV), C::BOX_BYTES, 1024, SWZ);
+                const uint64_t dq0 = smem_desc(smem_u32(sQ), 16, 8 * C::SWB, SWZ);
+                const uint64_t dk0 = smem_desc(smem_u32(sK), 16, 8 * C::SWB, SWZ);
+                const uint64_t dv0 = smem_desc(smem_u32(sV), C::BOX_BYTES, 8 * C::SWB, SWZ);
                 const uint32_t dq_lo = (uint32_t)dq0, dq_hi = (uint32_t)(dq0 >> 32);
                 const uint32_t dk_lo = (uint32_t)dk0, dk_hi = (uint32_t)(dk0 >> 32);
                 const uint32_t dv_lo = (uint32_t)dv0, dv_hi = (uint32_t)(dv0 >> 32);
                 auto issue_qk = [&](int q, int slot) {
-                    const uint32_t qa = dq_lo + (uint32_t)q * (C::TILE_BYTES >> 4);
+                    const uint32_t qa = dq_lo + (KSPLIT ? 0u : (uint32_t)q * (C::TILE_BYTES >> 4));
                     const uint32_t ka = dk_lo + (uint32_t)slot * (C::TILE_BYTES >> 4);
                     const uint32_t tS = tmem_base + q * 128;
                     #pragma unroll
@@ -280,13 +303,58 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 };
                 auto issue_pv = [&](int q, int slot, uint32_t acc0, int half) {
                     const uint32_t va = dv_lo + (uint32_t)slot * (C::TILE_BYTES >> 4);
-                    const uint32_t tS = tmem_base + q * 128, tO = tmem_base + 256 + q * 128;
+                    const uint32_t tP = tmem_base + (AHEAD ? 320 : 0) + q * 128, tO = tmem_base + 256 + q * 128;
                     #pragma unroll
                     for (int ks = half * 4; ks < half * 4 + 4; ks++)
-                        tc_mma_ts_lh(tO, tS + ks * 8, va + ((ks * 16 * 128) >> 4), dv_hi, IDESC_PV, ks > 0 ? 1u : acc0);
+                        tc_mma_ts_lh(tO, tP + ks * 8, va + ((ks * 16 * C::SWB) >> 4), dv_hi, IDESC_PV, ks > 0 ? 1u : acc0);
                 };
                 bool ok = true;
-                if (nblk_max > 0) {
+                if constexpr (ISSUERS == 2) {
+                    // One issuer per tile. Without KSPLIT both tiles use every stage's slots, so both issuers follow
+                    // every stage to its end, also where the tile itself has no keys left.
+                    const int q = warp - 9;
+                    const int n = KSPLIT ? (nblk[0] + 1 - q) / 2 : nblk[q];      // stages with work for this tile
+                    const int n_follow = KSPLIT ? n : nblk_max;
+                    auto stage = [&](int i) { return KSPLIT ? 2 * i + q : i; };
+                    if (n > 0) ok = mbar_wait(&q_full[KSPLIT ? 0 : q], 0, &abort_word, 24);
+                    // S(i) = Q K^T of stage i. With P in columns of its own, S(i - 1) only has to be in registers.
+                    auto step_qk = [&](int i) -> bool {
+                        if (i >= n_follow) return true;
+                        const int j = stage(i), sk = j % NSK;
+                        if (!mbar_wait(&k_full[sk], (uint32_t)((j / NSK) & 1), &abort_word, 27)) return false;
+                        if (i < n) {
+                            if (AHEAD && i > 0 && !mbar_wait(&s_read[q], (uint32_t)((i - 1) & 1), &abort_word, 23)) return false;
+                            tc_fence_after_sync();
+                            issue_qk(q, sk);
+                            tc_commit(&s_full[q]);
+                        }
+                        tc_commit(&k_empty[sk]);
+                        return true;
+                    };
+                    auto step_pv = [&](int i) -> bool {
+                        const int j = stage(i), sv = j % NSV;
+                        if (!mbar_wait(&v_full[sv], (uint32_t)((j / NSV) & 1), &abort_word, 25)) return false;
+                        if (i < n) {
+                            if (!mbar_wait(&p_full[q][0], (uint32_t)(i & 1), &abort_word, 26)) return false;
+                            tc_fence_after_sync();
+                            issue_pv(q, sv, i > 0 ? 1u : 0u, 0);
+                            if (!mbar_wait(&p_full[q][1], (uint32_t)(i & 1), &abort_word, 29)) return false;
+                            tc_fence_after_sync();
+                            issue_pv(q, sv, 1u, 1);
+                            if (AHEAD || i == n - 1) tc_commit(&o_done[q]);
+                        }
+                        tc_commit(&v_empty[sv]);
+                        return true;
+                    };
+                    ok = ok && step_qk(0);
+                    for (int i = 0; i < n_follow && ok; i++)
+                        ok = AHEAD ? step_qk(i + 1) && step_pv(i) : step_pv(i) && step_qk(i + 1);
+                    // The last commit has to land before the barriers are rebuilt for the next work item.
+                    if (ok && n_follow > 0) {
+                        const int j = stage(n_follow - 1);
+                        mbar_wait(&v_empty[j % NSV], (uint32_t)((j / NSV) & 1), &abort_word, 28);
+                    }
+                } else if (nblk_max > 0) {
                     ok = mbar_wait(&k_full[0], 0, &abort_word, 23);
                     for (int q = 0; q < 2 && ok; q++) {
                         if (nblk[q] > 0) {
@@ -299,7 +367,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     }
                     if (ok) tc_commit(&k_empty[0]);
                 }
-                for (int j = 0; j < nblk_max && ok; j++) {
+                for (int j = 0; ISSUERS == 1 && j < nblk_max && ok; j++) {
                     const int sv = j % NSV;
                     ok = mbar_wait(&v_full[sv], (uint32_t)((j / NSV) & 1), &abort_word, 25);
                     if (!ok) break;
@@ -333,7 +401,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     if (j + 1 < nblk_max) tc_commit(&k_empty[(j + 1) % NSK]);
                 }
                 // The last commit has to land before the barriers are rebuilt for the next work item.
-                if (ok && nblk_max > 0)
+                if (ISSUERS == 1 && ok && nblk_max > 0)
                     mbar_wait(&v_empty[(nblk_max - 1) % NSV], (uint32_t)(((nblk_max - 1) / NSV) & 1), &abort_word, 28);
             }
             end_item();
@@ -352,9 +420,10 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             const int row = tid - q * WS_BM;
             const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
             const uint32_t tmem_S = tmem_base + q * 128 + lane_base;
+            const uint32_t tmem_P = tmem_S + (AHEAD ? 320 : 0);
             const uint32_t tmem_O = tmem_base + 256 + q * 128 + lane_base;
             const int my_rows = rows_q[q];
-            const int my_nblk = nblk[q];
+            const int my_nblk = KSPLIT ? (nblk[0] + 1 - q) / 2 : nblk[q];
             const int my_abs0 = q_abs0[q];
 
             float m_ref = kNegInfW;     // exponent offset in use (a past row maximum), scaled by scale*log2(e)
@@ -363,7 +432,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             bool ok = true;
 
             for (int j = 0; j < my_nblk; j++) {
-                const int kb = kv_lo + j * WS_BN;
+                const int kb = kv_lo + (KSPLIT ? 2 * j + q : j) * WS_BN;
                 ok = __all_sync(0xffffffffu, mbar_wait(&s_full[q], (uint32_t)(j & 1), &abort_word, 31));
                 if (!ok) break;
                 tc_fence_after_sync();
@@ -372,6 +441,11 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 #pragma unroll
                 for (int c = 0; c < 4; c++) tmem_ld32(tmem_S + c * 32, su[c]);
                 tmem_wait_ld();
+                if constexpr (AHEAD) {                       // S(j) is in registers: its columns may take S(j+1)
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&s_read[q]);
+                }
 
                 const bool need_mask = (kb + WS_BN > kv_hi) || (a.causal && kb + WS_BN - 1 > my_abs0);
                 if (need_mask) {
@@ -406,17 +480,34 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 }
                 const float m_off = (m_ref == kNegInfW) ? 0.f : m_ref;
 
-                // S(j) complete implies PV(j-1) of this tile complete (the tensor pipe runs in order), and no
-                // part of PV(j) is issued before this thread's first arrival below: O may be rescaled here.
+                // O may be rescaled and P overwritten once PV(j-1) of this tile is complete: no part of PV(j) is issued
+                // before this warp's first arrival below. With P in S's columns, S(j) complete implies it (the
+                // tensor pipe runs in issue order); with Q*K^T a stage ahead it is waited for.
+                if constexpr (AHEAD) {
+                    if (j > 0) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], (uint32_t)((j - 1) & 1), &abort_word, 33));
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                    }
+                }
                 if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                    #pragma unroll
-                    for (int c = 0; c < D / 32; c++) {
-                        uint32_t o[32];
-                        tmem_ld32(tmem_O + c * 32, o);
+                    if constexpr (D >= 32) {
+                        #pragma unroll
+                        for (int c = 0; c < D / 32; c++) {
+                            uint32_t o[32];
+                            tmem_ld32(tmem_O + c * 32, o);
+                            tmem_wait_ld();
+                            #pragma unroll
+                            for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                            tmem_st32(tmem_O + c * 32, o);
+                        }
+                    } else {
+                        uint32_t o[16];
+                        tmem_ld16(tmem_O, o);
                         tmem_wait_ld();
                         #pragma unroll
-                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st32(tmem_O + c * 32, o);
+                        for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st16(tmem_O, o);
                     }
                 }
 
@@ -435,11 +526,12 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                         psum2[i & 1] = add2(psum2[i & 1], pack2(q0, q1));
                         pk[i] = pack_f16x2(q0, q1);
                     }
-                    tmem_st16(tmem_S + c * 16, pk);
+                    tmem_st16(tmem_P + c * 16, pk);
                     if (c == 1 || c == 3) {
                         tmem_wait_st();
                         tc_fence_before_sync();
-                        mbar_arrive(&p_full[q][c >> 1]);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&p_full[q][c >> 1]);
                     }
                 }
                 float ps0, ps1;
@@ -454,14 +546,34 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             }
 
             if (ok && my_nblk > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], 0, &abort_word, 32));
+                ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], AHEAD ? (uint32_t)((my_nblk - 1) & 1) : 0u, &abort_word, 32));
                 tc_fence_after_sync();
             }
+
+            // KSPLIT: both warpgroups learn each other's offset, maximum and sum; each then merges half of the columns.
+            float w_own = 1.f, w_other = 0.f;
+            if constexpr (KSPLIT) {
+                float (*xchg)[2 * WS_BM] = reinterpret_cast<float (*)[2 * WS_BM]>(sQ + C::TILE_BYTES);   // the second Q tile's place
+                xchg[0][tid] = m_ref; xchg[1][tid] = m_true; xchg[2][tid] = l_run;
+                tc_fence_before_sync();
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                tc_fence_after_sync();
+                ok = __all_sync(0xffffffffu, ok && abort_word == 0);
+                const float m_ref_o = xchg[0][tid ^ WS_BM], l_o = xchg[2][tid ^ WS_BM];
+                const float m_all = fmaxf(m_ref, m_ref_o);
+                w_own   = (m_ref == kNegInfW) ? 0.f : ex2(m_ref - m_all);
+                w_other = (m_ref_o == kNegInfW) ? 0.f : ex2(m_ref_o - m_all);
+                m_true = fmaxf(m_true, xchg[1][tid ^ WS_BM]);
+                l_run = l_run * w_own + l_o * w_other;
+                m_ref = m_all;
+            }
+            // Columns [c_lo, c_hi) in steps of 16 (D = 16: the first warpgroup takes the one step).
+            const int c_lo = KSPLIT && q == 1 ? (D + 16) / 32 : 0, c_hi = KSPLIT && q == 0 ? (D + 16) / 32 : D / 16;
 
             // ---- epilogue: this thread's row (warps take this branch as a whole: my_rows is 0, 64 or 128)
             if (ok && (warp & 3) * 32 < my_rows) {
                 const size_t ld_o = (size_t)a.H_local * D;
-                const size_t orow = (size_t)block_row0 + q * WS_BM + row;
+                const size_t orow = (size_t)block_row0 + (KSPLIT ? 0 : q * WS_BM) + row;
                 float mult;
                 float*  dst32 = nullptr;
                 __half* dst16 = nullptr;
@@ -474,11 +586,14 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     mult = (m_true == kNegInfW) ? 0.f : ex2(m_ref - m_true);
                     dst32 = a.O_part + ((size_t)split * a.part_rows + orow) * ld_o + (size_t)head * D;
                     const size_t s0 = ((size_t)split * a.part_rows + orow) * a.H_local + head;
-                    a.m_part[s0] = m_true;
-                    a.l_part[s0] = l_run * mult;
+                    if (!KSPLIT || q == 0) {
+                        a.m_part[s0] = m_true;
+                        a.l_part[s0] = l_run * mult;
+                    }
                 }
                 #pragma unroll
                 for (int c = 0; c < D / 16; c++) {
+                    if (KSPLIT && (c < c_lo || c >= c_hi)) continue;
                     uint32_t o[16];
                     if (my_nblk > 0) {
                         tmem_ld16(tmem_O + c * 16, o);
@@ -486,6 +601,17 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     } else {
                         #pragma unroll
                         for (int i = 0; i < 16; i++) o[i] = 0u;
+                    }
+                    if constexpr (KSPLIT) {
+                        uint32_t o2[16];
+                        const bool other_ran = (nblk[0] + q) / 2 > 0;            // stages of the other warpgroup
+                        if (other_ran) {
+                            tmem_ld16(tmem_base + 256 + (q ^ 1) * 128 + lane_base + c * 16, o2);
+                            tmem_wait_ld();
+                        }
+                        #pragma unroll
+                        for (int i = 0; i < 16; i++)
+                            o[i] = __float_as_uint(__uint_as_float(o[i]) * w_own + (other_ran ? __uint_as_float(o2[i]) * w_other : 0.f));
                     }
                     if (dst16) {
                         uint4 v0, v1;
@@ -510,15 +636,15 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 }
 
                 // ---- completion signal: one count per finished 64-row block, after its rows are visible.
-                // A 64-row block is two warps; the second of them to get here publishes the count.
+                // A 64-row block is two warps (KSPLIT: of each warpgroup); the last of them to get here publishes the count.
                 if (a.tile_counters != nullptr) {
                     if (a.counters_sys) __threadfence_system(); else __threadfence();
                     __syncwarp();
                     if (lane == 0) {
                         const int half = (warp & 3) >> 1;
-                        if (atomicAdd(&half_done[q][half], 1) == 1) {
+                        if (atomicAdd(&half_done[KSPLIT ? 0 : q][half], 1) == (KSPLIT ? 3 : 1)) {
                             if (a.counters_sys) __threadfence_system(); else __threadfence();
-                            atomicAdd(a.tile_counters + (block_row0 + q * WS_BM + half * 64) / a.tile_rows, 1);
+                            atomicAdd(a.tile_counters + (block_row0 + (KSPLIT ? 0 : q * WS_BM) + half * 64) / a.tile_rows, 1);
                         }
                     }
                 }
@@ -544,22 +670,23 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
-template <int D, bool OUT_F16, bool PERSIST>
+template <int D, bool OUT_F16, bool PERSIST, bool KSPLIT = false>
 int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args,
-              int reserve_sms, cudaStream_t stream)
+              int reserve_sms, cudaStream_t stream, int blocks = 0 /* of a 1-D grid; 0: all */)
 {
     using C = WsCfg<D>;
     static bool configured[64] = {};
     int dev = 0;
     EFA_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, PERSIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, PERSIST, KSPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         configured[dev] = true;
     }
     const int items_x = args.H_local * args.nsplit;
-    const int items_y = (args.q_rows + 2 * WS_BM - 1) / (2 * WS_BM);
+    const int item_rows = KSPLIT ? WS_BM : 2 * WS_BM;
+    const int items_y = (args.q_rows + item_rows - 1) / item_rows;
     const int total = items_x * items_y;
-    if (PERSIST) {
+    if constexpr (PERSIST) {
         int sms = 148;
         EFA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         int ctas = sms - reserve_sms;
@@ -568,32 +695,45 @@ int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
         int* counter = work_counter_slot();
         if (!counter) { set_error("no device memory for the work counter"); return 1; }
         EFA_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), stream));
-        fa_fwd_ws_kernel<D, OUT_F16, true><<<ctas, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, counter, items_x, total);
+        fa_fwd_ws_kernel<D, OUT_F16, true, KSPLIT><<<ctas, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, counter, items_x, total);
     } else {
-        dim3 grid(items_x, items_y);
-        fa_fwd_ws_kernel<D, OUT_F16, false><<<grid, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, nullptr, items_x, total);
+        const dim3 grid = blocks > 0 ? dim3(blocks) : dim3(items_x, items_y);
+        fa_fwd_ws_kernel<D, OUT_F16, false, KSPLIT><<<grid, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, nullptr, items_x, KSPLIT && blocks > 0 ? blocks : total);
     }
     EFA_CUDA(cudaGetLastError());
     return 0;
 }
 
+template <int D>
+int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a, bool out_f16,
+                int reserve_sms, cudaStream_t stream)
+{
+    if constexpr (D >= 64)
+        if (reserve_sms > 0) return out_f16 ? launch_ws<D, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<D, false, true>(tq, tk, tv, a, reserve_sms, stream);
+    // 128-row items with their keys split over the two warpgroups where the launch is short of items: an item takes
+    // half as long as a 256-row one, so waves * 1 against waves * 2. A row block that has a K/V stage to itself
+    // reads it twice as often from L2, so near-ties stay with 256 rows.
+    const long heads = (long)a.H_local * a.nsplit;
+    const long waves256 = (heads * ((a.q_rows + 255) / 256) + 147) / 148, waves128 = (heads * ((a.q_rows + 127) / 128) + 147) / 148;
+    if (a.order_tab == nullptr && waves128 * 4 <= waves256 * 2 * 3)
+        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false, true>(tq, tk, tv, a, 0, stream);
+    return out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream);
+}
+
 }  // namespace
 
 // Launch of the warp-specialised kernel; the caller has validated the arguments and built the maps.
-// reserve_sms > 0 selects the persistent form with that many SMs left free.
+// reserve_sms > 0 selects the persistent form with that many SMs left free (d_h 64 and 128).
 int fa_forward_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a,
                   int d_h, bool out_f16, int reserve_sms, cudaStream_t stream)
 {
-    const bool persist = reserve_sms > 0;
-    if (d_h == 64) {
-        if (persist) return out_f16 ? launch_ws<64, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<64, false, true>(tq, tk, tv, a, reserve_sms, stream);
-        return out_f16 ? launch_ws<64, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<64, false, false>(tq, tk, tv, a, 0, stream);
+    switch (d_h) {
+        case 16:  return launch_form<16>(tq, tk, tv, a, out_f16, reserve_sms, stream);
+        case 32:  return launch_form<32>(tq, tk, tv, a, out_f16, reserve_sms, stream);
+        case 64:  return launch_form<64>(tq, tk, tv, a, out_f16, reserve_sms, stream);
+        case 128: return launch_form<128>(tq, tk, tv, a, out_f16, reserve_sms, stream);
     }
-    if (d_h == 128) {
-        if (persist) return out_f16 ? launch_ws<128, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<128, false, true>(tq, tk, tv, a, reserve_sms, stream);
-        return out_f16 ? launch_ws<128, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<128, false, false>(tq, tk, tv, a, 0, stream);
-    }
-    set_error("fa_forward_ws: d_h=%d is not handled by the warp-specialised kernel", d_h);
+    set_error("fa_forward_ws: d_h=%d is not 16, 32, 64 or 128", d_h);
     return 2;
 }
 
@@ -611,12 +751,18 @@ template <class K> int touch_kernel(K kernel)
 
 // Loads the code of every instantiation now. A kernel's first launch may otherwise have to wait for the device to go
 // idle, which it never does while a stream sits in a front-end wait on a counter that is not coming.
+template <int D>
+static int touch_forms()
+{
+    return touch_kernel(fa_fwd_ws_kernel<D, true, false, false>) || touch_kernel(fa_fwd_ws_kernel<D, false, false, false>) ||
+           touch_kernel(fa_fwd_ws_kernel<D, true, false, true>) || touch_kernel(fa_fwd_ws_kernel<D, false, false, true>);
+}
+
 int fa_ws_preload()
 {
-    return touch_kernel(fa_fwd_ws_kernel<64, true, false>) || touch_kernel(fa_fwd_ws_kernel<64, false, false>) ||
-           touch_kernel(fa_fwd_ws_kernel<64, true, true>) || touch_kernel(fa_fwd_ws_kernel<64, false, true>) ||
-           touch_kernel(fa_fwd_ws_kernel<128, true, false>) || touch_kernel(fa_fwd_ws_kernel<128, false, false>) ||
-           touch_kernel(fa_fwd_ws_kernel<128, true, true>) || touch_kernel(fa_fwd_ws_kernel<128, false, true>);
+    return touch_forms<16>() || touch_forms<32>() || touch_forms<64>() || touch_forms<128>() ||
+           touch_kernel(fa_fwd_ws_kernel<64, true, true, false>) || touch_kernel(fa_fwd_ws_kernel<64, false, true, false>) ||
+           touch_kernel(fa_fwd_ws_kernel<128, true, true, false>) || touch_kernel(fa_fwd_ws_kernel<128, false, true, false>);
 }
 
 }  // namespace efa

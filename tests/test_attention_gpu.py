@@ -156,3 +156,34 @@ def test_full_size_rank_shards_on_sampled_rows(pkg, oracle, torch_cuda, S, H_loc
     ones = torch.ones((H_local, S, d_h), dtype=torch.float16, device="cuda")
     O1, _ = run_attention(pkg, torch, p, [dev[0], dev[1], ones], 0, S, pkg.F32)
     assert float((O1 - 1.0).abs().max()) < 2e-3
+
+
+# Key stages per 128-row block at which the two softmax warpgroups get none, one, an odd and an even number; few heads
+# take the form that splits the keys between them, many the form with 256 rows per block (H * split in (74, 148]).
+@pytest.mark.parametrize("H", [3, 40])
+@pytest.mark.parametrize("d_h", [16, 32, 64, 128])
+@pytest.mark.parametrize("S,q_start,q_rows,split,causal", [
+    (64, 0, 64, 1, 0), (128, 0, 128, 1, 1), (192, 64, 128, 1, 1), (320, 64, 256, 1, 0), (512, 128, 256, 2, 1),
+    (512, 0, 192, 2, 1), (640, 0, 64, 2, 1), (896, 448, 448, 2, 1)])
+def test_both_block_forms_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal):
+    torch = torch_cuda
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
+    g = torch.Generator(device="cuda").manual_seed(S + d_h + H)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    # rows whose maximum keeps growing along the keys: the exponent offset moves after the first stages too
+    dev[1] *= torch.linspace(0.5, 6.0, S, device="cuda", dtype=torch.float16)[None, :, None]
+    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
+    q, k, v = (t.double() for t in dev)
+    s = q[:, q_start:q_start + q_rows] @ k.transpose(1, 2) * p.flash_tc.scale
+    if causal:
+        rows = torch.arange(q_start, q_start + q_rows, device="cuda")[:, None]
+        s = s.masked_fill(torch.arange(S, device="cuda")[None, :] > rows, float("-inf"))
+    w = torch.softmax(s, dim=-1)
+    ref = (w @ v).permute(1, 0, 2).reshape(q_rows, H * d_h)
+    # Every softmax weight is rounded to fp16 (2^-11 of it) or, below 2^-14 of the largest, to a multiple of 2^-25; the
+    # offset may lag the maximum by 2^8. fp32 scores of up to about 100 carry 1e-5 of relative error into the weights.
+    bound = ((w * 2 ** -11 + 2.0 ** -24) @ v.abs()).permute(1, 0, 2).reshape(q_rows, H * d_h) + 1e-4 * ref.abs().max()
+    err = (O.double() - ref).abs()
+    assert torch.isfinite(O).all()
+    assert bool((err <= bound).all()), float((err - bound).max())
+    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)

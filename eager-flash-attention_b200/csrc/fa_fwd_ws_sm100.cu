@@ -717,6 +717,17 @@ int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     const long waves256 = (heads * ((a.q_rows + 255) / 256) + 147) / 148, waves128 = (heads * ((a.q_rows + 127) / 128) + 147) / 148;
     if (a.order_tab == nullptr && waves128 * 4 <= waves256 * 2 * 3)
         return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false, true>(tq, tk, tv, a, 0, stream);
+    // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
+    // is at most half of a wave it goes as 128-row items behind the full waves: 0.6 of a wave instead of one. From 4096 keys
+    // on, where that is worth ten times the second launch.
+    const long total = heads * ((a.q_rows + 255) / 256), rest = total % 148;
+    if (!a.causal && a.order_tab == nullptr && total > 148 && rest > 0 && rest * 2 <= 148 && a.kv_len >= 4096) {
+        FaArgs t = a;
+        t.tail_first = (int)(total - rest);
+        t.tail_total = (int)total;
+        if (int rc = out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream, t.tail_first) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream, t.tail_first)) return rc;
+        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, t, 0, stream, (int)rest * 2) : launch_ws<D, false, false, true>(tq, tk, tv, t, 0, stream, (int)rest * 2);
+    }
     return out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream);
 }
 

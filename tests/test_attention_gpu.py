@@ -187,3 +187,25 @@ def test_both_block_forms_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q
     assert torch.isfinite(O).all()
     assert bool((err <= bound).all()), float((err - bound).max())
     assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
+
+
+@pytest.mark.parametrize("d_h", [16, 64, 128])
+@pytest.mark.parametrize("H,q_start,q_rows,split", [(50, 64, 704, 1), (50, 0, 576, 1), (19, 2048, 2048, 1), (38, 0, 1024, 2)])
+def test_a_short_last_wave(pkg, torch_cuda, d_h, H, q_start, q_rows, split):
+    """Launches whose last wave is at most half full take its 256-row items as 128-row ones: ragged last blocks among
+    them, one with nothing in its second half."""
+    torch = torch_cuda
+    S = 4096 * split
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, 0)
+    g = torch.Generator(device="cuda").manual_seed(H + q_rows + d_h)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
+    assert torch.isfinite(O).all()
+    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
+    for h in range(H):
+        q, k, v = (t[h].double() for t in dev)
+        w = torch.softmax(q[q_start:q_start + q_rows] @ k.T * p.flash_tc.scale, dim=-1)
+        ref = w @ v
+        bound = (w * 2 ** -11 + 2.0 ** -24) @ v.abs() + 1e-4 * ref.abs().max()      # as above: softmax weights in fp16
+        err = (O[:, h * d_h:(h + 1) * d_h].double() - ref).abs()
+        assert bool((err <= bound).all()), (h, float((err - bound).max()))

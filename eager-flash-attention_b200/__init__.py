@@ -75,6 +75,12 @@ class Weights(C.Structure):
     _fields_ = [("Qh", C.c_void_p), ("Kh", C.c_void_p), ("Vh", C.c_void_p), ("W_O", C.c_void_p)]
 
 
+class FlashPlan(C.Structure):
+    """efa_flash_plan: the work items of an attention launch, and the K/V stages they keep in shared memory."""
+    _fields_ = [("items_256", C.c_int), ("items_128", C.c_int), ("k_slots", C.c_int), ("v_slots", C.c_int),
+                ("stage_step", C.c_int)]
+
+
 class StreamGroup(C.Structure):
     """efa_stream_group: tiles [first_tile, first_tile + ntiles) share one projection and one AllReduce."""
     _fields_ = [("first_tile", C.c_int), ("ntiles", C.c_int)]
@@ -98,6 +104,7 @@ _SIGNATURES = {
     "efa_flash_attn_tc_combine": (C.c_int, [C.POINTER(FlashPartials), C.c_void_p, C.c_int, C.c_int, C.c_int,
                                             C.POINTER(FlashParams), C.c_void_p]),
     "efa_flash_attn_tc_check_params": (C.c_char_p, [C.POINTER(FlashParams), C.c_int]),
+    "efa_flash_attn_tc_plan": (C.c_int, [C.POINTER(FlashParams), C.c_int, C.POINTER(FlashPlan)]),
     "efa_convert_f32_to_f16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "efa_project_f16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "efa_compute_qkv_f16": (C.c_int, [C.c_void_p] * 7 + [C.c_int] * 4 + [C.c_void_p]),
@@ -196,6 +203,13 @@ def attn_check_params(p: Params) -> Optional[str]:
 def flash_attn_tc_check_params(fp: FlashParams, q_rows: int) -> Optional[str]:
     why = lib().efa_flash_attn_tc_check_params(C.byref(fp), q_rows)
     return None if why is None else why.decode()
+
+
+def flash_attn_tc_plan(fp: FlashParams, q_rows: int) -> FlashPlan:
+    """The work items that flash_attn_tc_forward cuts a launch of ``q_rows`` rows into. Host arithmetic."""
+    plan = FlashPlan()
+    _check(lib().efa_flash_attn_tc_plan(C.byref(fp), q_rows, C.byref(plan)), "flash_attn_tc_plan")
+    return plan
 
 
 def blocks_per_tile(p: Params) -> int:

@@ -54,6 +54,14 @@ extern "C" const char* efa_flash_attn_tc_check_params(const efa_flash_params* p,
     return fa_check_params(*p, q_rows);
 }
 
+extern "C" int efa_flash_attn_tc_plan(const efa_flash_params* p, int q_rows, efa_flash_plan* out)
+{
+    if (!p || !out) { set_error("efa_flash_attn_tc_plan: null argument"); return 2; }
+    if (const char* why = fa_check_params(*p, q_rows)) { set_error("efa_flash_attn_tc_plan: %s", why); return 2; }
+    fa_plan(*p, q_rows, out);
+    return 0;
+}
+
 extern "C" int efa_convert_f32_to_f16(const float* in, void* out, size_t n, void* stream)
 {
     if ((!in || !out) && n) { set_error("efa_convert_f32_to_f16: null argument"); return 2; }

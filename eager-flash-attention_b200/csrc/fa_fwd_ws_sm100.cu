@@ -63,7 +63,7 @@ constexpr int WS_THREADS = 384;
 constexpr float kNegInfW = -INFINITY;
 constexpr float kRescaleThreshold = 8.0f;   // log2 units
 
-template <int D>
+template <int D, bool KSPLIT>
 struct WsCfg {
     static constexpr int SWB        = D >= 64 ? 128 : D * 2;      // swizzle width = TMA box row, bytes
     static constexpr int BOXC       = SWB / 2;
@@ -71,9 +71,16 @@ struct WsCfg {
     static constexpr int BOX_BYTES  = 128 * SWB;
     static constexpr int TILE_BYTES = 128 * D * 2;
     static constexpr int NSTAGE_K   = D == 128 ? 2 : 4;           // K(j+1) is wanted a whole stage after its slot is freed,
-    static constexpr int NSTAGE_V   = D == 128 ? 3 : 4;           // V(j) right at the start of the stage: the deeper ring
-    static constexpr int SMEM_BYTES = TILE_BYTES * (2 + NSTAGE_K + NSTAGE_V) + 1024;
+    static constexpr int NSTAGE_V   = D == 128 && !KSPLIT ? 3 : 4; // V(j) right at the start of the stage: the deeper ring
+    static constexpr int QTILES     = KSPLIT ? 1 : 2;
+    static constexpr int SMEM_BYTES = TILE_BYTES * (QTILES + NSTAGE_K + NSTAGE_V) + 1024;
     static constexpr int TMEM_COLS  = 512;
+    // A wait by parity only holds for a thread that waits for every phase of a slot in turn: one that skips a phase
+    // finds the parity it wants while the slot is still a phase behind. With KSPLIT an issuer takes every second stage, so
+    // each slot has to belong to one issuer.
+    static constexpr int STAGE_STEP = KSPLIT ? 2 : 1;
+    static_assert(NSTAGE_K % STAGE_STEP == 0 && NSTAGE_V % STAGE_STEP == 0, "an issuer would skip phases of a slot");
+    static_assert(!KSPLIT || 3 * WS_BM * (int)sizeof(float) <= TILE_BYTES, "the merge's exchange fits a K slot");
 };
 
 __device__ __forceinline__ float max3(float a, float b, float c)
@@ -129,7 +136,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                  const __grid_constant__ CUtensorMap tmV,
                  const FaArgs a, int* work_counter, int items_x, int items_total)
 {
-    using C = WsCfg<D>;
+    using C = WsCfg<D, KSPLIT>;
     constexpr uint32_t SWZ = swizzle_code(C::SWB);
     constexpr uint32_t IDESC_QK = idesc_f16_f32(WS_BM, WS_BN, 0, 0);
     constexpr uint32_t IDESC_PV = idesc_f16_f32(WS_BM, D, 0, 1);
@@ -145,8 +152,8 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* sQ = smem;                                   // 2 tiles
-    uint8_t* sK = sQ + 2 * C::TILE_BYTES;                 // NSK stages
+    uint8_t* sQ = smem;                                   // QTILES tiles
+    uint8_t* sK = sQ + C::QTILES * C::TILE_BYTES;         // NSK stages
     uint8_t* sV = sK + NSK * C::TILE_BYTES;               // NSV stages
 
     __shared__ __align__(8) uint64_t q_full[2];
@@ -273,7 +280,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     for (int b = 0; b < C::NBOX; b++)
                         tma_load_3d(dst + b * C::BOX_BYTES, tm, bar, b * C::BOXC, row, head);
                 };
-                for (int q = 0; q < (KSPLIT ? 1 : 2); q++)
+                for (int q = 0; q < C::QTILES; q++)
                     if (nblk[q] > 0) load_tile(sQ + q * C::TILE_BYTES, &tmQ, &q_full[q], q_abs0[q]);
                 for (int j = 0; j < nblk_max; j++) {
                     const int sk = j % NSK, uk = j / NSK, sv = j % NSV, uv = j / NSV;
@@ -550,20 +557,22 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 tc_fence_after_sync();
             }
 
-            // KSPLIT: both warpgroups learn each other's offset, maximum and sum; each then merges half of the columns.
+            // KSPLIT: both warpgroups learn each other's offset, maximum and sum; each then merges half of the columns. The
+            // exchange goes through K slot q, which only this warpgroup's stages used: all of them are consumed here.
             float w_own = 1.f, w_other = 0.f;
             if constexpr (KSPLIT) {
-                float (*xchg)[2 * WS_BM] = reinterpret_cast<float (*)[2 * WS_BM]>(sQ + C::TILE_BYTES);   // the second Q tile's place
-                xchg[0][tid] = m_ref; xchg[1][tid] = m_true; xchg[2][tid] = l_run;
+                float* own = reinterpret_cast<float*>(sK + q * C::TILE_BYTES) + row;
+                const float* other = reinterpret_cast<const float*>(sK + (q ^ 1) * C::TILE_BYTES) + row;
+                own[0] = m_ref; own[WS_BM] = m_true; own[2 * WS_BM] = l_run;
                 tc_fence_before_sync();
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 tc_fence_after_sync();
                 ok = __all_sync(0xffffffffu, ok && abort_word == 0);
-                const float m_ref_o = xchg[0][tid ^ WS_BM], l_o = xchg[2][tid ^ WS_BM];
+                const float m_ref_o = other[0], l_o = other[2 * WS_BM];
                 const float m_all = fmaxf(m_ref, m_ref_o);
                 w_own   = (m_ref == kNegInfW) ? 0.f : ex2(m_ref - m_all);
                 w_other = (m_ref_o == kNegInfW) ? 0.f : ex2(m_ref_o - m_all);
-                m_true = fmaxf(m_true, xchg[1][tid ^ WS_BM]);
+                m_true = fmaxf(m_true, other[WS_BM]);
                 l_run = l_run * w_own + l_o * w_other;
                 m_ref = m_all;
             }
@@ -674,7 +683,7 @@ template <int D, bool OUT_F16, bool PERSIST, bool KSPLIT = false>
 int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args,
               int reserve_sms, cudaStream_t stream, int blocks = 0 /* of a 1-D grid; 0: all */)
 {
-    using C = WsCfg<D>;
+    using C = WsCfg<D, KSPLIT>;
     static bool configured[64] = {};
     int dev = 0;
     EFA_CUDA(cudaGetDevice(&dev));
@@ -710,28 +719,62 @@ int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
 {
     if constexpr (D >= 64)
         if (reserve_sms > 0) return out_f16 ? launch_ws<D, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<D, false, true>(tq, tk, tv, a, reserve_sms, stream);
-    // 128-row items with their keys split over the two warpgroups where the launch is short of items: an item takes
-    // half as long as a 256-row one, so waves * 1 against waves * 2. A row block that has a K/V stage to itself
-    // reads it twice as often from L2, so near-ties stay with 256 rows.
-    const long heads = (long)a.H_local * a.nsplit;
-    const long waves256 = (heads * ((a.q_rows + 255) / 256) + 147) / 148, waves128 = (heads * ((a.q_rows + 127) / 128) + 147) / 148;
-    if (a.order_tab == nullptr && waves128 * 4 <= waves256 * 2 * 3)
+    const FaPlan plan = fa_ws_plan(a, D, reserve_sms);
+    if (plan.items256 == 0)
         return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false, true>(tq, tk, tv, a, 0, stream);
-    // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
-    // is at most half of a wave it goes as 128-row items behind the full waves: 0.6 of a wave instead of one. From 4096 keys
-    // on, where that is worth ten times the second launch.
-    const long total = heads * ((a.q_rows + 255) / 256), rest = total % 148;
-    if (!a.causal && a.order_tab == nullptr && total > 148 && rest > 0 && rest * 2 <= 148 && a.kv_len >= 4096) {
+    if (plan.items128 > 0) {
         FaArgs t = a;
-        t.tail_first = (int)(total - rest);
-        t.tail_total = (int)total;
+        t.tail_first = plan.items256;
+        t.tail_total = plan.items256 + plan.items128 / 2;
         if (int rc = out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream, t.tail_first) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream, t.tail_first)) return rc;
-        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, t, 0, stream, (int)rest * 2) : launch_ws<D, false, false, true>(tq, tk, tv, t, 0, stream, (int)rest * 2);
+        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, t, 0, stream, plan.items128) : launch_ws<D, false, false, true>(tq, tk, tv, t, 0, stream, plan.items128);
     }
     return out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream);
 }
 
+template <int D, bool KSPLIT>
+void ring_of(FaPlan& plan)
+{
+    using C = WsCfg<D, KSPLIT>;
+    plan.k_slots = C::NSTAGE_K;
+    plan.v_slots = C::NSTAGE_V;
+    plan.stage_step = C::STAGE_STEP;
+}
+
 }  // namespace
+
+// Which items a launch goes as. Host arithmetic only.
+FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
+{
+    // 128-row items with their keys split over the two warpgroups where the launch is short of items: an item takes
+    // half as long as a 256-row one, so waves * 1 against waves * 2. A row block that has a K/V stage to itself
+    // reads it twice as often from L2, so near-ties stay with 256 rows.
+    const long heads = (long)a.H_local * a.nsplit;
+    const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
+    const long waves256 = (total + 147) / 148, waves128 = (total128 + 147) / 148, rest = total % 148;
+    const bool free_form = a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64);
+    FaPlan plan;
+    plan.items256 = (int)total;
+    plan.items128 = 0;
+    if (free_form && waves128 * 4 <= waves256 * 2 * 3) {
+        plan.items256 = 0;
+        plan.items128 = (int)total128;
+    // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
+    // is at most half of a wave it goes as 128-row items behind the full waves: 0.6 of a wave instead of one. From 4096 keys
+    // on, where that is worth ten times the second launch.
+    } else if (free_form && !a.causal && total > 148 && rest > 0 && rest * 2 <= 148 && a.kv_len >= 4096) {
+        plan.items256 = (int)(total - rest);
+        plan.items128 = (int)rest * 2;
+    }
+    const bool ks = plan.items128 > 0;
+    switch (d_h) {
+        case 16:  ks ? ring_of<16, true>(plan)  : ring_of<16, false>(plan);  break;
+        case 32:  ks ? ring_of<32, true>(plan)  : ring_of<32, false>(plan);  break;
+        case 64:  ks ? ring_of<64, true>(plan)  : ring_of<64, false>(plan);  break;
+        case 128: ks ? ring_of<128, true>(plan) : ring_of<128, false>(plan); break;
+    }
+    return plan;
+}
 
 // Launch of the warp-specialised kernel; the caller has validated the arguments and built the maps.
 // reserve_sms > 0 selects the persistent form with that many SMs left free (d_h 64 and 128).

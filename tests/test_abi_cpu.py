@@ -157,6 +157,21 @@ def test_stream_plan_mixed_order(pkg):
     assert pkg.stream_row_blocks(q) == [] and pkg.stream_plan(q)[1] == 2048
 
 
+@pytest.mark.parametrize("d_h", [16, 32, 64, 128])
+@pytest.mark.parametrize("H", [2, 300])
+def test_every_issuing_thread_waits_for_all_phases_of_its_kv_slots(pkg, d_h, H):
+    """A wait by parity holds only for a thread that waits for each phase of the slot: the parity it wants also reads
+    as complete while the slot is one phase behind, so a phase left to another thread would let it pass early."""
+    plan = pkg.flash_attn_tc_plan(pkg.make_params(8192, H * d_h, H, 64, causal=1).flash_tc, 256)
+    assert (plan.items_256, plan.items_128) == ((0, 4) if H == 2 else (300, 0))
+    assert plan.stage_step == (2 if H == 2 else 1)
+    for slots in (plan.k_slots, plan.v_slots):
+        for first in range(plan.stage_step):
+            for slot in range(slots):
+                phases = [j // slots for j in range(first, 60, plan.stage_step) if j % slots == slot]
+                assert phases == list(range(len(phases))), (slots, first, slot)
+
+
 def test_stream_plan_counts_without_a_buffer_and_rejects_a_short_one(pkg):
     import ctypes as C
     p = pkg.make_params(32768, 4096, 32, 128, causal=1, world_size=1)

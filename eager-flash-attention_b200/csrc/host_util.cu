@@ -145,6 +145,14 @@ int* work_counter_slot()
     return ring[dev] + (next[dev]++ % kSlots);
 }
 
+bool own_device_memory(const void* p)
+{
+    int dev = -1;
+    cudaPointerAttributes attr;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&attr, p) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    return attr.type == cudaMemoryTypeDevice && attr.device == dev;
+}
+
 static int make_tmap(CUtensorMap* out, CUtensorMapDataType type, unsigned elem_bytes, const void* base, int rank,
                      const unsigned long long* dims, const unsigned long long* strides_bytes, const unsigned* box)
 {

@@ -59,6 +59,9 @@ int* kernel_status_word();
 // ring handed out round-robin; the caller clears its slot on the launch stream.
 int* work_counter_slot();
 
+// Whether p is memory of the current device itself: not mapped host memory, managed memory or another GPU's.
+bool own_device_memory(const void* p);
+
 // fp16 tensor map over a row-major tensor viewed as up to 3 dimensions (dim 0 fastest).
 // `box` rows x `box_cols` columns, swizzle chosen from box_cols * 2 bytes (32, 64 or 128).
 int make_tmap_f16(CUtensorMap* out, const void* base, int rank,

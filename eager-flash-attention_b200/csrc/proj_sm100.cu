@@ -27,7 +27,7 @@ constexpr int PJ_BM = 128;
 constexpr int PJ_BK = 64;
 constexpr int PJ_EPI_WARPS = 4;
 
-template <int BN>
+template <int BN, bool LOOP>
 struct PjCfg {
     static constexpr int A_BYTES    = PJ_BM * PJ_BK * 2;          // 16 KB
     static constexpr int B_BOX      = PJ_BK * 64 * 2;             // one [64 k][64 n] box, 8 KB
@@ -35,13 +35,21 @@ struct PjCfg {
     static constexpr int STAGE      = A_BYTES + B_BYTES;
     static constexpr int NSTAGE     = BN == 256 ? 4 : 6;
     static constexpr int OUT_BOX    = 32 * 128;                   // 32 rows of 128 bytes: one TMA store of one warp
-    static constexpr int OUT_BYTES  = PJ_EPI_WARPS * 2 * OUT_BOX; // two per warp
+    static constexpr int OUT_BYTES  = LOOP ? PJ_EPI_WARPS * 2 * OUT_BOX : 0;   // two per warp
+    static constexpr int ACCS       = LOOP ? 2 : 1;
     static constexpr int SMEM_BYTES = STAGE * NSTAGE + OUT_BYTES + 1024;
 };
+
+__device__ __forceinline__ uint4 pack8(const uint32_t* x)
+{
+    return make_uint4(pack_f16x2(__uint_as_float(x[0]), __uint_as_float(x[1])), pack_f16x2(__uint_as_float(x[2]), __uint_as_float(x[3])),
+                      pack_f16x2(__uint_as_float(x[4]), __uint_as_float(x[5])), pack_f16x2(__uint_as_float(x[6]), __uint_as_float(x[7])));
+}
 
 struct PjArgs {
     int M, N, K;
     int heads, d_h;     // HEADS: N = 3 * heads * d_h
+    void* out;          // without LOOP: fp16 or fp32 [M][N]
     int* status;
 };
 
@@ -50,16 +58,25 @@ struct PjArgs {
 // result is [heads][M][d_h]. d_h is a multiple of 64, so every 64-column box lies in one head of one tensor, and a
 // tile may span heads and tensors: A is read once for all of them, and narrow heads still fill wide tiles. Measured,
 // 8192 x 4096 to Q, K and V of four heads of 128: 297 us as twelve launches of 64 tiles each, 98 us as one of 384.
+// LOOP = false: a block per tile, stored row by row from registers with plain stores, which go wherever the kernel may
+// write. Nothing promises that for bulk tensor stores: outputs in mapped host memory, managed memory or another GPU's
+// memory take this form.
+template <int TENSORS, bool LOOP>
 struct PjMaps {
-    CUtensorMap A, W[3], out[3];
+    CUtensorMap A, W[TENSORS], out[TENSORS];
+};
+template <int TENSORS>
+struct PjMaps<TENSORS, false> {
+    CUtensorMap A, W[TENSORS];
 };
 
-template <int BN, bool OUT_F32, bool HEADS>
+template <int BN, bool OUT_F32, bool HEADS, bool LOOP>
 __global__ void __launch_bounds__(192, 1)
-proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
+proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const PjArgs a)
 {
     static_assert(!(OUT_F32 && HEADS), "Q, K and V are fp16");
-    using C = PjCfg<BN>;
+    static_assert(LOOP || !HEADS, "the plain stores know one output");
+    using C = PjCfg<BN, LOOP>;
     constexpr uint32_t IDESC = idesc_f16_f32(PJ_BM, BN, 0, 1);
     constexpr uint32_t SWZ = swizzle_code(128);
 
@@ -91,10 +108,13 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
         }
         mbar_fence_init();
         tma_prefetch_desc(&maps.A);
-        for (int t = 0; t < (HEADS ? 3 : 1); t++) { tma_prefetch_desc(&maps.W[t]); tma_prefetch_desc(&maps.out[t]); }
+        for (int t = 0; t < (HEADS ? 3 : 1); t++) {
+            tma_prefetch_desc(&maps.W[t]);
+            if constexpr (LOOP) tma_prefetch_desc(&maps.out[t]);
+        }
     }
     __syncwarp();
-    if (warp == 1) tmem_alloc(&tmem_base_smem, 2 * BN);
+    if (warp == 1) tmem_alloc(&tmem_base_smem, C::ACCS * BN);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -103,7 +123,7 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
     // Tile of round `it`: the CTA's own block first, then the answer to request it - 1. false: no more (or gave up).
     auto next = [&](int it, int& bx, int& by) -> bool {
         const int s = it & 1;
-        if (!mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
+        if (!LOOP || !mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
         return clc_query(&next_tile[s], bx, by);
     };
 
@@ -124,8 +144,10 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
             for (int it = 0; ok; it++) {
                 const int ns = it & 1;
                 if (it >= 2 && !mbar_wait(&next_empty[ns], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 15)) break;
-                mbar_expect_tx(&next_full[ns], 16);
-                clc_try_cancel(&next_tile[ns], &next_full[ns]);
+                if constexpr (LOOP) {
+                    mbar_expect_tx(&next_full[ns], 16);
+                    clc_try_cancel(&next_tile[ns], &next_full[ns]);
+                }
                 const int n0 = bx * BN, m0 = by * PJ_BM;
                 const int nbox = min(BN / 64, (a.N - n0) / 64);   // N is a multiple of 64
                 int wt[BN / 64], wh[BN / 64], wx[BN / 64];
@@ -202,49 +224,64 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (uint32_t)((it >> 1) & 1), &abort_word, 13))) break;
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(lane_grp * 32) << 16);
-            #pragma unroll 1
-            for (int c = 0; c < BN / COLS; c++, stores++) {
-                if (n0 + c * COLS >= a.N) break;
-                uint4 v[8];                                       // this lane's row: eight 16-byte chunks
-                if constexpr (OUT_F32) {
+            if constexpr (!LOOP) {
+                const int cols = row0 < a.M ? min(BN, a.N - n0) : 0;   // row0 and M are multiples of 32, columns of 64
+                #pragma unroll 1
+                for (int c = 0; c < cols / 32; c++) {
+                    const int col = n0 + c * 32;
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
                     tmem_wait_ld();
-                    #pragma unroll
-                    for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                } else {
-                    uint32_t r[2][32];
-                    tmem_ld32(taddr + c * 64, r[0]);
-                    tmem_ld32(taddr + c * 64 + 32, r[1]);
-                    tmem_wait_ld();
-                    #pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const uint32_t* x = &r[q >> 2][8 * (q & 3)];
-                        v[q].x = pack_f16x2(__uint_as_float(x[0]), __uint_as_float(x[1]));
-                        v[q].y = pack_f16x2(__uint_as_float(x[2]), __uint_as_float(x[3]));
-                        v[q].z = pack_f16x2(__uint_as_float(x[4]), __uint_as_float(x[5]));
-                        v[q].w = pack_f16x2(__uint_as_float(x[6]), __uint_as_float(x[7]));
+                    const size_t at = (size_t)(row0 + lane) * a.N + col;
+                    if constexpr (OUT_F32) {
+                        uint4* dst = reinterpret_cast<uint4*>(static_cast<float*>(a.out) + at);
+                        #pragma unroll
+                        for (int q = 0; q < 8; q++) dst[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    } else {
+                        uint4* dst = reinterpret_cast<uint4*>(static_cast<__half*>(a.out) + at);
+                        #pragma unroll
+                        for (int q = 0; q < 4; q++) dst[q] = pack8(&r[8 * q]);
                     }
                 }
-                uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
-                if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
-                __syncwarp();
-                #pragma unroll
-                for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
-                    *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    if (row0 < a.M) {
-                        if constexpr (HEADS) {
-                            int t, head, x;
-                            locate(n0 + c * COLS, t, head, x);
-                            tma_store_3d(&maps.out[t], box, x, row0, head);
-                        } else {
-                            tma_store_2d(&maps.out[0], box, n0 + c * COLS, row0);
-                        }
+            } else {
+                #pragma unroll 1
+                for (int c = 0; c < BN / COLS; c++, stores++) {
+                    if (n0 + c * COLS >= a.N) break;
+                    uint4 v[8];                                       // this lane's row: eight 16-byte chunks
+                    if constexpr (OUT_F32) {
+                        uint32_t r[32];
+                        tmem_ld32(taddr + c * 32, r);
+                        tmem_wait_ld();
+                        #pragma unroll
+                        for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    } else {
+                        uint32_t r[2][32];
+                        tmem_ld32(taddr + c * 64, r[0]);
+                        tmem_ld32(taddr + c * 64 + 32, r[1]);
+                        tmem_wait_ld();
+                        #pragma unroll
+                        for (int q = 0; q < 8; q++) v[q] = pack8(&r[q >> 2][8 * (q & 3)]);
                     }
-                    tma_store_commit();                           // also without a store: the waits above count groups
+                    uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
+                    if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
+                    __syncwarp();
+                    #pragma unroll
+                    for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
+                        *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (row0 < a.M) {
+                            if constexpr (HEADS) {
+                                int t, head, x;
+                                locate(n0 + c * COLS, t, head, x);
+                                tma_store_3d(&maps.out[t], box, x, row0, head);
+                            } else {
+                                tma_store_2d(&maps.out[0], box, n0 + c * COLS, row0);
+                            }
+                        }
+                        tma_store_commit();                           // also without a store: the waits above count groups
+                    }
                 }
             }
             tc_fence_before_sync();
@@ -256,7 +293,7 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
             if (lane == 0) mbar_arrive(&next_empty[it & 1]);
             if (!more) break;
         }
-        if (lane == 0) tma_store_wait_all();
+        if (LOOP && lane == 0) tma_store_wait_all();
     }
 
     __syncwarp();
@@ -272,24 +309,31 @@ proj_gemm_kernel(const __grid_constant__ PjMaps maps, const PjArgs a)
         }
         __syncthreads();
     }
-    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == 1) tmem_dealloc(tmem_base, C::ACCS * BN);
 }
 
-template <int BN, bool OUT_F32, bool HEADS>
-int launch_proj(const PjMaps& maps, const PjArgs& args, cudaStream_t stream)
+template <int BN, bool OUT_F32, bool HEADS, bool LOOP>
+int launch_proj(const PjMaps<HEADS ? 3 : 1, LOOP>& maps, const PjArgs& args, cudaStream_t stream)
 {
-    using C = PjCfg<BN>;
+    using C = PjCfg<BN, LOOP>;
     static bool configured[64] = {};
     int dev = 0;
     EFA_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        EFA_CUDA(cudaFuncSetAttribute(proj_gemm_kernel<BN, OUT_F32, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        EFA_CUDA(cudaFuncSetAttribute(proj_gemm_kernel<BN, OUT_F32, HEADS, LOOP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         configured[dev] = true;
     }
     dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
-    proj_gemm_kernel<BN, OUT_F32, HEADS><<<grid, 192, C::SMEM_BYTES, stream>>>(maps, args);
+    proj_gemm_kernel<BN, OUT_F32, HEADS, LOOP><<<grid, 192, C::SMEM_BYTES, stream>>>(maps, args);
     EFA_CUDA(cudaGetLastError());
     return 0;
+}
+
+template <bool LOOP>
+int launch_form(const PjMaps<1, LOOP>& maps, const PjArgs& a, bool wide, bool f32, cudaStream_t stream)
+{
+    if (f32) return wide ? launch_proj<256, true, false, LOOP>(maps, a, stream) : launch_proj<128, true, false, LOOP>(maps, a, stream);
+    return wide ? launch_proj<256, false, false, LOOP>(maps, a, stream) : launch_proj<128, false, false, LOOP>(maps, a, stream);
 }
 
 // Tile width: the one that leaves the busiest SM less to fetch. What bounds the kernel is the rate at which tiles come
@@ -320,13 +364,13 @@ int input_map(CUtensorMap* out, const void* A, int rows, int k)
 
 }  // namespace
 
-int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype)
+int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out)
 {
     if (out_dtype != EFA_F16 && out_dtype != EFA_F32) { set_error("project: unknown output type %d", out_dtype); return 2; }
     if (int rc = check_shape(rows, d_local, d)) return rc;
     if (!A || !W || !out) { set_error("project: null pointer"); return 2; }
 
-    PjMaps maps;
+    PjMaps<1, true> maps;
     if (input_map(&maps.A, A, rows, d_local)) return 1;
     {
         unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)d_local};
@@ -334,17 +378,17 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
         unsigned box[2] = {64u, 64u};
         if (make_tmap_f16(&maps.W[0], W, 2, dims, strides, box)) return 1;
     }
-    {
-        const bool f32 = out_dtype == EFA_F32;
-        unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)rows};
-        unsigned long long strides[1] = {(unsigned long long)d * (f32 ? 4ull : 2ull)};
-        unsigned box[2] = {f32 ? 32u : 64u, 32u};
-        if (f32 ? make_tmap_f32(&maps.out[0], out, 2, dims, strides, box) : make_tmap_f16(&maps.out[0], out, 2, dims, strides, box)) return 1;
+    const bool f32 = out_dtype == EFA_F32, wide = wide_tiles(rows, d);
+    PjArgs a{rows, d, d_local, 1, d, out, kernel_status_word()};
+    if (!own_out && !own_device_memory(out)) {
+        if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
+        return launch_form<false>({maps.A, {maps.W[0]}}, a, wide, f32, stream);
     }
-    PjArgs a{rows, d, d_local, 1, d, kernel_status_word()};
-    const bool wide = wide_tiles(rows, d);
-    if (out_dtype == EFA_F32) return wide ? launch_proj<256, true, false>(maps, a, stream) : launch_proj<128, true, false>(maps, a, stream);
-    return wide ? launch_proj<256, false, false>(maps, a, stream) : launch_proj<128, false, false>(maps, a, stream);
+    unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)rows};
+    unsigned long long strides[1] = {(unsigned long long)d * (f32 ? 4ull : 2ull)};
+    unsigned box[2] = {f32 ? 32u : 64u, 32u};
+    if (f32 ? make_tmap_f32(&maps.out[0], out, 2, dims, strides, box) : make_tmap_f16(&maps.out[0], out, 2, dims, strides, box)) return 1;
+    return launch_form<true>(maps, a, wide, f32, stream);
 }
 
 int project_heads_f16(const void* X, const void* const W[3], void* const out[3], int rows, int d, int heads, int d_h,
@@ -352,7 +396,16 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
 {
     if (int rc = check_shape(rows, d, d_h)) return rc;
     if ((long)3 * heads * d_h > 0x7fffff00l) { set_error("project: %d heads of %d are too many columns", heads, d_h); return 2; }
-    PjMaps maps;
+    if (!own_device_memory(out[0]) || !own_device_memory(out[1]) || !own_device_memory(out[2])) {
+        // where the staged stores cannot go: head by head
+        for (int h = 0; h < heads; h++)
+            for (int t = 0; t < 3; t++)
+                if (int rc = project_f16(X, static_cast<const __half*>(W[t]) + (size_t)h * d * d_h,
+                                         static_cast<__half*>(out[t]) + (size_t)h * rows * d_h, rows, d, d_h, stream))
+                    return rc;
+        return 0;
+    }
+    PjMaps<3, true> maps;
     if (input_map(&maps.A, X, rows, d)) return 1;
     for (int t = 0; t < 3; t++) {
         // three dimensions, so that rows past d read as zero and not as the next head's
@@ -366,8 +419,8 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
         if (make_tmap_f16(&maps.out[t], out[t], 3, odims, ostrides, obox)) return 1;
     }
     const int cols = 3 * heads * d_h;
-    PjArgs a{rows, cols, d, heads, d_h, kernel_status_word()};
-    return wide_tiles(rows, cols) ? launch_proj<256, false, true>(maps, a, stream) : launch_proj<128, false, true>(maps, a, stream);
+    PjArgs a{rows, cols, d, heads, d_h, nullptr, kernel_status_word()};
+    return wide_tiles(rows, cols) ? launch_proj<256, false, true, true>(maps, a, stream) : launch_proj<128, false, true, true>(maps, a, stream);
 }
 
 
@@ -382,9 +435,11 @@ template <class K> int touch_kernel(K kernel)
 
 int proj_preload()
 {
-    return touch_kernel(proj_gemm_kernel<128, false, false>) || touch_kernel(proj_gemm_kernel<128, true, false>) ||
-           touch_kernel(proj_gemm_kernel<256, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false>) ||
-           touch_kernel(proj_gemm_kernel<128, false, true>) || touch_kernel(proj_gemm_kernel<256, false, true>);
+    return touch_kernel(proj_gemm_kernel<128, false, false, true>) || touch_kernel(proj_gemm_kernel<128, true, false, true>) ||
+           touch_kernel(proj_gemm_kernel<256, false, false, true>) || touch_kernel(proj_gemm_kernel<256, true, false, true>) ||
+           touch_kernel(proj_gemm_kernel<128, false, false, false>) || touch_kernel(proj_gemm_kernel<128, true, false, false>) ||
+           touch_kernel(proj_gemm_kernel<256, false, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false, false>) ||
+           touch_kernel(proj_gemm_kernel<128, false, true, true>) || touch_kernel(proj_gemm_kernel<256, false, true, true>);
 }
 
 }  // namespace efa

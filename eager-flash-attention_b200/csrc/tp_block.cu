@@ -110,17 +110,13 @@ struct Run {
 
     // One rank: its partial sum is the result, so the projection writes `output` itself and nothing is reduced. A
     // one-rank AllReduce is a copy (0.5 GB read and written at 32k rows of d = 4096) and, tile by tile, a launch and several
-    // microseconds of host time per group. Not where the kernel's TMA stores could not go (an output that is
-    // not this GPU's own memory or not 16-byte aligned) or where writing early would disturb W_O.
+    // microseconds of host time per group. Not for an output that is not this GPU's own memory (the copy then
+    // crosses to it once, behind the projections) or not 16-byte aligned, or where writing early would disturb W_O.
     bool direct = false;
     void choose_direct(const void* output)
     {
         if (p.R != 1 || p.skip_comm || p.skip_proj || p.reduce == EFA_REDUCE_P2P || ((uintptr_t)output & 15) != 0) return;
-        int dev = -1;
-        if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return; }
-        cudaPointerAttributes attr;
-        if (cudaPointerGetAttributes(&attr, output) != cudaSuccess) { (void)cudaGetLastError(); return; }
-        if (attr.type != cudaMemoryTypeDevice || attr.device != dev) return;
+        if (!own_device_memory(output)) return;
         const char* o = static_cast<const char*>(output);
         const char* wo = static_cast<const char*>(static_cast<const void*>(w.W_O));
         if (o < wo + (size_t)p.d_local * p.d * sizeof(__half) && wo < o + (size_t)p.S * row_bytes()) return;
@@ -167,7 +163,8 @@ struct Run {
     {
         if (p.skip_proj) return 0;
         launches++;
-        return project_f16(O_tile, w.W_O, out, rows, p.d_local, p.d, c->proj_stream, wire_f32() ? EFA_F32 : EFA_F16);
+        return project_f16(O_tile, w.W_O, out, rows, p.d_local, p.d, c->proj_stream, wire_f32() ? EFA_F32 : EFA_F16,
+                           /* send buffers are, and a direct output has been looked at: */ true);
     }
     // allreduce (run_drivers.cu:26-30): sum of n partial sums at `send` (a place in the send buffer) over the ranks
     // into `recv` (a place in `output`), on communicator / stream `slot`.

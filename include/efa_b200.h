@@ -119,7 +119,8 @@ int efa_convert_f32_to_f16(const float* in, void* out, size_t n, void* stream);
 
 /* project (attn_main.cuh:62-65, attn_main.cu:262-273) for the fp16 data path:
  * out[rows][d] = O_tile[rows][d_local] * W_O[d_local][d], fp16 operands, fp32 accumulate, fp16 out.
- * rows must be a multiple of 64, d_local a multiple of 16, d a multiple of 64. */
+ * rows must be a multiple of 64, d_local a multiple of 16, d a multiple of 64. out: any 16-byte aligned memory that the
+ * GPU may write (its own, mapped host memory, managed memory, a peer's). */
 int efa_project_f16(const void* O_tile, const void* W_O, void* out,
                     int rows, int d_local, int d, void* stream);
 
@@ -127,7 +128,8 @@ int efa_project_f16(const void* O_tile, const void* W_O, void* out,
  * per local head h, Q_h[S][d_h] = X[S][d] * W_q_h[d][d_h] (and K, V alike) with the projection kernel,
  * fp32 accumulate, written as fp16 head-major [H_local][S][d_h] directly (the reference computes in
  * fp32 with cuBLAS and converts in a second pass). X fp16 [S][d]; W_q/W_k/W_v fp16 [H_local][d][d_h].
- * d_h must be 64 or 128, S a multiple of 64, d a multiple of 16. Untimed in the reference. */
+ * d_h must be 64 or 128, S a multiple of 64, d a multiple of 16; outputs as for efa_project_f16. Untimed in the
+ * reference. */
 int efa_compute_qkv_f16(const void* X, const void* W_q, const void* W_k, const void* W_v,
                         void* Qh, void* Kh, void* Vh, int S, int d, int H_local, int d_h, void* stream);
 

@@ -28,6 +28,43 @@ def test_projection_matches_float64(pkg, torch_cuda, rows, d_local, d):
     assert bool((err <= bound).all()), float((err - bound).max())
 
 
+# Ragged last rows and columns, one tile and several per SM, both tile widths; heads that share a tile.
+@pytest.mark.parametrize("rows,d_local,d", [(64, 16, 64), (192, 80, 448), (320, 256, 4096), (19136, 48, 320)])
+def test_projection_into_mapped_host_memory(pkg, torch_cuda, rows, d_local, d):
+    """An output that is not this GPU's own memory gets the same values as one that is."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows + d)
+    A = torch.randn(rows, d_local, generator=g, device="cuda").to(torch.float16)
+    W = (torch.randn(d_local, d, generator=g, device="cuda") / d ** 0.5).to(torch.float16)
+    out = torch.full((rows + 1, d), float("nan"), dtype=torch.float16, device="cuda")
+    host = torch.full((rows + 1, d), float("nan"), dtype=torch.float16).pin_memory()
+    pkg.kernel_status_reset()
+    for o in (out, host):
+        pkg.project(A, W, o, rows, d_local, d)
+    torch.cuda.synchronize()
+    assert pkg.kernel_status()[0] == 0
+    assert torch.isfinite(out[:rows]).all() and torch.equal(out[:rows].cpu(), host[:rows])
+    assert torch.isnan(host[rows]).all()                         # nothing behind the last row
+    with pytest.raises(pkg.EfaError, match="16-byte"):
+        pkg.project(A, W, host.view(-1)[1:], rows, d_local, d)
+
+
+@pytest.mark.parametrize("S,d,H_local,d_h", [(192, 80, 3, 64), (4160, 96, 3, 128)])
+def test_compute_qkv_into_mapped_host_memory(pkg, torch_cuda, S, d, H_local, d_h):
+    """One of the three outputs in host memory is enough for all of them to be written the plain way."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S + d)
+    X = torch.randn(S, d, generator=g, device="cuda").to(torch.float16)
+    W = [torch.randn(H_local, d, d_h, generator=g, device="cuda").to(torch.float16) * 0.1 for _ in range(3)]
+    out = [torch.full((H_local, S, d_h), float("nan"), dtype=torch.float16, device="cuda") for _ in range(3)]
+    mixed = [out[0].clone(), out[1].cpu().pin_memory(), out[2].clone()]
+    for o in (out, mixed):
+        pkg.compute_qkv(X, *W, *o, S, d, H_local, d_h)
+    torch.cuda.synchronize()
+    for a, b in zip(out, mixed):
+        assert torch.isfinite(a).all() and torch.equal(a.cpu(), b.cpu())
+
+
 def test_projection_rejects_bad_shapes(pkg, torch_cuda):
     torch = torch_cuda
     A = torch.zeros(128, 64, dtype=torch.float16, device="cuda")

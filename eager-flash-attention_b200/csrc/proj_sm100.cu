@@ -27,7 +27,7 @@ constexpr int PJ_BM = 128;
 constexpr int PJ_BK = 64;
 constexpr int PJ_EPI_WARPS = 4;
 
-template <int BN, bool LOOP>
+template <int BN, bool STAGED>
 struct PjCfg {
     static constexpr int A_BYTES    = PJ_BM * PJ_BK * 2;          // 16 KB
     static constexpr int B_BOX      = PJ_BK * 64 * 2;             // one [64 k][64 n] box, 8 KB
@@ -35,8 +35,7 @@ struct PjCfg {
     static constexpr int STAGE      = A_BYTES + B_BYTES;
     static constexpr int NSTAGE     = BN == 256 ? 4 : 6;
     static constexpr int OUT_BOX    = 32 * 128;                   // 32 rows of 128 bytes: one TMA store of one warp
-    static constexpr int OUT_BYTES  = LOOP ? PJ_EPI_WARPS * 2 * OUT_BOX : 0;   // two per warp
-    static constexpr int ACCS       = LOOP ? 2 : 1;
+    static constexpr int OUT_BYTES  = STAGED ? PJ_EPI_WARPS * 2 * OUT_BOX : 0;   // two per warp
     static constexpr int SMEM_BYTES = STAGE * NSTAGE + OUT_BYTES + 1024;
 };
 
@@ -49,7 +48,6 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* x)
 struct PjArgs {
     int M, N, K;
     int heads, d_h;     // HEADS: N = 3 * heads * d_h
-    void* out;          // without LOOP: fp16 or fp32 [M][N]
     int* status;
 };
 
@@ -58,25 +56,17 @@ struct PjArgs {
 // result is [heads][M][d_h]. d_h is a multiple of 64, so every 64-column box lies in one head of one tensor, and a
 // tile may span heads and tensors: A is read once for all of them, and narrow heads still fill wide tiles. Measured,
 // 8192 x 4096 to Q, K and V of four heads of 128: 297 us as twelve launches of 64 tiles each, 98 us as one of 384.
-// LOOP = false: a block per tile, stored row by row from registers with plain stores, which go wherever the kernel may
-// write. Nothing promises that for bulk tensor stores: outputs in mapped host memory, managed memory or another GPU's
-// memory take this form.
-template <int TENSORS, bool LOOP>
+template <int TENSORS>
 struct PjMaps {
     CUtensorMap A, W[TENSORS], out[TENSORS];
 };
-template <int TENSORS>
-struct PjMaps<TENSORS, false> {
-    CUtensorMap A, W[TENSORS];
-};
 
-template <int BN, bool OUT_F32, bool HEADS, bool LOOP>
+template <int BN, bool OUT_F32, bool HEADS>
 __global__ void __launch_bounds__(192, 1)
-proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const PjArgs a)
+proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjArgs a)
 {
     static_assert(!(OUT_F32 && HEADS), "Q, K and V are fp16");
-    static_assert(LOOP || !HEADS, "the plain stores know one output");
-    using C = PjCfg<BN, LOOP>;
+    using C = PjCfg<BN, true>;
     constexpr uint32_t IDESC = idesc_f16_f32(PJ_BM, BN, 0, 1);
     constexpr uint32_t SWZ = swizzle_code(128);
 
@@ -108,13 +98,10 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
         }
         mbar_fence_init();
         tma_prefetch_desc(&maps.A);
-        for (int t = 0; t < (HEADS ? 3 : 1); t++) {
-            tma_prefetch_desc(&maps.W[t]);
-            if constexpr (LOOP) tma_prefetch_desc(&maps.out[t]);
-        }
+        for (int t = 0; t < (HEADS ? 3 : 1); t++) { tma_prefetch_desc(&maps.W[t]); tma_prefetch_desc(&maps.out[t]); }
     }
     __syncwarp();
-    if (warp == 1) tmem_alloc(&tmem_base_smem, C::ACCS * BN);
+    if (warp == 1) tmem_alloc(&tmem_base_smem, 2 * BN);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -123,7 +110,7 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
     // Tile of round `it`: the CTA's own block first, then the answer to request it - 1. false: no more (or gave up).
     auto next = [&](int it, int& bx, int& by) -> bool {
         const int s = it & 1;
-        if (!LOOP || !mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
+        if (!mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
         return clc_query(&next_tile[s], bx, by);
     };
 
@@ -144,10 +131,8 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
             for (int it = 0; ok; it++) {
                 const int ns = it & 1;
                 if (it >= 2 && !mbar_wait(&next_empty[ns], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 15)) break;
-                if constexpr (LOOP) {
-                    mbar_expect_tx(&next_full[ns], 16);
-                    clc_try_cancel(&next_tile[ns], &next_full[ns]);
-                }
+                mbar_expect_tx(&next_full[ns], 16);
+                clc_try_cancel(&next_tile[ns], &next_full[ns]);
                 const int n0 = bx * BN, m0 = by * PJ_BM;
                 const int nbox = min(BN / 64, (a.N - n0) / 64);   // N is a multiple of 64
                 int wt[BN / 64], wh[BN / 64], wx[BN / 64];
@@ -224,64 +209,43 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (uint32_t)((it >> 1) & 1), &abort_word, 13))) break;
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(lane_grp * 32) << 16);
-            if constexpr (!LOOP) {
-                const int cols = row0 < a.M ? min(BN, a.N - n0) : 0;   // row0 and M are multiples of 32, columns of 64
-                #pragma unroll 1
-                for (int c = 0; c < cols / 32; c++) {
-                    const int col = n0 + c * 32;
+            #pragma unroll 1
+            for (int c = 0; c < BN / COLS; c++, stores++) {
+                if (n0 + c * COLS >= a.N) break;
+                uint4 v[8];                                       // this lane's row: eight 16-byte chunks
+                if constexpr (OUT_F32) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c * 32, r);
                     tmem_wait_ld();
-                    const size_t at = (size_t)(row0 + lane) * a.N + col;
-                    if constexpr (OUT_F32) {
-                        uint4* dst = reinterpret_cast<uint4*>(static_cast<float*>(a.out) + at);
-                        #pragma unroll
-                        for (int q = 0; q < 8; q++) dst[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                    } else {
-                        uint4* dst = reinterpret_cast<uint4*>(static_cast<__half*>(a.out) + at);
-                        #pragma unroll
-                        for (int q = 0; q < 4; q++) dst[q] = pack8(&r[8 * q]);
-                    }
-                }
-            } else {
-                #pragma unroll 1
-                for (int c = 0; c < BN / COLS; c++, stores++) {
-                    if (n0 + c * COLS >= a.N) break;
-                    uint4 v[8];                                       // this lane's row: eight 16-byte chunks
-                    if constexpr (OUT_F32) {
-                        uint32_t r[32];
-                        tmem_ld32(taddr + c * 32, r);
-                        tmem_wait_ld();
-                        #pragma unroll
-                        for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                    } else {
-                        uint32_t r[2][32];
-                        tmem_ld32(taddr + c * 64, r[0]);
-                        tmem_ld32(taddr + c * 64 + 32, r[1]);
-                        tmem_wait_ld();
-                        #pragma unroll
-                        for (int q = 0; q < 8; q++) v[q] = pack8(&r[q >> 2][8 * (q & 3)]);
-                    }
-                    uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
-                    if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
-                    __syncwarp();
                     #pragma unroll
-                    for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
-                        *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (row0 < a.M) {
-                            if constexpr (HEADS) {
-                                int t, head, x;
-                                locate(n0 + c * COLS, t, head, x);
-                                tma_store_3d(&maps.out[t], box, x, row0, head);
-                            } else {
-                                tma_store_2d(&maps.out[0], box, n0 + c * COLS, row0);
-                            }
+                    for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                } else {
+                    uint32_t r[2][32];
+                    tmem_ld32(taddr + c * 64, r[0]);
+                    tmem_ld32(taddr + c * 64 + 32, r[1]);
+                    tmem_wait_ld();
+                    #pragma unroll
+                    for (int q = 0; q < 8; q++) v[q] = pack8(&r[q >> 2][8 * (q & 3)]);
+                }
+                uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
+                if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
+                __syncwarp();
+                #pragma unroll
+                for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
+                    *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (row0 < a.M) {
+                        if constexpr (HEADS) {
+                            int t, head, x;
+                            locate(n0 + c * COLS, t, head, x);
+                            tma_store_3d(&maps.out[t], box, x, row0, head);
+                        } else {
+                            tma_store_2d(&maps.out[0], box, n0 + c * COLS, row0);
                         }
-                        tma_store_commit();                           // also without a store: the waits above count groups
                     }
+                    tma_store_commit();                           // also without a store: the waits above count groups
                 }
             }
             tc_fence_before_sync();
@@ -293,7 +257,7 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
             if (lane == 0) mbar_arrive(&next_empty[it & 1]);
             if (!more) break;
         }
-        if (LOOP && lane == 0) tma_store_wait_all();
+        if (lane == 0) tma_store_wait_all();
     }
 
     __syncwarp();
@@ -309,31 +273,171 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1, LOOP> maps, const
         }
         __syncthreads();
     }
-    if (warp == 1) tmem_dealloc(tmem_base, C::ACCS * BN);
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
 }
 
-template <int BN, bool OUT_F32, bool HEADS, bool LOOP>
-int launch_proj(const PjMaps<HEADS ? 3 : 1, LOOP>& maps, const PjArgs& args, cudaStream_t stream)
+template <int BN, bool OUT_F32, bool HEADS>
+int launch_proj(const PjMaps<HEADS ? 3 : 1>& maps, const PjArgs& args, cudaStream_t stream)
 {
-    using C = PjCfg<BN, LOOP>;
+    using C = PjCfg<BN, true>;
     static bool configured[64] = {};
     int dev = 0;
     EFA_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        EFA_CUDA(cudaFuncSetAttribute(proj_gemm_kernel<BN, OUT_F32, HEADS, LOOP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        EFA_CUDA(cudaFuncSetAttribute(proj_gemm_kernel<BN, OUT_F32, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         configured[dev] = true;
     }
     dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
-    proj_gemm_kernel<BN, OUT_F32, HEADS, LOOP><<<grid, 192, C::SMEM_BYTES, stream>>>(maps, args);
+    proj_gemm_kernel<BN, OUT_F32, HEADS><<<grid, 192, C::SMEM_BYTES, stream>>>(maps, args);
     EFA_CUDA(cudaGetLastError());
     return 0;
 }
 
-template <bool LOOP>
-int launch_form(const PjMaps<1, LOOP>& maps, const PjArgs& a, bool wide, bool f32, cudaStream_t stream)
+// A block per tile, stored row by row from registers with plain stores, which go wherever the kernel may write. Nothing
+// promises that for bulk tensor stores: outputs in mapped host memory, managed memory or another GPU's memory take this
+// kernel, and launches that are over in one wave (block_per_tile).
+struct PjTileArgs {
+    void* out;          // fp16 or fp32 [M][N]
+    int M, N, K;
+    int* status;
+};
+
+template <int BN, bool OUT_F32>
+__global__ void __launch_bounds__(192)
+proj_tile_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const PjTileArgs a)
 {
-    if (f32) return wide ? launch_proj<256, true, false, LOOP>(maps, a, stream) : launch_proj<128, true, false, LOOP>(maps, a, stream);
-    return wide ? launch_proj<256, false, false, LOOP>(maps, a, stream) : launch_proj<128, false, false, LOOP>(maps, a, stream);
+    using C = PjCfg<BN, false>;
+    constexpr uint32_t IDESC = idesc_f16_f32(PJ_BM, BN, 0, 1);
+    constexpr uint32_t SWZ = swizzle_code(128);
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+
+    __shared__ __align__(8) uint64_t bar_full[C::NSTAGE];
+    __shared__ __align__(8) uint64_t bar_empty[C::NSTAGE];
+    __shared__ __align__(8) uint64_t bar_acc;
+    __shared__ uint32_t tmem_base_smem;
+    __shared__ int abort_word;
+
+    const int tid  = threadIdx.x;
+    const int warp = tid >> 5;
+    const int lane = tid & 31;
+    const int n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * PJ_BM;
+    const int num_k = (a.K + PJ_BK - 1) / PJ_BK;
+
+    if (tid == 0) {
+        abort_word = 0;
+        for (int s = 0; s < C::NSTAGE; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        mbar_init(&bar_acc, 1);
+        mbar_fence_init();
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmW);
+    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc(&tmem_base_smem, BN);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_acc = tmem_base_smem;
+
+    if (warp == 0) {
+        // ---- TMA producer
+        if (lane == 0) {
+            for (int kb = 0; kb < num_k; kb++) {
+                const int s = kb % C::NSTAGE;
+                const int use = kb / C::NSTAGE;
+                if (use > 0 && !mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), &abort_word, 11)) break;
+                uint8_t* sa = smem + s * C::STAGE;
+                uint8_t* sb = sa + C::A_BYTES;
+                mbar_expect_tx(&bar_full[s], C::STAGE);
+                tma_load_2d(sa, &tmA, &bar_full[s], kb * PJ_BK, m0);
+                #pragma unroll
+                for (int nb = 0; nb < BN / 64; nb++)
+                    tma_load_2d(sb + nb * C::B_BOX, &tmW, &bar_full[s], n0 + nb * 64, kb * PJ_BK);
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer
+        if (lane == 0) {
+            bool ok = true;
+            for (int kb = 0; kb < num_k && ok; kb++) {
+                const int s = kb % C::NSTAGE;
+                ok = mbar_wait(&bar_full[s], (uint32_t)((kb / C::NSTAGE) & 1), &abort_word, 12);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t sa = smem_u32(smem + s * C::STAGE);
+                const uint32_t sb = sa + C::A_BYTES;
+                #pragma unroll
+                for (int ks = 0; ks < PJ_BK / 16; ks++) {
+                    tc_mma_ss(tmem_acc,
+                              smem_desc(sa + ks * 32, 16, 1024, SWZ),                    // K-major: 32 B per 16 k
+                              smem_desc(sb + ks * 16 * 128, C::B_BOX, 1024, SWZ),        // MN-major: 16 k rows of 128 B
+                              IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+                }
+                tc_commit(&bar_empty[s]);
+            }
+            if (ok) tc_commit(&bar_acc);
+        }
+    } else {
+        // ---- epilogue: warps 2..5 own TMEM lanes 32*(warp % 4) .. +31
+        const int lane_grp = warp & 3;
+        const int row = m0 + lane_grp * 32 + lane;
+        if (mbar_wait(&bar_acc, 0, &abort_word, 13)) {
+            tc_fence_after_sync();
+            const uint32_t taddr = tmem_acc + ((uint32_t)(lane_grp * 32) << 16);
+            #pragma unroll 1
+            for (int c = 0; c < BN / 32; c++) {
+                uint32_t r[32];
+                tmem_ld32(taddr + c * 32, r);
+                tmem_wait_ld();
+                const int col = n0 + c * 32;
+                if (OUT_F32) {
+                    if (row < a.M && col < a.N) {
+                        uint4* dst = reinterpret_cast<uint4*>(static_cast<float*>(a.out) + (size_t)row * a.N + col);
+                        #pragma unroll
+                        for (int q = 0; q < 8; q++) dst[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    }
+                } else if (row < a.M && col < a.N) {   // N is a multiple of 64, so a 32-column chunk is all in or all out
+                    uint4* dst = reinterpret_cast<uint4*>(static_cast<__half*>(a.out) + (size_t)row * a.N + col);
+                    #pragma unroll
+                    for (int q = 0; q < 4; q++) dst[q] = pack8(&r[8 * q]);
+                }
+            }
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (abort_word != 0) {
+        for (int i = 0; i < 64; i++) __nanosleep(100000);
+        if (tid == 0 && a.status != nullptr) {
+            if (atomicCAS(a.status, 0, (int)KS_WAIT_TIMEOUT) == 0) {
+                a.status[1] = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+                a.status[2] = abort_word;
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 1) tmem_dealloc(tmem_acc, BN);
+}
+
+template <int BN, bool OUT_F32>
+int launch_tile(const CUtensorMap& ta, const CUtensorMap& tw, const PjTileArgs& args, cudaStream_t stream)
+{
+    using C = PjCfg<BN, false>;
+    static bool configured[64] = {};
+    int dev = 0;
+    EFA_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        EFA_CUDA(cudaFuncSetAttribute(proj_tile_kernel<BN, OUT_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        configured[dev] = true;
+    }
+    dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
+    proj_tile_kernel<BN, OUT_F32><<<grid, 192, C::SMEM_BYTES, stream>>>(ta, tw, args);
+    EFA_CUDA(cudaGetLastError());
+    return 0;
 }
 
 // Tile width: the one that leaves the busiest SM less to fetch. What bounds the kernel is the rate at which tiles come
@@ -344,6 +448,19 @@ bool wide_tiles(int rows, int cols)
     const long row_tiles = (rows + PJ_BM - 1) / PJ_BM;
     auto waves = [&](int bn) { return (row_tiles * ((cols + bn - 1) / bn) + 147) / 148; };
     return waves(256) * 3 <= waves(128) * 2;
+}
+
+// A block per tile where one wave of narrow tiles is the whole launch, so that there is nothing to take over, and
+// - there are 64 rows: half of every tile's staged stores would be of nothing (64 x 1024 x 1024: 8.7 against 9.5 us), or
+// - d is a power of two and d_local at least 512: the 64 rows of a W box then lie a power of two apart and come in slowly,
+//   the k loop is the time, and it runs 3 to 6 % faster in the smaller kernel (256 x 4096 x 1024: 24.5 against 25.9 us;
+//   4416 x 1536 x 512: 13.2 against 13.9).
+// Otherwise the coalesced stores of the other kernel are worth more (2496 x 512 x 576: 7.7 against 8.8 us; 256 x 704 x 2304:
+// 8.4 against 9.1), and in more than one wave always. Durations of single launches.
+bool block_per_tile(int rows, int d_local, int d)
+{
+    const long tiles = (long)((rows + PJ_BM - 1) / PJ_BM) * ((d + 127) / 128);
+    return tiles <= 148 && !wide_tiles(rows, d) && (rows <= 64 || (d_local >= 512 && (d & (d - 1)) == 0));
 }
 
 int check_shape(int rows, int d_local, int d)
@@ -370,7 +487,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     if (int rc = check_shape(rows, d_local, d)) return rc;
     if (!A || !W || !out) { set_error("project: null pointer"); return 2; }
 
-    PjMaps<1, true> maps;
+    PjMaps<1> maps;
     if (input_map(&maps.A, A, rows, d_local)) return 1;
     {
         unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)d_local};
@@ -379,16 +496,19 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
         if (make_tmap_f16(&maps.W[0], W, 2, dims, strides, box)) return 1;
     }
     const bool f32 = out_dtype == EFA_F32, wide = wide_tiles(rows, d);
-    PjArgs a{rows, d, d_local, 1, d, out, kernel_status_word()};
-    if (!own_out && !own_device_memory(out)) {
+    if (block_per_tile(rows, d_local, d) || (!own_out && !own_device_memory(out))) {
         if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
-        return launch_form<false>({maps.A, {maps.W[0]}}, a, wide, f32, stream);
+        const PjTileArgs a{out, rows, d, d_local, kernel_status_word()};
+        if (f32) return launch_tile<128, true>(maps.A, maps.W[0], a, stream);
+        return wide ? launch_tile<256, false>(maps.A, maps.W[0], a, stream) : launch_tile<128, false>(maps.A, maps.W[0], a, stream);
     }
     unsigned long long dims[2] = {(unsigned long long)d, (unsigned long long)rows};
     unsigned long long strides[1] = {(unsigned long long)d * (f32 ? 4ull : 2ull)};
     unsigned box[2] = {f32 ? 32u : 64u, 32u};
     if (f32 ? make_tmap_f32(&maps.out[0], out, 2, dims, strides, box) : make_tmap_f16(&maps.out[0], out, 2, dims, strides, box)) return 1;
-    return launch_form<true>(maps, a, wide, f32, stream);
+    const PjArgs a{rows, d, d_local, 1, d, kernel_status_word()};
+    if (f32) return wide ? launch_proj<256, true, false>(maps, a, stream) : launch_proj<128, true, false>(maps, a, stream);
+    return wide ? launch_proj<256, false, false>(maps, a, stream) : launch_proj<128, false, false>(maps, a, stream);
 }
 
 int project_heads_f16(const void* X, const void* const W[3], void* const out[3], int rows, int d, int heads, int d_h,
@@ -405,7 +525,7 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
                     return rc;
         return 0;
     }
-    PjMaps<3, true> maps;
+    PjMaps<3> maps;
     if (input_map(&maps.A, X, rows, d)) return 1;
     for (int t = 0; t < 3; t++) {
         // three dimensions, so that rows past d read as zero and not as the next head's
@@ -419,8 +539,8 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
         if (make_tmap_f16(&maps.out[t], out[t], 3, odims, ostrides, obox)) return 1;
     }
     const int cols = 3 * heads * d_h;
-    PjArgs a{rows, cols, d, heads, d_h, nullptr, kernel_status_word()};
-    return wide_tiles(rows, cols) ? launch_proj<256, false, true, true>(maps, a, stream) : launch_proj<128, false, true, true>(maps, a, stream);
+    PjArgs a{rows, cols, d, heads, d_h, kernel_status_word()};
+    return wide_tiles(rows, cols) ? launch_proj<256, false, true>(maps, a, stream) : launch_proj<128, false, true>(maps, a, stream);
 }
 
 
@@ -435,11 +555,11 @@ template <class K> int touch_kernel(K kernel)
 
 int proj_preload()
 {
-    return touch_kernel(proj_gemm_kernel<128, false, false, true>) || touch_kernel(proj_gemm_kernel<128, true, false, true>) ||
-           touch_kernel(proj_gemm_kernel<256, false, false, true>) || touch_kernel(proj_gemm_kernel<256, true, false, true>) ||
-           touch_kernel(proj_gemm_kernel<128, false, false, false>) || touch_kernel(proj_gemm_kernel<128, true, false, false>) ||
-           touch_kernel(proj_gemm_kernel<256, false, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false, false>) ||
-           touch_kernel(proj_gemm_kernel<128, false, true, true>) || touch_kernel(proj_gemm_kernel<256, false, true, true>);
+    return touch_kernel(proj_gemm_kernel<128, false, false>) || touch_kernel(proj_gemm_kernel<128, true, false>) ||
+           touch_kernel(proj_gemm_kernel<256, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false>) ||
+           touch_kernel(proj_gemm_kernel<128, false, true>) || touch_kernel(proj_gemm_kernel<256, false, true>) ||
+           touch_kernel(proj_tile_kernel<128, false>) || touch_kernel(proj_tile_kernel<128, true>) ||
+           touch_kernel(proj_tile_kernel<256, false>);
 }
 
 }  // namespace efa

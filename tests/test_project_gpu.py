@@ -9,6 +9,9 @@ pytestmark = pytest.mark.gpu
                                              (256, 1024, 1024), (192, 32, 256), (2048, 512, 512), (4096, 256, 4096),
                                              (128, 4096, 4096), (19072, 128, 1024),
                                              # several tiles per SM, with ragged last rows and columns, one k-block and many
+                                             # a block per tile (up to 148 narrow tiles: 64 rows, or d a power of two and
+                                             # d_local from 512 on) and just not
+                                             (64, 48, 448), (192, 512, 256), (192, 496, 256), (192, 512, 320), (4736, 528, 512), (4800, 528, 512),
                                              (19136, 48, 320), (9536, 16, 704), (4160, 512, 4096), (64, 80, 448)])
 def test_projection_matches_float64(pkg, torch_cuda, rows, d_local, d):
     torch = torch_cuda

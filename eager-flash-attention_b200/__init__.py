@@ -104,7 +104,7 @@ _SIGNATURES = {
     "efa_flash_attn_tc_combine": (C.c_int, [C.POINTER(FlashPartials), C.c_void_p, C.c_int, C.c_int, C.c_int,
                                             C.POINTER(FlashParams), C.c_void_p]),
     "efa_flash_attn_tc_check_params": (C.c_char_p, [C.POINTER(FlashParams), C.c_int]),
-    "efa_flash_attn_tc_plan": (C.c_int, [C.POINTER(FlashParams), C.c_int, C.POINTER(FlashPlan)]),
+    "efa_flash_attn_tc_plan": (C.c_int, [C.POINTER(FlashParams), C.c_int, C.c_int, C.POINTER(FlashPlan)]),
     "efa_convert_f32_to_f16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "efa_project_f16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "efa_compute_qkv_f16": (C.c_int, [C.c_void_p] * 7 + [C.c_int] * 4 + [C.c_void_p]),
@@ -205,10 +205,10 @@ def flash_attn_tc_check_params(fp: FlashParams, q_rows: int) -> Optional[str]:
     return None if why is None else why.decode()
 
 
-def flash_attn_tc_plan(fp: FlashParams, q_rows: int) -> FlashPlan:
-    """The work items that flash_attn_tc_forward cuts a launch of ``q_rows`` rows into. Host arithmetic."""
+def flash_attn_tc_plan(fp: FlashParams, q_start: int, q_rows: int) -> FlashPlan:
+    """The work items that flash_attn_tc_forward cuts rows [q_start, q_start + q_rows) into. Host arithmetic."""
     plan = FlashPlan()
-    _check(lib().efa_flash_attn_tc_plan(C.byref(fp), q_rows, C.byref(plan)), "flash_attn_tc_plan")
+    _check(lib().efa_flash_attn_tc_plan(C.byref(fp), q_start, q_rows, C.byref(plan)), "flash_attn_tc_plan")
     return plan
 
 

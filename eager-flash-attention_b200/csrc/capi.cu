@@ -54,11 +54,12 @@ extern "C" const char* efa_flash_attn_tc_check_params(const efa_flash_params* p,
     return fa_check_params(*p, q_rows);
 }
 
-extern "C" int efa_flash_attn_tc_plan(const efa_flash_params* p, int q_rows, efa_flash_plan* out)
+extern "C" int efa_flash_attn_tc_plan(const efa_flash_params* p, int q_start, int q_rows, efa_flash_plan* out)
 {
     if (!p || !out) { set_error("efa_flash_attn_tc_plan: null argument"); return 2; }
     if (const char* why = fa_check_params(*p, q_rows)) { set_error("efa_flash_attn_tc_plan: %s", why); return 2; }
-    fa_plan(*p, q_rows, out);
+    if (q_start < 0 || q_start + q_rows > p->S) { set_error("efa_flash_attn_tc_plan: rows outside [0, %d)", p->S); return 2; }
+    fa_plan(*p, q_start, q_rows, out);
     return 0;
 }
 

@@ -124,9 +124,10 @@ const char* fa_check_params(const efa_flash_params& p, int q_rows)
     return nullptr;
 }
 
-void fa_plan(const efa_flash_params& p, int q_rows, efa_flash_plan* out)
+void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan* out)
 {
     FaArgs a{};
+    a.q_start = q_start; a.S = p.S;
     a.H_local = p.H_local; a.nsplit = p.split; a.q_rows = q_rows; a.kv_len = p.S / p.split; a.causal = p.causal;
     const FaPlan plan = fa_ws_plan(a, p.d_h, 0);
     *out = efa_flash_plan{plan.items256, plan.items128, plan.k_slots, plan.v_slots, plan.stage_step};

@@ -19,8 +19,8 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
                                        // the first; -1 = last first exactly when there are no counters and the mask is causal
                const short* order_tab = nullptr);  // band_rows == 0: the order of the 256-row blocks (device memory)
 
-// How fa_forward of p over q_rows rows is cut into work items (fa_ws_plan); the caller has checked p.
-void fa_plan(const efa_flash_params& p, int q_rows, efa_flash_plan* out);
+// How fa_forward of p over rows q_start .. q_start+q_rows is cut into work items (fa_ws_plan); the caller has checked p.
+void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan* out);
 
 // Split-KV attention + merge with the partials in a fixed device array (no allocation anywhere).
 int fa_forward_noalloc(const void* Q, const void* K, const void* V, void* O, int o_dtype,

@@ -746,17 +746,22 @@ void ring_of(FaPlan& plan)
 // Which items a launch goes as. Host arithmetic only.
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
 {
-    // 128-row items with their keys split over the two warpgroups where the launch is short of items: an item takes
-    // half as long as a 256-row one, so waves * 1 against waves * 2. A row block that has a K/V stage to itself
-    // reads it twice as often from L2, so near-ties stay with 256 rows.
+    // 128-row items with their keys split over the two warpgroups where one wave of them is the whole launch (d_h 16 /
+    // 64 / 128, 74 items of 256 rows and 32 key stages: 33 / 35 / 49 us against 61 / 57 / 64). Three waves of them against
+    // two of 256 rows are worth it only where items are long and the tensor pipe is not what an item waits for. In us:
+    // 53 against 63 (d_h 16, 16 stages), 57 against 62 (64, 16 stages), even at 8 stages (64), 27 against 25 (64, 4 stages),
+    // 19 against 17 (16, 2 stages), 80 against 75 (128, 16 stages).
     const long heads = (long)a.H_local * a.nsplit;
     const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
     const long waves256 = (total + 147) / 148, waves128 = (total128 + 147) / 148, rest = total % 148;
+    const double keys = a.causal ? a.q_start + 0.5 * (a.q_rows + 256) : a.S;
+    const double stages = keys / ((double)WS_BN * a.nsplit);                   // of an average item
+    const bool long_items = d_h < 128 && stages >= 8;
     const bool free_form = a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64);
     FaPlan plan;
     plan.items256 = (int)total;
     plan.items128 = 0;
-    if (free_form && waves128 * 4 <= waves256 * 2 * 3) {
+    if (free_form && (waves128 <= 1 || (long_items && waves128 * 4 <= waves256 * 2 * 3))) {
         plan.items256 = 0;
         plan.items128 = (int)total128;
     // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest

@@ -77,7 +77,7 @@ class Weights(C.Structure):
 
 class FlashPlan(C.Structure):
     """efa_flash_plan: the work items of an attention launch, and the K/V stages they keep in shared memory."""
-    _fields_ = [("items_256", C.c_int), ("items_128", C.c_int), ("k_slots", C.c_int), ("v_slots", C.c_int),
+    _fields_ = [("items_256", C.c_int), ("items_128", C.c_int), ("tiles", C.c_int), ("k_slots", C.c_int), ("v_slots", C.c_int),
                 ("stage_step", C.c_int)]
 
 

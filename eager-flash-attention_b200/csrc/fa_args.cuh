@@ -41,11 +41,17 @@ __device__ __forceinline__ float ex2(float x)
 int fa_ws_kv_box_rows();
 int fa_ws_preload();    // loads the code of every instantiation of the kernel on the current device
 // How a launch is cut into work items: items256 of 256 rows, then items128 of 128 rows (a launch of their own where
-// there are both); and the stages of K and V that the last of them keeps, of which an issuing thread takes every
-// stage_step-th.
-struct FaPlan { int items256, items128, k_slots, v_slots, stage_step; };
+// there are both), or tiles blocks of the one-tile kernel; and the stages of K and V that the last of them keeps, of which
+// an issuing thread takes every stage_step-th.
+struct FaPlan { int items256, items128, tiles, k_slots, v_slots, stage_step; };
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms);
 int fa_forward_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a,
                   int d_h, bool out_f16, int reserve_sms, cudaStream_t stream);
+
+
+// One-tile kernel (fa_fwd_tile_sm100.cu), d_h 16 and 32; the same maps.
+int fa_tile_preload();
+int fa_forward_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a,
+                    int d_h, bool out_f16, cudaStream_t stream);
 
 }  // namespace efa

@@ -1,6 +1,6 @@
 // The attention launch interface (flash_attn_tc_forward of eager-flash-attention, flash_attn_tc.cu:363-399): argument
-// checks, tensor maps, the merge of split-KV partials and the entry that allocates nothing. The kernel is in
-// fa_fwd_ws_sm100.cu.
+// checks, tensor maps, the merge of split-KV partials and the entry that allocates nothing. The kernels are in
+// fa_fwd_ws_sm100.cu (which also says which launch takes which) and fa_fwd_tile_sm100.cu.
 #include "fa_fwd_sm100.cuh"
 #include "fa_args.cuh"
 #include "host_util.h"
@@ -130,7 +130,7 @@ void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan*
     a.q_start = q_start; a.S = p.S;
     a.H_local = p.H_local; a.nsplit = p.split; a.q_rows = q_rows; a.kv_len = p.S / p.split; a.causal = p.causal;
     const FaPlan plan = fa_ws_plan(a, p.d_h, 0);
-    *out = efa_flash_plan{plan.items256, plan.items128, plan.k_slots, plan.v_slots, plan.stage_step};
+    *out = efa_flash_plan{plan.items256, plan.items128, plan.tiles, plan.k_slots, plan.v_slots, plan.stage_step};
 }
 
 int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype,
@@ -353,7 +353,7 @@ template <class K> int touch_kernel(K kernel)
 int fa_preload()
 {
     return touch_kernel(combine_splits_kernel<true>) || touch_kernel(combine_splits_kernel<false>) ||
-           touch_kernel(f32_to_f16_kernel) || fa_ws_preload();
+           touch_kernel(f32_to_f16_kernel) || fa_ws_preload() || fa_tile_preload();
 }
 
 }  // namespace efa

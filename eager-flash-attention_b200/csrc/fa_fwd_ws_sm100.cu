@@ -3,8 +3,9 @@
 // interface: same tensor layouts, split-KV partial format (row max in the log2 domain) and completion counters.
 //
 // Described for two tiles of d_h = 64 or 128. Small heads (AHEAD) and few rows (KSPLIT) use it with the differences
-// stated at those two constants; they had a kernel of one tile per block before: 4032 rows of eight heads of 32,
-// 71.5 -> 63 us; 128 rows against 16384 keys in eight splits (16 heads of 64), 55 -> 41.5 us.
+// stated at those two constants. Against a kernel of one tile per block (fa_fwd_tile_sm100.cu, which keeps the small heads'
+// launches of few keys): 4032 rows of eight heads of 32, 71.5 -> 58.6 us; 128 rows against 16384 keys in eight splits (16
+// heads of 64), 55 -> 41.5 us.
 //
 // One CTA = 256 query rows (two 128-row Q tiles) of one (head, split), 384 threads:
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
@@ -720,6 +721,7 @@ int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     if constexpr (D >= 64)
         if (reserve_sms > 0) return out_f16 ? launch_ws<D, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<D, false, true>(tq, tk, tv, a, reserve_sms, stream);
     const FaPlan plan = fa_ws_plan(a, D, reserve_sms);
+    if (plan.tiles > 0) return fa_forward_tile(tq, tk, tv, a, D, out_f16, stream);
     if (plan.items256 == 0)
         return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false, true>(tq, tk, tv, a, 0, stream);
     if (plan.items128 > 0) {
@@ -760,7 +762,15 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     const bool free_form = a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64);
     FaPlan plan;
     plan.items256 = (int)total;
-    plan.items128 = 0;
+    plan.items128 = plan.tiles = 0;
+    if (d_h < 64 && free_form && total128 > 148 && stages <= 6) {
+        // few keys and more than one wave of anything: two small blocks to an SM (the figures are in fa_fwd_tile_sm100.cu)
+        plan.items256 = 0;
+        plan.tiles = (int)total128;
+        plan.k_slots = plan.v_slots = 2;
+        plan.stage_step = 1;
+        return plan;
+    }
     if (free_form && (waves128 <= 1 || (long_items && waves128 * 4 <= waves256 * 2 * 3))) {
         plan.items256 = 0;
         plan.items128 = (int)total128;

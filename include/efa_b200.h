@@ -109,9 +109,9 @@ const char* efa_flash_attn_tc_check_params(const efa_flash_params* p, int q_rows
 
 /* How efa_flash_attn_tc_forward cuts rows q_start .. q_start+q_rows into work items: items_256 items of 256 query rows of one
  * head and split, then items_128 items of 128 rows whose keys two warpgroups share (in a launch of their own where
- * there are both). k_slots and v_slots: the 128-key stages of K and V that the last of them keeps in shared memory, of which
+ * there are both); or tiles blocks of 128 rows of the kernel for small heads and few keys. k_slots and v_slots: the 128-key stages of K and V that the last of them keeps in shared memory, of which
  * one issuing thread takes every stage_step-th. Host arithmetic only; no counterpart in the reference. */
-typedef struct efa_flash_plan { int items_256, items_128, k_slots, v_slots, stage_step; } efa_flash_plan;
+typedef struct efa_flash_plan { int items_256, items_128, tiles, k_slots, v_slots, stage_step; } efa_flash_plan;
 int efa_flash_attn_tc_plan(const efa_flash_params* p, int q_start, int q_rows, efa_flash_plan* out);
 
 /* convert_f32_to_f16 (flash_attn_tc.cuh:62, flash_attn_tc.cu:411-424), round to nearest even. */

@@ -162,7 +162,7 @@ def test_stream_plan_mixed_order(pkg):
 def test_every_issuing_thread_waits_for_all_phases_of_its_kv_slots(pkg, d_h, H):
     """A wait by parity holds only for a thread that waits for each phase of the slot: the parity it wants also reads
     as complete while the slot is one phase behind, so a phase left to another thread would let it pass early."""
-    plan = pkg.flash_attn_tc_plan(pkg.make_params(8192, H * d_h, H, 64, causal=1).flash_tc, 0, 256)
+    plan = pkg.flash_attn_tc_plan(pkg.make_params(8192, H * d_h, H, 64, causal=1).flash_tc, 7936, 256)
     assert (plan.items_256, plan.items_128) == ((0, 4) if H == 2 else (300, 0))
     assert plan.stage_step == (2 if H == 2 else 1)
     for slots in (plan.k_slots, plan.v_slots):
@@ -177,7 +177,7 @@ def test_every_issuing_thread_waits_for_all_phases_of_its_kv_slots(pkg, d_h, H):
     (16, 74, 512, 256, 1, 0, (0, 148)), (128, 37, 4096, 512, 1, 1, (0, 148)), (64, 18, 4096, 192, 4, 0, (0, 144)), (64, 20, 4096, 192, 4, 0, (80, 0)),
     (64, 75, 512, 256, 1, 0, (75, 0)), (128, 148, 4096, 256, 1, 0, (148, 0)),
     # three waves against two: long items of small heads only
-    (16, 75, 1024, 512, 1, 0, (0, 300)), (16, 75, 512, 512, 1, 0, (150, 0)), (16, 111, 1024, 512, 1, 1, (222, 0)),
+    (16, 75, 1024, 512, 1, 0, (0, 300)), (16, 111, 1024, 512, 1, 1, (222, 0)), (32, 111, 896, 512, 1, 0, (222, 0)),
     (32, 111, 2048, 512, 1, 1, (0, 444)), (64, 111, 1024, 512, 1, 1, (222, 0)), (64, 111, 1024, 512, 1, 0, (0, 444)),
     (128, 75, 2048, 512, 1, 0, (150, 0)), (128, 111, 2048, 512, 1, 1, (222, 0)),
     # a last wave that is at most half full, from 4096 keys on and without a mask
@@ -186,7 +186,16 @@ def test_every_issuing_thread_waits_for_all_phases_of_its_kv_slots(pkg, d_h, H):
 def test_work_items_of_an_attention_launch(pkg, d_h, H, S, q_rows, split, causal, want):
     p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
     plan = pkg.flash_attn_tc_plan(p.flash_tc, S - q_rows, q_rows)
-    assert (plan.items_256, plan.items_128) == want
+    assert (plan.items_256, plan.items_128) == want and plan.tiles == 0
+
+
+@pytest.mark.parametrize("d_h,H,S,q_rows,split,causal,want", [
+    (16, 100, 256, 256, 1, 0, 200), (32, 75, 768, 512, 1, 0, 300), (32, 8, 4096, 4096, 8, 0, 2048), (16, 111, 1024, 512, 1, 1, 0),
+    (16, 74, 256, 256, 1, 0, 0), (32, 75, 896, 512, 1, 0, 0), (64, 100, 256, 256, 1, 0, 0), (16, 8, 4096, 4096, 4, 0, 0)])
+def test_small_heads_with_few_keys_go_as_single_tiles(pkg, d_h, H, S, q_rows, split, causal, want):
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
+    plan = pkg.flash_attn_tc_plan(p.flash_tc, S - q_rows, q_rows)
+    assert plan.tiles == want and (plan.items_256 + plan.items_128 == 0) == (want > 0)
 
 
 def test_stream_plan_counts_without_a_buffer_and_rejects_a_short_one(pkg):

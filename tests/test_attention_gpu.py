@@ -158,6 +158,42 @@ def test_full_size_rank_shards_on_sampled_rows(pkg, oracle, torch_cuda, S, H_loc
     assert float((O1 - 1.0).abs().max()) < 2e-3
 
 
+def check_against_float64(pkg, torch, H, d_h, S, q_start, q_rows, split, causal):
+    """One launch with counters of 64 rows against float64, on rows whose maximum keeps growing along the keys, so that
+    the exponent offset moves after the first stages too."""
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
+    g = torch.Generator(device="cuda").manual_seed(S + d_h + H)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev[1] *= torch.linspace(0.5, 6.0, S, device="cuda", dtype=torch.float16)[None, :, None]
+    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
+    assert torch.isfinite(O).all()
+    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
+    rows = torch.arange(q_start, q_start + q_rows, device="cuda")[:, None]
+    for h in range(H):
+        q, k, v = (t[h].double() for t in dev)
+        s = q[q_start:q_start + q_rows] @ k.T * p.flash_tc.scale
+        if causal:
+            s = s.masked_fill(torch.arange(S, device="cuda")[None, :] > rows, float("-inf"))
+        w = torch.softmax(s, dim=-1)
+        ref = w @ v
+        # Every softmax weight is rounded to fp16 (2^-11 of it) or, below 2^-14 of the largest, to a multiple of 2^-25; the
+        # offset may lag the maximum by 2^8. fp32 scores of up to about 100 carry 1e-5 of relative error into the weights.
+        bound = (w * 2 ** -11 + 2.0 ** -24) @ v.abs() + 1e-4 * ref.abs().max()
+        err = (O[:, h * d_h:(h + 1) * d_h].double() - ref).abs()
+        assert bool((err <= bound).all()), (h, float((err - bound).max()))
+
+
+# One to six key stages, ragged last blocks, rows that see no key of a split, both directions of the mask.
+@pytest.mark.parametrize("d_h", [16, 32])
+@pytest.mark.parametrize("H,S,q_start,q_rows,split,causal", [
+    (160, 64, 0, 64, 1, 0), (100, 256, 0, 256, 1, 1), (152, 192, 64, 128, 1, 1), (60, 640, 320, 320, 1, 0), (40, 768, 0, 768, 1, 0),
+    (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (16, 1536, 192, 576, 2, 0)])
+def test_single_tiles_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal):
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
+    assert pkg.flash_attn_tc_plan(p.flash_tc, q_start, q_rows).tiles > 0
+    check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
+
+
 # Key stages per 128-row block at which the two softmax warpgroups get none, one, an odd and an even number; few heads
 # take the form that splits the keys between them, many the form with 256 rows per block (H * split in (74, 148]).
 @pytest.mark.parametrize("H", [3, 40])

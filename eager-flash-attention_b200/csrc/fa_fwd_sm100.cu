@@ -136,7 +136,7 @@ void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan*
 int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype,
                const efa_flash_partials* part, int q_start, int q_rows,
                const efa_flash_params& p, cudaStream_t stream, int* tile_counters, int tile_rows, int reserve_sms,
-               int band_rows, int heavy_first, const short* order_tab)
+               int band_rows, int heavy_first, const short* order_tab, int* launches)
 {
     if (const char* why = fa_check_params(p, q_rows)) { set_error("flash_attn_tc_forward: %s", why); return 2; }
     if (q_start < 0 || q_start % 64 != 0 || q_start + q_rows > p.S) {
@@ -189,6 +189,10 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
     a.order_tab = order_tab;
     a.heavy_first = heavy_first >= 0 ? (heavy_first ? 1 : 0) : ((tile_counters == nullptr && p.causal) ? 1 : 0);
 
+    if (launches) {
+        const FaPlan plan = fa_ws_plan(a, p.d_h, reserve_sms);
+        *launches += plan.items256 > 0 && plan.items128 > 0 ? 2 : 1;
+    }
     const bool f16 = (o_dtype == EFA_F16);
     return fa_forward_ws(tq, tk, tv, a, p.d_h, f16, reserve_sms, stream);
 }

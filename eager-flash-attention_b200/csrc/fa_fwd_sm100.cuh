@@ -17,7 +17,8 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
                                        // order is free and whole heads are processed one after another.
                int heavy_first = -1,  // 1 = take the row blocks (or bands) from the last to the first, 0 = from
                                        // the first; -1 = last first exactly when there are no counters and the mask is causal
-               const short* order_tab = nullptr);  // band_rows == 0: the order of the 256-row blocks (device memory)
+               const short* order_tab = nullptr,  // band_rows == 0: the order of the 256-row blocks (device memory)
+               int* launches = nullptr);          // counts the kernels launched
 
 // How fa_forward of p over rows q_start .. q_start+q_rows is cut into work items (fa_ws_plan); the caller has checked p.
 void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan* out);

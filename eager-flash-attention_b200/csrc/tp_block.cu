@@ -142,9 +142,8 @@ struct Run {
             q.m_part += (size_t)ws_row0 * p.H_local;
             q.l_part += (size_t)ws_row0 * p.H_local;
         }
-        launches++;
         return fa_forward(w.Qh, w.Kh, w.Vh, O, EFA_F16, &q, q_start, q_rows, p.flash_tc, s, counters, tile_rows, reserve_sms,
-                          band_rows, heavy_first, order_tab);
+                          band_rows, heavy_first, order_tab, &launches);
     }
     // launch_combine (attn_main.cu:247-252): no-op when split == 1.
     int combine(__half* O, int ws_rows, int row0, int rows, cudaStream_t s)

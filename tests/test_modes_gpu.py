@@ -221,6 +221,22 @@ def test_residual_is_added_to_every_reduced_group(pkg, oracle, torch_cuda, ctx, 
         assert_close(oracle, plain.float().cpu().numpy(), ref, f"{name} without residual")
 
 
+@pytest.mark.parametrize("mode,more", [("attn", 0), ("megatron", 1)])
+@pytest.mark.parametrize("H,d_h,S,want", [(13, 128, 4096, 2), (13, 128, 2048, 1), (3, 64, 4096, 1), (40, 32, 512, 1)])
+def test_every_launch_of_the_attention_is_counted(pkg, torch_cuda, ctx, H, d_h, S, want, mode, more):
+    """A launch whose short last wave goes as one of its own counts as two."""
+    torch = torch_cuda
+    p = pkg.make_params(S, H * d_h, H, 64)
+    dev = [torch.zeros((H, S, d_h), dtype=torch.float16, device="cuda") for _ in range(3)]
+    dev.append(torch.zeros((H * d_h, H * d_h), dtype=torch.float16, device="cuda"))
+    out = torch.zeros((S, H * d_h), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    st = pkg.run_mode(ctx, pkg.parse_mode(mode), pkg.Weights(*(t.data_ptr() for t in dev)), out, p)
+    plan = pkg.flash_attn_tc_plan(p.flash_tc, 0, S)
+    assert (2 if plan.items_256 and plan.items_128 else 1) == want
+    assert st.kernel_launches == want + more
+
+
 def test_residual_is_rejected_where_no_block_output_exists(pkg, oracle, torch_cuda, ctx):
     torch = torch_cuda
     S, d, H, tile = 512, 256, 4, 128

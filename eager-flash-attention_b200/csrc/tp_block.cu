@@ -111,15 +111,20 @@ struct Run {
     // One rank: its partial sum is the result, so the projection writes `output` itself and nothing is reduced. A
     // one-rank AllReduce is a copy (0.5 GB read and written at 32k rows of d = 4096) and, tile by tile, a launch and several
     // microseconds of host time per group. Not for an output that is not this GPU's own memory (the copy then
-    // crosses to it once, behind the projections) or not 16-byte aligned, or where writing early would disturb W_O.
+    // crosses to it once, behind the projections) or not 16-byte aligned, or where writing early would disturb W_O or rows
+    // of the residual that are added later.
     bool direct = false;
     void choose_direct(const void* output)
     {
         if (p.R != 1 || p.skip_comm || p.skip_proj || p.reduce == EFA_REDUCE_P2P || ((uintptr_t)output & 15) != 0) return;
         if (!own_device_memory(output)) return;
         const char* o = static_cast<const char*>(output);
-        const char* wo = static_cast<const char*>(static_cast<const void*>(w.W_O));
-        if (o < wo + (size_t)p.d_local * p.d * sizeof(__half) && wo < o + (size_t)p.S * row_bytes()) return;
+        auto overlaps = [&](const void* x, size_t bytes) {
+            const char* b = static_cast<const char*>(x);
+            return o < b + bytes && b < o + (size_t)p.S * row_bytes();
+        };
+        if (overlaps(w.W_O, (size_t)p.d_local * p.d * sizeof(__half))) return;
+        if (residual && overlaps(residual, (size_t)p.S * p.d * sizeof(__half))) return;
         direct = true;
     }
 

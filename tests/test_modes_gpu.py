@@ -237,6 +237,31 @@ def test_every_launch_of_the_attention_is_counted(pkg, torch_cuda, ctx, H, d_h, 
     assert st.kernel_launches == want + more
 
 
+@pytest.mark.parametrize("mode", ["sync", "overlap", "stream"])
+def test_residual_rows_inside_the_output(pkg, torch_cuda, mode):
+    """With one communication stream the rows are reduced and added to in order, so a residual that lies a group of
+    rows further on in the output buffer is read before the block overwrites it."""
+    torch = torch_cuda
+    S, d, H, tile = 1024, 512, 8, 128
+    p = pkg.make_params(S, d, H, tile)
+    p.row_order = pkg.ROWS_ASCENDING
+    g = torch.Generator(device="cuda").manual_seed(11)
+    dev = [torch.randn(H, S, d // H, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev.append(torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5)
+    w = pkg.Weights(*(t.data_ptr() for t in dev))
+    residual = torch.randn(S, d, generator=g, device="cuda", dtype=torch.float16)
+    buf = torch.zeros(S + tile, d, dtype=torch.float16, device="cuda")
+    buf[tile:] = residual
+    apart = torch.zeros(S, d, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    one = pkg.make_ctx(pkg.World(), ncomm=1)
+    pkg.run_mode_residual(one, pkg.parse_mode(mode), w, residual, apart, p)
+    pkg.run_mode_residual(one, pkg.parse_mode(mode), w, buf[tile:], buf[:S], p)
+    torch.cuda.synchronize()
+    pkg.destroy_ctx(one)
+    assert torch.equal(buf[:S], apart)
+
+
 def test_residual_is_rejected_where_no_block_output_exists(pkg, oracle, torch_cuda, ctx):
     torch = torch_cuda
     S, d, H, tile = 512, 256, 4, 128

@@ -680,24 +680,39 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
+// The first launch of a head size and output type on a device loads and configures every form of it: which one a launch
+// takes depends on its shape, and a later one may be inside a stream capture or find no device memory left.
+template <int D, bool OUT_F16>
+int configure_forms()
+{
+    static bool configured[64] = {};
+    int dev = 0;
+    EFA_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || configured[dev]) return 0;
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, false>, attr, WsCfg<D, false>::SMEM_BYTES));
+    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, true>, attr, WsCfg<D, true>::SMEM_BYTES));
+    if constexpr (D >= 64) {
+        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, true, false>, attr, WsCfg<D, false>::SMEM_BYTES));
+    } else if (fa_tile_preload()) {
+        return 1;
+    }
+    configured[dev] = true;
+    return 0;
+}
+
 template <int D, bool OUT_F16, bool PERSIST, bool KSPLIT = false>
 int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args,
               int reserve_sms, cudaStream_t stream, int blocks = 0 /* of a 1-D grid; 0: all */)
 {
     using C = WsCfg<D, KSPLIT>;
-    static bool configured[64] = {};
-    int dev = 0;
-    EFA_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, PERSIST, KSPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
-        configured[dev] = true;
-    }
     const int items_x = args.H_local * args.nsplit;
     const int item_rows = KSPLIT ? WS_BM : 2 * WS_BM;
     const int items_y = (args.q_rows + item_rows - 1) / item_rows;
     const int total = items_x * items_y;
     if constexpr (PERSIST) {
-        int sms = 148;
+        int dev = 0, sms = 148;
+        EFA_CUDA(cudaGetDevice(&dev));
         EFA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         int ctas = sms - reserve_sms;
         if (ctas < 1) ctas = 1;
@@ -718,6 +733,7 @@ template <int D>
 int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a, bool out_f16,
                 int reserve_sms, cudaStream_t stream)
 {
+    if (out_f16 ? configure_forms<D, true>() : configure_forms<D, false>()) return 1;
     if constexpr (D >= 64)
         if (reserve_sms > 0) return out_f16 ? launch_ws<D, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<D, false, true>(tq, tk, tv, a, reserve_sms, stream);
     const FaPlan plan = fa_ws_plan(a, D, reserve_sms);

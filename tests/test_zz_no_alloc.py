@@ -6,10 +6,13 @@ keeps the split-KV partials in a fixed array inside the library instead of a cal
 This file is collected last on purpose, so that a failure here cannot hide a failure elsewhere.
 Two calls in a row, with different shapes and data, check that what the first call left in the
 shared array does not leak into the second."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
-from conftest import ABS_TOL, REL_TOL
+from conftest import ABS_TOL, REL_TOL, ROOT
 from helpers import assert_close, ref_inputs_f16, to_dev
 
 pytestmark = pytest.mark.gpu
@@ -56,6 +59,50 @@ def test_two_calls_in_a_row_match_the_ordinary_entry_point(pkg, oracle, torch_cu
         assert diff <= ABS_TOL and diff <= REL_TOL * float(np.abs(w).max()), diff
         rows = np.arange(q_start, q_start + q_rows, dtype=np.int32)
         assert_close(oracle, g, oracle.attention_rows(vals[0], vals[1], vals[2], causal, rows))
+
+
+CAPTURE = """
+import sys
+import torch
+sys.path.insert(0, sys.argv[1])
+import __graft_entry__ as entry
+pkg = entry.load_package()
+d_h, S = int(sys.argv[2]), int(sys.argv[3])
+torch.manual_seed(1)
+def case(H, rows):
+    p = pkg.make_params(S, H * d_h, H, 64)
+    qkv = [torch.randn(H, S, d_h, device="cuda", dtype=torch.float16) for _ in range(3)]
+    return p, qkv, torch.zeros(rows, H * d_h, device="cuda", dtype=torch.float16)
+def kinds(p, rows):
+    plan = pkg.flash_attn_tc_plan(p.flash_tc, 0, rows)
+    return [n > 0 for n in (plan.items_256, plan.items_128, plan.tiles)]
+few, many = case(2, 64), case(150, 256)
+assert kinds(few[0], 64) != kinds(many[0], 256)
+def call(c, stream=None):
+    p, qkv, O = c
+    pkg.flash_attn_tc_forward_noalloc(*qkv, O, 0, O.shape[0], p.flash_tc, stream)
+call(few)                                             # the first call on the device
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    call(many, torch.cuda.current_stream())           # another form of the same head size, captured
+graph.replay()
+torch.cuda.synchronize()
+got = many[2].clone()
+many[2].zero_()
+call(many)
+torch.cuda.synchronize()
+assert bool(got.any()) and torch.equal(got, many[2])
+assert pkg.flash_attn_tc_noalloc_status()[0] == 0
+"""
+
+
+@pytest.mark.parametrize("d_h,S", [(16, 256), (32, 512), (64, 512), (128, 512)])
+def test_after_the_first_call_every_form_can_be_captured(torch_cuda, d_h, S):
+    """Few and many rows take different forms of the kernel; the first call of a head size has prepared them all. In a
+    process of its own: nothing may have been loaded before."""
+    run = subprocess.run([sys.executable, "-c", CAPTURE, ROOT, str(d_h), str(S)], capture_output=True, text=True, timeout=180)
+    assert run.returncode == 0, run.stderr[-2000:]
 
 
 def test_shapes_beyond_the_fixed_array_are_rejected(pkg, torch_cuda):

@@ -711,10 +711,7 @@ int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
     const int items_y = (args.q_rows + item_rows - 1) / item_rows;
     const int total = items_x * items_y;
     if constexpr (PERSIST) {
-        int dev = 0, sms = 148;
-        EFA_CUDA(cudaGetDevice(&dev));
-        EFA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        int ctas = sms - reserve_sms;
+        int ctas = device_sms() - reserve_sms;
         if (ctas < 1) ctas = 1;
         if (ctas > total) ctas = total;
         int* counter = work_counter_slot();
@@ -771,7 +768,8 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     // 19 against 17 (16, 2 stages), 80 against 75 (128, 16 stages).
     const long heads = (long)a.H_local * a.nsplit;
     const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
-    const long waves256 = (total + 147) / 148, waves128 = (total128 + 147) / 148, rest = total % 148;
+    const long sms = device_sms();
+    const long waves256 = (total + sms - 1) / sms, waves128 = (total128 + sms - 1) / sms, rest = total % sms;
     const double keys = a.causal ? a.q_start + 0.5 * (a.q_rows + 256) : a.S;
     const double stages = keys / ((double)WS_BN * a.nsplit);                   // of an average item
     const bool long_items = d_h < 128 && stages >= 8;
@@ -779,7 +777,7 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     FaPlan plan;
     plan.items256 = (int)total;
     plan.items128 = plan.tiles = 0;
-    if (d_h < 64 && free_form && total128 > 148 && stages <= 6) {
+    if (d_h < 64 && free_form && total128 > sms && stages <= 6) {
         // few keys and more than one wave of anything: two small blocks to an SM (the figures are in fa_fwd_tile_sm100.cu)
         plan.items256 = 0;
         plan.tiles = (int)total128;
@@ -793,7 +791,7 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
     // is at most half of a wave it goes as 128-row items behind the full waves: 0.6 of a wave instead of one. From 4096 keys
     // on, where that is worth ten times the second launch.
-    } else if (free_form && !a.causal && total > 148 && rest > 0 && rest * 2 <= 148 && a.kv_len >= 4096) {
+    } else if (free_form && !a.causal && total > sms && rest > 0 && rest * 2 <= sms && a.kv_len >= 4096) {
         plan.items256 = (int)(total - rest);
         plan.items128 = (int)rest * 2;
     }

@@ -145,6 +145,20 @@ int* work_counter_slot()
     return ring[dev] + (next[dev]++ % kSlots);
 }
 
+int device_sms()
+{
+    constexpr int kB200 = 148;
+    static int sms[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return kB200; }
+    if (sms[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) { (void)cudaGetLastError(); return kB200; }
+        sms[dev] = n;
+    }
+    return sms[dev];
+}
+
 bool own_device_memory(const void* p)
 {
     int dev = -1;

@@ -59,6 +59,9 @@ int* kernel_status_word();
 // ring handed out round-robin; the caller clears its slot on the launch stream.
 int* work_counter_slot();
 
+// Number of SMs of the current device (148, a B200, where there is none: plans are also made on machines without a GPU).
+int device_sms();
+
 // Whether p is memory of the current device itself: not mapped host memory, managed memory or another GPU's.
 bool own_device_memory(const void* p);
 

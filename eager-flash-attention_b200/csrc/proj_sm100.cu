@@ -446,7 +446,8 @@ int launch_tile(const CUtensorMap& ta, const CUtensorMap& tw, const PjTileArgs& 
 bool wide_tiles(int rows, int cols)
 {
     const long row_tiles = (rows + PJ_BM - 1) / PJ_BM;
-    auto waves = [&](int bn) { return (row_tiles * ((cols + bn - 1) / bn) + 147) / 148; };
+    const long sms = device_sms();
+    auto waves = [&](int bn) { return (row_tiles * ((cols + bn - 1) / bn) + sms - 1) / sms; };
     return waves(256) * 3 <= waves(128) * 2;
 }
 
@@ -460,7 +461,7 @@ bool wide_tiles(int rows, int cols)
 bool block_per_tile(int rows, int d_local, int d)
 {
     const long tiles = (long)((rows + PJ_BM - 1) / PJ_BM) * ((d + 127) / 128);
-    return tiles <= 148 && !wide_tiles(rows, d) && (rows <= 64 || (d_local >= 512 && (d & (d - 1)) == 0));
+    return tiles <= device_sms() && !wide_tiles(rows, d) && (rows <= 64 || (d_local >= 512 && (d & (d - 1)) == 0));
 }
 
 int check_shape(int rows, int d_local, int d)

@@ -158,16 +158,18 @@ def test_full_size_rank_shards_on_sampled_rows(pkg, oracle, torch_cuda, S, H_loc
     assert float((O1 - 1.0).abs().max()) < 2e-3
 
 
-def check_against_float64(pkg, torch, H, d_h, S, q_start, q_rows, split, causal):
-    """One launch with counters of 64 rows against float64, on rows whose maximum keeps growing along the keys, so that
-    the exponent offset moves after the first stages too."""
+def check_against_float64(pkg, torch, H, d_h, S, q_start, q_rows, split, causal, growing=True, tile_rows=64):
+    """One launch against float64; growing: on rows whose maximum keeps growing along the keys, so that the exponent
+    offset moves after the first stages too."""
     p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
     g = torch.Generator(device="cuda").manual_seed(S + d_h + H)
     dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
-    dev[1] *= torch.linspace(0.5, 6.0, S, device="cuda", dtype=torch.float16)[None, :, None]
-    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
+    if growing:
+        dev[1] *= torch.linspace(0.5, 6.0, S, device="cuda", dtype=torch.float16)[None, :, None]
+    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=tile_rows)
     assert torch.isfinite(O).all()
-    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
+    if tile_rows:
+        assert counters.cpu().tolist() == [H * split * tile_rows // 64] * (q_rows // tile_rows)
     rows = torch.arange(q_start, q_start + q_rows, device="cuda")[:, None]
     for h in range(H):
         q, k, v = (t[h].double() for t in dev)
@@ -183,65 +185,57 @@ def check_against_float64(pkg, torch, H, d_h, S, q_start, q_rows, split, causal)
         assert bool((err <= bound).all()), (h, float((err - bound).max()))
 
 
+def form(pkg, H, d_h, S, q_start, q_rows, split, causal):
+    """The kernel forms that a launch takes: "256", "128", both behind one another, or "tiles"."""
+    plan = pkg.flash_attn_tc_plan(pkg.make_params(S, H * d_h, H, 64, 2, split, causal).flash_tc, q_start, q_rows)
+    return "+".join(n for n, items in (("256", plan.items_256), ("128", plan.items_128), ("tiles", plan.tiles)) if items)
+
+
 # One to six key stages, ragged last blocks, rows that see no key of a split, both directions of the mask.
 @pytest.mark.parametrize("d_h", [16, 32])
 @pytest.mark.parametrize("H,S,q_start,q_rows,split,causal", [
     (160, 64, 0, 64, 1, 0), (100, 256, 0, 256, 1, 1), (152, 192, 64, 128, 1, 1), (60, 640, 320, 320, 1, 0), (40, 768, 0, 768, 1, 0),
     (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (16, 1536, 192, 576, 2, 0)])
 def test_single_tiles_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal):
-    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
-    assert pkg.flash_attn_tc_plan(p.flash_tc, q_start, q_rows).tiles > 0
+    assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == "tiles"
     check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
 
 
-# Key stages per 128-row block at which the two softmax warpgroups get none, one, an odd and an even number; few heads
-# take the form that splits the keys between them, many the form with 256 rows per block (H * split in (74, 148]).
+# Key stages per 128-row block at which the two softmax warpgroups of a 128-row item get none, one, an odd and an even
+# number: three heads take that form. Forty heads take it where they are at most 148 such items (the shapes of one split, and
+# 64 rows), else single tiles (d_h 16 and 32) or 256-row items (d_h 64 and 128).
 @pytest.mark.parametrize("H", [3, 40])
 @pytest.mark.parametrize("d_h", [16, 32, 64, 128])
 @pytest.mark.parametrize("S,q_start,q_rows,split,causal", [
     (64, 0, 64, 1, 0), (128, 0, 128, 1, 1), (192, 64, 128, 1, 1), (320, 64, 256, 1, 0), (512, 128, 256, 2, 1),
     (512, 0, 192, 2, 1), (640, 0, 64, 2, 1), (896, 448, 448, 2, 1)])
 def test_both_block_forms_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal):
-    torch = torch_cuda
-    p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
-    g = torch.Generator(device="cuda").manual_seed(S + d_h + H)
-    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
-    # rows whose maximum keeps growing along the keys: the exponent offset moves after the first stages too
-    dev[1] *= torch.linspace(0.5, 6.0, S, device="cuda", dtype=torch.float16)[None, :, None]
-    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
-    q, k, v = (t.double() for t in dev)
-    s = q[:, q_start:q_start + q_rows] @ k.transpose(1, 2) * p.flash_tc.scale
-    if causal:
-        rows = torch.arange(q_start, q_start + q_rows, device="cuda")[:, None]
-        s = s.masked_fill(torch.arange(S, device="cuda")[None, :] > rows, float("-inf"))
-    w = torch.softmax(s, dim=-1)
-    ref = (w @ v).permute(1, 0, 2).reshape(q_rows, H * d_h)
-    # Every softmax weight is rounded to fp16 (2^-11 of it) or, below 2^-14 of the largest, to a multiple of 2^-25; the
-    # offset may lag the maximum by 2^8. fp32 scores of up to about 100 carry 1e-5 of relative error into the weights.
-    bound = ((w * 2 ** -11 + 2.0 ** -24) @ v.abs()).permute(1, 0, 2).reshape(q_rows, H * d_h) + 1e-4 * ref.abs().max()
-    err = (O.double() - ref).abs()
-    assert torch.isfinite(O).all()
-    assert bool((err <= bound).all()), float((err - bound).max())
-    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
+    few = H * split * ((q_rows + 127) // 128) <= 148
+    assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == ("128" if few else "tiles" if d_h < 64 else "256")
+    check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
 
 
-@pytest.mark.parametrize("d_h", [16, 64, 128])
-@pytest.mark.parametrize("H,q_start,q_rows,split", [(50, 64, 704, 1), (50, 0, 576, 1), (19, 2048, 2048, 1), (38, 0, 1024, 2)])
-def test_a_short_last_wave(pkg, torch_cuda, d_h, H, q_start, q_rows, split):
-    """Launches whose last wave is at most half full take its 256-row items as 128-row ones: ragged last blocks among
-    them, one with nothing in its second half."""
-    torch = torch_cuda
+# Seven to 32 key stages, more than any ring of K/V slots holds: 256-row items whose two tiles have the same number of stages,
+# one more in the second, or 64 rows in the second; 128-row items whose warpgroups get an odd and an even number.
+@pytest.mark.parametrize("d_h", [16, 32, 64, 128])
+@pytest.mark.parametrize("H,S,q_start,q_rows,split,causal,want", [
+    (80, 1024, 768, 256, 1, 0, "256"), (90, 1152, 832, 256, 1, 1, "256"), (76, 1024, 832, 192, 1, 0, "256"),
+    (40, 2304, 1984, 256, 2, 1, "256"), (100, 1024, 960, 64, 1, 1, "128"), (5, 4096, 2880, 1216, 1, 1, "128"),
+    (18, 2176, 64, 448, 2, 0, "128")])
+def test_rings_that_wrap_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal, want):
+    assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == want
+    check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
+
+
+@pytest.mark.parametrize("d_h", [16, 32, 64, 128])
+@pytest.mark.parametrize("tile_rows", [64, None])
+@pytest.mark.parametrize("H,q_start,q_rows,split", [(50, 64, 704, 1), (50, 0, 576, 1), (19, 2048, 2048, 1), (38, 0, 1024, 2),
+                                                    (100, 64, 704, 1), (120, 0, 576, 1), (60, 128, 448, 3)])
+def test_a_short_last_wave(pkg, torch_cuda, d_h, H, q_start, q_rows, split, tile_rows):
+    """Launches whose last wave is at most half full: from two full waves on (the last four shapes; at d_h 128 from one)
+    its 256-row items go as 128-row ones, last blocks of 192 and 64 rows among them, of which the second half has 64 rows
+    or none; below that the whole launch goes as 128-row items."""
     S = 4096 * split
-    p = pkg.make_params(S, H * d_h, H, 64, 2, split, 0)
-    g = torch.Generator(device="cuda").manual_seed(H + q_rows + d_h)
-    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
-    O, counters = run_attention(pkg, torch, p, dev, q_start, q_rows, pkg.F32, tile_rows=64)
-    assert torch.isfinite(O).all()
-    assert counters.cpu().tolist() == [H * split] * (q_rows // 64)
-    for h in range(H):
-        q, k, v = (t[h].double() for t in dev)
-        w = torch.softmax(q[q_start:q_start + q_rows] @ k.T * p.flash_tc.scale, dim=-1)
-        ref = w @ v
-        bound = (w * 2 ** -11 + 2.0 ** -24) @ v.abs() + 1e-4 * ref.abs().max()      # as above: softmax weights in fp16
-        err = (O[:, h * d_h:(h + 1) * d_h].double() - ref).abs()
-        assert bool((err <= bound).all()), (h, float((err - bound).max()))
+    items = H * split * ((q_rows + 255) // 256)
+    assert form(pkg, H, d_h, S, q_start, q_rows, split, 0) == ("256+128" if items > 296 or d_h == 128 else "128")
+    check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, 0, growing=False, tile_rows=tile_rows)

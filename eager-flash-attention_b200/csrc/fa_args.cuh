@@ -23,7 +23,8 @@ struct FaArgs {
     int     counters_sys;   // the tile counters live in host memory: order the rows before the count at system scope
     const short* order_tab; // strict-order launches only: order_tab[k] = the 256-row block taken k-th
                             // (device memory, one entry per block); nullptr = first to last (or last to first, below)
-    int tail_first = -1, tail_total = 0;   // >= 0: the launch covers, as 128-row items, the 256-row items of a launch of tail_total from this one on
+    int     tail_first = -1, tail_total = 0;   // >= 0: the launch covers, as 128-row items, the 256-row items of a launch of tail_total from this one on
+    float   rescale_above;  // log2 units by which a row maximum may outgrow the exponent offset in use
     int     heavy_first;    // take the row blocks (or bands) from the last to the first; with a causal
                             // mask the last rows sweep the most keys, so the longest items start first
 };

@@ -84,6 +84,12 @@ __global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restri
     for (; i < n; i += stride) out[i] = __float2half_rn(in[i]);
 }
 
+// How far (log2 units) a row maximum may outgrow the exponent offset before the accumulator is rescaled. With the
+// maximum itself as the offset the largest softmax weight of a row is exactly 1; under a lagging one it is rounded to fp16
+// like the others. Long sweeps of the larger heads lag; small heads (few columns to rescale) and the allocation-free
+// entry do not: 2 to 8 % less error against float64 (d_h 32, 4032 keys: 1.94e-4 against 2.07e-4, 2-norm).
+constexpr float kRescaleLag = 8.f;
+
 // Tensor maps depend only on (pointer, S, H_local, d_h); drivers launch the same tensors over and over.
 struct TmapKey {
     const void* ptr; int S, H, D, rows;
@@ -173,6 +179,7 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
     a.q_start = q_start; a.q_rows = q_rows; a.S = p.S; a.H_local = p.H_local;
     a.nsplit = p.split; a.kv_len = p.S / p.split; a.causal = p.causal;
     a.scale_log2e = p.scale * 1.4426950408889634f;
+    a.rescale_above = p.d_h >= 64 ? kRescaleLag : 0.f;
     a.tile_counters = tile_counters; a.tile_rows = tile_rows;
     a.counters_sys = 0;
     if (tile_counters != nullptr) {
@@ -320,6 +327,7 @@ int fa_forward_noalloc(const void* Q, const void* K, const void* V, void* O, int
     a.q_start = q_start; a.q_rows = q_rows; a.S = p.S; a.H_local = p.H_local;
     a.nsplit = p.split; a.kv_len = p.S / p.split; a.causal = p.causal;
     a.scale_log2e = p.scale * 1.4426950408889634f;
+    a.rescale_above = 0.f;
     a.tile_counters = nullptr; a.tile_rows = 0;
     a.counters_sys = 0;
     a.status = status;                       // a word of the module, see noalloc_status()

@@ -3,9 +3,10 @@
 //
 // What bounds such a launch is the turnover of its blocks: tensor-memory allocation, barriers, the Q load, the first Q*K^T and
 // the epilogue of a row block that has only a few 128-key stages. Two of these small blocks share an SM and hide each
-// other's; the kernel of 256 rows has the SM to itself. Its item takes 3.5 us and 1.7 a stage (d_h 16; 4.2 and 1.7 at d_h
-// 32), the same rows here 2.0 and 1.9 (1.7 and 2.1). 222 items of 256 rows: 2 stages 14.4 against 16.5 us, 4 stages 20.6
-// against 22.8, 8 stages 35 against 34 (d_h 16); 14.5 / 22.4 / 37 against 18.5 / 24.7 / 35 (d_h 32).
+// other's; the kernel of 256 rows has the SM to itself. Its item takes about 4 us and 1.7 a stage, the same rows here 2 us
+// and 2 a stage. Without a mask the line lies at five stages: 222 items of 256 rows, d_h 16, take 14.4 us here against 16.5
+// (2 stages), 20.6 against 22.8 (4), 35 against 34 (8). Under a causal mask the smaller blocks also end more evenly: up to
+// ten stages on average, 16 heads x 2048 rows 37.0 against 49.2 us (d_h 16), 39.0 against 52.0 (d_h 32).
 //
 // One CTA = 128 query rows of one (head, split). K and V stream through shared memory in 128-key stages filled by TMA
 // (32- or 64-byte swizzle). S = Q K^T is a tcgen05.mma with both operands in shared memory and the 128x128 fp32 result

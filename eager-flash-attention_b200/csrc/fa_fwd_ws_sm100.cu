@@ -4,8 +4,10 @@
 //
 // Described for two tiles of d_h = 64 or 128. Small heads (AHEAD) and few rows (KSPLIT) use it with the differences
 // stated at those two constants. Against a kernel of one tile per block (fa_fwd_tile_sm100.cu, which keeps the small heads'
-// launches of few keys): 4032 rows of eight heads of 32, 71.5 -> 58.6 us; 128 rows against 16384 keys in eight splits (16
-// heads of 64), 55 -> 41.5 us.
+// launches of few keys): 4032 rows of eight heads of 32, 71.5 -> 61.4 us; 128 rows against 16384 keys in eight splits (16
+// heads of 64), 55 -> 42.5 us. Both figures with the row maximum itself as the exponent offset (58.6 and 41.2 under a
+// lagging one, at 6 and 3 % more error), and with the wait for P*V and the rescaling behind the first half's exponentials
+// (63.7 and 43.0 before them).
 //
 // One CTA = 256 query rows (two 128-row Q tiles) of one (head, split), 384 threads:
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
@@ -34,7 +36,7 @@
 // registers, with its exponentials under the offset in use while the maximum is still being found: the halves'
 // MMAs fetch Q twice (d_h = 128, S = 32768, four heads, causal: 1.27 ms against 1.02).
 // Tensor memory (512 columns): S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+D) O1 [384,384+D).
-// O is rescaled in tensor memory by the softmax warps themselves, and only when a row maximum grew
+// O is rescaled in tensor memory by the softmax warps themselves, and for d_h 64 and 128 only when a row maximum grew
 // by more than 2^8 since the value last used as the exponent offset (P then stays below 256, well
 // inside fp16); the final division by the row sum makes the result independent of the offset.
 // P reaches the MMA warp in two 64-key halves, each on its own mbarrier, so the first four k-steps of
@@ -62,7 +64,6 @@ constexpr int WS_BM = 128;          // rows per Q tile
 constexpr int WS_BN = 128;          // keys per stage
 constexpr int WS_THREADS = 384;
 constexpr float kNegInfW = -INFINITY;
-constexpr float kRescaleThreshold = 8.0f;   // log2 units
 
 template <int D, bool KSPLIT>
 struct WsCfg {
@@ -480,7 +481,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
 
                 // Move the exponent offset only when the maximum grew by more than the threshold.
                 float alpha = 1.f;
-                if (m_true - m_ref > kRescaleThreshold || m_ref == kNegInfW) {     // (-inf) - (-inf) is NaN: second test
+                if (m_true - m_ref > a.rescale_above || m_ref == kNegInfW) {     // (-inf) - (-inf) is NaN: second test
                     const float m_new = m_true;
                     const float m_use = (m_new == kNegInfW) ? 0.f : m_new;
                     alpha = (m_ref == kNegInfW) ? 0.f : ex2(m_ref - m_use);
@@ -488,9 +489,26 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 }
                 const float m_off = (m_ref == kNegInfW) ? 0.f : m_ref;
 
+                // P is handed to the MMA warp in two halves of 64 keys: the first four k-steps of P*V run on
+                // the tensor pipe while the exponentials of the second half are still being computed.
+                const uint64_t scale2 = pack2(a.scale_log2e, a.scale_log2e), off2 = pack2(-m_off, -m_off);
+                uint64_t psum2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+                auto weights = [&](int c, uint32_t (&pk)[16]) {
+                    #pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        float x0, x1;
+                        unpack2(fma2(pack2(__uint_as_float(su[c][2 * i]), __uint_as_float(su[c][2 * i + 1])), scale2, off2), x0, x1);
+                        const float q0 = ex2(x0), q1 = ex2(x1);
+                        psum2[i & 1] = add2(psum2[i & 1], pack2(q0, q1));
+                        pk[i] = pack_f16x2(q0, q1);
+                    }
+                };
+                uint32_t pk[2][16];
+                if constexpr (AHEAD) { weights(0, pk[0]); weights(1, pk[1]); }
+
                 // O may be rescaled and P overwritten once PV(j-1) of this tile is complete: no part of PV(j) is issued
                 // before this warp's first arrival below. With P in S's columns, S(j) complete implies it (the
-                // tensor pipe runs in issue order); with Q*K^T a stage ahead it is waited for.
+                // tensor pipe runs in issue order); with Q*K^T a stage ahead it is waited for, behind the first half's exponentials.
                 if constexpr (AHEAD) {
                     if (j > 0) {
                         ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], (uint32_t)((j - 1) & 1), &abort_word, 33));
@@ -519,22 +537,10 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     }
                 }
 
-                // P is handed to the MMA warp in two halves of 64 keys: the first four k-steps of P*V run on
-                // the tensor pipe while the exponentials of the second half are still being computed.
-                const uint64_t scale2 = pack2(a.scale_log2e, a.scale_log2e), off2 = pack2(-m_off, -m_off);
-                uint64_t psum2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
                 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    uint32_t pk[16];
-                    #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        float x0, x1;
-                        unpack2(fma2(pack2(__uint_as_float(su[c][2 * i]), __uint_as_float(su[c][2 * i + 1])), scale2, off2), x0, x1);
-                        const float q0 = ex2(x0), q1 = ex2(x1);
-                        psum2[i & 1] = add2(psum2[i & 1], pack2(q0, q1));
-                        pk[i] = pack_f16x2(q0, q1);
-                    }
-                    tmem_st16(tmem_P + c * 16, pk);
+                    if (!AHEAD || c >= 2) weights(c, pk[c & 1]);
+                    tmem_st16(tmem_P + c * 16, pk[c & 1]);
                     if (c == 1 || c == 3) {
                         tmem_wait_st();
                         tc_fence_before_sync();
@@ -777,7 +783,7 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     FaPlan plan;
     plan.items256 = (int)total;
     plan.items128 = plan.tiles = 0;
-    if (d_h < 64 && free_form && total128 > sms && stages <= 6) {
+    if (d_h < 64 && free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
         // few keys and more than one wave of anything: two small blocks to an SM (the figures are in fa_fwd_tile_sm100.cu)
         plan.items256 = 0;
         plan.tiles = (int)total128;

@@ -177,7 +177,7 @@ def test_every_issuing_thread_waits_for_all_phases_of_its_kv_slots(pkg, d_h, H):
     (16, 74, 512, 256, 1, 0, (0, 148)), (128, 37, 4096, 512, 1, 1, (0, 148)), (64, 18, 4096, 192, 4, 0, (0, 144)), (64, 20, 4096, 192, 4, 0, (80, 0)),
     (64, 75, 512, 256, 1, 0, (75, 0)), (128, 148, 4096, 256, 1, 0, (148, 0)),
     # three waves against two: long items of small heads only
-    (16, 75, 1024, 512, 1, 0, (0, 300)), (16, 111, 1024, 512, 1, 1, (222, 0)), (32, 111, 896, 512, 1, 0, (222, 0)),
+    (16, 75, 1024, 512, 1, 0, (0, 300)), (16, 148, 1536, 256, 1, 1, (148, 0)), (32, 111, 896, 512, 1, 0, (222, 0)),
     (32, 111, 2048, 512, 1, 1, (0, 444)), (64, 111, 1024, 512, 1, 1, (222, 0)), (64, 111, 1024, 512, 1, 0, (0, 444)),
     (128, 75, 2048, 512, 1, 0, (150, 0)), (128, 111, 2048, 512, 1, 1, (222, 0)),
     # a last wave that is at most half full, from 4096 keys on and without a mask
@@ -190,8 +190,9 @@ def test_work_items_of_an_attention_launch(pkg, d_h, H, S, q_rows, split, causal
 
 
 @pytest.mark.parametrize("d_h,H,S,q_rows,split,causal,want", [
-    (16, 100, 256, 256, 1, 0, 200), (32, 75, 768, 512, 1, 0, 300), (32, 8, 4096, 4096, 8, 0, 2048), (16, 111, 1024, 512, 1, 1, 0),
-    (16, 74, 256, 256, 1, 0, 0), (32, 75, 896, 512, 1, 0, 0), (64, 100, 256, 256, 1, 0, 0), (16, 8, 4096, 4096, 4, 0, 0)])
+    (16, 100, 256, 256, 1, 0, 200), (32, 75, 640, 512, 1, 0, 300), (32, 8, 4096, 4096, 8, 0, 2048), (16, 111, 1024, 512, 1, 1, 444),
+    (16, 16, 2048, 2048, 1, 1, 256), (16, 111, 1536, 512, 1, 1, 0), (16, 74, 256, 256, 1, 0, 0), (32, 75, 768, 512, 1, 0, 0),
+    (64, 100, 256, 256, 1, 0, 0), (16, 8, 4096, 4096, 4, 0, 0)])
 def test_small_heads_with_few_keys_go_as_single_tiles(pkg, d_h, H, S, q_rows, split, causal, want):
     p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)
     plan = pkg.flash_attn_tc_plan(p.flash_tc, S - q_rows, q_rows)

@@ -117,10 +117,6 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
     return d;
 }
 
-
-
-
-
 __device__ __forceinline__ void setmaxnreg_dec_56() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
 __device__ __forceinline__ void setmaxnreg_inc_224() { asm volatile("setmaxnreg.inc.sync.aligned.u32 224;"); }
 
@@ -768,10 +764,10 @@ void ring_of(FaPlan& plan)
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
 {
     // 128-row items with their keys split over the two warpgroups where one wave of them is the whole launch (d_h 16 /
-    // 64 / 128, 74 items of 256 rows and 32 key stages: 33 / 35 / 49 us against 61 / 57 / 64). Three waves of them against
-    // two of 256 rows are worth it only where items are long and the tensor pipe is not what an item waits for. In us:
-    // 53 against 63 (d_h 16, 16 stages), 57 against 62 (64, 16 stages), even at 8 stages (64), 27 against 25 (64, 4 stages),
-    // 19 against 17 (16, 2 stages), 80 against 75 (128, 16 stages).
+    // 64 / 128, 74 items of 256 rows and 16 key stages: 20 / 21 / 29 us against 31 / 33 / 37). Three waves of them against
+    // two of 256 rows are worth it only where items are long and the tensor pipe is not what an item waits for. In us, 222
+    // items of 256 rows: 51 against 58 (d_h 16, 16 stages), 59 against 63 (64, 16 stages), even at 8 stages (64), 27 against
+    // 25 (64, 4 stages), 82 against 76 (128, 16 stages).
     const long heads = (long)a.H_local * a.nsplit;
     const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
     const long sms = device_sms();
@@ -795,8 +791,10 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
         plan.items256 = 0;
         plan.items128 = (int)total128;
     // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
-    // is at most half of a wave it goes as 128-row items behind the full waves: 0.6 of a wave instead of one. From 4096 keys
-    // on, where that is worth ten times the second launch.
+    // is at most half of a wave it goes as 128-row items behind the full waves (two of them at least, one at d_h 128: shorter
+    // launches are decided above). A wave of 128-row items takes 0.54 / 0.60 / 0.60 / 0.67 of one of 256 rows (d_h 16 / 32 / 64 /
+    // 128, 32 stages); behind three full waves of 65536 keys, with the second launch, 0.75: 3.13 -> 2.95 ms (d_h 64). From
+    // 4096 keys on, where that is worth ten times a launch: 111 heads x 512 rows of d_h 128 140 -> 133 us.
     } else if (free_form && !a.causal && total > sms && rest > 0 && rest * 2 <= sms && a.kv_len >= 4096) {
         plan.items256 = (int)(total - rest);
         plan.items128 = (int)rest * 2;

@@ -23,8 +23,8 @@
 //
 // With one rank there is nothing to reduce: the GEMM epilogue writes the output directly.
 //
-// Co-residency: a CTA of this kernel requests enough shared memory that no CTA of the two-tile
-// attention kernel (which needs all 512 tensor-memory columns) can share its SM, so a tensor-memory
+// Co-residency: a CTA of this kernel requests enough shared memory that no CTA of the attention
+// kernels (which need 256 or all 512 tensor-memory columns) can share its SM, so a tensor-memory
 // allocation can never block on a CTA that only ends when the whole run ends.
 //
 // Every wait (mbarrier, tile counter, arrival flag, done flag) is bounded; on expiry the CTA records

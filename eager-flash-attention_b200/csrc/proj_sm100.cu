@@ -14,7 +14,7 @@
 // (a 128 x 256 tile of d_local = 512 is 4k cycles of MMA). Unlike a grid of one CTA per SM with a fixed share of the
 // tiles, it also suits the launch that starts beside the attention kernel: SMs that come free late find only the
 // tiles that nobody has taken. Measured, 4160 x 512 x 4096 (17.4 GFLOP): 30.7 us with a block per tile and row-wise
-// stores from registers, 24.2 us like this.
+// stores from registers, 24.6 us like this.
 #include "fa_fwd_sm100.cuh"
 #include "host_util.h"
 #include "sm100_ptx.cuh"
@@ -55,7 +55,7 @@ struct PjArgs {
 // HEADS = true: the N columns are those of three weight tensors [heads][K][d_h] side by side, and each tensor's
 // result is [heads][M][d_h]. d_h is a multiple of 64, so every 64-column box lies in one head of one tensor, and a
 // tile may span heads and tensors: A is read once for all of them, and narrow heads still fill wide tiles. Measured,
-// 8192 x 4096 to Q, K and V of four heads of 128: 297 us as twelve launches of 64 tiles each, 98 us as one of 384.
+// 8192 x 4096 to Q, K and V of four heads of 128: 297 us as twelve launches of 64 tiles each, 100 us as one of 384.
 template <int TENSORS>
 struct PjMaps {
     CUtensorMap A, W[TENSORS], out[TENSORS];

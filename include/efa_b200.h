@@ -208,7 +208,7 @@ typedef struct efa_params {
                                    EFA_WIRE_F32 = the fp32 accumulators are summed (the reference's types, run_drivers.cu:26-30)
                                    and the sum is rounded once into the fp16 output. EFA_WIRE_AUTO = fp32. */
     int debug_target_bias;      /* test hook, 0 in normal use: added on the HOST to the counter target that stream mode's
-                                   consumers wait for (the cuStreamWaitValue32 of the projection stream, the polling of
+                                   consumers wait for (the front-end waits of the projection stream, the polling of
                                    the persistent kernel), so that a guarded wait runs out and its recovery can be
                                    tested without any fault on the GPU */
     efa_flash_params flash_tc;
@@ -223,7 +223,7 @@ int efa_blocks_per_tile(const efa_params* p);
 
 /* The launch plan of stream mode (the loop of run_stream, run_drivers.cu:227-240, which there is one tile per
  * iteration): consecutive tiles [first_tile, first_tile + ntiles) share one projection launch and one reduction
- * after a cuStreamWaitValue32 on each of their counters. Groups are returned in the order in which they are
+ * after front-end waits on all of their counters. Groups are returned in the order in which they are
  * waited for: first to last rows, (*descending = 1) last to first, or for EFA_ROWS_MIXED (S/16 rows per group) in the
  * order in which a list schedule of the work items on the device's SMs completes them.
  * group_tiles > 0: groups of that many tiles (1 = the reference's schedule). group_tiles == 0: about S/8

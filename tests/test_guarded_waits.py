@@ -63,7 +63,7 @@ def test_persistent_kernel_gives_up_waiting_for_counters_and_recovers(pkg, oracl
 
 @pytest.mark.gpu
 def test_pending_stream_waits_are_released_after_the_host_limit(pkg, oracle, torch_cuda):
-    """Stream mode with front-end waits (cuStreamWaitValue32) on a target that is one too high: the projection
+    """Stream mode with front-end waits (cuStreamBatchMemOp) on a target that is one too high: the projection
     stream never gets past its first wait. After the context's host limit (300 ms here) run_mode overwrites the
     counters from another stream, which releases every pending wait, drains the streams and reports the failure."""
     torch = torch_cuda

@@ -32,6 +32,8 @@ combine_splits_kernel(const float* __restrict__ O_part, const float* __restrict_
                       int row0, int rows, int ws_rows, int d_local, int H_local, int d_h, int split)
 {
     extern __shared__ float weight[];                       // [CB_ROWS][H_local][split]
+    pdl_wait();
+    pdl_trigger();
     const int first = blockIdx.x * CB_ROWS;
     const int nrows = min(CB_ROWS, rows - first);
 
@@ -213,12 +215,11 @@ int fa_combine(const efa_flash_partials& part, void* O, int o_dtype, int row0, i
     const size_t smem = (size_t)CB_ROWS * p.H_local * p.split * sizeof(float);
     if (smem > 48 * 1024) { set_error("flash_attn_tc_combine: H_local * split = %d is too large", p.H_local * p.split); return 2; }
     if (o_dtype == EFA_F16)
-        combine_splits_kernel<true><<<blocks, 256, smem, stream>>>(part.O_part, part.m_part, part.l_part, O,
-                                                                   row0, rows, part.rows, d_local, p.H_local, p.d_h, p.split);
+        EFA_CUDA(launch_early(combine_splits_kernel<true>, dim3(blocks), 256, smem, stream, part.O_part, part.m_part, part.l_part, O,
+                              row0, rows, part.rows, d_local, p.H_local, p.d_h, p.split));
     else
-        combine_splits_kernel<false><<<blocks, 256, smem, stream>>>(part.O_part, part.m_part, part.l_part, O,
-                                                                    row0, rows, part.rows, d_local, p.H_local, p.d_h, p.split);
-    EFA_CUDA(cudaGetLastError());
+        EFA_CUDA(launch_early(combine_splits_kernel<false>, dim3(blocks), 256, smem, stream, part.O_part, part.m_part, part.l_part, O,
+                              row0, rows, part.rows, d_local, p.H_local, p.d_h, p.split));
     return 0;
 }
 

@@ -95,6 +95,8 @@ fa_fwd_tile_kernel(const __grid_constant__ CUtensorMap tmQ,
     __syncthreads();
     tc_fence_after_sync();
 
+    pdl_wait();
+    pdl_trigger();
     const uint32_t tmem_base = tmem_base_smem;
     const uint32_t tmem_S = tmem_base;            // fp32 S, 128 columns; P (fp16 pairs) reuses columns 0..63
     const uint32_t tmem_O = tmem_base + 128;      // fp32 O, D columns
@@ -332,8 +334,7 @@ int launch_tile(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     using C = FaCfg<D>;
     static_assert(C::SMEM_BYTES <= 48 * 1024, "no opt-in to larger shared memory needed");
     const dim3 grid(args.H_local * args.nsplit, (args.q_rows + FA_BM - 1) / FA_BM);
-    fa_fwd_tile_kernel<D, OUT_F16><<<grid, 128, C::SMEM_BYTES, stream>>>(tq, tk, tv, args);
-    EFA_CUDA(cudaGetLastError());
+    EFA_CUDA(launch_early(fa_fwd_tile_kernel<D, OUT_F16>, grid, 128, C::SMEM_BYTES, stream, tq, tk, tv, args));
     return 0;
 }
 

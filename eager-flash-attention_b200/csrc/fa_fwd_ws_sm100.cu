@@ -178,6 +178,9 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_smem;
+    const bool behind = KSPLIT && a.tail_first >= 0;     // the rest of the launch before this one: no need to wait for that
+    if (!behind) pdl_wait();
+    pdl_trigger();
     const int kv_len = a.kv_len;
 
     struct ItemInfo { int head, split, block_row0, kv_lo, kv_hi, nblk_max; int q_abs0[2], rows_q[2], nblk[2]; };
@@ -680,6 +683,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
         __syncthreads();
     }
     if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
+    if (behind) pdl_wait();
 }
 
 // The first launch of a head size and output type on a device loads and configures every form of it: which one a launch
@@ -719,12 +723,11 @@ int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
         int* counter = work_counter_slot();
         if (!counter) { set_error("no device memory for the work counter"); return 1; }
         EFA_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), stream));
-        fa_fwd_ws_kernel<D, OUT_F16, true, KSPLIT><<<ctas, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, counter, items_x, total);
+        EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, true, KSPLIT>, dim3(ctas), WS_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, counter, items_x, total));
     } else {
         const dim3 grid = blocks > 0 ? dim3(blocks) : dim3(items_x, items_y);
-        fa_fwd_ws_kernel<D, OUT_F16, false, KSPLIT><<<grid, WS_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, args, nullptr, items_x, KSPLIT && blocks > 0 ? blocks : total);
+        EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, false, KSPLIT>, grid, WS_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, (int*)nullptr, items_x, KSPLIT && blocks > 0 ? blocks : total));
     }
-    EFA_CUDA(cudaGetLastError());
     return 0;
 }
 

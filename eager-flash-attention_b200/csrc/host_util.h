@@ -65,6 +65,28 @@ int device_sms();
 // Whether p is memory of the current device itself: not mapped host memory, managed memory or another GPU's.
 bool own_device_memory(const void* p);
 
+#ifdef __CUDACC__
+// A launch whose blocks may start while the kernel before it in the stream still runs, as soon as all blocks of that one have
+// said so or ended: its set-up (barriers, tensor memory, descriptors) and the launch itself then cost nothing. For kernels
+// that wait (pdl_wait) before they touch memory. Call after call: projection 4160 x 512 x 4096 24.6 -> 23.2 us, attention of
+// 4032 rows, eight heads of 32, 61.5 -> 59.5 us, of 16384 rows, four heads of 64 in four splits with the merge 266 -> 262 us.
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#endif
+
 // fp16 tensor map over a row-major tensor viewed as up to 3 dimensions (dim 0 fastest).
 // `box` rows x `box_cols` columns, swizzle chosen from box_cols * 2 bytes (32, 64 or 128).
 int make_tmap_f16(CUtensorMap* out, const void* base, int rank,

@@ -49,6 +49,7 @@ struct PjArgs {
     int M, N, K;
     int heads, d_h;     // HEADS: N = 3 * heads * d_h
     int* status;
+    int behind = 0;     // the launch before it in the stream is a projection of other rows of the same A (project_f16)
 };
 
 // HEADS = false: one W [K][N] and one out [M][N].
@@ -106,6 +107,8 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjArg
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_smem;
+    if (!a.behind) pdl_wait();
+    pdl_trigger();
 
     // Tile of round `it`: the CTA's own block first, then the answer to request it - 1. false: no more (or gave up).
     auto next = [&](int it, int& bx, int& by) -> bool {
@@ -274,6 +277,7 @@ proj_gemm_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjArg
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    if (a.behind) pdl_wait();
 }
 
 template <int BN, bool OUT_F32, bool HEADS>
@@ -288,8 +292,7 @@ int launch_proj(const PjMaps<HEADS ? 3 : 1>& maps, const PjArgs& args, cudaStrea
         configured[dev] = true;
     }
     dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
-    proj_gemm_kernel<BN, OUT_F32, HEADS><<<grid, 192, C::SMEM_BYTES, stream>>>(maps, args);
-    EFA_CUDA(cudaGetLastError());
+    EFA_CUDA(launch_early(proj_gemm_kernel<BN, OUT_F32, HEADS>, grid, 192, C::SMEM_BYTES, stream, maps, args));
     return 0;
 }
 
@@ -300,6 +303,7 @@ struct PjTileArgs {
     void* out;          // fp16 or fp32 [M][N]
     int M, N, K;
     int* status;
+    int behind = 0;
 };
 
 template <int BN, bool OUT_F32>
@@ -340,6 +344,8 @@ proj_tile_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_acc = tmem_base_smem;
+    if (!a.behind) pdl_wait();
+    pdl_trigger();
 
     if (warp == 0) {
         // ---- TMA producer
@@ -421,6 +427,7 @@ proj_tile_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem_acc, BN);
+    if (a.behind) pdl_wait();
 }
 
 template <int BN, bool OUT_F32>
@@ -435,8 +442,7 @@ int launch_tile(const CUtensorMap& ta, const CUtensorMap& tw, const PjTileArgs& 
         configured[dev] = true;
     }
     dim3 grid((args.N + BN - 1) / BN, (args.M + PJ_BM - 1) / PJ_BM);
-    proj_tile_kernel<BN, OUT_F32><<<grid, 192, C::SMEM_BYTES, stream>>>(ta, tw, args);
-    EFA_CUDA(cudaGetLastError());
+    EFA_CUDA(launch_early(proj_tile_kernel<BN, OUT_F32>, grid, 192, C::SMEM_BYTES, stream, ta, tw, args));
     return 0;
 }
 
@@ -482,7 +488,7 @@ int input_map(CUtensorMap* out, const void* A, int rows, int k)
 
 }  // namespace
 
-int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out)
+int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out, bool behind)
 {
     if (out_dtype != EFA_F16 && out_dtype != EFA_F32) { set_error("project: unknown output type %d", out_dtype); return 2; }
     if (int rc = check_shape(rows, d_local, d)) return rc;
@@ -499,7 +505,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     const bool f32 = out_dtype == EFA_F32, wide = wide_tiles(rows, d);
     if (block_per_tile(rows, d_local, d) || (!own_out && !own_device_memory(out))) {
         if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
-        const PjTileArgs a{out, rows, d, d_local, kernel_status_word()};
+        const PjTileArgs a{out, rows, d, d_local, kernel_status_word(), behind};
         if (f32) return launch_tile<128, true>(maps.A, maps.W[0], a, stream);
         return wide ? launch_tile<256, false>(maps.A, maps.W[0], a, stream) : launch_tile<128, false>(maps.A, maps.W[0], a, stream);
     }
@@ -507,7 +513,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     unsigned long long strides[1] = {(unsigned long long)d * (f32 ? 4ull : 2ull)};
     unsigned box[2] = {f32 ? 32u : 64u, 32u};
     if (f32 ? make_tmap_f32(&maps.out[0], out, 2, dims, strides, box) : make_tmap_f16(&maps.out[0], out, 2, dims, strides, box)) return 1;
-    const PjArgs a{rows, d, d_local, 1, d, kernel_status_word()};
+    const PjArgs a{rows, d, d_local, 1, d, kernel_status_word(), behind};
     if (f32) return wide ? launch_proj<256, true, false>(maps, a, stream) : launch_proj<128, true, false>(maps, a, stream);
     return wide ? launch_proj<256, false, false>(maps, a, stream) : launch_proj<128, false, false>(maps, a, stream);
 }

@@ -156,6 +156,18 @@ __device__ __forceinline__ void tma_store_wait_read_but_one() { asm volatile("cp
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------
+// Launches that overlap the kernel before them (launch_early)
+// ---------------------------------------------------------------------------------------------
+// The kernels before this one in the stream are complete and their memory is visible. In every block, ahead of the first
+// access to memory that any of them reads or writes; a kernel that belongs to the one before it (works on the same inputs and
+// other outputs) has it at its end instead, so that it never completes before its predecessor.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// From here on blocks of the next kernel of the stream may start where there is room, once every block of this one is here.
+// Behind pdl_wait, so that one which belongs to this finds its inputs complete, and behind the allocation of tensor
+// memory: a block that came early must not take it from one that the GPU still has to finish.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
 // Cluster launch control: take over a block of this grid that has not started
 // ---------------------------------------------------------------------------------------------
 // The answer (16 bytes) arrives at `answer` and counts as 16 transaction bytes on `bar`. Not to be called again

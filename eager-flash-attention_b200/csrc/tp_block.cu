@@ -163,12 +163,13 @@ struct Run {
         return combine(O, ws_rows, 0, q_rows, s);
     }
     // project (attn_main.cu:262-273) on the projection stream; `out` is a place in the send buffer.
-    int project(const __half* O_tile, void* out, int rows)
+    int project(const __half* O_tile, void* out, int rows) { return project(O_tile, out, rows, c->proj_stream, false); }
+    int project(const __half* O_tile, void* out, int rows, cudaStream_t s, bool behind)
     {
         if (p.skip_proj) return 0;
         launches++;
-        return project_f16(O_tile, w.W_O, out, rows, p.d_local, p.d, c->proj_stream, wire_f32() ? EFA_F32 : EFA_F16,
-                           /* send buffers are, and a direct output has been looked at: */ true);
+        return project_f16(O_tile, w.W_O, out, rows, p.d_local, p.d, s, wire_f32() ? EFA_F32 : EFA_F16,
+                           /* send buffers are, and a direct output has been looked at: */ true, behind);
     }
     // allreduce (run_drivers.cu:26-30): sum of n partial sums at `send` (a place in the send buffer) over the ranks
     // into `recv` (a place in `output`), on communicator / stream `slot`.
@@ -415,6 +416,30 @@ int run_overlap(Run& r, char* output, efa_run_stats* st)
     return finish_timing(c, t0, st, false, false, r.launches);
 }
 
+// Stream mode where nothing follows the projection (one rank that writes `output` itself, no residual): there is nothing to
+// start early for, and the projection of rows that are finished first only takes SMs from the attention of the others. The
+// projections follow the attention on its own stream, without counters, front-end waits and events (a group of them costs 18 to
+// 21 us: its waits and a launch on an idle GPU). One launch for all rows where a group would be the library's choice; where a
+// tile is more than S/16 rows, the caller's tiles stay launches of their own, side by side. Blocks, before and with this:
+// S=1024, eight heads of 64 76 -> 41 us; S=4096, 16 heads of 64 216 -> 141; S=32768, 32 heads of 128 9310 -> 9050.
+int run_stream_alone(Run& r, char* output, efa_run_stats* st)
+{
+    efa_ctx* c = r.c; const efa_params& p = r.p;
+    if (scratch(c, r, p.S, 0, 0, p.S, 0)) return 1;
+    __half* O_all = static_cast<__half*>(c->O_all);
+    if (world_barrier(c->world)) return 1;
+    const double t0 = now_ms();
+    EFA_CUDA(cudaEventRecord(c->ev_t0, c->compute_stream));
+    if (r.attention_raw(O_all, p.S, 0, p.S, c->compute_stream, nullptr, 0)) return 1;
+    EFA_CUDA(cudaEventRecord(c->ev_t1, c->compute_stream));
+    if (r.combine(O_all, p.S, 0, p.S, c->compute_stream)) return 1;
+    const int step = p.S / 8 >= 2 * p.tile ? p.num_tiles : 1;
+    for (int t = 0; t < p.num_tiles; t += step)
+        if (r.project(O_all + (size_t)t * p.tile * p.d_local, output + (size_t)t * p.tile * r.row_bytes(), step * p.tile, c->compute_stream, t > 0)) return 1;
+    if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
+    return finish_timing(c, t0, st, true, false, r.launches);
+}
+
 // run_stream (run_drivers.cu:201-255): one attention launch over all rows; the kernel counts finished
 // 64-row blocks per tile; the projection stream holds, for every tile, a front-end wait on that
 // tile's counter (cuStreamBatchMemOp, no SM involved), the split combine, the projection and an
@@ -441,6 +466,9 @@ int run_stream(Run& r, char* output, efa_run_stats* st)
     // timeline on stderr after the run, relative to the start of the attention kernel. Diagnostic; the events
     // cost a few microseconds each, so traced runs are not benchmark numbers.
     const bool trace = p.trace != 0 && !fused;
+    if (r.direct && !r.residual && !trace && p.debug_target_bias == 0 && p.group_tiles <= 0 && p.reserve_sms <= 0 &&
+        p.row_order == EFA_ROWS_AUTO && p.band_rows == 0)
+        return run_stream_alone(r, output, st);
     if (trace && ensure_trace_events(c, (size_t)3 * ngroups)) return 1;
     if (fused) {
         // One persistent kernel does projection and reduction of every tile beside the attention kernel:

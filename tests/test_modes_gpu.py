@@ -336,3 +336,31 @@ def test_outputs_that_the_projection_cannot_write_itself(pkg, torch_cuda, ctx, m
         results.append(out.cpu())
     assert bool(results[0].any()) and torch.isfinite(results[0]).all()
     assert torch.equal(results[0], results[1])
+
+
+# Tiles of S/16 rows (one launch for all), just larger ones (launches side by side), one tile; splits; fp32.
+@pytest.mark.parametrize("S,tile,d_h,split,f32", [(1024, 64, 64, 1, 0), (1088, 64, 64, 1, 1), (960, 64, 32, 1, 0), (2048, 256, 128, 2, 0),
+                                                  (768, 768, 64, 3, 1), (4096, 256, 64, 1, 0)])
+def test_stream_mode_alone_matches_its_groups(pkg, torch_cuda, ctx, S, tile, d_h, split, f32):
+    """One rank without a residual projects behind the attention; with groups asked for it projects beside it."""
+    torch = torch_cuda
+    H = 4
+    d = H * d_h
+    p = pkg.make_params(S, d, H, tile, 2, split, 1)
+    p.proj_f32 = f32
+    g = torch.Generator(device="cuda").manual_seed(S)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev.append(torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5)
+    w = pkg.Weights(*(t.data_ptr() for t in dev))
+    results = []
+    for groups in (0, 1):
+        p.group_tiles = groups
+        out = torch.full((S, d), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
+        pkg.kernel_status_reset()
+        torch.cuda.synchronize()
+        for _ in range(3):
+            st = pkg.run_mode(ctx, pkg.MODE_STREAM, w, out, p)
+        assert pkg.kernel_status()[0] == 0 and st.attn_kernel_ms > 0
+        results.append((out, st.kernel_launches))
+    assert torch.isfinite(results[0][0]).all() and torch.equal(results[0][0], results[1][0])
+    assert results[0][1] <= results[1][1]

@@ -266,3 +266,27 @@ def test_the_largest_weight_of_a_row_is_not_rounded(pkg, torch_cuda, entry, d_h,
     ref = torch.softmax(s, dim=-1)[:, 300]
     assert 2 ** -8 < float((1 / ref - 1).min()) < float((1 / ref - 1).max()) < 2 ** -2.9
     assert float((O.double() / ref[:, None] - 1).abs().max()) < 5e-6
+
+
+# One row to a block (few rows), several with a ragged last block (1024 rows: three), and the most (from 2368 rows on).
+@pytest.mark.parametrize("rows", [64, 576, 640, 1024, 2368, 2432])
+@pytest.mark.parametrize("split,H,d_h", [(2, 3, 16), (5, 2, 64)])
+def test_merge_of_partials_by_number_of_rows(pkg, torch_cuda, rows, split, H, d_h):
+    """flash_attn_tc_combine alone, from given partials, with rows before and behind those that are merged."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    ws = rows + 128
+    O = torch.randn(split, ws, H, d_h, generator=g, device="cuda")
+    m = torch.randn(split, ws, H, generator=g, device="cuda") * 4
+    l = torch.rand(split, ws, H, generator=g, device="cuda") + 1
+    m[0, ::3] = float("-inf")                                  # a split without keys
+    l[0, ::3] = 0
+    O[0, ::3] = 0
+    fp = pkg.FlashParams(64 * split * 64, d_h, H, split, 0, 1.0)
+    out = torch.full((rows, H * d_h), float("nan"), device="cuda")
+    pkg.flash_attn_tc_combine(pkg.FlashPartials(O.data_ptr(), m.data_ptr(), l.data_ptr(), ws), out, 64, rows, fp, None, pkg.F32)
+    torch.cuda.synchronize()
+    w = torch.exp2(m.double() - m.double().amax(0))
+    want = ((w[..., None] * O.double()).sum(0) / (w * l.double()).sum(0)[..., None])[64:64 + rows].reshape(rows, -1)
+    # sums of `split` fp32 terms and weights from exp2f: a few units in the last place of the largest term
+    assert bool(((out.double() - want).abs() <= 16 * 2 ** -24 * (1 + want.abs().max())).all())

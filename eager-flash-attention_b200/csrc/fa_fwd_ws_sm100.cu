@@ -13,7 +13,7 @@
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
 //   warps 4-7   softmax of Q tile 1
 //   warp  8     TMA producer: Q tiles once, then K and V 128-key stages through two rings
-//   warp  9     tcgen05.mma issuer; owns the tensor-memory allocation
+//   warp  9     tcgen05.mma issuer (one elected lane); owns the tensor-memory allocation
 //   warp  10    the second issuer where there is one, else idle; warp 11 idle (they give their registers to the softmax)
 // Both Q tiles share each K/V stage, which halves the L2 -> shared-memory traffic per FLOP. Each tile is a
 // chain  S(j) -> softmax -> P(j) -> P(j)*V(j) -> Q*K^T(j+1) -> S(j+1)  (P overwrites S in tensor memory, and the
@@ -163,7 +163,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     __shared__ int s_item;
 
     const int tid  = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // known to be one value for the warp
     const int lane = tid & 31;
 
     // ---- once per CTA
@@ -177,7 +177,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_smem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
     const bool behind = KSPLIT && a.tail_first >= 0;     // the rest of the launch before this one: no need to wait for that
     if (!behind) pdl_wait();
     pdl_trigger();
@@ -209,7 +209,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             mbar_fence_init();
         }
         __syncthreads();
-        const int item = s_item;
+        const int item = PERSIST ? __shfl_sync(0xffffffffu, s_item, 0) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
         if (item >= items_total || abort_word != 0) return false;
 
         // Work order. Strict row order (heads fastest) makes every head's K/V stream live at once, far more than
@@ -231,7 +231,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             item_y = b * band + rem % nb;
             // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
             // is worth up to one item's duration (a fifth of the launch with four heads per GPU at 32k rows).
-            if (a.order_tab != nullptr && band == 1) item_y = a.order_tab[item_y];
+            if (a.order_tab != nullptr && band == 1) item_y = __shfl_sync(0xffffffffu, (int)a.order_tab[item_y], 0);
             else if (a.heavy_first) item_y = items_y - 1 - item_y;
         }
         it.head  = item_x % a.H_local;
@@ -290,127 +290,105 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     if (uv > 0 && !mbar_wait(&v_empty[sv], (uint32_t)((uv - 1) & 1), &abort_word, 22)) break;
                     load_tile(sV + sv * C::TILE_BYTES, &tmV, &v_full[sv], kv_lo + j * WS_BN);
                 }
-            } else if (warp >= 9 && warp < 9 + ISSUERS && lane == 0) {
-                // ---- MMA issuer. Descriptors as (low, high) words; a k-step or a ring slot only moves the address
-                // field of the low word.
+            } else if (warp >= 9 && warp < 9 + ISSUERS) {
+                // ---- MMA issuer. The whole warp runs the loop, so that the descriptors are values of the warp (uniform registers,
+                // which is where the instruction wants them), and one elected lane issues: always the same, since a commit
+                // covers what the thread that executes it has issued. Descriptors as (low, high) words; a k-step or a ring
+                // slot only moves the address field of the low word.
+                // A commit costs this warp 200 to 300 cycles (time stamps: 630 of a period of 3284 at d_h 128 and of 2968 at d_h 64 went
+                // into two of them, while a P was waiting), so there is one per tile and stage (s_full; with P in its own
+                // columns also o_done). S = 65536, two heads of 64: 2903 -> 2830 us; S = 32768, four heads of 128, causal: 1035 -> 1002;
+                // 4032 rows, eight heads of 32: 59.3 -> 55.2. Ring slots are given back by the softmax warps that see it: S(j) complete means
+                // that all that was issued before is, QK(j) and PV(j-1) of both tiles among it.
                 const uint64_t dq0 = smem_desc(smem_u32(sQ), 16, 8 * C::SWB, SWZ);
                 const uint64_t dk0 = smem_desc(smem_u32(sK), 16, 8 * C::SWB, SWZ);
                 const uint64_t dv0 = smem_desc(smem_u32(sV), C::BOX_BYTES, 8 * C::SWB, SWZ);
                 const uint32_t dq_lo = (uint32_t)dq0, dq_hi = (uint32_t)(dq0 >> 32);
                 const uint32_t dk_lo = (uint32_t)dk0, dk_hi = (uint32_t)(dk0 >> 32);
                 const uint32_t dv_lo = (uint32_t)dv0, dv_hi = (uint32_t)(dv0 >> 32);
+                auto wait = [&](uint64_t* bar, int phase, int site) -> bool {
+                    const bool done = __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(phase & 1), &abort_word, site));
+                    tc_fence_after_sync();
+                    return done;
+                };
                 auto issue_qk = [&](int q, int slot) {
                     const uint32_t qa = dq_lo + (KSPLIT ? 0u : (uint32_t)q * (C::TILE_BYTES >> 4));
                     const uint32_t ka = dk_lo + (uint32_t)slot * (C::TILE_BYTES >> 4);
                     const uint32_t tS = tmem_base + q * 128;
-                    #pragma unroll
-                    for (int ks = 0; ks < D / 16; ks++) {
-                        const uint32_t off = ((uint32_t)((ks * 16) / C::BOXC) * C::BOX_BYTES + (uint32_t)((ks * 16) % C::BOXC) * 2u) >> 4;
-                        tc_mma_ss_lh(tS, qa + off, dq_hi, ka + off, dk_hi, IDESC_QK, ks > 0 ? 1u : 0u);
+                    if (elect_one()) {
+                        #pragma unroll
+                        for (int ks = 0; ks < D / 16; ks++) {
+                            const uint32_t off = ((uint32_t)((ks * 16) / C::BOXC) * C::BOX_BYTES + (uint32_t)((ks * 16) % C::BOXC) * 2u) >> 4;
+                            tc_mma_ss_lh(tS, qa + off, dq_hi, ka + off, dk_hi, IDESC_QK, ks > 0 ? 1u : 0u);
+                        }
+                        tc_commit(&s_full[q]);
                     }
                 };
-                auto issue_pv = [&](int q, int slot, uint32_t acc0, int half) {
+                auto issue_pv = [&](int q, int slot, uint32_t acc0, int half, bool last) {
                     const uint32_t va = dv_lo + (uint32_t)slot * (C::TILE_BYTES >> 4);
                     const uint32_t tP = tmem_base + (AHEAD ? 320 : 0) + q * 128, tO = tmem_base + 256 + q * 128;
-                    #pragma unroll
-                    for (int ks = half * 4; ks < half * 4 + 4; ks++)
-                        tc_mma_ts_lh(tO, tP + ks * 8, va + ((ks * 16 * C::SWB) >> 4), dv_hi, IDESC_PV, ks > 0 ? 1u : acc0);
+                    if (elect_one()) {
+                        #pragma unroll
+                        for (int ks = half * 4; ks < half * 4 + 4; ks++)
+                            tc_mma_ts_lh(tO, tP + ks * 8, va + ((ks * 16 * C::SWB) >> 4), dv_hi, IDESC_PV, ks > 0 ? 1u : acc0);
+                        if (last) tc_commit(&o_done[q]);
+                    }
                 };
                 bool ok = true;
                 if constexpr (ISSUERS == 2) {
-                    // One issuer per tile. Without KSPLIT both tiles use every stage's slots, so both issuers follow
-                    // every stage to its end, also where the tile itself has no keys left.
+                    // One issuer per tile.
                     const int q = warp - 9;
-                    const int n = KSPLIT ? (nblk[0] + 1 - q) / 2 : nblk[q];      // stages with work for this tile
-                    const int n_follow = KSPLIT ? n : nblk_max;
+                    const int n = KSPLIT ? (nblk[0] + 1 - q) / 2 : q ? nblk[1] : nblk[0];      // stages with work for this tile
                     auto stage = [&](int i) { return KSPLIT ? 2 * i + q : i; };
-                    if (n > 0) ok = mbar_wait(&q_full[KSPLIT ? 0 : q], 0, &abort_word, 24);
+                    if (n > 0) ok = wait(&q_full[KSPLIT ? 0 : q], 0, 24);
                     // S(i) = Q K^T of stage i. With P in columns of its own, S(i - 1) only has to be in registers.
                     auto step_qk = [&](int i) -> bool {
-                        if (i >= n_follow) return true;
+                        if (i >= n) return true;
                         const int j = stage(i), sk = j % NSK;
-                        if (!mbar_wait(&k_full[sk], (uint32_t)((j / NSK) & 1), &abort_word, 27)) return false;
-                        if (i < n) {
-                            if (AHEAD && i > 0 && !mbar_wait(&s_read[q], (uint32_t)((i - 1) & 1), &abort_word, 23)) return false;
-                            tc_fence_after_sync();
-                            issue_qk(q, sk);
-                            tc_commit(&s_full[q]);
-                        }
-                        tc_commit(&k_empty[sk]);
+                        if (!wait(&k_full[sk], j / NSK, 27)) return false;
+                        if (AHEAD && i > 0 && !wait(&s_read[q], i - 1, 23)) return false;
+                        issue_qk(q, sk);
                         return true;
                     };
                     auto step_pv = [&](int i) -> bool {
                         const int j = stage(i), sv = j % NSV;
-                        if (!mbar_wait(&v_full[sv], (uint32_t)((j / NSV) & 1), &abort_word, 25)) return false;
-                        if (i < n) {
-                            if (!mbar_wait(&p_full[q][0], (uint32_t)(i & 1), &abort_word, 26)) return false;
-                            tc_fence_after_sync();
-                            issue_pv(q, sv, i > 0 ? 1u : 0u, 0);
-                            if (!mbar_wait(&p_full[q][1], (uint32_t)(i & 1), &abort_word, 29)) return false;
-                            tc_fence_after_sync();
-                            issue_pv(q, sv, 1u, 1);
-                            if (AHEAD || i == n - 1) tc_commit(&o_done[q]);
-                        }
-                        tc_commit(&v_empty[sv]);
+                        if (!wait(&v_full[sv], j / NSV, 25)) return false;
+                        if (!wait(&p_full[q][0], i, 26)) return false;
+                        issue_pv(q, sv, i > 0 ? 1u : 0u, 0, false);
+                        if (!wait(&p_full[q][1], i, 29)) return false;
+                        issue_pv(q, sv, 1u, 1, AHEAD || i == n - 1);
                         return true;
                     };
                     ok = ok && step_qk(0);
-                    for (int i = 0; i < n_follow && ok; i++)
+                    for (int i = 0; i < n && ok; i++)
                         ok = AHEAD ? step_qk(i + 1) && step_pv(i) : step_pv(i) && step_qk(i + 1);
-                    // The last commit has to land before the barriers are rebuilt for the next work item.
-                    if (ok && n_follow > 0) {
-                        const int j = stage(n_follow - 1);
-                        mbar_wait(&v_empty[j % NSV], (uint32_t)((j / NSV) & 1), &abort_word, 28);
-                    }
-                } else if (nblk_max > 0) {
-                    ok = mbar_wait(&k_full[0], 0, &abort_word, 23);
-                    for (int q = 0; q < 2 && ok; q++) {
-                        if (nblk[q] > 0) {
-                            ok = mbar_wait(&q_full[q], 0, &abort_word, 24);
-                            if (!ok) break;
-                            tc_fence_after_sync();
-                            issue_qk(q, 0);
-                            tc_commit(&s_full[q]);
+                } else {
+                    if (nblk_max > 0) {
+                        ok = wait(&k_full[0], 0, 23);
+                        #pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            if (nblk[q] == 0 || !ok) continue;
+                            ok = wait(&q_full[q], 0, 24);
+                            if (ok) issue_qk(q, 0);
                         }
                     }
-                    if (ok) tc_commit(&k_empty[0]);
-                }
-                for (int j = 0; ISSUERS == 1 && j < nblk_max && ok; j++) {
-                    const int sv = j % NSV;
-                    ok = mbar_wait(&v_full[sv], (uint32_t)((j / NSV) & 1), &abort_word, 25);
-                    if (!ok) break;
-                    bool k_next_ready = false;
-                    for (int q = 0; q < 2 && ok; q++) {
-                        if (j >= nblk[q]) continue;
-                        ok = mbar_wait(&p_full[q][0], (uint32_t)(j & 1), &abort_word, 26);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        issue_pv(q, sv, j > 0 ? 1u : 0u, 0);
-                        ok = mbar_wait(&p_full[q][1], (uint32_t)(j & 1), &abort_word, 29);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        issue_pv(q, sv, 1u, 1);
-                        if (j + 1 < nblk[q]) {
-                            const int sk = (j + 1) % NSK;
-                            if (!k_next_ready) {
-                                ok = mbar_wait(&k_full[sk], (uint32_t)(((j + 1) / NSK) & 1), &abort_word, 27);
-                                if (!ok) break;
-                                tc_fence_after_sync();
-                                k_next_ready = true;
-                            }
-                            issue_qk(q, sk);
-                            tc_commit(&s_full[q]);
-                        } else {
-                            tc_commit(&o_done[q]);
+                    for (int j = 0; j < nblk_max && ok; j++) {
+                        const int sv = j % NSV, sk = (j + 1) % NSK;
+                        ok = wait(&v_full[sv], j / NSV, 25);
+                        if (ok && j + 1 < nblk_max) ok = wait(&k_full[sk], (j + 1) / NSK, 27);
+                        #pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            if (j >= nblk[q] || !ok) continue;
+                            ok = wait(&p_full[q][0], j, 26);
+                            if (!ok) continue;
+                            issue_pv(q, sv, j > 0 ? 1u : 0u, 0, false);
+                            ok = wait(&p_full[q][1], j, 29);
+                            if (!ok) continue;
+                            issue_pv(q, sv, 1u, 1, j + 1 == nblk[q]);
+                            if (j + 1 < nblk[q]) issue_qk(q, sk);
                         }
                     }
-                    if (!ok) break;
-                    tc_commit(&v_empty[sv]);
-                    if (j + 1 < nblk_max) tc_commit(&k_empty[(j + 1) % NSK]);
                 }
-                // The last commit has to land before the barriers are rebuilt for the next work item.
-                if (ISSUERS == 1 && ok && nblk_max > 0)
-                    mbar_wait(&v_empty[(nblk_max - 1) % NSV], (uint32_t)(((nblk_max - 1) / NSV) & 1), &abort_word, 28);
             }
             end_item();
             if (!PERSIST) break;
@@ -430,9 +408,19 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             const uint32_t tmem_S = tmem_base + q * 128 + lane_base;
             const uint32_t tmem_P = tmem_S + (AHEAD ? 320 : 0);
             const uint32_t tmem_O = tmem_base + 256 + q * 128 + lane_base;
-            const int my_rows = rows_q[q];
-            const int my_nblk = KSPLIT ? (nblk[0] + 1 - q) / 2 : nblk[q];
-            const int my_abs0 = q_abs0[q];
+            const int my_rows = q ? rows_q[1] : rows_q[0];
+            const int my_nblk = KSPLIT ? (nblk[0] + 1 - q) / 2 : q ? nblk[1] : nblk[0];
+            const int my_abs0 = q ? q_abs0[1] : q_abs0[0];
+            // Who gives ring slots back: with an issuer per tile each tile for its part (one that has the slots to itself for
+            // both), else the tile that is issued last. Tile 1 sweeps at most one stage more than tile 0, its very last one, whose slots
+            // nothing waits for.
+            const bool gives_back = (warp & 3) == 0 && lane == 0 && (ISSUERS == 2 || q == (nblk[1] > 0 ? 1 : 0));
+            const bool both_parts = SLOT_USERS == 2 && (nblk[0] == 0 || nblk[1] == 0);
+            auto give_back = [&](uint64_t* bar) {
+                mbar_arrive(bar);
+                if (both_parts) mbar_arrive(bar);
+            };
+            auto stage_of = [&](int j) { return KSPLIT ? 2 * j + q : j; };
 
             float m_ref = kNegInfW;     // exponent offset in use (a past row maximum), scaled by scale*log2(e)
             float m_true = kNegInfW;    // true running row maximum, same scaling
@@ -444,6 +432,10 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 ok = __all_sync(0xffffffffu, mbar_wait(&s_full[q], (uint32_t)(j & 1), &abort_word, 31));
                 if (!ok) break;
                 tc_fence_after_sync();
+                if (gives_back) {
+                    give_back(&k_empty[stage_of(j) % NSK]);
+                    if (!AHEAD && j > 0) give_back(&v_empty[stage_of(j - 1) % NSV]);
+                }
 
                 uint32_t su[4][32];
                 #pragma unroll
@@ -513,6 +505,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                         ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], (uint32_t)((j - 1) & 1), &abort_word, 33));
                         if (!ok) break;
                         tc_fence_after_sync();
+                        if (gives_back) give_back(&v_empty[stage_of(j - 1) % NSV]);
                     }
                 }
                 if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {

@@ -296,6 +296,266 @@ int launch_proj(const PjMaps<HEADS ? 3 : 1>& maps, const PjArgs& args, cudaStrea
     return 0;
 }
 
+// The same with two CTAs to a tile of 256 rows: a pair of neighbouring SMs runs one tcgen05.mma (cta_group::2, 256 x 256 x 16).
+// Each CTA stages its own 128 rows of A and HALF of the columns of W, so an SM fetches 32 KB per 64 k instead of 48
+// and reads W's part of an operand from shared memory half as often, which is both what bounds the one-CTA form and a good part
+// of its power. Rank 0 of the pair issues the MMAs and owns the barriers that they wait for (bar_full, acc_empty); its
+// commits arrive in both CTAs. Each CTA keeps its 128 rows of the accumulator and writes them as above. A tile is
+// taken over by the pair as a whole (the answer of try_cancel goes to both). 8192 x 4096 x 4096: 200 -> 178 us (1545 TFLOP/s),
+// 32768 x 4096 x 4096: 820 -> 727, both under the power cap; 8192 x 4096 to Q, K and V of four heads of 128: 84 -> 76.
+struct PjPairCfg {
+    static constexpr int BN         = 256;
+    static constexpr int A_BYTES    = PJ_BM * PJ_BK * 2;          // 16 KB
+    static constexpr int B_BOX      = PJ_BK * 64 * 2;             // one [64 k][64 n] box, 8 KB
+    static constexpr int NBOX       = BN / 128;                   // boxes of W in each CTA
+    static constexpr int STAGE      = A_BYTES + B_BOX * NBOX;
+    static constexpr int NSTAGE     = 6;
+    static constexpr int OUT_BOX    = 32 * 128;
+    static constexpr int OUT_BYTES  = PJ_EPI_WARPS * 2 * OUT_BOX;
+    static constexpr int SMEM_BYTES = STAGE * NSTAGE + OUT_BYTES + 1024;
+};
+
+template <bool OUT_F32, bool HEADS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+proj_pair_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjArgs a)
+{
+    static_assert(!(OUT_F32 && HEADS), "Q, K and V are fp16");
+    using C = PjPairCfg;
+    constexpr int BN = C::BN;
+    constexpr uint32_t IDESC = idesc_f16_f32(2 * PJ_BM, BN, 0, 1);
+    constexpr uint32_t SWZ = swizzle_code(128);
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sOut = smem + C::NSTAGE * C::STAGE;
+
+    __shared__ __align__(8) uint64_t bar_full[C::NSTAGE];         // used in rank 0 only: both CTAs' copies count there
+    __shared__ __align__(8) uint64_t bar_empty[C::NSTAGE];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];   // acc_empty: rank 0
+    __shared__ __align__(8) uint64_t next_full[2], next_empty[2]; // next_empty: rank 0
+    __shared__ __align__(16) uint4 next_tile[2];                  // answers of try_cancel
+    __shared__ uint32_t tmem_base_smem;
+    __shared__ int abort_word;
+
+    const int tid  = threadIdx.x;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // known to be one value for the warp
+    const int lane = tid & 31;
+    const int rank = (int)cluster_rank();
+    const int num_k = (a.K + PJ_BK - 1) / PJ_BK;
+
+    if (tid == 0) {
+        abort_word = 0;
+        for (int s = 0; s < C::NSTAGE; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 2 * PJ_EPI_WARPS);
+            mbar_init(&next_full[s], 1);
+            mbar_init(&next_empty[s], 2 * PJ_EPI_WARPS + 2);      // both epilogues, the issuer, rank 1's producer
+        }
+        mbar_fence_init();
+        tma_prefetch_desc(&maps.A);
+        for (int t = 0; t < (HEADS ? 3 : 1); t++) { tma_prefetch_desc(&maps.W[t]); tma_prefetch_desc(&maps.out[t]); }
+    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc_pair(&tmem_base_smem, 2 * BN);
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync();                                               // the other CTA's barriers are there
+    tc_fence_after_sync();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
+    if (!a.behind) pdl_wait();
+    pdl_trigger();
+
+    // Tile of round `it`: the pair's own block first, then the answer to request it - 1. false: no more (or gave up).
+    auto next = [&](int it, int& bx, int& by) -> bool {
+        const int s = it & 1;
+        if (!mbar_wait(&next_full[s], (uint32_t)((it >> 1) & 1), &abort_word, 14)) return false;
+        int x;
+        if (!clc_query(&next_tile[s], x, by)) return false;
+        bx = x >> 1;                                              // the pair's first block
+        return true;
+    };
+
+    // HEADS: tensor, head and column within the head of a column of the whole.
+    auto locate = [&](int col, int& t, int& head, int& x) {
+        const int h_all = col / a.d_h;
+        t = h_all / a.heads;
+        head = h_all - t * a.heads;
+        x = col - h_all * a.d_h;
+    };
+
+    if (warp == 0) {
+        // ---- TMA producer of each CTA; rank 0's also asks for the next tile at the start of every tile
+        if (lane == 0) {
+            int bx = blockIdx.x >> 1, by = blockIdx.y;
+            int g = 0;                                            // stages filled so far, over all tiles
+            bool ok = true;
+            for (int it = 0; ok; it++) {
+                const int ns = it & 1;
+                if (rank == 0 && it >= 2 && !mbar_wait(&next_empty[ns], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 15)) { ok = false; break; }
+                mbar_expect_tx(&next_full[ns], 16);
+                if (rank == 0) clc_try_cancel_cluster(&next_tile[ns], &next_full[ns]);
+                const int n0 = bx * BN + rank * (BN / 2), m0 = (by * 2 + rank) * PJ_BM;
+                int wt[C::NBOX], wh[C::NBOX], wx[C::NBOX];
+                if constexpr (HEADS) {
+                    #pragma unroll
+                    for (int nb = 0; nb < C::NBOX; nb++) locate(min(n0 + nb * 64, a.N - 64), wt[nb], wh[nb], wx[nb]);
+                }
+                for (int kb = 0; kb < num_k; kb++, g++) {
+                    const int s = g % C::NSTAGE;
+                    const int use = g / C::NSTAGE;
+                    if (use > 0 && !mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), &abort_word, 11)) { ok = false; break; }
+                    uint8_t* sa = smem + s * C::STAGE;
+                    uint8_t* sb = sa + C::A_BYTES;
+                    const uint32_t full = cluster_addr(&bar_full[s], 0);
+                    if (rank == 0) mbar_expect_tx(&bar_full[s], 2 * C::STAGE);
+                    tma_load_2d_pair(sa, &maps.A, full, kb * PJ_BK, m0);      // rows and columns past the end read as zeros
+                    #pragma unroll
+                    for (int nb = 0; nb < C::NBOX; nb++) {
+                        if constexpr (HEADS) tma_load_3d_pair(sb + nb * C::B_BOX, &maps.W[wt[nb]], full, wx[nb], kb * PJ_BK, wh[nb]);
+                        else                 tma_load_2d_pair(sb + nb * C::B_BOX, &maps.W[0], full, n0 + nb * 64, kb * PJ_BK);
+                    }
+                }
+                if (!ok || !next(it, bx, by)) break;
+                fence_proxy_async_smem();
+                if (rank != 0) mbar_arrive_cluster(cluster_addr(&next_empty[it & 1], 0));
+            }
+            // rank 0's commits arrive here as well: none may be on its way when this CTA ends
+            for (int s = max(0, g - C::NSTAGE); ok && s < g; s++)
+                ok = mbar_wait(&bar_empty[s % C::NSTAGE], (uint32_t)((s / C::NSTAGE) & 1), &abort_word, 17);
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer of the pair
+        if (rank == 0 && lane == 0) {
+            const uint64_t da = smem_desc(smem_u32(smem), 16, 1024, SWZ);                          // K-major
+            const uint64_t db = smem_desc(smem_u32(smem) + C::A_BYTES, C::B_BOX, 1024, SWZ);       // MN-major: 16 k rows of 128 B
+            const uint32_t da_lo = (uint32_t)da, da_hi = (uint32_t)(da >> 32), db_lo = (uint32_t)db, db_hi = (uint32_t)(db >> 32);
+            int bx = 0, by = 0, g = 0;
+            bool ok = true;
+            for (int it = 0; ok; it++) {
+                const int acc = it & 1;
+                if (it >= 2) {
+                    ok = mbar_wait(&acc_empty[acc], (uint32_t)(((it >> 1) - 1) & 1), &abort_word, 16);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                }
+                const uint32_t tmem_acc = tmem_base + acc * BN;
+                for (int kb = 0; kb < num_k && ok; kb++, g++) {
+                    const int s = g % C::NSTAGE;
+                    ok = mbar_wait(&bar_full[s], (uint32_t)((g / C::NSTAGE) & 1), &abort_word, 12);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const uint32_t off = (uint32_t)(s * (C::STAGE >> 4));
+                    #pragma unroll
+                    for (int ks = 0; ks < PJ_BK / 16; ks++)
+                        tc_mma_ss_pair(tmem_acc, da_lo + off + ks * 2, da_hi, db_lo + off + ks * 128, db_hi,
+                                       IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+                    tc_commit_pair(&bar_empty[s]);
+                }
+                if (!ok) break;
+                tc_commit_pair(&acc_full[acc]);
+                const bool more = next(it, bx, by);
+                fence_proxy_async_smem();
+                mbar_arrive(&next_empty[it & 1]);
+                if (!more) break;
+            }
+        }
+    } else {
+        // ---- epilogue of this CTA's 128 rows: warps 2..5 own TMEM lanes 32*(warp % 4) .. +31
+        constexpr int COLS = OUT_F32 ? 32 : 64;                   // columns in 128 bytes
+        const int lane_grp = warp & 3;
+        uint8_t* box0 = sOut + lane_grp * 2 * C::OUT_BOX;
+        int bx = blockIdx.x >> 1, by = blockIdx.y;
+        int stores = 0;
+        for (int it = 0; ; it++) {
+            const int acc = it & 1;
+            const int row0 = (by * 2 + rank) * PJ_BM + lane_grp * 32, n0 = bx * BN;
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (uint32_t)((it >> 1) & 1), &abort_word, 13))) break;
+            tc_fence_after_sync();
+            const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(lane_grp * 32) << 16);
+            #pragma unroll 1
+            for (int c = 0; c < BN / COLS; c++, stores++) {
+                if (n0 + c * COLS >= a.N || row0 >= a.M) break;
+                uint4 v[8];                                       // this lane's row: eight 16-byte chunks
+                if constexpr (OUT_F32) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + c * 32, r);
+                    tmem_wait_ld();
+                    #pragma unroll
+                    for (int q = 0; q < 8; q++) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                } else {
+                    uint32_t r[2][32];
+                    tmem_ld32(taddr + c * 64, r[0]);
+                    tmem_ld32(taddr + c * 64 + 32, r[1]);
+                    tmem_wait_ld();
+                    #pragma unroll
+                    for (int q = 0; q < 8; q++) v[q] = pack8(&r[q >> 2][8 * (q & 3)]);
+                }
+                uint8_t* box = box0 + (stores & 1) * C::OUT_BOX;
+                if (lane == 0) tma_store_wait_read_but_one();     // the store before last has left this box
+                __syncwarp();
+                #pragma unroll
+                for (int q = 0; q < 8; q++)                       // 128-byte swizzle: eight rows hit eight bank groups
+                    *reinterpret_cast<uint4*>(box + lane * 128 + ((q ^ (lane & 7)) << 4)) = v[q];
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if constexpr (HEADS) {
+                        int t, head, x;
+                        locate(n0 + c * COLS, t, head, x);
+                        tma_store_3d(&maps.out[t], box, x, row0, head);
+                    } else {
+                        tma_store_2d(&maps.out[0], box, n0 + c * COLS, row0);
+                    }
+                    tma_store_commit();
+                }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[acc], 0));
+            const bool more = __all_sync(0xffffffffu, next(it, bx, by));
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(&next_empty[it & 1], 0));
+            if (!more) break;
+        }
+        if (lane == 0) tma_store_wait_all();
+    }
+
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (abort_word != 0) {
+        for (int i = 0; i < 64; i++) __nanosleep(100000);
+        if (tid == 0 && a.status != nullptr) {
+            if (atomicCAS(a.status, 0, (int)KS_WAIT_TIMEOUT) == 0) {
+                a.status[1] = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+                a.status[2] = abort_word;
+            }
+        }
+        __syncthreads();
+    }
+    cluster_sync();                                               // arrivals and MMAs of the pair reach into both CTAs
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 2 * BN);
+    if (a.behind) pdl_wait();
+}
+
+template <bool OUT_F32, bool HEADS>
+int launch_pair(const PjMaps<HEADS ? 3 : 1>& maps, const PjArgs& args, cudaStream_t stream)
+{
+    using C = PjPairCfg;
+    static bool configured[64] = {};
+    int dev = 0;
+    EFA_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        EFA_CUDA(cudaFuncSetAttribute(proj_pair_kernel<OUT_F32, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        configured[dev] = true;
+    }
+    dim3 grid(2 * ((args.N + C::BN - 1) / C::BN), (args.M + 2 * PJ_BM - 1) / (2 * PJ_BM));
+    EFA_CUDA(launch_early(proj_pair_kernel<OUT_F32, HEADS>, grid, 192, C::SMEM_BYTES, stream, maps, args));
+    return 0;
+}
+
 // A block per tile, stored row by row from registers with plain stores, which go wherever the kernel may write. Nothing
 // promises that for bulk tensor stores: outputs in mapped host memory, managed memory or another GPU's memory take this
 // kernel, and launches that are over in one wave (block_per_tile).
@@ -470,6 +730,16 @@ bool block_per_tile(int rows, int d_local, int d)
     return tiles <= device_sms() && !wide_tiles(rows, d) && (rows <= 64 || (d_local >= 512 && (d & (d - 1)) == 0));
 }
 
+// A pair of CTAs to a tile costs a cluster's start and a hand-over between two SMs per tile, which is worth it where wide tiles are
+// and their k loop is long: from d_local 832 on where there are more tiles than pairs of SMs (12224 x 848 x 2688: 55.8 -> 53.7 us, 16384 x
+// 1024 x 1024: 33.2 -> 31.5, 25728 x 2864 x 1344: 179 -> 159, but 4160 x 512 x 4096: 20.6 -> 21.2, 9024 x 368 x 1600: 17.2 -> 18.4,
+// 29952 x 176 x 1984: 39 -> 50), from 2048 on also with fewer (1024 x 4096 x 4096: 29.9 -> 29.1; 4096 x 1024 x 1024: 10.7 -> 11.2).
+bool in_pairs(int rows, int d_local, int cols)
+{
+    const long tiles = (long)((rows + 255) / 256) * ((cols + 255) / 256);
+    return wide_tiles(rows, cols) && (d_local >= 2048 ? rows >= 256 : d_local >= 832 && tiles > device_sms() / 2);
+}
+
 int check_shape(int rows, int d_local, int d)
 {
     if (rows <= 0 || rows % 64 != 0) { set_error("project: rows (%d) must be a positive multiple of 64", rows); return 2; }
@@ -488,7 +758,7 @@ int input_map(CUtensorMap* out, const void* A, int rows, int k)
 
 }  // namespace
 
-int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out, bool behind)
+int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out, bool behind, bool beside)
 {
     if (out_dtype != EFA_F16 && out_dtype != EFA_F32) { set_error("project: unknown output type %d", out_dtype); return 2; }
     if (int rc = check_shape(rows, d_local, d)) return rc;
@@ -514,6 +784,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     unsigned box[2] = {f32 ? 32u : 64u, 32u};
     if (f32 ? make_tmap_f32(&maps.out[0], out, 2, dims, strides, box) : make_tmap_f16(&maps.out[0], out, 2, dims, strides, box)) return 1;
     const PjArgs a{rows, d, d_local, 1, d, kernel_status_word(), behind};
+    if (!beside && in_pairs(rows, d_local, d)) return f32 ? launch_pair<true, false>(maps, a, stream) : launch_pair<false, false>(maps, a, stream);
     if (f32) return wide ? launch_proj<256, true, false>(maps, a, stream) : launch_proj<128, true, false>(maps, a, stream);
     return wide ? launch_proj<256, false, false>(maps, a, stream) : launch_proj<128, false, false>(maps, a, stream);
 }
@@ -547,6 +818,7 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
     }
     const int cols = 3 * heads * d_h;
     PjArgs a{rows, cols, d, heads, d_h, kernel_status_word()};
+    if (in_pairs(rows, d, cols)) return launch_pair<false, true>(maps, a, stream);
     return wide_tiles(rows, cols) ? launch_proj<256, false, true>(maps, a, stream) : launch_proj<128, false, true>(maps, a, stream);
 }
 
@@ -565,6 +837,7 @@ int proj_preload()
     return touch_kernel(proj_gemm_kernel<128, false, false>) || touch_kernel(proj_gemm_kernel<128, true, false>) ||
            touch_kernel(proj_gemm_kernel<256, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false>) ||
            touch_kernel(proj_gemm_kernel<128, false, true>) || touch_kernel(proj_gemm_kernel<256, false, true>) ||
+           touch_kernel(proj_pair_kernel<false, false>) || touch_kernel(proj_pair_kernel<true, false>) || touch_kernel(proj_pair_kernel<false, true>) ||
            touch_kernel(proj_tile_kernel<128, false>) || touch_kernel(proj_tile_kernel<128, true>) ||
            touch_kernel(proj_tile_kernel<256, false>);
 }

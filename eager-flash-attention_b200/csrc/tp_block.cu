@@ -163,13 +163,13 @@ struct Run {
         return combine(O, ws_rows, 0, q_rows, s);
     }
     // project (attn_main.cu:262-273) on the projection stream; `out` is a place in the send buffer.
-    int project(const __half* O_tile, void* out, int rows) { return project(O_tile, out, rows, c->proj_stream, false); }
-    int project(const __half* O_tile, void* out, int rows, cudaStream_t s, bool behind)
+    int project(const __half* O_tile, void* out, int rows) { return project(O_tile, out, rows, c->proj_stream, false, true); }
+    int project(const __half* O_tile, void* out, int rows, cudaStream_t s, bool behind, bool beside)
     {
         if (p.skip_proj) return 0;
         launches++;
         return project_f16(O_tile, w.W_O, out, rows, p.d_local, p.d, s, wire_f32() ? EFA_F32 : EFA_F16,
-                           /* send buffers are, and a direct output has been looked at: */ true, behind);
+                           /* send buffers are, and a direct output has been looked at: */ true, behind, beside);
     }
     // allreduce (run_drivers.cu:26-30): sum of n partial sums at `send` (a place in the send buffer) over the ranks
     // into `recv` (a place in `output`), on communicator / stream `slot`.
@@ -342,7 +342,7 @@ int run_megatron(Run& r, char* output, efa_run_stats* st)
 
     EFA_CUDA(cudaStreamWaitEvent(c->proj_stream, attn_done, 0));
     EFA_CUDA(cudaEventRecord(c->ev_t2, c->proj_stream));
-    if (r.project(O_all, send_buf, p.S)) return 1;
+    if (r.project(O_all, send_buf, p.S, c->proj_stream, false, false)) return 1;
     EFA_CUDA(cudaEventRecord(c->ev_t3, c->proj_stream));
     EFA_CUDA(cudaEventRecord(proj_done, c->proj_stream));
 
@@ -366,7 +366,7 @@ int run_sync(Run& r, char* output, efa_run_stats* st)
         if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
         char* out_t = output + (size_t)t * p.tile * r.row_bytes();
         char* send = r.direct ? out_t : send_buf;
-        if (r.project(O_tile, send, p.tile)) return 1;
+        if (r.project(O_tile, send, p.tile, c->proj_stream, false, false)) return 1;
         if (sync_stream(c, c->proj_stream, nullptr, 0)) return 1;
         if (r.allreduce(0, send, out_t, (size_t)p.tile * p.d)) return 1;
         if (sync_stream(c, c->comm_streams[0], nullptr, 0)) return 1;
@@ -435,7 +435,7 @@ int run_stream_alone(Run& r, char* output, efa_run_stats* st)
     if (r.combine(O_all, p.S, 0, p.S, c->compute_stream)) return 1;
     const int step = p.S / 8 >= 2 * p.tile ? p.num_tiles : 1;
     for (int t = 0; t < p.num_tiles; t += step)
-        if (r.project(O_all + (size_t)t * p.tile * p.d_local, output + (size_t)t * p.tile * r.row_bytes(), step * p.tile, c->compute_stream, t > 0)) return 1;
+        if (r.project(O_all + (size_t)t * p.tile * p.d_local, output + (size_t)t * p.tile * r.row_bytes(), step * p.tile, c->compute_stream, t > 0, false)) return 1;
     if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
     return finish_timing(c, t0, st, true, false, r.launches);
 }

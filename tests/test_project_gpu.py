@@ -100,3 +100,54 @@ def test_compute_qkv_matches_float64(pkg, torch_cuda, S, d, H_local, d_h):
         assert bool((err <= ref.abs() * 2 ** -10 + 1e-4 * ref.abs().max()).all())
     with pytest.raises(pkg.EfaError, match="d_h"):
         pkg.compute_qkv(X, W[0], W[1], W[2], out[0], out[1], out[2], S, d, H_local, 32)
+
+
+# Pairs of CTAs to a tile (see in_pairs): one row past a tile's first half, ragged rows, columns and k; fewer tiles than pairs of SMs
+# and several per pair; just below the limits.
+@pytest.mark.parametrize("rows,d_local,d", [(256, 2048, 4096), (320, 2064, 8192), (2048, 2048, 2048), (9408, 832, 640), (9536, 848, 704),
+                                            (9408, 816, 640), (4160, 4080, 1088), (19136, 1040, 576)])
+def test_projection_by_pairs_matches_float64(pkg, torch_cuda, rows, d_local, d):
+    test_projection_matches_float64(pkg, torch_cuda, rows, d_local, d)
+
+
+@pytest.mark.parametrize("S,d,H_local,d_h", [(6464, 848, 8, 64), (8256, 1040, 5, 64), (1088, 2064, 16, 128), (4160, 2048, 3, 128)])
+def test_compute_qkv_by_pairs_matches_float64(pkg, torch_cuda, S, d, H_local, d_h):
+    """Tiles whose two CTAs take columns of different heads and tensors."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S + d)
+    X = torch.randn(S, d, generator=g, device="cuda").to(torch.float16)
+    W = [(torch.randn(H_local, d, d_h, generator=g, device="cuda") * d ** -0.5).to(torch.float16) for _ in range(3)]
+    out = [torch.full((H_local, S, d_h), float("nan"), dtype=torch.float16, device="cuda") for _ in range(3)]
+    pkg.kernel_status_reset()
+    for _ in range(3):
+        pkg.compute_qkv(X, W[0], W[1], W[2], out[0], out[1], out[2], S, d, H_local, d_h)
+    torch.cuda.synchronize()
+    assert pkg.kernel_status()[0] == 0
+    for t in range(3):
+        ref = torch.einsum("sk,hkj->hsj", X.double(), W[t].double())
+        err = (out[t].double() - ref).abs()
+        assert torch.isfinite(out[t]).all()
+        assert bool((err <= ref.abs() * 2 ** -10 + 1e-4 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("S,H,d_h", [(4096, 16, 128), (20480, 14, 64)])
+def test_fp32_projection_by_pairs(pkg, torch_cuda, S, H, d_h):
+    """fp32 sums of the block's projection: the fp16 result is their rounding."""
+    torch = torch_cuda
+    d = H * d_h
+    p = pkg.make_params(S, d, H, 64)
+    g = torch.Generator(device="cuda").manual_seed(S)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev.append(torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5)
+    w = pkg.Weights(*(t.data_ptr() for t in dev))
+    ctx = pkg.make_ctx(pkg.World(), ncomm=1)
+    try:
+        half = torch.full((S, d), float("nan"), dtype=torch.float16, device="cuda")
+        full = torch.full((S, d), float("nan"), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        pkg.run_mode(ctx, pkg.MODE_MEGATRON, w, half, p)
+        p.proj_f32 = 1
+        pkg.run_mode(ctx, pkg.MODE_MEGATRON, w, full, p)
+    finally:
+        pkg.destroy_ctx(ctx)
+    assert torch.isfinite(full).all() and torch.equal(full.to(torch.float16), half)

@@ -364,3 +364,28 @@ def test_stream_mode_alone_matches_its_groups(pkg, torch_cuda, ctx, S, tile, d_h
         results.append((out, st.kernel_launches))
     assert torch.isfinite(results[0][0]).all() and torch.equal(results[0][0], results[1][0])
     assert results[0][1] <= results[1][1]
+
+
+# One buffer (one lane), two and more; an odd number of tiles, a single one; splits, whose partials of two tiles lie side by side.
+@pytest.mark.parametrize("S,tile,nbuf,split,d_h", [(960, 64, 1, 1, 64), (960, 64, 2, 3, 32), (1152, 128, 3, 2, 128), (512, 512, 2, 4, 64), (4096, 64, 2, 1, 16)])
+def test_overlap_mode_alone_matches_the_one_launch(pkg, torch_cuda, ctx, S, tile, nbuf, split, d_h):
+    """One rank without a residual runs the tiles on two streams; per row it is the same attention and projection."""
+    torch = torch_cuda
+    H = 4
+    d = H * d_h
+    p = pkg.make_params(S, d, H, tile, nbuf, split, 1)
+    g = torch.Generator(device="cuda").manual_seed(S + tile)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)]
+    dev.append(torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5)
+    w = pkg.Weights(*(t.data_ptr() for t in dev))
+    zero = torch.zeros((S, d), dtype=torch.float16, device="cuda")
+    lanes = torch.full((S, d), float("nan"), dtype=torch.float16, device="cuda")
+    events = torch.full((S, d), float("nan"), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    pkg.kernel_status_reset()
+    for _ in range(3):
+        pkg.run_mode(ctx, pkg.MODE_OVERLAP, w, lanes, p)
+    pkg.run_mode_residual(ctx, pkg.MODE_OVERLAP, w, zero, events, p)
+    torch.cuda.synchronize()
+    assert pkg.kernel_status()[0] == 0
+    assert torch.isfinite(lanes).all() and torch.equal(lanes, events)

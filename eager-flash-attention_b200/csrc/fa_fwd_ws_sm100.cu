@@ -30,9 +30,7 @@
 // in registers as (low, high) words, so that an MMA costs the issuing thread two additions and the instruction
 // (it shares its scheduler with two softmax warps); a V ring one slot deeper than the K ring (V(j) is wanted
 // right at the start of stage j, K(j+1) a whole stage after its slot is freed); packed fp32 pairs in the softmax.
-// Computing a share of the exponentials with a polynomial on the FMA pipes lengthens the softmax and with it the
-// chain; it was measured slower at every share (d_h = 64 with Q*K^T a stage ahead, a quarter of them: 3.36 against 3.14 ms
-// at S = 65536, two heads). So was Q*K^T in two 64-key halves, the upper one issued as soon as its columns of S are in
+// Slower were: Q*K^T in two 64-key halves, the upper one issued as soon as its columns of S are in
 // registers, with its exponentials under the offset in use while the maximum is still being found: the halves'
 // MMAs fetch Q twice (d_h = 128, S = 32768, four heads, causal: 1.27 ms against 1.02).
 // Tensor memory (512 columns): S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+D) O1 [384,384+D).
@@ -110,11 +108,41 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
 {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
+}
+
+// Two exponentials 2^x on the FMA and integer pipes: x = n + f with n the nearest integer, 2^f as a polynomial of degree 5 (a
+// least-maximum fit of the relative error on [-1/2, 1/2] with value 1 at 0; off by at most 1.7e-7 in fp32, as much as ex2.approx).
+// Below -127 the result is 0, NaN stays NaN.
+__device__ __forceinline__ uint64_t exp2_poly2(uint64_t x)
+{
+    float x0, x1;
+    unpack2(x, x0, x1);
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.f));
+    x = pack2(x0, x1);
+    const uint64_t t = add2(x, pack2(12582912.f, 12582912.f));           // 1.5 * 2^23: n in the low bits
+    const uint64_t n = add2(t, pack2(-12582912.f, -12582912.f));
+    const uint64_t f = fma2(n, pack2(-1.f, -1.f), x);
+    uint64_t p = pack2(0x1.5bba14p-10f, 0x1.5bba14p-10f);
+    p = fma2(p, f, pack2(0x1.3cea88p-7f, 0x1.3cea88p-7f));
+    p = fma2(p, f, pack2(0x1.c6b752p-5f, 0x1.c6b752p-5f));
+    p = fma2(p, f, pack2(0x1.ebf9bcp-3f, 0x1.ebf9bcp-3f));
+    p = fma2(p, f, pack2(0x1.62e42ap-1f, 0x1.62e42ap-1f));
+    p = fma2(p, f, pack2(1.f, 1.f));
+    float t0, t1;
+    unpack2(t, t0, t1);
+    return mul2(p, pack2(__uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u), __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u)));
 }
 
 __device__ __forceinline__ void setmaxnreg_dec_56() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
@@ -146,6 +174,12 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     constexpr bool AHEAD = D < 64 || (KSPLIT && D == 64);
     constexpr int ISSUERS = AHEAD || KSPLIT ? 2 : 1;    // issuing threads: one per tile where the tiles need not alternate
     constexpr int SLOT_USERS = AHEAD && !KSPLIT ? 2 : 1; // issuers that read one K/V slot
+    // Every fourth pair of exponentials as a polynomial where one tile's chain is what an item waits for and the special-function
+    // unit has time to spare: d_h 128 (S = 32768, four heads, causal 1008 -> 1000 us; 2048 rows, eight heads 25.3 -> 24.5; ten heads x
+    // 8192 rows 310 -> 302) and 128-row items of small heads (1024 rows, eight heads of 32 11.0 -> 10.6). Elsewhere the instructions
+    // cost more than the unit gains (65536 rows, two heads of 64 2666 -> 2836; 4032 rows, eight heads of 32 56.4 -> 60.4; 128-row
+    // items of 64 -2 % in a single wave, +2 % behind full ones); a third of the pairs is worse everywhere (d_h 128: +3 %).
+    constexpr bool POLY = D == 128 || (KSPLIT && D < 64);
     constexpr int ITEM_ROWS = KSPLIT ? WS_BM : 2 * WS_BM;
 
     extern __shared__ uint8_t smem_raw[];
@@ -487,6 +521,14 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 auto weights = [&](int c, uint32_t (&pk)[16]) {
                     #pragma unroll
                     for (int i = 0; i < 16; i++) {
+                        if (POLY && i % 4 == 3) {
+                            const uint64_t e = exp2_poly2(fma2(pack2(__uint_as_float(su[c][2 * i]), __uint_as_float(su[c][2 * i + 1])), scale2, off2));
+                            float e0, e1;
+                            unpack2(e, e0, e1);
+                            psum2[i & 1] = add2(psum2[i & 1], e);
+                            pk[i] = pack_f16x2(e0, e1);
+                            continue;
+                        }
                         float x0, x1;
                         unpack2(fma2(pack2(__uint_as_float(su[c][2 * i]), __uint_as_float(su[c][2 * i + 1])), scale2, off2), x0, x1);
                         const float q0 = ex2(x0), q1 = ex2(x1);

@@ -290,3 +290,26 @@ def test_merge_of_partials_by_number_of_rows(pkg, torch_cuda, rows, split, H, d_
     want = ((w[..., None] * O.double()).sum(0) / (w * l.double()).sum(0)[..., None])[64:64 + rows].reshape(rows, -1)
     # sums of `split` fp32 terms and weights from exp2f: a few units in the last place of the largest term
     assert bool(((out.double() - want).abs() <= 16 * 2 ** -24 * (1 + want.abs().max())).all())
+
+
+# Launches that compute a share of the exponentials as a polynomial (d_h 128, and 128-row items of the other sizes), and one that does not.
+@pytest.mark.parametrize("S,H,d_h,split", [(512, 2, 128, 1), (4096, 13, 128, 1), (256, 4, 64, 1), (512, 2, 16, 1), (256, 2, 32, 2), (4096, 12, 64, 1)])
+def test_weights_over_the_whole_exponent_range(pkg, torch_cuda, S, H, d_h, split):
+    """Scores spread over several hundred powers of two, so that most weights vanish, some of them below the smallest number;
+    and a NaN in the keys reaches every row, whichever way its exponential is computed."""
+    torch = torch_cuda
+    p = pkg.make_params(S, H * d_h, H, 64, 2, split, 0)
+    g = torch.Generator(device="cuda").manual_seed(S + d_h)
+    dev = [torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) * f for f in (8, 8, 1)]
+    O, _ = run_attention(pkg, torch, p, dev, 0, S, pkg.F32)
+    for h in range(H):
+        q, k, v = (x[h].double() for x in dev)
+        want = torch.softmax(q @ k.T * p.flash_tc.scale, 1) @ v
+        got = O.view(S, H, d_h)[:, h].double()
+        # fp16 weights (2^-11 each) of values up to max |V|, fp32 scores of up to 2^9: 2^-24 * 2^9 in the exponent
+        assert bool(((got - want).abs() <= (2 ** -11 + 2 ** -13) * v.abs().max()).all())
+    for key in (S - 128 + 70, 5):                              # of pairs that go the one way and the other
+        bad = [x.clone() for x in dev]
+        bad[1][:, key, 3] = float("nan")
+        O, _ = run_attention(pkg, torch, p, bad, 0, S, pkg.F32)
+        assert torch.isnan(O).all()

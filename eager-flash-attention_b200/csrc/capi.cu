@@ -71,7 +71,7 @@ extern "C" int efa_convert_f32_to_f16(const float* in, void* out, size_t n, void
 
 extern "C" int efa_project_f16(const void* O_tile, const void* W_O, void* out, int rows, int d_local, int d, void* stream)
 {
-    return project_f16(O_tile, W_O, out, rows, d_local, d, (cudaStream_t)stream);
+    return project_f16(O_tile, W_O, out, rows, d_local, d, (cudaStream_t)stream, EFA_F16, false, false, false, true);
 }
 
 extern "C" int efa_compute_qkv_f16(const void* X, const void* W_q, const void* W_k, const void* W_v,

@@ -40,7 +40,8 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
                 int out_dtype = EFA_F16, bool own_out = false /* the caller knows `out` to be this GPU's own memory */,
                 bool behind = false /* the launch before it in the stream is a projection whose output this one does not touch, and
                                        whose inputs were complete when it started: this one need not wait for it to end */,
-                bool beside = false /* runs while an attention kernel holds the SMs, which come free one by one and not in pairs */);
+                bool beside = false /* runs while an attention kernel holds the SMs, which come free one by one and not in pairs */,
+                bool in_parts = false /* k may be summed in parts (fp16 results; the blocks of all modes sum it in one go, to the same bits) */);
 
 // Three projections of one input in one launch: out[t][head][rows][d_h] = X[rows][d] * W[t][head][d][d_h], all fp16.
 int project_heads_f16(const void* X, const void* const W[3], void* const out[3], int rows, int d, int heads, int d_h,

@@ -706,6 +706,202 @@ int launch_tile(const CUtensorMap& ta, const CUtensorMap& tw, const PjTileArgs& 
     return 0;
 }
 
+// Few tiles and a long k loop: the tiles leave most SMs idle while each of the others waits for its own copies (about 0.37 us per
+// 64 k, whatever the tile's width). A cluster of CTAs shares a 128 x 128 tile, each with its part of k; the partial sums meet in shared
+// memory, where every CTA adds its share of the rows over all of them, in rank order in fp32, and stores it:
+// 64 x 3776 x 3712 20.8 -> 10.7 us, 128 x 4096 x 4096 22.5 -> 11.5; 1216 x 2752 to Q, K and V of one head of 64 17.4 -> 10.7.
+struct PjSplitCfg {
+    static constexpr int BN         = 128;
+    static constexpr int A_BYTES    = PJ_BM * PJ_BK * 2;
+    static constexpr int B_BOX      = PJ_BK * 64 * 2;
+    static constexpr int STAGE      = A_BYTES + 2 * B_BOX;        // 32 KB
+    static constexpr int NSTAGE     = 6;
+    static constexpr int PITCH      = BN + 4;                     // floats between rows of partial sums: 16 bytes off the banks per row
+    static constexpr int SMEM_BYTES = STAGE * NSTAGE + 1024;
+    static_assert(PJ_BM * PITCH * 4 <= STAGE * NSTAGE, "the partial sums take the ring's place");
+};
+
+struct PjSplitArgs {
+    void* out[3];       // fp16 [M][N]; HEADS: of Q, K and V [heads][M][d_h]
+    int M, N, K;
+    int heads, d_h;
+    int* status;
+    int behind;
+};
+
+template <bool HEADS>
+__global__ void __launch_bounds__(192)
+proj_split_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjSplitArgs a)
+{
+    using C = PjSplitCfg;
+    constexpr uint32_t IDESC = idesc_f16_f32(PJ_BM, C::BN, 0, 1);
+    constexpr uint32_t SWZ = swizzle_code(128);
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+
+    __shared__ __align__(8) uint64_t bar_full[C::NSTAGE];
+    __shared__ __align__(8) uint64_t bar_empty[C::NSTAGE];
+    __shared__ __align__(8) uint64_t bar_acc;
+    __shared__ uint32_t tmem_base_smem;
+    __shared__ int abort_word;
+
+    const int tid  = threadIdx.x;
+    const int warp = tid >> 5;
+    const int lane = tid & 31;
+    const int rank = (int)cluster_rank(), parts = (int)gridDim.z;  // the cluster is the grid's third dimension
+    const int n0 = blockIdx.x * C::BN;
+    const int m0 = blockIdx.y * PJ_BM;
+    const int all_k = (a.K + PJ_BK - 1) / PJ_BK;
+    const int kb0 = rank * all_k / parts, num_k = (rank + 1) * all_k / parts - kb0;       // at least one: parts <= all_k
+
+    // HEADS: tensor, head and column within the head of a column of the whole.
+    auto locate = [&](int col, int& t, int& head, int& x) {
+        const int h_all = col / a.d_h;
+        t = h_all / a.heads;
+        head = h_all - t * a.heads;
+        x = col - h_all * a.d_h;
+    };
+
+    if (tid == 0) {
+        abort_word = 0;
+        for (int s = 0; s < C::NSTAGE; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        mbar_init(&bar_acc, 1);
+        mbar_fence_init();
+        tma_prefetch_desc(&maps.A);
+        for (int t = 0; t < (HEADS ? 3 : 1); t++) tma_prefetch_desc(&maps.W[t]);
+    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc(&tmem_base_smem, C::BN);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_acc = tmem_base_smem;
+    if (!a.behind) pdl_wait();
+    pdl_trigger();
+
+    if (warp == 0) {
+        // ---- TMA producer
+        if (lane == 0) {
+            int wt[2], wh[2], wx[2];
+            if constexpr (HEADS) {
+                #pragma unroll
+                for (int nb = 0; nb < 2; nb++) locate(min(n0 + nb * 64, a.N - 64), wt[nb], wh[nb], wx[nb]);
+            }
+            for (int kb = 0; kb < num_k; kb++) {
+                const int s = kb % C::NSTAGE;
+                const int use = kb / C::NSTAGE;
+                if (use > 0 && !mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), &abort_word, 11)) break;
+                uint8_t* sa = smem + s * C::STAGE;
+                uint8_t* sb = sa + C::A_BYTES;
+                mbar_expect_tx(&bar_full[s], C::STAGE);
+                tma_load_2d(sa, &maps.A, &bar_full[s], (kb0 + kb) * PJ_BK, m0);
+                #pragma unroll
+                for (int nb = 0; nb < 2; nb++) {
+                    if constexpr (HEADS) tma_load_3d(sb + nb * C::B_BOX, &maps.W[wt[nb]], &bar_full[s], wx[nb], (kb0 + kb) * PJ_BK, wh[nb]);
+                    else                 tma_load_2d(sb + nb * C::B_BOX, &maps.W[0], &bar_full[s], n0 + nb * 64, (kb0 + kb) * PJ_BK);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer
+        if (lane == 0) {
+            bool ok = true;
+            for (int kb = 0; kb < num_k && ok; kb++) {
+                const int s = kb % C::NSTAGE;
+                ok = mbar_wait(&bar_full[s], (uint32_t)((kb / C::NSTAGE) & 1), &abort_word, 12);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t sa = smem_u32(smem + s * C::STAGE);
+                const uint32_t sb = sa + C::A_BYTES;
+                #pragma unroll
+                for (int ks = 0; ks < PJ_BK / 16; ks++) {
+                    tc_mma_ss(tmem_acc,
+                              smem_desc(sa + ks * 32, 16, 1024, SWZ),                    // K-major: 32 B per 16 k
+                              smem_desc(sb + ks * 16 * 128, C::B_BOX, 1024, SWZ),        // MN-major: 16 k rows of 128 B
+                              IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
+                }
+                tc_commit(&bar_empty[s]);
+            }
+            if (ok) tc_commit(&bar_acc);
+        }
+    } else if (__all_sync(0xffffffffu, mbar_wait(&bar_acc, 0, &abort_word, 13))) {
+        // ---- warps 2..5 own TMEM lanes 32*(warp % 4) .. +31: a row of partial sums per thread, to where the ring was (the MMAs
+        // that read it are complete)
+        tc_fence_after_sync();
+        const int lane_grp = warp & 3;
+        float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem) + (lane_grp * 32 + lane) * C::PITCH);
+        const uint32_t taddr = tmem_acc + ((uint32_t)(lane_grp * 32) << 16);
+        #pragma unroll 1
+        for (int c = 0; c < C::BN / 32; c++) {
+            uint32_t r[32];
+            tmem_ld32(taddr + c * 32, r);
+            tmem_wait_ld();
+            #pragma unroll
+            for (int q = 0; q < 8; q++)
+                dst[c * 8 + q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync();                                               // everybody's partial sums are there
+    const int share = PJ_BM / parts;                              // parts is 2, 4 or 8
+    for (int e = tid; e < share * (C::BN / 4); e += 192) {
+        const int r = rank * share + e / (C::BN / 4), c = (e % (C::BN / 4)) * 4;
+        const int row = m0 + r, col = n0 + c;
+        if (row >= a.M || col >= a.N) continue;
+        const uint32_t at = smem_u32(reinterpret_cast<float*>(smem) + r * C::PITCH + c);
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < parts; i++) {
+            float4 v;
+            uint32_t peer;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(i));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer) : "memory");
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        size_t off = (size_t)row * a.N + col;
+        int t = 0;
+        if constexpr (HEADS) {
+            int head, x;
+            locate(col, t, head, x);
+            off = ((size_t)head * a.M + row) * a.d_h + x;
+        }
+        *reinterpret_cast<uint2*>(static_cast<__half*>(a.out[t]) + off) = make_uint2(pack_f16x2(sum.x, sum.y), pack_f16x2(sum.z, sum.w));
+    }
+    __syncwarp();
+    cluster_sync();                                               // nobody reads this CTA's memory any more
+    if (abort_word != 0) {
+        for (int i = 0; i < 64; i++) __nanosleep(100000);
+        if (tid == 0 && a.status != nullptr) {
+            if (atomicCAS(a.status, 0, (int)KS_WAIT_TIMEOUT) == 0) {
+                a.status[1] = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+                a.status[2] = abort_word;
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 1) tmem_dealloc(tmem_acc, C::BN);
+    if (a.behind) pdl_wait();
+}
+
+template <bool HEADS>
+int launch_split(const PjMaps<HEADS ? 3 : 1>& maps, const PjSplitArgs& args, int parts, cudaStream_t stream)
+{
+    using C = PjSplitCfg;
+    static bool configured[64] = {};
+    int dev = 0;
+    EFA_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+        EFA_CUDA(cudaFuncSetAttribute(proj_split_kernel<HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        configured[dev] = true;
+    }
+    const dim3 grid((args.N + C::BN - 1) / C::BN, (args.M + PJ_BM - 1) / PJ_BM, parts);
+    EFA_CUDA(launch_early_cluster(parts, proj_split_kernel<HEADS>, grid, 192, C::SMEM_BYTES, stream, maps, args));
+    return 0;
+}
+
 // Tile width: the one that leaves the busiest SM less to fetch. What bounds the kernel is the rate at which tiles come
 // from L2 (48 KB per 64 k for a wide tile, 32 KB for a narrow one, 512 and 256 cycles of MMA), so wide tiles count 3, narrow
 // ones 2: 4096 x 4096 x 4096 keeps wide tiles although narrow ones would leave the busiest SM fewer columns.
@@ -740,6 +936,22 @@ bool in_pairs(int rows, int d_local, int cols)
     return wide_tiles(rows, cols) && (d_local >= 2048 ? rows >= 256 : d_local >= 832 && tiles > device_sms() / 2);
 }
 
+// Parts of k for a tile. A cluster and the sum over it cost 2.5 to 3 us, a k-block that an SM has no longer to wait for gives 0.3:
+// two parts from 40 k-blocks on (256 x 4096 x 4096: 22.8 -> 17.5 us, but 2048 x 1472 to Q, K and V of one head of 128: 11.3 -> 12.8), four
+// from 16 (512 x 1024 x 1024: 8.1 -> 7.6; 512 x 2048 x 1024: 12.8 -> 8.9), while there are SMs for them in clusters (128: a cluster's
+// SMs are neighbours, and not every one finds a cluster); eight for at most eight tiles (64 x 2608 x 320: 15.0 -> 7.2; sixteen
+// clusters of eight are not on the GPU at a time: 18.6 -> 15.4, the like of it in fours 17.4 -> 10.7).
+int k_parts(int rows, int d_local, int cols)
+{
+    const long tiles = (long)((rows + PJ_BM - 1) / PJ_BM) * ((cols + 127) / 128);
+    const int num_k = (d_local + PJ_BK - 1) / PJ_BK;
+    const long clustered = device_sms() * 128l / 148;
+    if (tiles <= 8 && num_k >= 32) return 8;
+    if (tiles * 4 <= clustered && num_k >= 16) return 4;
+    if (tiles * 2 <= clustered && num_k >= 40) return 2;
+    return 1;
+}
+
 int check_shape(int rows, int d_local, int d)
 {
     if (rows <= 0 || rows % 64 != 0) { set_error("project: rows (%d) must be a positive multiple of 64", rows); return 2; }
@@ -758,7 +970,7 @@ int input_map(CUtensorMap* out, const void* A, int rows, int k)
 
 }  // namespace
 
-int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out, bool behind, bool beside)
+int project_f16(const void* A, const void* W, void* out, int rows, int d_local, int d, cudaStream_t stream, int out_dtype, bool own_out, bool behind, bool beside, bool in_parts)
 {
     if (out_dtype != EFA_F16 && out_dtype != EFA_F32) { set_error("project: unknown output type %d", out_dtype); return 2; }
     if (int rc = check_shape(rows, d_local, d)) return rc;
@@ -773,6 +985,11 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
         if (make_tmap_f16(&maps.W[0], W, 2, dims, strides, box)) return 1;
     }
     const bool f32 = out_dtype == EFA_F32, wide = wide_tiles(rows, d);
+    if (const int parts = in_parts && !f32 ? k_parts(rows, d_local, d) : 1; parts > 1) {
+        if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
+        const PjSplitArgs a{{out, nullptr, nullptr}, rows, d, d_local, 1, d, kernel_status_word(), behind};
+        return launch_split<false>(maps, a, parts, stream);
+    }
     if (block_per_tile(rows, d_local, d) || (!own_out && !own_device_memory(out))) {
         if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
         const PjTileArgs a{out, rows, d, d_local, kernel_status_word(), behind};
@@ -817,6 +1034,10 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
         if (make_tmap_f16(&maps.out[t], out[t], 3, odims, ostrides, obox)) return 1;
     }
     const int cols = 3 * heads * d_h;
+    if (const int parts = k_parts(rows, d, cols); parts > 1) {
+        const PjSplitArgs s{{out[0], out[1], out[2]}, rows, cols, d, heads, d_h, kernel_status_word(), 0};
+        return launch_split<true>(maps, s, parts, stream);
+    }
     PjArgs a{rows, cols, d, heads, d_h, kernel_status_word()};
     if (in_pairs(rows, d, cols)) return launch_pair<false, true>(maps, a, stream);
     return wide_tiles(rows, cols) ? launch_proj<256, false, true>(maps, a, stream) : launch_proj<128, false, true>(maps, a, stream);
@@ -838,6 +1059,7 @@ int proj_preload()
            touch_kernel(proj_gemm_kernel<256, false, false>) || touch_kernel(proj_gemm_kernel<256, true, false>) ||
            touch_kernel(proj_gemm_kernel<128, false, true>) || touch_kernel(proj_gemm_kernel<256, false, true>) ||
            touch_kernel(proj_pair_kernel<false, false>) || touch_kernel(proj_pair_kernel<true, false>) || touch_kernel(proj_pair_kernel<false, true>) ||
+           touch_kernel(proj_split_kernel<false>) || touch_kernel(proj_split_kernel<true>) ||
            touch_kernel(proj_tile_kernel<128, false>) || touch_kernel(proj_tile_kernel<128, true>) ||
            touch_kernel(proj_tile_kernel<256, false>);
 }

@@ -151,3 +151,21 @@ def test_fp32_projection_by_pairs(pkg, torch_cuda, S, H, d_h):
     finally:
         pkg.destroy_ctx(ctx)
     assert torch.isfinite(full).all() and torch.equal(full.to(torch.float16), half)
+
+
+# A cluster per tile (see k_parts): eight, four and two parts of k, also of unequal length and with a ragged last k-block; ragged rows
+# and columns; at the limits of each and just past them.
+@pytest.mark.parametrize("rows,d_local,d", [(64, 4080, 64), (128, 2048, 1024), (128, 2032, 1088), (192, 1040, 448), (2048, 1024, 256), (2112, 1024, 256),
+                                            (320, 976, 704), (320, 960, 704), (4096, 2560, 256), (4160, 2560, 256), (1984, 2512, 448), (1984, 2480, 448)])
+def test_projection_by_parts_of_k_matches_float64(pkg, torch_cuda, rows, d_local, d):
+    for _ in range(3):
+        test_projection_matches_float64(pkg, torch_cuda, rows, d_local, d)
+
+
+@pytest.mark.parametrize("S,d,H_local,d_h", [(1024, 3008, 1, 64), (192, 1040, 3, 64), (64, 2064, 2, 128)])
+def test_compute_qkv_by_parts_of_k_matches_float64(pkg, torch_cuda, S, d, H_local, d_h):
+    test_compute_qkv_by_pairs_matches_float64(pkg, torch_cuda, S, d, H_local, d_h)
+
+
+def test_projection_by_parts_of_k_into_mapped_host_memory(pkg, torch_cuda):
+    test_projection_into_mapped_host_memory(pkg, torch_cuda, 192, 1040, 448)

@@ -37,8 +37,9 @@ NVLINK_GBS = 900.0      # per direction and GPU, nominal: the link bound the blo
 REDUCE_BY_RANKS = {1: "nccl", 2: "pull", 4: "pull", 8: "pull"}
 
 # DRAM bytes (read + written) of one attention launch of the benchmark shape with all 32 heads on one GPU, by
-# (mode, rows taken last-first): ncu captures, one launch each.
-ATTN_TRAFFIC_32_HEADS = {("stream", False): 5.105e9, ("stream", True): 5.212e9}
+# (mode, rows taken last-first): ncu captures, one launch each. "alone": whole heads in turn, as every launch without tile
+# counters takes them (stream mode on one rank with the library's own plan).
+ATTN_TRAFFIC_32_HEADS = {("stream", False): 5.105e9, ("stream", True): 5.212e9, ("alone", True): 1.061e9}
 
 
 def measured_peaks():
@@ -295,6 +296,10 @@ def main():
     p.reserve_sms = args.reserve_sms
     mode = pkg.parse_mode(args.mode)
     descending = bool(pkg.stream_plan(p)[2])
+    # one rank with the library's own plan: the projection follows an attention launch without tile counters
+    alone = (args.mode == "stream" and world_size == 1 and p.group_tiles <= 0 and p.reserve_sms <= 0 and p.band_rows == 0
+             and args.order == "auto" and p.reduce != pkg.REDUCE_P2P)
+    order = "alone" if alone else args.mode
 
     # Synthetic inputs in pinned host memory (N(0,1) Q/K/V, W_O ~ N(0, 1/d)), then resident copies.
     qkv_shape = (p.H_local, p.S, p.d_h)
@@ -420,7 +425,7 @@ def main():
             data="synthetic",
             config=dict(workload=f"S={p.S} H={p.H} d_h={p.d_h} causal tile={p.tile} ncomm={W['ncomm']} TP={world_size}",
                         mode=args.mode, split=p.split, reduce=(reduce_note or args.reduce), reduce_ctas=(args.reduce_ctas or "default"), reserve_sms=args.reserve_sms, numa_node=numa_node, wire=args.wire, row_order=args.order,
-                        group_tiles=args.group_tiles or "auto (S/8 rows per launch)",
+                        group_tiles=args.group_tiles or ("one launch behind the attention" if order == "alone" else "auto (S/8 rows per launch)"),
                         l2="256 MB buffer written between steps",
                         e2e="pinned host Q/K/V/W_O copied in by every rank, the fp16 [S][d] result (identical on all ranks) copied "
                             "out once, S/N rows by each rank; copy-in, compute and copy-out pipelined over row chunks; bytes "
@@ -437,9 +442,9 @@ def main():
                           # dram__bytes_read.sum + dram__bytes_write.sum of this kernel's launch, from one ncu capture of
                           # the benchmark shape on one rank (32 heads); heads are independent, so a rank's traffic is
                           # that figure times H_local / 32. Shapes that were not captured report null.
-                          traffic=(ATTN_TRAFFIC_32_HEADS.get((args.mode, descending)) * p.H_local / 32
+                          traffic=(ATTN_TRAFFIC_32_HEADS.get((order, descending)) * p.H_local / 32
                                    if (p.S == 32768 and p.d_h == 128 and p.causal and p.split == 1
-                                       and (args.mode, descending) in ATTN_TRAFFIC_32_HEADS) else None),
+                                       and (order, descending) in ATTN_TRAFFIC_32_HEADS) else None),
                           algorithmic_bytes=2.0 * p.S * p.d_local * 4),      # Q, K, V read once, O written once (fp16)
             cpu_baseline=cpu,
             e2e=dict(value=e2e_ms, unit="ms", h2d_bytes_per_step=h2d, d2h_bytes_per_step=d2h),

@@ -24,8 +24,8 @@ namespace {
 // into shared memory; then every thread merges 16-byte column chunks with them, so the row maxima and
 // denominators are read and exponentiated once per head and row, not once per output element. HBM-bound:
 // (split + 1/2 or 1) * rows * d_local * 4 bytes. With few rows it is a chain of loads that counts: up to CB_ROWS rows to a
-// block, but no more than leave two blocks to every SM (128 rows of 16 heads of 64 in eight splits: 24 us with 16 blocks of eight
-// rows, under 10 with one of each; the whole call 42.4 -> 29.1 us).
+// block, but no more than leave two blocks to every SM (128 rows of 16 heads of 64 in eight splits: 24 us as 16 blocks of eight
+// rows; attention and merge together 42.4 us so, 29.1 as blocks of one row).
 constexpr int CB_ROWS = 8;
 
 template <bool OUT_F16>

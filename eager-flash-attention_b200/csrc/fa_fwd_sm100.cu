@@ -25,13 +25,13 @@ namespace {
 // denominators are read and exponentiated once per head and row, not once per output element. HBM-bound:
 // (split + 1/2 or 1) * rows * d_local * 4 bytes. With few rows it is a chain of loads that counts: up to CB_ROWS rows to a
 // block, but no more than leave two blocks to every SM (128 rows of 16 heads of 64 in eight splits: 24 us as 16 blocks of eight
-// rows; attention and merge together 42.4 us so, 29.1 as blocks of one row).
+// rows; attention and merge together 42.4 us so, 29.1 as blocks of one row). The partials are written while this kernel may already be
+// on the GPU (launch_early): the pointers promise nothing, and the loads are ordinary ones, past L1 for what is read once.
 constexpr int CB_ROWS = 8;
 
 template <bool OUT_F16>
 __global__ void __launch_bounds__(256)
-combine_splits_kernel(const float* __restrict__ O_part, const float* __restrict__ m_part,
-                      const float* __restrict__ l_part, void* __restrict__ O,
+combine_splits_kernel(const float* O_part, const float* m_part, const float* l_part, void* O,
                       int row0, int rows, int ws_rows, int d_local, int H_local, int d_h, int split, int per_block)
 {
     extern __shared__ float weight[];                       // [per_block][H_local][split]
@@ -67,7 +67,7 @@ combine_splits_kernel(const float* __restrict__ O_part, const float* __restrict_
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         #pragma unroll 4
         for (int i = 0; i < split; i++) {
-            const float4 v = __ldg(src + i * step4);
+            const float4 v = __ldcg(src + i * step4);
             acc.x = fmaf(w[i], v.x, acc.x); acc.y = fmaf(w[i], v.y, acc.y);
             acc.z = fmaf(w[i], v.z, acc.z); acc.w = fmaf(w[i], v.w, acc.w);
         }

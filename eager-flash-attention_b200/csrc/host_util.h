@@ -68,7 +68,9 @@ bool own_device_memory(const void* p);
 #ifdef __CUDACC__
 // A launch whose blocks may start while the kernel before it in the stream still runs, as soon as all blocks of that one have
 // said so or ended: its set-up (barriers, tensor memory, descriptors) and the launch itself then cost nothing. For kernels
-// that wait (pdl_wait) before they touch memory. Call after call: projection 4160 x 512 x 4096 24.6 -> 23.2 us, attention of
+// that wait (pdl_wait) before they touch memory, and that read it with ordinary loads or TMA only: what the kernel before it
+// writes is not read-only for as long as such a kernel is on the GPU, so no __ldg, no ld.global.nc and no __restrict__ parameter, which
+// lets the compiler choose them and move them ahead of the wait. Call after call: projection 4160 x 512 x 4096 24.6 -> 23.2 us, attention of
 // 4032 rows, eight heads of 32, 61.5 -> 59.5 us, of 16384 rows, four heads of 64 in four splits with the merge 266 -> 262 us.
 // cluster > 1: the blocks along the grid's third dimension, all of them, are a cluster.
 template <class... P, class... A>

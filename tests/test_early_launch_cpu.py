@@ -1,0 +1,55 @@
+"""Kernels that may be on the GPU before the kernel ahead of them has ended (launch_early) read memory that is still being
+written when they start. Loads that presume read-only memory are no option for them: the sources are looked through."""
+import glob
+import os
+import re
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "eager-flash-attention_b200", "csrc")
+
+
+def _sources():
+    text = {}
+    for path in glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")):
+        with open(path) as f:
+            text[path] = re.sub(r"//[^\n]*", "", f.read())
+    return text
+
+
+def _definition(text, name):
+    """Parameters and body of the kernel `name`, or None."""
+    at = re.search(r"__global__[^;{]*?\b" + name + r"\(", text)
+    if not at:
+        return None
+    depth, i = 0, text.index("{", at.end())
+    for k in range(i, len(text)):
+        depth += (text[k] == "{") - (text[k] == "}")
+        if depth == 0:
+            return text[at.start():k + 1]
+    raise AssertionError(f"{name}: no end")
+
+
+def _early_kernels():
+    found = {}
+    for path, text in _sources().items():
+        for name in re.findall(r"launch_early(?:_cluster)?\((?:\w+,\s*)?(\w+_kernel)\b", text):
+            found[name] = _definition(text, name)
+    return found
+
+
+def test_kernels_that_start_early_are_found():
+    assert set(_early_kernels()) == {"combine_splits_kernel", "fa_fwd_ws_kernel", "fa_fwd_tile_kernel", "proj_gemm_kernel", "proj_pair_kernel",
+                                     "proj_tile_kernel", "proj_split_kernel"}
+
+
+def test_kernels_that_start_early_presume_no_read_only_memory():
+    for name, body in _early_kernels().items():
+        assert body, name
+        assert not re.search(r"__restrict__|__ldg\b|\.nc\b|__constant__", body), name
+        assert "pdl_wait()" in body and "pdl_trigger()" in body, name
+
+
+def test_helpers_that_kernels_share_presume_no_read_only_memory():
+    with open(os.path.join(CSRC, "sm100_ptx.cuh")) as f:
+        assert not re.search(r"__restrict__|__ldg\b|global\.nc\b", f.read())

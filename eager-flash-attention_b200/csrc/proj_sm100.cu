@@ -1011,7 +1011,10 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
 {
     if (int rc = check_shape(rows, d, d_h)) return rc;
     if ((long)3 * heads * d_h > 0x7fffff00l) { set_error("project: %d heads of %d are too many columns", heads, d_h); return 2; }
-    if (!own_device_memory(out[0]) || !own_device_memory(out[1]) || !own_device_memory(out[2])) {
+    const int cols = 3 * heads * d_h;
+    const int parts = k_parts(rows, d, cols);
+    // The clusters along k write with plain stores, which go anywhere: whether k is summed in parts does not depend on the memory.
+    if (parts == 1 && (!own_device_memory(out[0]) || !own_device_memory(out[1]) || !own_device_memory(out[2]))) {
         // where the staged stores cannot go: head by head
         for (int h = 0; h < heads; h++)
             for (int t = 0; t < 3; t++)
@@ -1028,13 +1031,14 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
         unsigned long long wstrides[2] = {(unsigned long long)d_h * 2ull, (unsigned long long)d * d_h * 2ull};
         unsigned wbox[3] = {64u, 64u, 1u};
         if (make_tmap_f16(&maps.W[t], W[t], 3, wdims, wstrides, wbox)) return 1;
+        if (((uintptr_t)out[t] & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
+        if (parts > 1) continue;
         unsigned long long odims[3] = {(unsigned long long)d_h, (unsigned long long)rows, (unsigned long long)heads};
         unsigned long long ostrides[2] = {(unsigned long long)d_h * 2ull, (unsigned long long)rows * d_h * 2ull};
         unsigned obox[3] = {64u, 32u, 1u};
         if (make_tmap_f16(&maps.out[t], out[t], 3, odims, ostrides, obox)) return 1;
     }
-    const int cols = 3 * heads * d_h;
-    if (const int parts = k_parts(rows, d, cols); parts > 1) {
+    if (parts > 1) {
         const PjSplitArgs s{{out[0], out[1], out[2]}, rows, cols, d, heads, d_h, kernel_status_word(), 0};
         return launch_split<true>(maps, s, parts, stream);
     }

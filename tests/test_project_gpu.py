@@ -169,3 +169,20 @@ def test_compute_qkv_by_parts_of_k_matches_float64(pkg, torch_cuda, S, d, H_loca
 
 def test_projection_by_parts_of_k_into_mapped_host_memory(pkg, torch_cuda):
     test_projection_into_mapped_host_memory(pkg, torch_cuda, 192, 1040, 448)
+
+
+@pytest.mark.parametrize("S,d,H_local,d_h", [(192, 1040, 3, 64), (1024, 3008, 1, 64), (64, 2064, 2, 128)])
+def test_compute_qkv_by_parts_of_k_into_mapped_host_memory(pkg, torch_cuda, S, d, H_local, d_h):
+    """Where k is summed in parts it is so for any output memory: the same bits. Nothing is written past the last row, and an output that
+    is not 16-byte aligned is refused."""
+    torch = torch_cuda
+    test_compute_qkv_into_mapped_host_memory(pkg, torch, S, d, H_local, d_h)
+    X = torch.ones(S, d, dtype=torch.float16, device="cuda")
+    W = [torch.ones(H_local, d, d_h, dtype=torch.float16, device="cuda") for _ in range(3)]
+    host = [torch.full((H_local * S * d_h + 64,), float("nan"), dtype=torch.float16).pin_memory() for _ in range(3)]
+    pkg.compute_qkv(X, *W, *host, S, d, H_local, d_h)
+    torch.cuda.synchronize()
+    for o in host:
+        assert bool((o[:-64] == d).all()) and torch.isnan(o[-64:]).all()
+    with pytest.raises(pkg.EfaError, match="16-byte"):
+        pkg.compute_qkv(X, *W, host[0], host[1].view(-1)[1:], host[2], S, d, H_local, d_h)

@@ -89,7 +89,9 @@ cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, u
     attr[1].val.clusterDim.z = (unsigned)cluster;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();        // reported here: not once more by whoever asks next
+    return e;
 }
 template <class... P, class... A>
 cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)

@@ -81,6 +81,23 @@ def test_projection_rejects_bad_shapes(pkg, torch_cuda):
         pkg.project(A, W, out, 128, 64, 96)
 
 
+def test_a_launch_that_is_refused_leaves_no_error_behind(pkg, torch_cuda):
+    """More row tiles than a grid has (65535): the call fails, and the next one does not inherit the error."""
+    torch = torch_cuda
+    rows = 65536 * 128
+    A = torch.zeros(rows, 16, dtype=torch.float16, device="cuda")
+    W = torch.zeros(16, 64, dtype=torch.float16, device="cuda")
+    out = torch.zeros(rows, 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(pkg.EfaError, match="proj_gemm_kernel"):
+        pkg.project(A, W, out, rows, 16, 64)
+    x = torch.arange(64, dtype=torch.float32, device="cuda")
+    y = torch.empty(64, dtype=torch.float16, device="cuda")
+    pkg.convert_f32_to_f16(x, y, 64)
+    assert torch.equal(y, x.half())
+    pkg.project(A, W, out, 128, 16, 64)
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("S,d,H_local,d_h", [(512, 512, 4, 128), (1024, 1024, 2, 64), (2048, 256, 4, 64),
                                             # tiles that span heads and tensors, ragged rows, columns and k; several tiles per SM
                                             (192, 80, 3, 64), (64, 16, 1, 64), (320, 144, 1, 128), (8256, 208, 5, 64), (4160, 96, 3, 128)])

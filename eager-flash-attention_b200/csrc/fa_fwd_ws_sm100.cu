@@ -121,9 +121,10 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
     return d;
 }
 
-// Two exponentials 2^x on the FMA and integer pipes: x = n + f with n the nearest integer, 2^f as a polynomial of degree 5 (a
-// least-maximum fit of the relative error on [-1/2, 1/2] with value 1 at 0; off by at most 1.7e-7 in fp32, as much as ex2.approx).
-// Below -127 the result is 0, NaN stays NaN.
+// Two exponentials 2^x on the FMA and integer pipes: x = n + f with n the nearest integer, 2^f as a polynomial of degree 5: the
+// minimax fit of the relative error on [-1/2, 1/2] with the constant term 1 (a linear program over Chebyshev nodes, its coefficients
+// rounded to fp32). Off by at most 1.8e-7 with the fp32 roundings below; ex2.approx is specified to 2^-22 = 2.4e-7. Below -127 the result
+// is 0, NaN stays NaN.
 __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x)
 {
     float x0, x1;

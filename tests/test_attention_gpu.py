@@ -292,7 +292,8 @@ def test_merge_of_partials_by_number_of_rows(pkg, torch_cuda, rows, split, H, d_
     assert bool(((out.double() - want).abs() <= 16 * 2 ** -24 * (1 + want.abs().max())).all())
 
 
-# Launches that compute a share of the exponentials as a polynomial (d_h 128, and 128-row items of the other sizes), and one that does not.
+# Launches that compute a share of the exponentials as a polynomial (d_h 128, and 128-row items of 16 and 32), and two that do not (d_h 64,
+# one wave of 128-row items and three).
 @pytest.mark.parametrize("S,H,d_h,split", [(512, 2, 128, 1), (4096, 13, 128, 1), (256, 4, 64, 1), (512, 2, 16, 1), (256, 2, 32, 2), (4096, 12, 64, 1)])
 def test_weights_over_the_whole_exponent_range(pkg, torch_cuda, S, H, d_h, split):
     """Scores spread over several hundred powers of two, so that most weights vanish, some of them below the smallest number;
@@ -313,3 +314,44 @@ def test_weights_over_the_whole_exponent_range(pkg, torch_cuda, S, H, d_h, split
         bad[1][:, key, 3] = float("nan")
         O, _ = run_attention(pkg, torch, p, bad, 0, S, pkg.F32)
         assert torch.isnan(O).all()
+
+
+# A share of the exponentials as a polynomial (columns 6 and 7 of every eight): items of 256 rows at d_h 128, of 128 rows at 32 and 16; d_h 64
+# has none. One position of the key to a head and split, so that all eight columns occur.
+@pytest.mark.parametrize("S,H,d_h,poly,items128", [(4096, 8, 128, True, False), (1024, 4, 128, True, True), (1024, 4, 32, True, True),
+                                                  (1024, 4, 16, True, True), (4096, 8, 64, False, False)])
+def test_each_weight_is_as_exact_as_its_exponential(pkg, torch_cuda, S, H, d_h, poly, items128):
+    """Two keys per row and split carry weight, the maximum (weight 1) and one of 2^x, x from -1 to 0 over the rows: the fp32
+    denominator shows the exponential itself, with one rounding."""
+    torch = torch_cuda
+    split = 2
+    fp = pkg.FlashParams(S, d_h, H, split, 0, 1.0)
+    plan = pkg.flash_attn_tc_plan(fp, 0, S)
+    assert (plan.items_128 > 0) == items128 and (plan.items_256 > 0) != items128 and plan.tiles == 0
+    g = torch.Generator(device="cuda").manual_seed(d_h)
+    Q = torch.zeros(H, S, d_h, device="cuda", dtype=torch.float16)
+    Q[..., 0] = (torch.rand(H, S, generator=g, device="cuda") * 0.69).half()
+    Q[..., 1] = torch.randint(0, 1024, (H, S), generator=g, device="cuda").half() / 1024
+    Q[..., 2] = 1
+    K = torch.zeros(H, S, d_h, device="cuda", dtype=torch.float16)
+    K[..., 2] = -1000                                           # no weight
+    V = torch.zeros(H, S, d_h, device="cuda", dtype=torch.float16)
+    column = torch.empty(split, H, dtype=torch.int64)
+    for i in range(split):
+        for h in range(H):
+            column[i, h] = (2 * h + i) % 8 + 8 * ((5 * h + 3 * i) % 16)
+            K[h, i * (S // split) + 9, 2] = 0                   # score 0, in the first stage of 128 keys
+            K[h, i * (S // split) + 256 + column[i, h], :3] = torch.tensor([-1, -2.0 ** -12, 0])
+    ws = [torch.full((n,), float("nan"), device="cuda") for n in (split * S * H * d_h, split * S * H, split * S * H)]
+    part = pkg.FlashPartials(*(w.data_ptr() for w in ws), S)
+    pkg.flash_attn_tc_forward(Q, K, V, None, part, 0, S, fp, o_dtype=pkg.F32)
+    torch.cuda.synchronize()
+    m, l = ws[1].view(split, S, H), ws[2].view(split, S, H)
+    assert bool((m == 0).all())
+    score = -(Q[..., 0].float() + Q[..., 1].float() * 2.0 ** -12).T          # exact in fp32
+    w = torch.exp2((score * 1.4426950408889634).double())                     # the argument rounded to fp32, as the kernel has it
+    err = (l.double() - (1 + w)).abs()
+    by_poly = (column % 8 >= 6).to(err.device)[:, None, :] & poly
+    # the error stated for either way, and the rounding of a sum between 1 and 2
+    bound = torch.where(by_poly, 1.8e-7, 2.0 ** -22) * w + 2.0 ** -24
+    assert bool((err <= bound).all()), float((err - bound).max())

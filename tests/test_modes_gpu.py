@@ -389,3 +389,42 @@ def test_overlap_mode_alone_matches_the_one_launch(pkg, torch_cuda, ctx, S, tile
     torch.cuda.synchronize()
     assert pkg.kernel_status()[0] == 0
     assert torch.isfinite(lanes).all() and torch.equal(lanes, events)
+
+
+# The projections behind the attention as launches side by side of pairs of CTAs (four tiles of 1024 rows), fp16 and fp32; one launch;
+# splits. In groups the projection of 4096 columns is one CTA to a tile: the same bits. Causal, so that no rows go as a short last wave of
+# 128-row items: which rows those are depends on the order of the items, and with it the rounding of their sums.
+@pytest.mark.parametrize("S,tile,H,d_h,split,causal,f32", [(4096, 1024, 32, 128, 1, 1, 0), (4096, 1024, 32, 128, 1, 1, 1), (1024, 64, 4, 64, 1, 1, 0),
+                                                          (1024, 256, 8, 64, 1, 1, 0), (2048, 128, 4, 128, 2, 1, 0)])
+def test_stream_mode_on_inputs_that_change_from_call_to_call(pkg, torch_cuda, ctx, S, tile, H, d_h, split, causal, f32):
+    """What a call reads too early would be of the call before: of other inputs. One launch behind the attention, groups of one tile
+    beside it, and the pipeline on host buffers."""
+    torch = torch_cuda
+    d = H * d_h
+    p = pkg.make_params(S, d, H, tile, 2, split, causal)
+    p.proj_f32 = f32
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    inputs = [[torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3)] +
+              [torch.randn(d, d, generator=g, device="cuda", dtype=torch.float16) * d ** -0.5] for _ in range(3)]
+    pkg.kernel_status_reset()
+
+    def run(i, mode, groups=0):
+        p.group_tiles = groups
+        out = torch.full((S, d), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        pkg.run_mode(ctx, mode, pkg.Weights(*(t.data_ptr() for t in inputs[i])), out, p)
+        return out
+
+    want = [run(i, pkg.MODE_MEGATRON) for i in (0, 1, 2)]
+    assert all(torch.isfinite(w).all() for w in want) and not torch.equal(want[0], want[1])
+    for groups in (0, 1):
+        for i in (0, 2, 1, 0):
+            assert torch.equal(run(i, pkg.MODE_STREAM, groups), want[i]), (groups, i)
+    if causal and not f32:
+        p.group_tiles = 0
+        for i in (1, 0, 2):
+            host = [t.cpu().pin_memory() for t in inputs[i]]
+            out = torch.full((S, d), float("nan"), dtype=torch.float16).pin_memory()
+            pkg.run_mode_host(ctx, pkg.MODE_STREAM, *host, out, p)
+            assert torch.equal(out, want[i].cpu()), ("host", i)
+    assert pkg.kernel_status()[0] == 0

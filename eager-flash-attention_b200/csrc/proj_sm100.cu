@@ -726,7 +726,6 @@ struct PjSplitArgs {
     int M, N, K;
     int heads, d_h;
     int* status;
-    int behind;
 };
 
 template <bool HEADS>
@@ -777,7 +776,7 @@ proj_split_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjSp
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_acc = tmem_base_smem;
-    if (!a.behind) pdl_wait();
+    pdl_wait();
     pdl_trigger();
 
     if (warp == 0) {
@@ -883,7 +882,6 @@ proj_split_kernel(const __grid_constant__ PjMaps<HEADS ? 3 : 1> maps, const PjSp
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem_acc, C::BN);
-    if (a.behind) pdl_wait();
 }
 
 template <bool HEADS>
@@ -987,7 +985,7 @@ int project_f16(const void* A, const void* W, void* out, int rows, int d_local, 
     const bool f32 = out_dtype == EFA_F32, wide = wide_tiles(rows, d);
     if (const int parts = in_parts && !f32 ? k_parts(rows, d_local, d) : 1; parts > 1) {
         if (((uintptr_t)out & 15) != 0) { set_error("project: output address not 16-byte aligned"); return 1; }
-        const PjSplitArgs a{{out, nullptr, nullptr}, rows, d, d_local, 1, d, kernel_status_word(), behind};
+        const PjSplitArgs a{{out, nullptr, nullptr}, rows, d, d_local, 1, d, kernel_status_word()};
         return launch_split<false>(maps, a, parts, stream);
     }
     if (block_per_tile(rows, d_local, d) || (!own_out && !own_device_memory(out))) {
@@ -1039,7 +1037,7 @@ int project_heads_f16(const void* X, const void* const W[3], void* const out[3],
         if (make_tmap_f16(&maps.out[t], out[t], 3, odims, ostrides, obox)) return 1;
     }
     if (parts > 1) {
-        const PjSplitArgs s{{out[0], out[1], out[2]}, rows, cols, d, heads, d_h, kernel_status_word(), 0};
+        const PjSplitArgs s{{out[0], out[1], out[2]}, rows, cols, d, heads, d_h, kernel_status_word()};
         return launch_split<true>(maps, s, parts, stream);
     }
     PjArgs a{rows, cols, d, heads, d_h, kernel_status_word()};

@@ -169,9 +169,9 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     constexpr uint32_t IDESC_PV = idesc_f16_f32(WS_BM, D, 0, 1);
     constexpr int NSK = C::NSTAGE_K, NSV = C::NSTAGE_V;
     // P in tensor-memory columns of its own (they fit beside S and O up to D = 64), so that Q*K^T runs a stage ahead of
-    // the softmax. Taken where there is one chain per tile and nothing alternates with it. With two tiles of D = 64 it is
-    // no faster (S = 65536, two heads: 3.14 ms either way; S = 16384, four splits: 274 us against 268): the
-    // special-function unit is busy 82 % of a working SM's time, and tiles that end together store together.
+    // the softmax. Taken where there is one chain per tile and nothing alternates with it. With two tiles of D = 64 it
+    // gives little (1.5 % on long launches, S = 65536, two heads: 2.67 -> 2.63 ms; split ones 0.3 % slower): the special-function
+    // unit is busy 75 to 84 % of a working SM's time already, and tiles that end together store together.
     constexpr bool AHEAD = D < 64 || (KSPLIT && D == 64);
     constexpr int ISSUERS = AHEAD || KSPLIT ? 2 : 1;    // issuing threads: one per tile where the tiles need not alternate
     constexpr int SLOT_USERS = AHEAD && !KSPLIT ? 2 : 1; // issuers that read one K/V slot

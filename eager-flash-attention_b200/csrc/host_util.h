@@ -71,7 +71,10 @@ bool own_device_memory(const void* p);
 // that wait (pdl_wait) before they touch memory, and that read it with ordinary loads or TMA only: what the kernel before it
 // writes is not read-only for as long as such a kernel is on the GPU, so no __ldg, no ld.global.nc and no __restrict__ parameter, which
 // lets the compiler choose them and move them ahead of the wait. Call after call: projection 4160 x 512 x 4096 24.6 -> 23.2 us, attention of
-// 4032 rows, eight heads of 32, 61.5 -> 59.5 us, of 16384 rows, four heads of 64 in four splits with the merge 266 -> 262 us.
+// 4032 rows, eight heads of 32, 61.5 -> 59.5 us, of 16384 rows, four heads of 64 in four splits with the merge 266 -> 262 us. A call of several
+// kernels gains by itself (on an idle GPU with a cold L2: the same attention with its merge 272 -> 269 us, a block of 1024 rows with four
+// projections 77 -> 55); a single kernel on an idle GPU has nothing ahead of it to start under and pays 0.2 to 0.3 us of host time for the
+// attribute and as much for the wait (projection 2496 x 576 x 512 16.4 -> 17.0 us from call to completion, 4160 x 512 x 4096 29.9 -> 30.4).
 // cluster > 1: the blocks along the grid's third dimension, all of them, are a cluster.
 template <class... P, class... A>
 cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)

@@ -914,8 +914,8 @@ bool wide_tiles(int rows, int cols)
 // A block per tile where one wave of narrow tiles is the whole launch, so that there is nothing to take over, and
 // - there are 64 rows: half of every tile's staged stores would be of nothing (64 x 1024 x 1024: 8.7 against 9.5 us), or
 // - d is a power of two and d_local at least 512: the 64 rows of a W box then lie a power of two apart and come in slowly,
-//   the k loop is the time, and it runs 3 to 6 % faster in the smaller kernel (256 x 4096 x 1024: 24.5 against 25.9 us;
-//   4416 x 1536 x 512: 13.2 against 13.9).
+//   the k loop is the time, and it runs 3 to 6 % faster in the smaller kernel (4416 x 1536 x 512: 13.2 against 13.9 us; where k is not
+//   summed in parts, as in the blocks, 256 x 4096 x 1024: 24.5 against 25.9).
 // Otherwise the coalesced stores of the other kernel are worth more (2496 x 512 x 576: 7.7 against 8.8 us; 256 x 704 x 2304:
 // 8.4 against 9.1), and in more than one wave always. Durations of single launches.
 bool block_per_tile(int rows, int d_local, int d)
@@ -938,7 +938,10 @@ bool in_pairs(int rows, int d_local, int cols)
 // two parts from 40 k-blocks on (256 x 4096 x 4096: 22.8 -> 17.5 us, but 2048 x 1472 to Q, K and V of one head of 128: 11.3 -> 12.8), four
 // from 16 (512 x 1024 x 1024: 8.1 -> 7.6; 512 x 2048 x 1024: 12.8 -> 8.9), while there are SMs for them in clusters (128: a cluster's
 // SMs are neighbours, and not every one finds a cluster); eight for at most eight tiles (64 x 2608 x 320: 15.0 -> 7.2; sixteen
-// clusters of eight are not on the GPU at a time: 18.6 -> 15.4, the like of it in fours 17.4 -> 10.7).
+// clusters of eight are not on the GPU at a time: 18.6 -> 15.4, the like of it in fours 17.4 -> 10.7). All this on a GPU that is
+// otherwise idle. Beside a kernel that holds every SM a cluster waits until its SMs come free together: on a stream of high priority beside
+// an attention of 16384 rows, eight heads of 128, 128 x 4096 x 4096 takes 59 us as one CTA per tile, 66 in two parts, 75 in four;
+// 64 x 2048 x 1024 29, 39, 45, and 60 in eight. Only the caller knows which it is; the blocks, which do run it so, do not ask for parts.
 int k_parts(int rows, int d_local, int cols)
 {
     const long tiles = (long)((rows + PJ_BM - 1) / PJ_BM) * ((cols + 127) / 128);

@@ -447,8 +447,10 @@ int run_overlap(Run& r, char* output, efa_run_stats* st)
 // Stream mode where nothing follows the projection (one rank that writes `output` itself, no residual): there is nothing to
 // start early for, and the projection of rows that are finished first only takes SMs from the attention of the others. The
 // projections follow the attention on its own stream, without counters, front-end waits and events (a group of them costs 18 to
-// 21 us: its waits and a launch on an idle GPU). One launch for all rows where a group would be the library's choice; where a
-// tile is more than S/16 rows, the caller's tiles stay launches of their own, side by side. Blocks, before and with this:
+// 21 us: its waits and a launch on an idle GPU). One launch for all rows where a group would be the library's choice. Where a
+// tile is more than S/16 rows, groups are the caller's tiles and each stays a launch: kernel_launches of a run is then less by num_tiles with
+// skip_proj, as in the grouped schedule. That is not for speed (one launch instead, us: S=1024, tiles of 256, eight heads of 64 43 -> 41;
+// S=4096, tiles of 512, 16 heads of 64 127 -> 117; tiles of 1024, 32 heads of 128 268 -> 258). Blocks, before and with this:
 // S=1024, eight heads of 64 76 -> 41 us; S=4096, 16 heads of 64 216 -> 141; S=32768, 32 heads of 128 9310 -> 9050.
 int run_stream_alone(Run& r, char* output, efa_run_stats* st)
 {

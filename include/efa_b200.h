@@ -120,7 +120,12 @@ int efa_convert_f32_to_f16(const float* in, void* out, size_t n, void* stream);
 /* project (attn_main.cuh:62-65, attn_main.cu:262-273) for the fp16 data path:
  * out[rows][d] = O_tile[rows][d_local] * W_O[d_local][d], fp16 operands, fp32 accumulate, fp16 out.
  * rows must be a multiple of 64, d_local a multiple of 16, d a multiple of 64. out: any 16-byte aligned memory that the
- * GPU may write (its own, mapped host memory, managed memory, a peer's). */
+ * GPU may write (its own, mapped host memory, managed memory, a peer's).
+ * The sum over d_local is taken in one go or, where there are few rows and columns, in 2, 4 or 8 parts that are added in order (fp32
+ * throughout). Which of them depends on rows, d_local, d and the number of SMs only: a call repeated gives the same bits, but a row
+ * may differ in its rounding between calls of different `rows`, and from what the run modes give for it, which never take parts.
+ * Parts occupy several neighbouring SMs at a time: much faster on an idle GPU, slower than one part beside a kernel that holds
+ * every SM (128 x 4096 x 4096: 25 -> 12 us idle, 59 -> 75 beside an attention launch). */
 int efa_project_f16(const void* O_tile, const void* W_O, void* out,
                     int rows, int d_local, int d, void* stream);
 
@@ -128,8 +133,8 @@ int efa_project_f16(const void* O_tile, const void* W_O, void* out,
  * per local head h, Q_h[S][d_h] = X[S][d] * W_q_h[d][d_h] (and K, V alike) with the projection kernel,
  * fp32 accumulate, written as fp16 head-major [H_local][S][d_h] directly (the reference computes in
  * fp32 with cuBLAS and converts in a second pass). X fp16 [S][d]; W_q/W_k/W_v fp16 [H_local][d][d_h].
- * d_h must be 64 or 128, S a multiple of 64, d a multiple of 16; outputs as for efa_project_f16. Untimed in the
- * reference. */
+ * d_h must be 64 or 128, S a multiple of 64, d a multiple of 16; outputs and parts of the sum over d as for efa_project_f16, with
+ * S rows and 3 * H_local * d_h columns. Untimed in the reference. */
 int efa_compute_qkv_f16(const void* X, const void* W_q, const void* W_k, const void* W_v,
                         void* Qh, void* Kh, void* Vh, int S, int d, int H_local, int d_h, void* stream);
 
@@ -180,7 +185,10 @@ typedef struct efa_params {
     int reduce;                 /* EFA_REDUCE_* */
     int group_tiles;            /* stream mode, NCCL reduction: consecutive tiles handled by one projection +
                                    AllReduce launch (each tile's counter is still waited on). 1 = the reference's
-                                   per-tile schedule; 0 = automatic (about S/8 rows per launch). */
+                                   per-tile schedule; 0 = automatic: about S/8 rows per launch; on one rank that writes
+                                   `output` itself and has no residual, with row_order, band_rows, reserve_sms and trace at their
+                                   defaults, no groups at all: the projection follows the attention on its stream, in one
+                                   launch (one per tile where a tile is more than S/16 rows), without counters. */
     int proj_f32;               /* 0 (default): the projection rounds its fp32 accumulator to fp16, the reduction sums
                                    fp16 and `output` is fp16. 1: partial sums, reduction and `output` are fp32 — the
                                    reference's types (attn_main.cu:262-273, run_drivers.cu:26-30), whose own --proj switch
@@ -193,14 +201,17 @@ typedef struct efa_params {
                                    a rush at the end. EFA_ROWS_MIXED (causal, strict row order) = two blocks from the end, one
                                    from the start, and so on: rows complete at a steady rate from both ends and the launch
                                    still ends on middle-weight items. AUTO = descending for a causal problem on one rank,
-                                   else ascending. */
+                                   else ascending; on one rank without groups (see group_tiles) whole heads in turn, last rows
+                                   first if causal. Any other value makes one rank work in groups. */
     int reduce_ctas;            /* thread blocks of the persistent kernel (P2P), 0 = chosen from the FLOP shares */
     int band_rows;              /* stream mode: rows within which the attention kernel may take its work head by head
-                                   instead of in strict row order (K/V reuse in L2); 0 = chosen by efa_stream_plan,
-                                   -1 = strict row order */
+                                   instead of in strict row order (K/V reuse in L2); 0 = chosen by efa_stream_plan (whole heads
+                                   on one rank without groups), -1 = strict row order */
     int reserve_sms;            /* stream mode, diagnostics: > 0 runs the attention kernel in its persistent form and
                                    leaves that many SMs without an attention CTA */
-    int trace;                  /* stream mode, diagnostics: 1 prints the timeline of the groups on stderr */
+    int trace;                  /* stream mode, diagnostics: 1 prints the timeline of the groups on stderr. A traced run always
+                                   works in groups, also on one rank, where an untraced one may not (see group_tiles): it
+                                   is then not the timeline of the untraced run. */
     int wire;                   /* element type of the partial sums that cross the links (NCCL and NVLS reductions):
                                    EFA_WIRE_F16 = the projection rounds its accumulator to fp16 and the reduction sums those
                                    (fp32 accumulation in the NVSwitch; one fp16 rounding per hop in NCCL) - half the bytes,
@@ -230,7 +241,9 @@ int efa_blocks_per_tile(const efa_params* p);
  * rows per group and the eighth that completes last cut into S/16, S/32, S/32, so that what remains after the
  * attention kernel ends is small. *band_rows (if not NULL): the band within which the attention kernel may take
  * its work head by head instead of in strict row order, 0 = strict order: bands are used when the K and V of all
- * local heads exceed what the L2 holds, and never exceed the smallest group. Host arithmetic only.
+ * local heads exceed what the L2 holds, and never exceed the smallest group. On one rank with everything at its default
+ * (see group_tiles) stream mode does not work in groups, and the plan is that of the same run with trace, a residual or an output
+ * that the projection cannot write itself. Host arithmetic only.
  * Returns the number of groups (groups may be NULL to count them), -1 on error. */
 typedef struct efa_stream_group { int first_tile, ntiles; } efa_stream_group;
 int efa_stream_plan(const efa_params* p, efa_stream_group* groups, int capacity, int* band_rows, int* descending);

@@ -203,3 +203,23 @@ def test_compute_qkv_by_parts_of_k_into_mapped_host_memory(pkg, torch_cuda, S, d
         assert bool((o[:-64] == d).all()) and torch.isnan(o[-64:]).all()
     with pytest.raises(pkg.EfaError, match="16-byte"):
         pkg.compute_qkv(X, *W, host[0], host[1].view(-1)[1:], host[2], S, d, H_local, d_h)
+
+
+# Eight, four and two parts of k.
+@pytest.mark.parametrize("rows,d_local,d", [(64, 4080, 64), (192, 1040, 448), (1984, 2512, 448)])
+def test_parts_of_k_give_the_same_bits_every_time(pkg, torch_cuda, rows, d_local, d):
+    """Whatever the stream and whatever runs beside, a call of the same sizes adds the parts in the same order."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    A = torch.randn(rows, d_local, generator=g, device="cuda").to(torch.float16)
+    W = (torch.randn(d_local, d, generator=g, device="cuda") / d ** 0.5).to(torch.float16)
+    outs = [torch.full((rows, d), float("nan"), dtype=torch.float16, device="cuda") for _ in range(8)]
+    streams = [torch.cuda.Stream(priority=-(i & 1)) for i in range(4)]
+    big = torch.randn(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        with torch.cuda.stream(streams[(i + 1) % 4]):
+            torch.mm(big, big)
+        pkg.project(A, W, out, rows, d_local, d, streams[i % 4])
+    torch.cuda.synchronize()
+    assert torch.isfinite(outs[0]).all() and all(torch.equal(o, outs[0]) for o in outs)

@@ -25,6 +25,7 @@ struct FaArgs {
                             // (device memory, one entry per block); nullptr = first to last (or last to first, below)
     int     tail_first = -1, tail_total = 0;   // >= 0: the launch covers, as 128-row items, the 256-row items of a launch of tail_total from this one on
     float   rescale_above;  // log2 units by which a row maximum may outgrow the exponent offset in use
+    int     group_heads = 0; // > 0 (no counters, causal): longest items first over groups of so many heads (work_order.h)
     int     heavy_first;    // take the row blocks (or bands) from the last to the first; with a causal
                             // mask the last rows sweep the most keys, so the longest items start first
 };

@@ -96,6 +96,22 @@ __global__ void f32_to_f16_kernel(const float* __restrict__ in, __half* __restri
 // entry do not: 2 to 8 % less error against float64 (d_h 32, 4032 keys: 1.94e-4 against 2.07e-4, 2-norm).
 constexpr float kRescaleLag = 8.f;
 
+// Heads that a causal launch without counters takes together, longest items first (work_order.h). One head after another, each from its
+// last rows, ends on the long items of the last head; row by row over all heads ends on short ones, but all heads' K and V are then live at
+// once. So as many as keep theirs in half of the L2, in groups of one size: heads in turn before, in groups now (us): S=8192,
+// 16 heads of 64 241 -> 191; S=16384, 16 heads of 64 787 -> 709; S=4096, 16 heads of 64 83.5 -> 53.7; S=8192, 32 heads of 128 540 -> 522; S=32768,
+// four heads of 128 928 -> 905; S=16384, four heads of 64 in four splits with the merge 252 -> 220. Groups of 24 or 140 MB are the same but
+// for 32 heads of 128 (560, 540). Finding an item takes two steps per split, hence the limit to those.
+constexpr size_t kGroupBytes = 64u << 20;
+int heads_together(const efa_flash_params& p)
+{
+    if (!p.causal || p.split > 16) return 0;
+    const size_t head_bytes = (size_t)p.S * p.d_h * 2 * sizeof(__half);
+    const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)p.H_local, kGroupBytes / head_bytes));
+    const int groups = (p.H_local + most - 1) / most;
+    return (p.H_local + groups - 1) / groups;
+}
+
 // Tensor maps depend only on (pointer, S, H_local, d_h); drivers launch the same tensors over and over.
 struct TmapKey {
     const void* ptr; int S, H, D, rows;
@@ -197,9 +213,10 @@ int fa_forward(const void* Q, const void* K, const void* V, void* O, int o_dtype
     a.status = kernel_status_word();
     a.band_blocks = (tile_counters == nullptr) ? (q_rows + 255) / 256 : band_rows / 256;
     // Nobody waits for particular rows of a launch without counters, so under a causal mask its longest work
-    // items (the last rows) go first and the launch ends on short ones; with counters the caller says in which
+    // items go first and the launch ends on short ones; with counters the caller says in which
     // order it will wait for them (first rows first unless told otherwise).
     a.order_tab = order_tab;
+    if (tile_counters == nullptr && order_tab == nullptr && heavy_first < 0) a.group_heads = heads_together(p);
     a.heavy_first = heavy_first >= 0 ? (heavy_first ? 1 : 0) : ((tile_counters == nullptr && p.causal) ? 1 : 0);
 
     if (launches) {
@@ -340,6 +357,7 @@ int fa_forward_noalloc(const void* Q, const void* K, const void* V, void* O, int
     a.band_blocks = (q_rows + 255) / 256;
     a.order_tab = nullptr;
     a.heavy_first = p.causal ? 1 : 0;
+    a.group_heads = heads_together(p);
 
     const int rc = fa_forward_ws(tq, tk, tv, a, p.d_h, o_dtype == EFA_F16, 0, stream);
     if (rc) return rc;

@@ -51,6 +51,7 @@
 #include "fa_args.cuh"
 #include "host_util.h"
 #include "sm100_ptx.cuh"
+#include "work_order.h"
 
 #include <cmath>
 
@@ -195,7 +196,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_word;
     __shared__ int half_done[2][2];                       // [tile][64-row half]: warps that finished their stores
-    __shared__ int s_item;
+    __shared__ int s_item, s_head, s_split, s_row0;       // the work item
 
     const int tid  = threadIdx.x;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // known to be one value for the warp
@@ -219,12 +220,11 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     const int kv_len = a.kv_len;
 
     struct ItemInfo { int head, split, block_row0, kv_lo, kv_hi, nblk_max; int q_abs0[2], rows_q[2], nblk[2]; };
-    // Next work item. Thread 0 rebuilds the barriers for every item: all threads are past the previous one.
+    // Next work item. Thread 0 rebuilds the barriers for every item (all threads are past the previous one), thread 32 finds the
+    // item for everybody (the divisions and what they leave in registers were worth 2 % of a launch at d_h 128).
     // Both role branches below call this the same number of times, so its __syncthreads pair up.
     auto fetch_item = [&](int round, ItemInfo& it) -> bool {
-        // ---- next work item; barriers are rebuilt for every item (all threads are past the previous one)
         if (tid == 0) {
-            s_item = PERSIST ? atomicAdd(work_counter, 1) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
             half_done[0][0] = half_done[0][1] = half_done[1][0] = half_done[1][1] = 0;
             if (round > 0) {
                 for (int q = 0; q < 2; q++) { mbar_inval(&q_full[q]); mbar_inval(&s_full[q]); mbar_inval(&s_read[q]); mbar_inval(&p_full[q][0]); mbar_inval(&p_full[q][1]); mbar_inval(&o_done[q]); }
@@ -243,35 +243,46 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], SLOT_USERS); }
             mbar_fence_init();
         }
-        __syncthreads();
-        const int item = PERSIST ? __shfl_sync(0xffffffffu, s_item, 0) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
-        if (item >= items_total || abort_word != 0) return false;
-
-        // Work order. Strict row order (heads fastest) makes every head's K/V stream live at once, far more than
-        // the L2 holds. With bands, the blocks of one band of rows are taken head by head: the CTAs in flight then
-        // share a few heads' K/V, and rows still complete band by band, which is all a consumer that handles
-        // groups of tiles needs.
-        int item_x, item_y;
-        {
-            const bool tail = KSPLIT && a.tail_first >= 0;         // halves of the 256-row items from tail_first on
-            const int units = tail ? a.tail_total : items_total, unit = tail ? a.tail_first + item / 2 : item;
-            const int items_y = units / items_x;
-            const int band_items = a.band_blocks * (KSPLIT && !tail ? 2 : 1);
-            const int band = band_items > 1 ? min(band_items, items_y) : 1;
-            const int per_band = items_x * band;
-            const int full = items_y / band;
-            int b = unit / per_band, rem = unit - b * per_band, nb = band;
-            if (b >= full) { b = full; rem = unit - full * per_band; nb = items_y - full * band; }
-            item_x = rem / nb;
-            item_y = b * band + rem % nb;
-            // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
-            // is worth up to one item's duration (a fifth of the launch with four heads per GPU at 32k rows).
-            if (a.order_tab != nullptr && band == 1) item_y = __shfl_sync(0xffffffffu, (int)a.order_tab[item_y], 0);
-            else if (a.heavy_first) item_y = items_y - 1 - item_y;
+        if (tid == 32) {
+            const int item = PERSIST ? atomicAdd(work_counter, 1) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
+            s_item = item;
+            if (item < items_total) {
+                // Causal and nobody waits for particular rows: longest items first over groups of heads (work_order.h). Else strict
+                // row order (heads fastest), which makes every head's K/V stream live at once, far more than the L2 holds, or
+                // bands: the blocks of one band of rows are taken head by head, so that the CTAs in flight share a few heads' K/V,
+                // and rows still complete band by band, which is all a consumer that handles groups of tiles needs.
+                int head, split, item_y;
+                const bool tail = KSPLIT && a.tail_first >= 0;         // halves of the 256-row items from tail_first on
+                if (a.group_heads > 0) {
+                    grouped_item(item, a.H_local, a.nsplit, items_total / items_x, a.group_heads, max(1, kv_len / ITEM_ROWS), head, split, item_y);
+                } else {
+                    const int units = tail ? a.tail_total : items_total, unit = tail ? a.tail_first + item / 2 : item;
+                    const int items_y = units / items_x;
+                    const int band_items = a.band_blocks * (KSPLIT && !tail ? 2 : 1);
+                    const int band = band_items > 1 ? min(band_items, items_y) : 1;
+                    const int per_band = items_x * band;
+                    const int full = items_y / band;
+                    int b = unit / per_band, rem = unit - b * per_band, nb = band;
+                    if (b >= full) { b = full; rem = unit - full * per_band; nb = items_y - full * band; }
+                    const int item_x = rem / nb;
+                    item_y = b * band + rem % nb;
+                    // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
+                    // is worth up to one item's duration (a fifth of the launch with four heads per GPU at 32k rows).
+                    if (a.order_tab != nullptr && band == 1) item_y = a.order_tab[item_y];
+                    else if (a.heavy_first) item_y = items_y - 1 - item_y;
+                    head  = item_x % a.H_local;
+                    split = item_x / a.H_local;
+                }
+                s_head = head;
+                s_split = split;
+                s_row0 = tail ? item_y * 2 * WS_BM + (item & 1) * WS_BM : item_y * ITEM_ROWS;
+            }
         }
-        it.head  = item_x % a.H_local;
-        it.split = item_x / a.H_local;
-        it.block_row0 = KSPLIT && a.tail_first >= 0 ? item_y * 2 * WS_BM + (item & 1) * WS_BM : item_y * ITEM_ROWS;
+        __syncthreads();
+        if (__shfl_sync(0xffffffffu, s_item, 0) >= items_total || abort_word != 0) return false;
+        it.head  = __shfl_sync(0xffffffffu, s_head, 0);
+        it.split = __shfl_sync(0xffffffffu, s_split, 0);
+        it.block_row0 = __shfl_sync(0xffffffffu, s_row0, 0);
         const int rows_valid = min(ITEM_ROWS, a.q_rows - it.block_row0);      // 64, 128, 192 or 256 (in a tail also none)
         it.kv_lo = it.split * kv_len;
         it.kv_hi = it.kv_lo + kv_len;
@@ -623,6 +634,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
 
             // ---- epilogue: this thread's row (warps take this branch as a whole: my_rows is 0, 64 or 128)
             if (ok && (warp & 3) * 32 < my_rows) {
+                const int head = *(volatile int*)&s_head, split = *(volatile int*)&s_split, block_row0 = *(volatile int*)&s_row0;   // not kept in registers through the loop
                 const size_t ld_o = (size_t)a.H_local * D;
                 const size_t orow = (size_t)block_row0 + (KSPLIT ? 0 : q * WS_BM) + row;
                 float mult;

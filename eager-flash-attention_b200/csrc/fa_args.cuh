@@ -5,6 +5,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "work_order.h"
+
 namespace efa {
 
 struct FaArgs {
@@ -35,6 +37,38 @@ __device__ __forceinline__ float ex2(float x)
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Work item `item` of a launch: head, split and first row. tail: 128-row items that are halves of the 256-row ones from a.tail_first on.
+__device__ __forceinline__ void pick_item(int item, const FaArgs& a, int items_x, int items_total, int item_rows, bool tail,
+                                          int& head, int& split, int& row0)
+{
+    // Causal and nobody waits for particular rows: longest items first over groups of heads (work_order.h). Else strict
+    // row order (heads fastest), which makes every head's K/V stream live at once, far more than the L2 holds, or
+    // bands: the blocks of one band of rows are taken head by head, so that the CTAs in flight share a few heads' K/V,
+    // and rows still complete band by band, which is all a consumer that handles groups of tiles needs.
+    int item_y;
+    if (a.group_heads > 0) {
+        grouped_item(item, a.H_local, a.nsplit, items_total / items_x, a.group_heads, max(1, a.kv_len / item_rows), head, split, item_y);
+    } else {
+        const int units = tail ? a.tail_total : items_total, unit = tail ? a.tail_first + item / 2 : item;
+        const int items_y = units / items_x;
+        const int band_items = a.band_blocks * (item_rows == 128 && !tail ? 2 : 1);
+        const int band = band_items > 1 ? min(band_items, items_y) : 1;
+        const int per_band = items_x * band;
+        const int full = items_y / band;
+        int b = unit / per_band, rem = unit - b * per_band, nb = band;
+        if (b >= full) { b = full; rem = unit - full * per_band; nb = items_y - full * band; }
+        const int item_x = rem / nb;
+        item_y = b * band + rem % nb;
+        // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
+        // is worth up to one item's duration (a fifth of the launch with four heads per GPU at 32k rows).
+        if (a.order_tab != nullptr && band == 1) item_y = a.order_tab[item_y];
+        else if (a.heavy_first) item_y = items_y - 1 - item_y;
+        head  = item_x % a.H_local;
+        split = item_x / a.H_local;
+    }
+    row0 = tail ? item_y * 256 + (item & 1) * 128 : item_y * item_rows;
 }
 
 // Warp-specialised kernel (fa_fwd_ws_sm100.cu).

@@ -2,12 +2,8 @@
 // Stands in for flash_attn_tc_kernel (flash_attn_tc.cu:73-312 of eager-flash-attention) behind the same launch
 // interface: same tensor layouts, split-KV partial format (row max in the log2 domain) and completion counters.
 //
-// Described for two tiles of d_h = 64 or 128. Small heads (AHEAD) and few rows (KSPLIT) use it with the differences
-// stated at those two constants. Against a kernel of one tile per block (fa_fwd_tile_sm100.cu, which keeps the small heads'
-// launches of few keys): 4032 rows of eight heads of 32, 71.5 -> 61.4 us; 128 rows against 16384 keys in eight splits (16
-// heads of 64), 55 -> 42.5 us. Both figures with the row maximum itself as the exponent offset (58.6 and 41.2 under a
-// lagging one, at 6 and 3 % more error), and with the wait for P*V and the rescaling behind the first half's exponentials
-// (63.7 and 43.0 before them).
+// Two kernels of one name: this one for d_h = 128, where the tensor pipe and the exponentials are about even (and for d_h = 64 in the persistent
+// form), and that of four chains for d_h 16, 32 and 64 (fa_fwd_chains.cuh). Few rows (KSPLIT) use it with the differences stated there.
 //
 // One CTA = 256 query rows (two 128-row Q tiles) of one (head, split), 384 threads:
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
@@ -34,7 +30,7 @@
 // registers, with its exponentials under the offset in use while the maximum is still being found: the halves'
 // MMAs fetch Q twice (d_h = 128, S = 32768, four heads, causal: 1.27 ms against 1.02).
 // Tensor memory (512 columns): S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+D) O1 [384,384+D).
-// O is rescaled in tensor memory by the softmax warps themselves, and for d_h 64 and 128 only when a row maximum grew
+// O is rescaled in tensor memory by the softmax warps themselves, and at d_h 64 and 128 only when a row maximum grew
 // by more than 2^8 since the value last used as the exponent offset (P then stays below 256, well
 // inside fp16); the final division by the row sum makes the result independent of the offset.
 // P reaches the MMA warp in two 64-key halves, each on its own mbarrier, so the first four k-steps of
@@ -51,8 +47,8 @@
 #include "fa_args.cuh"
 #include "host_util.h"
 #include "sm100_ptx.cuh"
-#include "work_order.h"
 
+#include <algorithm>
 #include <cmath>
 
 namespace efa {
@@ -66,7 +62,8 @@ constexpr float kNegInfW = -INFINITY;
 
 template <int D, bool KSPLIT>
 struct WsCfg {
-    static constexpr int SWB        = D >= 64 ? 128 : D * 2;      // swizzle width = TMA box row, bytes
+    static_assert(D == 128 || (D == 64 && !KSPLIT), "smaller heads take the kernel of four chains");
+    static constexpr int SWB        = 128;                        // swizzle width = TMA box row, bytes
     static constexpr int BOXC       = SWB / 2;
     static constexpr int NBOX       = D / BOXC;
     static constexpr int BOX_BYTES  = 128 * SWB;
@@ -149,6 +146,11 @@ __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x)
 
 __device__ __forceinline__ void setmaxnreg_dec_56() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
 __device__ __forceinline__ void setmaxnreg_inc_224() { asm volatile("setmaxnreg.inc.sync.aligned.u32 224;"); }
+__device__ __forceinline__ void setmaxnreg_dec_40() { asm volatile("setmaxnreg.dec.sync.aligned.u32 40;"); }
+__device__ __forceinline__ void setmaxnreg_dec_24() { asm volatile("setmaxnreg.dec.sync.aligned.u32 24;"); }
+__device__ __forceinline__ void setmaxnreg_inc_104() { asm volatile("setmaxnreg.inc.sync.aligned.u32 104;"); }
+
+#include "fa_fwd_chains.cuh"
 
 // PERSIST = false: one work item (256 rows of one head/split) per CTA, grid (H_local*split, row blocks).
 // PERSIST = true: a 1-D grid of fewer CTAs than SMs; each CTA takes work items from a global counter in
@@ -169,19 +171,11 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     constexpr uint32_t IDESC_QK = idesc_f16_f32(WS_BM, WS_BN, 0, 0);
     constexpr uint32_t IDESC_PV = idesc_f16_f32(WS_BM, D, 0, 1);
     constexpr int NSK = C::NSTAGE_K, NSV = C::NSTAGE_V;
-    // P in tensor-memory columns of its own (they fit beside S and O up to D = 64), so that Q*K^T runs a stage ahead of
-    // the softmax. Taken where there is one chain per tile and nothing alternates with it. With two tiles of D = 64 it
-    // gives little (1.5 % on long launches, S = 65536, two heads: 2.67 -> 2.63 ms; split ones 0.3 % slower): the special-function
-    // unit is busy 75 to 84 % of a working SM's time already, and tiles that end together store together.
-    constexpr bool AHEAD = D < 64 || (KSPLIT && D == 64);
-    constexpr int ISSUERS = AHEAD || KSPLIT ? 2 : 1;    // issuing threads: one per tile where the tiles need not alternate
-    constexpr int SLOT_USERS = AHEAD && !KSPLIT ? 2 : 1; // issuers that read one K/V slot
-    // Every fourth pair of exponentials as a polynomial where one tile's chain is what an item waits for and the special-function
-    // unit has time to spare: d_h 128 (S = 32768, four heads, causal 1008 -> 1000 us; 2048 rows, eight heads 25.3 -> 24.5; ten heads x
-    // 8192 rows 310 -> 302) and 128-row items of small heads (1024 rows, eight heads of 32 11.0 -> 10.6). Elsewhere the instructions
-    // cost more than the unit gains (65536 rows, two heads of 64 2666 -> 2836; 4032 rows, eight heads of 32 56.4 -> 60.4; 128-row
-    // items of 64 -2 % in a single wave, +2 % behind full ones); a third of the pairs is worse everywhere (d_h 128: +3 %).
-    constexpr bool POLY = D == 128 || (KSPLIT && D < 64);
+    constexpr int ISSUERS = KSPLIT ? 2 : 1;             // issuing threads: one per warpgroup where the tiles need not alternate
+    // Every fourth pair of exponentials as a polynomial at d_h 128, where one tile's chain is what an item waits for and the special-function
+    // unit has time to spare: S = 32768, four heads, causal 1008 -> 1000 us; 2048 rows, eight heads 25.3 -> 24.5; ten heads x 8192 rows
+    // 310 -> 302; a third of the pairs is worse (+3 %).
+    constexpr bool POLY = D == 128;
     constexpr int ITEM_ROWS = KSPLIT ? WS_BM : 2 * WS_BM;
 
     extern __shared__ uint8_t smem_raw[];
@@ -192,7 +186,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
 
     __shared__ __align__(8) uint64_t q_full[2];
     __shared__ __align__(8) uint64_t k_full[NSK], k_empty[NSK], v_full[NSV], v_empty[NSV];
-    __shared__ __align__(8) uint64_t s_full[2], s_read[2], p_full[2][2], o_done[2];
+    __shared__ __align__(8) uint64_t s_full[2], p_full[2][2], o_done[2];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_word;
     __shared__ int half_done[2][2];                       // [tile][64-row half]: warps that finished their stores
@@ -227,55 +221,31 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
         if (tid == 0) {
             half_done[0][0] = half_done[0][1] = half_done[1][0] = half_done[1][1] = 0;
             if (round > 0) {
-                for (int q = 0; q < 2; q++) { mbar_inval(&q_full[q]); mbar_inval(&s_full[q]); mbar_inval(&s_read[q]); mbar_inval(&p_full[q][0]); mbar_inval(&p_full[q][1]); mbar_inval(&o_done[q]); }
+                for (int q = 0; q < 2; q++) { mbar_inval(&q_full[q]); mbar_inval(&s_full[q]); mbar_inval(&p_full[q][0]); mbar_inval(&p_full[q][1]); mbar_inval(&o_done[q]); }
                 for (int s = 0; s < NSK; s++) { mbar_inval(&k_full[s]); mbar_inval(&k_empty[s]); }
                 for (int s = 0; s < NSV; s++) { mbar_inval(&v_full[s]); mbar_inval(&v_empty[s]); }
             }
             for (int q = 0; q < 2; q++) {
                 mbar_init(&q_full[q], 1);
                 mbar_init(&s_full[q], 1);
-                mbar_init(&s_read[q], WS_BM / 32);
                 mbar_init(&p_full[q][0], WS_BM / 32);
                 mbar_init(&p_full[q][1], WS_BM / 32);
                 mbar_init(&o_done[q], 1);
             }
-            for (int s = 0; s < NSK; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], SLOT_USERS); }
-            for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], SLOT_USERS); }
+            for (int s = 0; s < NSK; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+            for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
             mbar_fence_init();
         }
         if (tid == 32) {
             const int item = PERSIST ? atomicAdd(work_counter, 1) : (int)(blockIdx.y * gridDim.x + blockIdx.x);
             s_item = item;
             if (item < items_total) {
-                // Causal and nobody waits for particular rows: longest items first over groups of heads (work_order.h). Else strict
-                // row order (heads fastest), which makes every head's K/V stream live at once, far more than the L2 holds, or
-                // bands: the blocks of one band of rows are taken head by head, so that the CTAs in flight share a few heads' K/V,
-                // and rows still complete band by band, which is all a consumer that handles groups of tiles needs.
-                int head, split, item_y;
-                const bool tail = KSPLIT && a.tail_first >= 0;         // halves of the 256-row items from tail_first on
-                if (a.group_heads > 0) {
-                    grouped_item(item, a.H_local, a.nsplit, items_total / items_x, a.group_heads, max(1, kv_len / ITEM_ROWS), head, split, item_y);
-                } else {
-                    const int units = tail ? a.tail_total : items_total, unit = tail ? a.tail_first + item / 2 : item;
-                    const int items_y = units / items_x;
-                    const int band_items = a.band_blocks * (KSPLIT && !tail ? 2 : 1);
-                    const int band = band_items > 1 ? min(band_items, items_y) : 1;
-                    const int per_band = items_x * band;
-                    const int full = items_y / band;
-                    int b = unit / per_band, rem = unit - b * per_band, nb = band;
-                    if (b >= full) { b = full; rem = unit - full * per_band; nb = items_y - full * band; }
-                    const int item_x = rem / nb;
-                    item_y = b * band + rem % nb;
-                    // Longest items first: list scheduling then ends on the shortest items instead of the longest, which
-                    // is worth up to one item's duration (a fifth of the launch with four heads per GPU at 32k rows).
-                    if (a.order_tab != nullptr && band == 1) item_y = a.order_tab[item_y];
-                    else if (a.heavy_first) item_y = items_y - 1 - item_y;
-                    head  = item_x % a.H_local;
-                    split = item_x / a.H_local;
-                }
+                const bool tail = KSPLIT && a.tail_first >= 0;
+                int head, split, row0;
+                pick_item(item, a, items_x, items_total, ITEM_ROWS, tail, head, split, row0);
                 s_head = head;
                 s_split = split;
-                s_row0 = tail ? item_y * 2 * WS_BM + (item & 1) * WS_BM : item_y * ITEM_ROWS;
+                s_row0 = row0;
             }
         }
         __syncthreads();
@@ -342,9 +312,8 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 // covers what the thread that executes it has issued. Descriptors as (low, high) words; a k-step or a ring
                 // slot only moves the address field of the low word.
                 // A commit costs this warp 200 to 300 cycles (time stamps: 630 of a period of 3284 at d_h 128 and of 2968 at d_h 64 went
-                // into two of them, while a P was waiting), so there is one per tile and stage (s_full; with P in its own
-                // columns also o_done). S = 65536, two heads of 64: 2903 -> 2830 us; S = 32768, four heads of 128, causal: 1035 -> 1002;
-                // 4032 rows, eight heads of 32: 59.3 -> 55.2. Ring slots are given back by the softmax warps that see it: S(j) complete means
+                // into two of them, while a P was waiting), so there is one per tile and stage (s_full): S = 32768, four heads of 128,
+                // causal, 1035 -> 1002 us. Ring slots are given back by the softmax warps that see it: S(j) complete means
                 // that all that was issued before is, QK(j) and PV(j-1) of both tiles among it.
                 const uint64_t dq0 = smem_desc(smem_u32(sQ), 16, 8 * C::SWB, SWZ);
                 const uint64_t dk0 = smem_desc(smem_u32(sK), 16, 8 * C::SWB, SWZ);
@@ -372,7 +341,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 };
                 auto issue_pv = [&](int q, int slot, uint32_t acc0, int half, bool last) {
                     const uint32_t va = dv_lo + (uint32_t)slot * (C::TILE_BYTES >> 4);
-                    const uint32_t tP = tmem_base + (AHEAD ? 320 : 0) + q * 128, tO = tmem_base + 256 + q * 128;
+                    const uint32_t tP = tmem_base + q * 128, tO = tmem_base + 256 + q * 128;
                     if (elect_one()) {
                         #pragma unroll
                         for (int ks = half * 4; ks < half * 4 + 4; ks++)
@@ -387,12 +356,11 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     const int n = KSPLIT ? (nblk[0] + 1 - q) / 2 : q ? nblk[1] : nblk[0];      // stages with work for this tile
                     auto stage = [&](int i) { return KSPLIT ? 2 * i + q : i; };
                     if (n > 0) ok = wait(&q_full[KSPLIT ? 0 : q], 0, 24);
-                    // S(i) = Q K^T of stage i. With P in columns of its own, S(i - 1) only has to be in registers.
+                    // S(i) = Q K^T of stage i.
                     auto step_qk = [&](int i) -> bool {
                         if (i >= n) return true;
                         const int j = stage(i), sk = j % NSK;
                         if (!wait(&k_full[sk], j / NSK, 27)) return false;
-                        if (AHEAD && i > 0 && !wait(&s_read[q], i - 1, 23)) return false;
                         issue_qk(q, sk);
                         return true;
                     };
@@ -402,12 +370,12 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                         if (!wait(&p_full[q][0], i, 26)) return false;
                         issue_pv(q, sv, i > 0 ? 1u : 0u, 0, false);
                         if (!wait(&p_full[q][1], i, 29)) return false;
-                        issue_pv(q, sv, 1u, 1, AHEAD || i == n - 1);
+                        issue_pv(q, sv, 1u, 1, i == n - 1);
                         return true;
                     };
                     ok = ok && step_qk(0);
                     for (int i = 0; i < n && ok; i++)
-                        ok = AHEAD ? step_qk(i + 1) && step_pv(i) : step_pv(i) && step_qk(i + 1);
+                        ok = step_pv(i) && step_qk(i + 1);
                 } else {
                     if (nblk_max > 0) {
                         ok = wait(&k_full[0], 0, 23);
@@ -452,20 +420,13 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             const int row = tid - q * WS_BM;
             const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
             const uint32_t tmem_S = tmem_base + q * 128 + lane_base;
-            const uint32_t tmem_P = tmem_S + (AHEAD ? 320 : 0);
             const uint32_t tmem_O = tmem_base + 256 + q * 128 + lane_base;
             const int my_rows = q ? rows_q[1] : rows_q[0];
             const int my_nblk = KSPLIT ? (nblk[0] + 1 - q) / 2 : q ? nblk[1] : nblk[0];
             const int my_abs0 = q ? q_abs0[1] : q_abs0[0];
-            // Who gives ring slots back: with an issuer per tile each tile for its part (one that has the slots to itself for
-            // both), else the tile that is issued last. Tile 1 sweeps at most one stage more than tile 0, its very last one, whose slots
-            // nothing waits for.
+            // Who gives ring slots back: with an issuer per warpgroup each for its part, else the tile that is issued last. Tile 1 sweeps at most
+            // one stage more than tile 0, its very last one, whose slots nothing waits for.
             const bool gives_back = (warp & 3) == 0 && lane == 0 && (ISSUERS == 2 || q == (nblk[1] > 0 ? 1 : 0));
-            const bool both_parts = SLOT_USERS == 2 && (nblk[0] == 0 || nblk[1] == 0);
-            auto give_back = [&](uint64_t* bar) {
-                mbar_arrive(bar);
-                if (both_parts) mbar_arrive(bar);
-            };
             auto stage_of = [&](int j) { return KSPLIT ? 2 * j + q : j; };
 
             float m_ref = kNegInfW;     // exponent offset in use (a past row maximum), scaled by scale*log2(e)
@@ -479,19 +440,14 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (gives_back) {
-                    give_back(&k_empty[stage_of(j) % NSK]);
-                    if (!AHEAD && j > 0) give_back(&v_empty[stage_of(j - 1) % NSV]);
+                    mbar_arrive(&k_empty[stage_of(j) % NSK]);
+                    if (j > 0) mbar_arrive(&v_empty[stage_of(j - 1) % NSV]);
                 }
 
                 uint32_t su[4][32];
                 #pragma unroll
                 for (int c = 0; c < 4; c++) tmem_ld32(tmem_S + c * 32, su[c]);
                 tmem_wait_ld();
-                if constexpr (AHEAD) {                       // S(j) is in registers: its columns may take S(j+1)
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&s_read[q]);
-                }
 
                 const bool need_mask = (kb + WS_BN > kv_hi) || (a.causal && kb + WS_BN - 1 > my_abs0);
                 if (need_mask) {
@@ -549,44 +505,25 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                     }
                 };
                 uint32_t pk[2][16];
-                if constexpr (AHEAD) { weights(0, pk[0]); weights(1, pk[1]); }
 
-                // O may be rescaled and P overwritten once PV(j-1) of this tile is complete: no part of PV(j) is issued
-                // before this warp's first arrival below. With P in S's columns, S(j) complete implies it (the
-                // tensor pipe runs in issue order); with Q*K^T a stage ahead it is waited for, behind the first half's exponentials.
-                if constexpr (AHEAD) {
-                    if (j > 0) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], (uint32_t)((j - 1) & 1), &abort_word, 33));
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        if (gives_back) give_back(&v_empty[stage_of(j - 1) % NSV]);
-                    }
-                }
+                // O may be rescaled and P overwritten once PV(j-1) of this tile is complete, which S(j) complete implies (the tensor pipe
+                // runs in issue order): no part of PV(j) is issued before this warp's first arrival below.
                 if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                    if constexpr (D >= 32) {
-                        #pragma unroll
-                        for (int c = 0; c < D / 32; c++) {
-                            uint32_t o[32];
-                            tmem_ld32(tmem_O + c * 32, o);
-                            tmem_wait_ld();
-                            #pragma unroll
-                            for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                            tmem_st32(tmem_O + c * 32, o);
-                        }
-                    } else {
-                        uint32_t o[16];
-                        tmem_ld16(tmem_O, o);
+                    #pragma unroll
+                    for (int c = 0; c < D / 32; c++) {
+                        uint32_t o[32];
+                        tmem_ld32(tmem_O + c * 32, o);
                         tmem_wait_ld();
                         #pragma unroll
-                        for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st16(tmem_O, o);
+                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st32(tmem_O + c * 32, o);
                     }
                 }
 
                 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    if (!AHEAD || c >= 2) weights(c, pk[c & 1]);
-                    tmem_st16(tmem_P + c * 16, pk[c & 1]);
+                    weights(c, pk[c & 1]);
+                    tmem_st16(tmem_S + c * 16, pk[c & 1]);
                     if (c == 1 || c == 3) {
                         tmem_wait_st();
                         tc_fence_before_sync();
@@ -606,7 +543,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
             }
 
             if (ok && my_nblk > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], AHEAD ? (uint32_t)((my_nblk - 1) & 1) : 0u, &abort_word, 32));
+                ok = __all_sync(0xffffffffu, mbar_wait(&o_done[q], 0u, &abort_word, 32));
                 tc_fence_after_sync();
             }
 
@@ -629,8 +566,8 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 l_run = l_run * w_own + l_o * w_other;
                 m_ref = m_all;
             }
-            // Columns [c_lo, c_hi) in steps of 16 (D = 16: the first warpgroup takes the one step).
-            const int c_lo = KSPLIT && q == 1 ? (D + 16) / 32 : 0, c_hi = KSPLIT && q == 0 ? (D + 16) / 32 : D / 16;
+            // Columns [c_lo, c_hi) in steps of 16.
+            const int c_lo = KSPLIT && q == 1 ? D / 32 : 0, c_hi = KSPLIT && q == 0 ? D / 32 : D / 16;
 
             // ---- epilogue: this thread's row (warps take this branch as a whole: my_rows is 0, 64 or 128)
             if (ok && (warp & 3) * 32 < my_rows) {
@@ -734,6 +671,18 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (behind) pdl_wait();
 }
 
+// The registers that the softmax warps take come out of what the block was launched with: with less than that they would wait for
+// ever, so it is looked at before the first launch.
+template <int D, bool OUT_F16, int WAYS>
+int configure_chains()
+{
+    cudaFuncAttributes attr;
+    EFA_CUDA(cudaFuncGetAttributes(&attr, fa_fwd_ws_kernel<D, OUT_F16, WAYS>));
+    if ((attr.numRegs + 7) / 8 * 8 * CH_THREADS < 512 * 104 + 128 * 40 + 128 * 24) { set_error("attention kernel compiled to %d registers", attr.numRegs); return 1; }
+    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, WAYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainCfg<D, WAYS>::SMEM_BYTES));
+    return 0;
+}
+
 // The first launch of a head size and output type on a device loads and configures every form of it: which one a launch
 // takes depends on its shape, and a later one may be inside a stream capture or find no device memory left.
 template <int D, bool OUT_F16>
@@ -744,69 +693,99 @@ int configure_forms()
     EFA_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || configured[dev]) return 0;
     constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, false>, attr, WsCfg<D, false>::SMEM_BYTES));
-    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, true>, attr, WsCfg<D, true>::SMEM_BYTES));
-    if constexpr (D >= 64) {
-        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, true, false>, attr, WsCfg<D, false>::SMEM_BYTES));
-    } else if (fa_tile_preload()) {
-        return 1;
+    if constexpr (D == 128) {
+        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, false>, attr, WsCfg<D, false>::SMEM_BYTES));
+        EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, false, true>, attr, WsCfg<D, true>::SMEM_BYTES));
+    } else {
+        if (configure_chains<D, OUT_F16, 2>() || configure_chains<D, OUT_F16, 4>()) return 1;
     }
+    if constexpr (D >= 64) EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, true, false>, attr, WsCfg<D, false>::SMEM_BYTES));
+    else if (fa_tile_preload()) return 1;
     configured[dev] = true;
     return 0;
 }
 
-template <int D, bool OUT_F16, bool PERSIST, bool KSPLIT = false>
-int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args,
-              int reserve_sms, cudaStream_t stream, int blocks = 0 /* of a 1-D grid; 0: all */)
+template <int D, bool OUT_F16, int WAYS>
+int launch_chains(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args, cudaStream_t stream, int blocks)
+{
+    using C = ChainCfg<D, WAYS>;
+    const int items_x = args.H_local * args.nsplit, rows = C::TILES * WS_BM;
+    const int items_y = (args.q_rows + rows - 1) / rows;
+    const dim3 grid = blocks > 0 ? dim3(blocks) : dim3(items_x, items_y);
+    EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, WAYS>, grid, CH_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, items_x, WAYS == 4 && blocks > 0 ? blocks : items_x * items_y));
+    return 0;
+}
+
+// reserve_sms >= 0: the persistent form on that many SMs less. blocks: of a 1-D grid; 0: all.
+template <int D, bool OUT_F16, bool KSPLIT = false>
+int launch_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args, cudaStream_t stream, int reserve_sms, int blocks)
 {
     using C = WsCfg<D, KSPLIT>;
     const int items_x = args.H_local * args.nsplit;
     const int item_rows = KSPLIT ? WS_BM : 2 * WS_BM;
     const int items_y = (args.q_rows + item_rows - 1) / item_rows;
     const int total = items_x * items_y;
-    if constexpr (PERSIST) {
-        int ctas = device_sms() - reserve_sms;
-        if (ctas < 1) ctas = 1;
-        if (ctas > total) ctas = total;
-        int* counter = work_counter_slot();
-        if (!counter) { set_error("no device memory for the work counter"); return 1; }
-        EFA_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), stream));
-        EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, true, KSPLIT>, dim3(ctas), WS_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, counter, items_x, total));
-    } else {
+    if constexpr (!KSPLIT) {
+        if (reserve_sms >= 0) {
+            const int ctas = std::min(total, std::max(1, device_sms() - reserve_sms));
+            int* counter = work_counter_slot();
+            if (!counter) { set_error("no device memory for the work counter"); return 1; }
+            EFA_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), stream));
+            EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, true, false>, dim3(ctas), WS_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, counter, items_x, total));
+            return 0;
+        }
+    }
+    if constexpr (D == 128) {
         const dim3 grid = blocks > 0 ? dim3(blocks) : dim3(items_x, items_y);
         EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, false, KSPLIT>, grid, WS_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, (int*)nullptr, items_x, KSPLIT && blocks > 0 ? blocks : total));
     }
     return 0;
 }
 
-template <int D>
-int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a, bool out_f16,
-                int reserve_sms, cudaStream_t stream)
+// Items of 256 rows (HALVES: 128); blocks: of a 1-D grid, 0: all.
+template <int D, bool OUT_F16, bool HALVES>
+int launch_items(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& args, cudaStream_t stream, int blocks = 0)
 {
-    if (out_f16 ? configure_forms<D, true>() : configure_forms<D, false>()) return 1;
+    if constexpr (D == 128) return launch_ws<D, OUT_F16, HALVES>(tq, tk, tv, args, stream, -1, blocks);
+    else return launch_chains<D, OUT_F16, HALVES ? 4 : 2>(tq, tk, tv, args, stream, blocks);
+}
+
+template <int D, bool OUT_F16>
+int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a, int reserve_sms, cudaStream_t stream)
+{
+    if (configure_forms<D, OUT_F16>()) return 1;
     if constexpr (D >= 64)
-        if (reserve_sms > 0) return out_f16 ? launch_ws<D, true, true>(tq, tk, tv, a, reserve_sms, stream) : launch_ws<D, false, true>(tq, tk, tv, a, reserve_sms, stream);
+        if (reserve_sms > 0) return launch_ws<D, OUT_F16>(tq, tk, tv, a, stream, reserve_sms, 0);
     const FaPlan plan = fa_ws_plan(a, D, reserve_sms);
-    if (plan.tiles > 0) return fa_forward_tile(tq, tk, tv, a, D, out_f16, stream);
-    if (plan.items256 == 0)
-        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false, true>(tq, tk, tv, a, 0, stream);
+    if (plan.tiles > 0) return fa_forward_tile(tq, tk, tv, a, D, OUT_F16, stream);
+    if (plan.items256 == 0) return launch_items<D, OUT_F16, true>(tq, tk, tv, a, stream);
     if (plan.items128 > 0) {
         FaArgs t = a;
         t.tail_first = plan.items256;
         t.tail_total = plan.items256 + plan.items128 / 2;
-        if (int rc = out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream, t.tail_first) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream, t.tail_first)) return rc;
-        return out_f16 ? launch_ws<D, true, false, true>(tq, tk, tv, t, 0, stream, plan.items128) : launch_ws<D, false, false, true>(tq, tk, tv, t, 0, stream, plan.items128);
+        if (int rc = launch_items<D, OUT_F16, false>(tq, tk, tv, a, stream, t.tail_first)) return rc;
+        return launch_items<D, OUT_F16, true>(tq, tk, tv, t, stream, plan.items128);
     }
-    return out_f16 ? launch_ws<D, true, false>(tq, tk, tv, a, 0, stream) : launch_ws<D, false, false>(tq, tk, tv, a, 0, stream);
+    return launch_items<D, OUT_F16, false>(tq, tk, tv, a, stream);
 }
 
-template <int D, bool KSPLIT>
-void ring_of(FaPlan& plan)
+template <int D>
+int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a, bool out_f16,
+                int reserve_sms, cudaStream_t stream)
 {
-    using C = WsCfg<D, KSPLIT>;
-    plan.k_slots = C::NSTAGE_K;
-    plan.v_slots = C::NSTAGE_V;
-    plan.stage_step = C::STAGE_STEP;
+    return out_f16 ? launch_form<D, true>(tq, tk, tv, a, reserve_sms, stream) : launch_form<D, false>(tq, tk, tv, a, reserve_sms, stream);
+}
+
+template <int D>
+void ring_of(FaPlan& plan, bool halves)
+{
+    if constexpr (D == 128) {
+        plan.k_slots = halves ? WsCfg<D, true>::NSTAGE_K : WsCfg<D, false>::NSTAGE_K;
+        plan.v_slots = halves ? WsCfg<D, true>::NSTAGE_V : WsCfg<D, false>::NSTAGE_V;
+    } else {
+        plan.k_slots = plan.v_slots = ChainCfg<D, 2>::NS;
+    }
+    plan.stage_step = halves ? 2 : 1;
 }
 
 }  // namespace
@@ -814,11 +793,11 @@ void ring_of(FaPlan& plan)
 // Which items a launch goes as. Host arithmetic only.
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
 {
-    // 128-row items with their keys split over the two warpgroups where one wave of them is the whole launch (d_h 16 /
-    // 64 / 128, 74 items of 256 rows and 16 key stages: 20 / 21 / 29 us against 31 / 33 / 37). Three waves of them against
+    // 128-row items with their keys split over all the warpgroups where one wave of them is the whole launch (d_h 16 / 32 /
+    // 64 / 128, 74 items of 256 rows and 16 key stages: 15 / 16 / 19 / 29 us against 25 / 27 / 28 / 37). Three waves of them against
     // two of 256 rows are worth it only where items are long and the tensor pipe is not what an item waits for. In us, 222
-    // items of 256 rows: 51 against 58 (d_h 16, 16 stages), 59 against 63 (64, 16 stages), even at 8 stages (64), 27 against
-    // 25 (64, 4 stages), 82 against 76 (128, 16 stages).
+    // items of 256 rows: 42 / 48 / 54 against 48 / 52 / 55 (d_h 16 / 32 / 64, 16 stages), 26 / 28 / 34 against 28 / 30 / 34 (8 stages), even at
+    // four, 82 against 76 (128, 16 stages).
     const long heads = (long)a.H_local * a.nsplit;
     const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
     const long sms = device_sms();
@@ -843,19 +822,18 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
         plan.items128 = (int)total128;
     // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
     // is at most half of a wave it goes as 128-row items behind the full waves (two of them at least, one at d_h 128: shorter
-    // launches are decided above). A wave of 128-row items takes 0.54 / 0.60 / 0.60 / 0.67 of one of 256 rows (d_h 16 / 32 / 64 /
-    // 128, 32 stages); behind three full waves of 65536 keys, with the second launch, 0.75: 3.13 -> 2.95 ms (d_h 64). From
-    // 4096 keys on, where that is worth ten times a launch: 111 heads x 512 rows of d_h 128 140 -> 133 us.
+    // launches are decided above). 65536 keys, two heads of 64, three full waves and 68 items: 2.75 -> 2.59 ms; 37 heads x 2560 rows x 4096 keys
+    // of d_h 64 / 32 141 -> 128 / 123 us. From 4096 keys on, where that is worth ten times a launch: 111 heads x 512 rows of d_h 128 140 -> 133 us.
     } else if (free_form && !a.causal && total > sms && rest > 0 && rest * 2 <= sms && a.kv_len >= 4096) {
         plan.items256 = (int)(total - rest);
         plan.items128 = (int)rest * 2;
     }
     const bool ks = plan.items128 > 0;
     switch (d_h) {
-        case 16:  ks ? ring_of<16, true>(plan)  : ring_of<16, false>(plan);  break;
-        case 32:  ks ? ring_of<32, true>(plan)  : ring_of<32, false>(plan);  break;
-        case 64:  ks ? ring_of<64, true>(plan)  : ring_of<64, false>(plan);  break;
-        case 128: ks ? ring_of<128, true>(plan) : ring_of<128, false>(plan); break;
+        case 16:  ring_of<16>(plan, ks);  break;
+        case 32:  ring_of<32>(plan, ks);  break;
+        case 64:  ring_of<64>(plan, ks);  break;
+        case 128: ring_of<128>(plan, ks); break;
     }
     return plan;
 }
@@ -889,18 +867,21 @@ template <class K> int touch_kernel(K kernel)
 
 // Loads the code of every instantiation now. A kernel's first launch may otherwise have to wait for the device to go
 // idle, which it never does while a stream sits in a front-end wait on a counter that is not coming.
-template <int D>
+template <int D, bool OUT_F16>
 static int touch_forms()
 {
-    return touch_kernel(fa_fwd_ws_kernel<D, true, false, false>) || touch_kernel(fa_fwd_ws_kernel<D, false, false, false>) ||
-           touch_kernel(fa_fwd_ws_kernel<D, true, false, true>) || touch_kernel(fa_fwd_ws_kernel<D, false, false, true>);
+    if constexpr (D >= 64)
+        if (touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, true, false>)) return 1;
+    if constexpr (D == 128)
+        return touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, false, false>) || touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, false, true>);
+    else
+        return touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, 2>) || touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, 4>);
 }
 
 int fa_ws_preload()
 {
-    return touch_forms<16>() || touch_forms<32>() || touch_forms<64>() || touch_forms<128>() ||
-           touch_kernel(fa_fwd_ws_kernel<64, true, true, false>) || touch_kernel(fa_fwd_ws_kernel<64, false, true, false>) ||
-           touch_kernel(fa_fwd_ws_kernel<128, true, true, false>) || touch_kernel(fa_fwd_ws_kernel<128, false, true, false>);
+    return touch_forms<16, true>() || touch_forms<16, false>() || touch_forms<32, true>() || touch_forms<32, false>() ||
+           touch_forms<64, true>() || touch_forms<64, false>() || touch_forms<128, true>() || touch_forms<128, false>();
 }
 
 }  // namespace efa

@@ -2,11 +2,11 @@
 // one wave. Same arguments, partials and completion counters as fa_fwd_ws_sm100.cu.
 //
 // What bounds such a launch is the turnover of its blocks: tensor-memory allocation, barriers, the Q load, the first Q*K^T and
-// the epilogue of a row block that has only a few 128-key stages. Two of these small blocks share an SM and hide each
-// other's; the kernel of 256 rows has the SM to itself. Its item takes about 4 us and 1.7 a stage, the same rows here 2 us
-// and 2 a stage. Without a mask the line lies at five stages: 222 items of 256 rows, d_h 16, take 14.4 us here against 16.5
-// (2 stages), 20.6 against 22.8 (4), 35 against 34 (8). Under a causal mask the smaller blocks also end more evenly: up to
-// ten stages on average, 16 heads x 2048 rows 37.0 against 49.2 us (d_h 16), 39.0 against 52.0 (d_h 32).
+// the epilogue of a row block that has only one or two 128-key stages. Two of these small blocks share an SM and hide each
+// other's; the kernel of four chains has the SM to itself, but is faster per stage. The line lies at two stages: 592 items of 256 rows, d_h 16 / 32,
+// 8.8 / 9.5 us here against 15.1 / 16.1 (one stage), 23.9 / 26.4 against 24.4 / 27.2 (two), 32.1 / 36.5 against 29.9 / 34.8 (three), 48 / 53 against
+// 41 / 47 (five); causal 200 heads x 256 rows 10.2 / 10.7 against 10.9 / 11.7, 64 heads x 512 rows 11.0 / 11.3 against 8.9 / 9.8, 16 x 2048
+// 32.7 / 34.0 against 16.4 / 17.7 (as 128-row items).
 //
 // One CTA = 128 query rows of one (head, split). K and V stream through shared memory in 128-key stages filled by TMA
 // (32- or 64-byte swizzle). S = Q K^T is a tcgen05.mma with both operands in shared memory and the 128x128 fp32 result

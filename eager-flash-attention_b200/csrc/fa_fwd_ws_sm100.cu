@@ -757,8 +757,8 @@ int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     if constexpr (D >= 64)
         if (reserve_sms > 0) return launch_ws<D, OUT_F16>(tq, tk, tv, a, stream, reserve_sms, 0);
     const FaPlan plan = fa_ws_plan(a, D, reserve_sms);
-    if (plan.tiles > 0) return fa_forward_tile(tq, tk, tv, a, D, OUT_F16, stream);
-    if (plan.items256 == 0) return launch_items<D, OUT_F16, true>(tq, tk, tv, a, stream);
+    if (plan.tiles > 0 && plan.tile_rows == 0) return fa_forward_tile(tq, tk, tv, a, D, OUT_F16, stream);
+    if (plan.items128 > 0 ? plan.items256 == 0 : plan.tile_rows == 128) return launch_items<D, OUT_F16, true>(tq, tk, tv, a, stream);
     if (plan.items128 > 0) {
         FaArgs t = a;
         t.tail_first = plan.items256;
@@ -804,20 +804,31 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     const long waves256 = (total + sms - 1) / sms, waves128 = (total128 + sms - 1) / sms, rest = total % sms;
     const double keys = a.causal ? a.q_start + 0.5 * (a.q_rows + 256) : a.S;
     const double stages = keys / ((double)WS_BN * a.nsplit);                   // of an average item
-    const bool long_items = d_h < 128 && stages >= 8;
     const bool free_form = a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64);
+    // Under a causal mask the longest item can be what a launch takes, and as 128-row items it is half of it. Time as the longer of
+    // the longest item and everything spread over the SMs, in stages of 256 rows; an item costs two of them besides, and 128 rows take 0.55 of
+    // a stage (0.67 at d_h 128). us, 256 against 128 rows, d_h 32 / 64 / 128: S=4096, 8 heads 47 / 47 / 56 against 27 / 28 / 43; S=8192, 4 heads 89 / 86 / 103
+    // against 49 / 46 / 78; S=1024, 32 heads 15.6 / 17.0 / 20.1 against 12.9 / 14.0 / 20.8; S=4096, 12 heads 48 / 48 / 59 against 44 / 45 / 71 (0.87 and 1.02 by
+    // this); S=2048, 24 heads 26.5 / 27.8 / 34.0 against 27.8 / 30.1 / 44.8 (1.0 and 1.2); nothing at four stages (S=512, 64 heads 9.7 against 10.4).
+    bool short_ends = false, even = true;                  // even: items of about one length, which come in waves
+    if (a.causal) {
+        const double longest = std::min<double>(a.kv_len, a.q_start + a.q_rows) / WS_BN, part = d_h < 128 ? 0.55 : 0.67, fixed = 2;
+        const double as256 = std::max(longest + fixed, total * (stages + fixed) / sms);
+        const double as128 = std::max(part * longest + fixed, 2 * total * (part * stages + fixed) / sms);
+        even = longest < 1.25 * stages;
+        short_ends = !even && longest >= 4 && as128 < 0.92 * as256;
+    }
+    const bool halves = free_form && (waves128 <= 1 || short_ends || (d_h < 128 && stages >= 8 && even && waves128 * 4 <= waves256 * 2 * 3));
     FaPlan plan;
     plan.items256 = (int)total;
-    plan.items128 = plan.tiles = 0;
+    plan.items128 = plan.tiles = plan.tile_rows = 0;
+    // Small heads with few keys and more than one wave of anything are counted in tiles. Up to two stages two small blocks to an SM are
+    // faster, above that items like the others' (the figures are in fa_fwd_tile_sm100.cu).
     if (d_h < 64 && free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
-        // few keys and more than one wave of anything: two small blocks to an SM (the figures are in fa_fwd_tile_sm100.cu)
         plan.items256 = 0;
         plan.tiles = (int)total128;
-        plan.k_slots = plan.v_slots = 2;
-        plan.stage_step = 1;
-        return plan;
-    }
-    if (free_form && (waves128 <= 1 || (long_items && waves128 * 4 <= waves256 * 2 * 3))) {
+        plan.tile_rows = stages <= 2 ? 0 : halves ? 128 : 256;
+    } else if (halves) {
         plan.items256 = 0;
         plan.items128 = (int)total128;
     // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
@@ -828,7 +839,12 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
         plan.items256 = (int)(total - rest);
         plan.items128 = (int)rest * 2;
     }
-    const bool ks = plan.items128 > 0;
+    if (plan.tiles > 0 && plan.tile_rows == 0) {
+        plan.k_slots = plan.v_slots = 2;
+        plan.stage_step = 1;
+        return plan;
+    }
+    const bool ks = plan.items128 > 0 || plan.tile_rows == 128;
     switch (d_h) {
         case 16:  ring_of<16>(plan, ks);  break;
         case 32:  ring_of<32>(plan, ks);  break;

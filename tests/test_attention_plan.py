@@ -1,0 +1,46 @@
+"""Which items a causal attention launch goes as: 128-row items where its longest 256-row item is what it takes, on the CPU; and the results of
+launches on both sides of that line, on the GPU."""
+import pytest
+
+
+@pytest.mark.parametrize("d_h,S,H,q_start,split,halves", [
+    (64, 4096, 8, 0, 1, True), (128, 8192, 4, 0, 1, True), (64, 1024, 32, 0, 1, True), (128, 1024, 32, 0, 1, False), (64, 2048, 20, 0, 1, True),
+    (64, 2048, 24, 0, 1, False), (128, 2048, 20, 0, 1, False), (64, 512, 64, 0, 1, False), (64, 4096, 8, 0, 2, False), (64, 16384, 16, 0, 1, False),
+    (64, 8192, 37, 7168, 1, False), (32, 4096, 8, 0, 1, True)])
+def test_items_under_a_mask(pkg, d_h, S, H, q_start, split, halves):
+    plan = pkg.flash_attn_tc_plan(pkg.FlashParams(S, d_h, H, split, 1, 1.0), q_start, S - q_start)
+    assert plan.tiles == 0 and (plan.items_128 > 0) == halves and (plan.items_256 > 0) != halves
+    assert plan.stage_step == (2 if halves else 1)
+
+
+@pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 4, 1),
+                                                       (16, 2048, 16, 1, 4, 2), (32, 1024, 32, 1, 4, 2), (32, 640, 160, 0, 4, 1)])
+def test_tiles_of_few_keys(pkg, d_h, S, H, causal, slots, step):
+    """Blocks of their own (two slots) up to two stages of keys, items of 256 or 128 rows (four slots) above that."""
+    plan = pkg.flash_attn_tc_plan(pkg.FlashParams(S, d_h, H, 1, causal, 1.0), 0, S)
+    assert plan.tiles == H * S // 128 and plan.items_256 == plan.items_128 == 0
+    assert (plan.k_slots, plan.v_slots, plan.stage_step) == (slots, slots, step)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d_h,S,H,causal", [(64, 2048, 20, 1), (128, 4096, 8, 1), (32, 1024, 32, 1), (16, 384, 200, 0), (32, 640, 160, 1), (16, 256, 200, 1)])
+def test_results(pkg, torch_cuda, d_h, S, H, causal):
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    q, k, v = (torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    fp = pkg.FlashParams(S, d_h, H, 1, causal, d_h ** -0.5)
+    out = torch.full((S, H * d_h), float("nan"), device="cuda")
+    pkg.kernel_status_reset()
+    pkg.flash_attn_tc_forward(q, k, v, out, None, 0, S, fp, o_dtype=pkg.F32)
+    torch.cuda.synchronize()
+    assert pkg.kernel_status()[0] == 0
+    for h in range(0, H, 7):
+        s = q[h].double() @ k[h].double().T * d_h ** -0.5
+        if causal:
+            s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+        w = torch.softmax(s, dim=-1)
+        ref = w @ v[h].double()
+        # every weight is rounded to fp16 (2^-11 of it) or, below 2^-14 of the largest, to a multiple of 2^-25 (the offset may lag the
+        # maximum by 2^8); fp32 scores of up to about 100 carry 1e-5 of relative error into the weights
+        bound = (w * 2 ** -11 + 2.0 ** -24) @ v[h].double().abs() + 1e-4 * ref.abs().max()
+        assert bool(((out[:, h * d_h:(h + 1) * d_h].double() - ref).abs() <= bound).all()), h

@@ -338,6 +338,14 @@ int run_megatron(Run& r, char* output, efa_run_stats* st)
     EFA_CUDA(cudaEventRecord(c->ev_t0, c->compute_stream));
     if (r.attention(O_all, p.S, 0, p.S, c->compute_stream)) return 1;
     EFA_CUDA(cudaEventRecord(c->ev_t1, c->compute_stream));
+    if (r.direct && !r.residual) {
+        // nothing follows the projection: it stays on the attention's stream, without the events between streams
+        EFA_CUDA(cudaEventRecord(c->ev_t2, c->compute_stream));
+        if (r.project(O_all, send_buf, p.S, c->compute_stream, false, false)) return 1;
+        EFA_CUDA(cudaEventRecord(c->ev_t3, c->compute_stream));
+        if (sync_stream(c, c->compute_stream, nullptr, 0)) return 1;
+        return finish_timing(c, t0, st, true, true, r.launches);
+    }
     EFA_CUDA(cudaEventRecord(attn_done, c->compute_stream));
 
     EFA_CUDA(cudaStreamWaitEvent(c->proj_stream, attn_done, 0));

@@ -927,11 +927,17 @@ bool block_per_tile(int rows, int d_local, int d)
 // A pair of CTAs to a tile costs a cluster's start and a hand-over between two SMs per tile, which is worth it where wide tiles are
 // and their k loop is long: from d_local 832 on where there are more tiles than pairs of SMs (12224 x 848 x 2688: 55.8 -> 53.7 us, 16384 x
 // 1024 x 1024: 33.2 -> 31.5, 25728 x 2864 x 1344: 179 -> 159, but 4160 x 512 x 4096: 20.6 -> 21.2, 9024 x 368 x 1600: 17.2 -> 18.4,
-// 29952 x 176 x 1984: 39 -> 50), from 2048 on also with fewer (1024 x 4096 x 4096: 29.9 -> 29.1; 4096 x 1024 x 1024: 10.7 -> 11.2).
+// 29952 x 176 x 1984: 39 -> 50), from 2048 on also with fewer (1024 x 4096 x 4096: 29.9 -> 29.1; 4096 x 1024 x 1024: 10.7 -> 11.2). From 576
+// to 832 the gain is 2 to 6 % (16384 x 576 x 4096: 74.1 -> 71.4, 25728 x 720 x 1344: 56.4 -> 52.9, 8192 x 768 x 2048: 26.1 -> 24.7, 8192 x 640 to Q, K and V of eight
+// heads of 128: 33.8 -> 32.2) unless the pairs take a round more than single CTAs (4736 x 640 x 4096, five against four: 24.3 -> 26.1).
 bool in_pairs(int rows, int d_local, int cols)
 {
-    const long tiles = (long)((rows + 255) / 256) * ((cols + 255) / 256);
-    return wide_tiles(rows, cols) && (d_local >= 2048 ? rows >= 256 : d_local >= 832 && tiles > device_sms() / 2);
+    const long wide = (cols + 255) / 256, pairs = device_sms() / 2;
+    const long tiles = (long)((rows + 255) / 256) * wide, halves = (long)((rows + PJ_BM - 1) / PJ_BM) * wide;
+    if (!wide_tiles(rows, cols)) return false;
+    if (d_local >= 2048) return rows >= 256;
+    if (tiles <= pairs) return false;
+    return d_local >= 832 || (d_local >= 576 && (tiles + pairs - 1) / pairs <= (halves + 2 * pairs - 1) / (2 * pairs));
 }
 
 // Parts of k for a tile. A cluster and the sum over it cost 2.5 to 3 us, a k-block that an SM has no longer to wait for gives 0.3:

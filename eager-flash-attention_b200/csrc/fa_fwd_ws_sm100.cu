@@ -822,12 +822,14 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
     FaPlan plan;
     plan.items256 = (int)total;
     plan.items128 = plan.tiles = plan.tile_rows = 0;
-    // Small heads with few keys and more than one wave of anything are counted in tiles. Up to two stages two small blocks to an SM are
-    // faster, above that items like the others' (the figures are in fa_fwd_tile_sm100.cu).
+    // Small heads with few keys and more than one wave of anything are counted in tiles. Two small blocks to an SM are faster up to two
+    // stages, and below four where the 256-row items are more than one wave and uneven or in a poorly filled last wave; else items like the
+    // others' (the figures are in fa_fwd_tile_sm100.cu).
     if (d_h < 64 && free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
         plan.items256 = 0;
         plan.tiles = (int)total128;
-        plan.tile_rows = stages <= 2 ? 0 : halves ? 128 : 256;
+        const bool blocks = stages <= 2 || (stages < 4 && waves256 > 1 && (a.causal || total * 10 < waves256 * sms * 7));
+        plan.tile_rows = blocks ? 0 : halves ? 128 : 256;
     } else if (halves) {
         plan.items256 = 0;
         plan.items128 = (int)total128;

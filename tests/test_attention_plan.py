@@ -13,10 +13,11 @@ def test_items_under_a_mask(pkg, d_h, S, H, q_start, split, halves):
     assert plan.stage_step == (2 if halves else 1)
 
 
-@pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 4, 1),
+@pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 2, 1), (32, 512, 64, 1, 4, 1), (16, 640, 75, 1, 2, 1), (16, 768, 100, 1, 4, 1),
+                                                       (32, 384, 148, 0, 4, 1), (32, 384, 222, 0, 4, 1),
                                                        (16, 2048, 16, 1, 4, 2), (32, 1024, 32, 1, 4, 2), (32, 640, 160, 0, 4, 1)])
 def test_tiles_of_few_keys(pkg, d_h, S, H, causal, slots, step):
-    """Blocks of their own (two slots) up to two stages of keys, items of 256 or 128 rows (four slots) above that."""
+    """Blocks of their own (two slots) up to two stages of keys, or four in uneven waves; items of 256 or 128 rows (four slots) above that."""
     plan = pkg.flash_attn_tc_plan(pkg.FlashParams(S, d_h, H, 1, causal, 1.0), 0, S)
     assert plan.tiles == H * S // 128 and plan.items_256 == plan.items_128 == 0
     assert (plan.k_slots, plan.v_slots, plan.stage_step) == (slots, slots, step)

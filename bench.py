@@ -37,8 +37,8 @@ NVLINK_GBS = 900.0      # per direction and GPU, nominal: the link bound the blo
 REDUCE_BY_RANKS = {1: "nccl", 2: "pull", 4: "pull", 8: "pull"}
 
 # DRAM bytes (read + written) of one attention launch of the benchmark shape with all 32 heads on one GPU, by
-# (mode, rows taken last-first): ncu captures, one launch each. "alone": whole heads in turn, as every launch without tile
-# counters takes them (stream mode on one rank with the library's own plan).
+# (mode, rows taken last-first): ncu captures, one launch each. "alone": longest items first over groups of heads, as every causal launch
+# without tile counters takes them (stream mode on one rank with the library's own plan); four times a launch of eight heads.
 ATTN_TRAFFIC_32_HEADS = {("stream", False): 5.105e9, ("stream", True): 5.212e9, ("alone", True): 1.389e9}
 
 

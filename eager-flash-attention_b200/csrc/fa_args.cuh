@@ -5,6 +5,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "work_order.h"
 
 namespace efa {
@@ -37,6 +39,18 @@ __device__ __forceinline__ float ex2(float x)
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// The denominator that goes into the partials of a split. +0 says that the mask leaves nothing of the split for the row: the merge does not read its O. A
+// row that has keys there, all of them with a score of -inf, has no sum either, but O is 0 * V, NaN where V is not finite: -0 for that.
+__device__ __forceinline__ float partial_sum(float l, bool has_keys)
+{
+    return has_keys && l == 0.f ? -0.f : l;
+}
+// ... and how the merge reads it.
+__device__ __forceinline__ bool no_keys(float m, float l)
+{
+    return m == -INFINITY && __float_as_uint(l) == 0u;
 }
 
 // Work item `item` of a launch: head, split and first row. tail: 128-row items that are halves of the 256-row ones from a.tail_first on.

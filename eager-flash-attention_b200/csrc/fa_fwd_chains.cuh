@@ -346,7 +346,7 @@ fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
                 const size_t s0 = ((size_t)split * a.part_rows + orow) * a.H_local + head;
                 if (way == 0) {
                     a.m_part[s0] = m_true;
-                    a.l_part[s0] = l_run * mult;
+                    a.l_part[s0] = partial_sum(l_run * mult, !a.causal || split * a.kv_len <= a.q_start + (int)orow);
                 }
             }
             if (c_lo < D) {

@@ -49,7 +49,7 @@ combine_splits_kernel(const float* O_part, const float* m_part, const float* l_p
         const size_t step = (size_t)ws_rows * H_local;      // distance between splits
         float top = -INFINITY, denom = 0.f;
         float* w = weight + (size_t)e * split;
-        // An empty split (the mask leaves nothing of it: O and denominator are zeros) gets -0 as its weight, and is not read below.
+        // An empty split (the mask leaves nothing of it, partial_sum) gets -0 as its weight, and is not read below.
         if constexpr (SPLIT > 0) {
             float m[SPLIT], l[SPLIT];
             #pragma unroll
@@ -60,7 +60,7 @@ combine_splits_kernel(const float* O_part, const float* m_part, const float* l_p
             for (int i = 0; i < SPLIT; i++) {
                 const float x = exp2f(m[i] - top);
                 denom += x * l[i];
-                m[i] = m[i] == -INFINITY && l[i] == 0.f ? -0.f : x;
+                m[i] = no_keys(m[i], l[i]) ? -0.f : x;
             }
             const float inv = 1.f / denom;
             #pragma unroll
@@ -70,7 +70,7 @@ combine_splits_kernel(const float* O_part, const float* m_part, const float* l_p
             for (int i = 0; i < split; i++) {
                 const float m = m_part[base + i * step], l = l_part[base + i * step], x = exp2f(m - top);
                 denom += x * l;
-                w[i] = m == -INFINITY && l == 0.f ? -0.f : x;
+                w[i] = no_keys(m, l) ? -0.f : x;
             }
             const float inv = 1.f / denom;
             for (int i = 0; i < split; i++) w[i] *= inv;

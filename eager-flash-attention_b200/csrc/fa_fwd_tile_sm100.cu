@@ -267,7 +267,7 @@ fa_fwd_tile_kernel(const __grid_constant__ CUtensorMap tmQ,
             dst32 = a.O_part + ((size_t)split * a.part_rows + row) * ld_o + (size_t)head * D;
             const size_t s0 = ((size_t)split * a.part_rows + row) * a.H_local + head;
             a.m_part[s0] = m_run;
-            a.l_part[s0] = l_run;
+            a.l_part[s0] = partial_sum(l_run, !a.causal || kv_lo <= q_abs0 + tid);
         }
         #pragma unroll
         for (int c = 0; c < D / 16; c++) {

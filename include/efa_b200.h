@@ -47,7 +47,8 @@ typedef struct efa_flash_params {
 
 /* Same fields, order and meaning as FlashAttnTCPartials (flash_attn_tc.cuh:25-34):
  *   O_part [split][rows][H_local*d_h] unnormalised, m_part / l_part [split][rows][H_local],
- *   row max in the log2 domain and row denominator. */
+ *   row max in the log2 domain and row denominator. Row max -inf and denominator +0: the row has no key in the
+ *   split, its O_part is not read by the merge; denominator -0: it has keys, all of which score -inf. */
 typedef struct efa_flash_partials {
     float* O_part;
     float* m_part;

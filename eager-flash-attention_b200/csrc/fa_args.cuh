@@ -7,6 +7,7 @@
 
 #include <cmath>
 
+#include "attention_plan.h"
 #include "work_order.h"
 
 namespace efa {
@@ -90,10 +91,6 @@ __device__ __forceinline__ void pick_item(int item, const FaArgs& a, int items_x
 // K and V maps for it have boxes of fa_ws_kv_box_rows() rows (its stage length); Q maps 128 rows.
 int fa_ws_kv_box_rows();
 int fa_ws_preload();    // loads the code of every instantiation of the kernel on the current device
-// How a launch is cut into work items: items256 of 256 rows, then items128 of 128 rows (a launch of their own where
-// there are both), or tiles of 128 rows: one to a block of the one-tile kernel (tile_rows 0) or as items of so many rows; and the stages of K and V that the last of them keeps, of which
-// an issuing thread takes every stage_step-th.
-struct FaPlan { int items256, items128, tiles, tile_rows, k_slots, v_slots, stage_step; };
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms);
 int fa_forward_ws(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FaArgs& a,
                   int d_h, bool out_f16, int reserve_sms, cudaStream_t stream);

@@ -204,6 +204,7 @@ void fa_plan(const efa_flash_params& p, int q_start, int q_rows, efa_flash_plan*
     FaArgs a{};
     a.q_start = q_start; a.S = p.S;
     a.H_local = p.H_local; a.nsplit = p.split; a.q_rows = q_rows; a.kv_len = p.S / p.split; a.causal = p.causal;
+    a.heavy_first = p.causal;                              // without counters
     const FaPlan plan = fa_ws_plan(a, p.d_h, 0);
     *out = efa_flash_plan{plan.items256, plan.items128, plan.tiles, plan.k_slots, plan.v_slots, plan.stage_step};
 }

@@ -790,57 +790,11 @@ void ring_of(FaPlan& plan, bool halves)
 
 }  // namespace
 
-// Which items a launch goes as. Host arithmetic only.
+// Which items a launch goes as (attention_plan.h) and the rings of their kernel. Host arithmetic only.
 FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
 {
-    // 128-row items with their keys split over all the warpgroups where one wave of them is the whole launch (d_h 16 / 32 /
-    // 64 / 128, 74 items of 256 rows and 16 key stages: 15 / 16 / 19 / 29 us against 25 / 27 / 28 / 37). Three waves of them against
-    // two of 256 rows are worth it only where items are long and the tensor pipe is not what an item waits for. In us, 222
-    // items of 256 rows: 42 / 48 / 54 against 48 / 52 / 55 (d_h 16 / 32 / 64, 16 stages), 26 / 28 / 34 against 28 / 30 / 34 (8 stages), even at
-    // four, 82 against 76 (128, 16 stages).
-    const long heads = (long)a.H_local * a.nsplit;
-    const long total = heads * ((a.q_rows + 255) / 256), total128 = heads * ((a.q_rows + 127) / 128);
-    const long sms = device_sms();
-    const long waves256 = (total + sms - 1) / sms, waves128 = (total128 + sms - 1) / sms, rest = total % sms;
-    const double keys = a.causal ? a.q_start + 0.5 * (a.q_rows + 256) : a.S;
-    const double stages = keys / ((double)WS_BN * a.nsplit);                   // of an average item
-    const bool free_form = a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64);
-    // Under a causal mask the longest item can be what a launch takes, and as 128-row items it is half of it. Time as the longer of
-    // the longest item and everything spread over the SMs, in stages of 256 rows; an item costs two of them besides, and 128 rows take 0.55 of
-    // a stage (0.67 at d_h 128). us, 256 against 128 rows, d_h 32 / 64 / 128: S=4096, 8 heads 47 / 47 / 56 against 27 / 28 / 43; S=8192, 4 heads 89 / 86 / 103
-    // against 49 / 46 / 78; S=1024, 32 heads 15.6 / 17.0 / 20.1 against 12.9 / 14.0 / 20.8; S=4096, 12 heads 48 / 48 / 59 against 44 / 45 / 71 (0.87 and 1.02 by
-    // this); S=2048, 24 heads 26.5 / 27.8 / 34.0 against 27.8 / 30.1 / 44.8 (1.0 and 1.2); nothing at four stages (S=512, 64 heads 9.7 against 10.4).
-    bool short_ends = false, even = true;                  // even: items of about one length, which come in waves
-    if (a.causal) {
-        const double longest = std::min<double>(a.kv_len, a.q_start + a.q_rows) / WS_BN, part = d_h < 128 ? 0.55 : 0.67, fixed = 2;
-        const double as256 = std::max(longest + fixed, total * (stages + fixed) / sms);
-        const double as128 = std::max(part * longest + fixed, 2 * total * (part * stages + fixed) / sms);
-        even = longest < 1.25 * stages;
-        short_ends = !even && longest >= 4 && as128 < 0.92 * as256;
-    }
-    const bool halves = free_form && (waves128 <= 1 || short_ends || (d_h < 128 && stages >= 8 && even && waves128 * 4 <= waves256 * 2 * 3));
-    FaPlan plan;
-    plan.items256 = (int)total;
-    plan.items128 = plan.tiles = plan.tile_rows = 0;
-    // Small heads with few keys and more than one wave of anything are counted in tiles. Two small blocks to an SM are faster up to two
-    // stages, and below four where the 256-row items are more than one wave and uneven or in a poorly filled last wave; else items like the
-    // others' (the figures are in fa_fwd_tile_sm100.cu).
-    if (d_h < 64 && free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
-        plan.items256 = 0;
-        plan.tiles = (int)total128;
-        const bool blocks = stages <= 2 || (stages < 4 && waves256 > 1 && (a.causal || total * 10 < waves256 * sms * 7));
-        plan.tile_rows = blocks ? 0 : halves ? 128 : 256;
-    } else if (halves) {
-        plan.items256 = 0;
-        plan.items128 = (int)total128;
-    // Items of equal length end in a wave of their own for the rest that does not fill the GPU. Where that rest
-    // is at most half of a wave it goes as 128-row items behind the full waves (two of them at least, one at d_h 128: shorter
-    // launches are decided above). 65536 keys, two heads of 64, three full waves and 68 items: 2.75 -> 2.59 ms; 37 heads x 2560 rows x 4096 keys
-    // of d_h 64 / 32 141 -> 128 / 123 us. From 4096 keys on, where that is worth ten times a launch: 111 heads x 512 rows of d_h 128 140 -> 133 us.
-    } else if (free_form && !a.causal && total > sms && rest > 0 && rest * 2 <= sms && a.kv_len >= 4096) {
-        plan.items256 = (int)(total - rest);
-        plan.items128 = (int)rest * 2;
-    }
+    FaPlan plan = plan_items(PlanShape{a.q_start, a.q_rows, a.S, a.H_local, a.nsplit, a.kv_len, a.causal, d_h,
+                                       a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64), a.group_heads > 0 || a.heavy_first != 0, device_sms()});
     if (plan.tiles > 0 && plan.tile_rows == 0) {
         plan.k_slots = plan.v_slots = 2;
         plan.stage_step = 1;

@@ -1,6 +1,37 @@
 """Which items a causal attention launch goes as: 128-row items where its longest 256-row item is what it takes, on the CPU; and the results of
 launches on both sides of that line, on the GPU."""
+import ctypes
+import os
+import subprocess
+
 import pytest
+
+from conftest import ROOT
+
+SOURCE = """
+#include "attention_plan.h"
+extern "C" void plan(int q_start, int q_rows, int S, int H, int split, int causal, int d_h, int longest_first, int* out)
+{
+    const efa::FaPlan p = efa::plan_items(efa::PlanShape{q_start, q_rows, S, H, split, S / split, causal, d_h, true, longest_first != 0, 148});
+    out[0] = p.items256; out[1] = p.items128; out[2] = p.tiles; out[3] = p.tile_rows;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plan_items(tmp_path_factory):
+    """The arithmetic of the plan, compiled for the CPU: (items of 256 rows, of 128 rows, tiles, rows that tiles go by)."""
+    d = tmp_path_factory.mktemp("plan")
+    (d / "plan.cpp").write_text(SOURCE)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "eager-flash-attention_b200", "csrc"),
+                    str(d / "plan.cpp"), "-o", str(d / "plan.so")], check=True)
+    lib = ctypes.CDLL(str(d / "plan.so"))
+
+    def run(*args):
+        out = (ctypes.c_int * 4)()
+        lib.plan(*args, out)
+        return tuple(out)
+    return run
 
 
 @pytest.mark.parametrize("d_h,S,H,q_start,split,halves", [
@@ -11,6 +42,16 @@ def test_items_under_a_mask(pkg, d_h, S, H, q_start, split, halves):
     plan = pkg.flash_attn_tc_plan(pkg.FlashParams(S, d_h, H, split, 1, 1.0), q_start, S - q_start)
     assert plan.tiles == 0 and (plan.items_128 > 0) == halves and (plan.items_256 > 0) != halves
     assert plan.stage_step == (2 if halves else 1)
+
+
+# With completion counters the rows go in order, and the longest item is the last to start.
+@pytest.mark.parametrize("d_h,S,H,q_start,longest_first,in_order", [
+    (128, 4096, 8, 0, True, False), (128, 8192, 4, 2048, True, False), (128, 2048, 12, 0, True, False), (128, 1024, 24, 0, True, False), (128, 4096, 5, 0, True, True),
+    (128, 8192, 3, 0, True, True), (128, 3072, 20, 1536, False, False), (64, 768, 32, 0, True, False), (64, 4096, 8, 0, True, True), (32, 4096, 20, 2048, True, True)])
+def test_items_under_a_mask_by_the_order_of_the_launch(plan_items, d_h, S, H, q_start, longest_first, in_order):
+    for first, halves in ((1, longest_first), (0, in_order)):
+        items256, items128, tiles, _ = plan_items(q_start, S - q_start, S, H, 1, 1, d_h, first)
+        assert ((items256 > 0), (items128 > 0), tiles) == (not halves, halves, 0), first
 
 
 @pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 2, 1), (32, 512, 64, 1, 4, 1), (16, 640, 75, 1, 2, 1), (16, 768, 100, 1, 4, 1),

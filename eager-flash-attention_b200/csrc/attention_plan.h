@@ -52,7 +52,7 @@ inline FaPlan plan_items(const PlanShape& a)
             if (in_turn) return waves * (most + fixed) - wave * waves * (waves - 1) / 2;
             return std::max({most + fixed, n * (cost * stages + fixed) / sms, waves == 2 ? 2 * (most - wave + fixed) : 0});
         };
-        const double line = a.d_h == 128 ? 0.88 : in_turn ? 0.99 : 0.92;
+        const double line = a.d_h == 128 ? 0.88 : in_turn ? 0.985 : 0.92;
         even = longest < 1.25 * stages;
         short_ends = !even && longest >= 4 && end(total128, part) < line * end(total, 1);
     }
@@ -60,12 +60,17 @@ inline FaPlan plan_items(const PlanShape& a)
     FaPlan plan;
     plan.items256 = (int)total;
     // Small heads with few keys and more than one wave of anything are counted in tiles. Two small blocks to an SM are faster up to two
-    // stages, and below four where the 256-row items are more than one wave and uneven or in a poorly filled last wave; else items like the
-    // others' (the figures are in fa_fwd_tile_sm100.cu).
+    // stages, and above that where the 256-row items are more than one wave and end less evenly; else items like the others' (the figures are in
+    // fa_fwd_tile_sm100.cu). Without a mask that is so where the last wave of items is poorly filled (below four stages), or where they take more
+    // waves than the tiles do two to an SM: a third more up to three stages, half as many again to five. Under a mask below four stages; below
+    // five where heads end on half an item and there are two waves of items (longest first) or half as many waves again as of tiles (in order).
     if (a.d_h < 64 && a.free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
         plan.items256 = 0;
         plan.tiles = (int)total128;
-        const bool blocks = stages <= 2 || (stages < 4 && waves256 > 1 && (a.causal || total * 10 < waves256 * sms * 7));
+        const long pairs = (total128 + 2 * sms - 1) / (2 * sms);               // waves of tiles
+        const bool uneven = a.causal ? stages < 4 || (stages < 5 && total * 2 > total128 && (a.longest_first ? total * 4 <= sms * 9 : waves256 * 2 >= pairs * 3))
+                                     : (stages < 4 && total * 10 < waves256 * sms * 7) || (stages <= 3 ? waves256 * 3 >= pairs * 4 : waves256 * 2 >= pairs * 3);
+        const bool blocks = stages <= 2 || (waves256 > 1 && uneven);
         plan.tile_rows = blocks ? 0 : halves ? 128 : 256;
     } else if (halves) {
         plan.items256 = 0;

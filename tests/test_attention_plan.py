@@ -54,6 +54,13 @@ def test_items_under_a_mask_by_the_order_of_the_launch(plan_items, d_h, S, H, q_
         assert ((items256 > 0), (items128 > 0), tiles) == (not halves, halves, 0), first
 
 
+# Without a mask by waves: of 256-row items against those of tiles, two to an SM. Under one, heads that end on half an item.
+@pytest.mark.parametrize("S,H,causal,rows", [(640, 50, 0, 0), (640, 110, 0, 0), (640, 60, 0, 256), (640, 160, 0, 256), (384, 160, 0, 0), (384, 250, 0, 0), (384, 200, 0, 256),
+                                             (576, 160, 0, 256), (512, 148, 0, 256), (896, 60, 1, 0), (896, 110, 1, 256), (768, 75, 1, 256)])
+def test_few_keys_by_waves(plan_items, S, H, causal, rows):
+    assert plan_items(0, S, S, H, 1, causal, 32, 1)[2:] == (H * ((S + 127) // 128), rows)
+
+
 @pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 2, 1), (32, 512, 64, 1, 4, 1), (16, 640, 75, 1, 2, 1), (16, 768, 100, 1, 4, 1),
                                                        (32, 384, 148, 0, 4, 1), (32, 384, 222, 0, 4, 1),
                                                        (16, 2048, 16, 1, 4, 2), (32, 1024, 32, 1, 4, 2), (32, 640, 160, 0, 4, 1)])

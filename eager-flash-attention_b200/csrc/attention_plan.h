@@ -5,10 +5,10 @@
 
 namespace efa {
 
-// How a launch is cut into work items: items256 of 256 rows, then items128 of 128 rows (a launch of their own where
-// there are both), or tiles of 128 rows: one to a block of the one-tile kernel (tile_rows 0) or as items of so many rows; and the stages of K and V that the last of them keeps, of which
-// an issuing thread takes every stage_step-th.
-struct FaPlan { int items256 = 0, items128 = 0, tiles = 0, tile_rows = 0, k_slots = 0, v_slots = 0, stage_step = 1; };
+// How a launch is cut into work items: items256 of 256 rows, then items128 of 128 rows (a launch of their own where there are both); or
+// tiles of 128 rows, one to a block of the one-tile kernel. And the stages of K and V that the last of them keeps, of which an issuing thread takes
+// every stage_step-th.
+struct FaPlan { int items256 = 0, items128 = 0, tiles = 0, k_slots = 0, v_slots = 0, stage_step = 1; };
 
 struct PlanShape {
     int q_start, q_rows, S, H_local, nsplit, kv_len, causal, d_h;
@@ -59,19 +59,18 @@ inline FaPlan plan_items(const PlanShape& a)
     const bool halves = a.free_form && (waves128 <= 1 || short_ends || (a.d_h < 128 && stages >= 8 && even && waves128 * 4 <= waves256 * 2 * 3));
     FaPlan plan;
     plan.items256 = (int)total;
-    // Small heads with few keys and more than one wave of anything are counted in tiles. Two small blocks to an SM are faster up to two
-    // stages, and above that where the 256-row items are more than one wave and end less evenly; else items like the others' (the figures are in
+    // Small heads with few keys and more than one wave of anything: the one-tile kernel. Two small blocks to an SM are faster up to two
+    // stages, and above that where the 256-row items are more than one wave and end less evenly (the figures are in
     // fa_fwd_tile_sm100.cu). Without a mask that is so where the last wave of items is poorly filled (below four stages), or where they take more
     // waves than the tiles do two to an SM: a third more up to three stages, half as many again to five. Under a mask below four stages; below
     // five where heads end on half an item and there are two waves of items (longest first) or half as many waves again as of tiles (in order).
-    if (a.d_h < 64 && a.free_form && total128 > sms && stages <= (a.causal ? 10 : 5)) {
+    const long pairs = (total128 + 2 * sms - 1) / (2 * sms);                   // waves of tiles
+    const bool half_more = waves256 * 2 >= pairs * 3;
+    const bool uneven = a.causal ? stages < 4 || (stages < 5 && total * 2 > total128 && (a.longest_first ? total * 4 <= sms * 9 : half_more))
+                                 : (stages < 4 && total * 10 < waves256 * sms * 7) || (stages <= 3 ? waves256 * 3 >= pairs * 4 : stages <= 5 && half_more);
+    if (a.d_h < 64 && a.free_form && total128 > sms && (stages <= 2 || (waves256 > 1 && uneven))) {
         plan.items256 = 0;
         plan.tiles = (int)total128;
-        const long pairs = (total128 + 2 * sms - 1) / (2 * sms);               // waves of tiles
-        const bool uneven = a.causal ? stages < 4 || (stages < 5 && total * 2 > total128 && (a.longest_first ? total * 4 <= sms * 9 : waves256 * 2 >= pairs * 3))
-                                     : (stages < 4 && total * 10 < waves256 * sms * 7) || (stages <= 3 ? waves256 * 3 >= pairs * 4 : waves256 * 2 >= pairs * 3);
-        const bool blocks = stages <= 2 || (waves256 > 1 && uneven);
-        plan.tile_rows = blocks ? 0 : halves ? 128 : 256;
     } else if (halves) {
         plan.items256 = 0;
         plan.items128 = (int)total128;

@@ -757,8 +757,8 @@ int launch_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     if constexpr (D >= 64)
         if (reserve_sms > 0) return launch_ws<D, OUT_F16>(tq, tk, tv, a, stream, reserve_sms, 0);
     const FaPlan plan = fa_ws_plan(a, D, reserve_sms);
-    if (plan.tiles > 0 && plan.tile_rows == 0) return fa_forward_tile(tq, tk, tv, a, D, OUT_F16, stream);
-    if (plan.items128 > 0 ? plan.items256 == 0 : plan.tile_rows == 128) return launch_items<D, OUT_F16, true>(tq, tk, tv, a, stream);
+    if (plan.tiles > 0) return fa_forward_tile(tq, tk, tv, a, D, OUT_F16, stream);
+    if (plan.items128 > 0 && plan.items256 == 0) return launch_items<D, OUT_F16, true>(tq, tk, tv, a, stream);
     if (plan.items128 > 0) {
         FaArgs t = a;
         t.tail_first = plan.items256;
@@ -795,12 +795,12 @@ FaPlan fa_ws_plan(const FaArgs& a, int d_h, int reserve_sms)
 {
     FaPlan plan = plan_items(PlanShape{a.q_start, a.q_rows, a.S, a.H_local, a.nsplit, a.kv_len, a.causal, d_h,
                                        a.order_tab == nullptr && !(reserve_sms > 0 && d_h >= 64), a.group_heads > 0 || a.heavy_first != 0, device_sms()});
-    if (plan.tiles > 0 && plan.tile_rows == 0) {
+    if (plan.tiles > 0) {
         plan.k_slots = plan.v_slots = 2;
         plan.stage_step = 1;
         return plan;
     }
-    const bool ks = plan.items128 > 0 || plan.tile_rows == 128;
+    const bool ks = plan.items128 > 0;
     switch (d_h) {
         case 16:  ring_of<16>(plan, ks);  break;
         case 32:  ring_of<32>(plan, ks);  break;

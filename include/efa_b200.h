@@ -110,10 +110,10 @@ const char* efa_flash_attn_tc_check_params(const efa_flash_params* p, int q_rows
 
 /* How efa_flash_attn_tc_forward cuts rows q_start .. q_start+q_rows into work items: items_256 items of 256 query rows of one
  * head and split, then items_128 items of 128 rows whose keys all warpgroups share (in a launch of their own where
- * there are both); or tiles of 128 rows for small heads with few keys, which go one to a block of a kernel of their own where there are two to four stages of keys
- * or fewer, as such items above that. k_slots and v_slots: the 128-key stages of K and V that the last of them keeps in shared memory, of which
- * one issuing thread takes every stage_step-th. This is what a launch without tile_counters takes; with them a causal one starts at the
- * first rows, and its items may be of the other size. Host arithmetic only; no counterpart in the reference. */
+ * there are both); or, for small heads with few keys, tiles of 128 rows, one to a block of a kernel of their own, and no items. k_slots and
+ * v_slots: the 128-key stages of K and V that the last of them keeps in shared memory, of which one issuing thread takes every
+ * stage_step-th. This is what a launch without tile_counters takes; with them a causal one starts at the
+ * first rows, and may go as another of the three. Host arithmetic only; no counterpart in the reference. */
 typedef struct efa_flash_plan { int items_256, items_128, tiles, k_slots, v_slots, stage_step; } efa_flash_plan;
 int efa_flash_attn_tc_plan(const efa_flash_params* p, int q_start, int q_rows, efa_flash_plan* out);
 

@@ -190,8 +190,10 @@ def test_work_items_of_an_attention_launch(pkg, d_h, H, S, q_rows, split, causal
 
 
 @pytest.mark.parametrize("d_h,H,S,q_rows,split,causal,want", [
-    (16, 100, 256, 256, 1, 0, 200), (32, 75, 640, 512, 1, 0, 300), (32, 8, 4096, 4096, 8, 0, 2048), (16, 111, 1024, 512, 1, 1, 444),
-    (16, 16, 2048, 2048, 1, 1, 256), (16, 111, 1536, 512, 1, 1, 0), (16, 74, 256, 256, 1, 0, 0), (32, 75, 768, 512, 1, 0, 0),
+    (16, 100, 256, 256, 1, 0, 200), (32, 80, 640, 320, 1, 0, 240), (32, 8, 4096, 4096, 16, 0, 4096), (16, 75, 640, 640, 1, 1, 375),
+    # more keys: items of 256 or 128 rows like the others'
+    (32, 75, 640, 512, 1, 0, 0), (32, 8, 4096, 4096, 8, 0, 0), (16, 111, 1024, 512, 1, 1, 0), (16, 16, 2048, 2048, 1, 1, 0),
+    (16, 111, 1536, 512, 1, 1, 0), (16, 74, 256, 256, 1, 0, 0), (32, 75, 768, 512, 1, 0, 0),
     (64, 100, 256, 256, 1, 0, 0), (16, 8, 4096, 4096, 4, 0, 0)])
 def test_small_heads_with_few_keys_go_as_single_tiles(pkg, d_h, H, S, q_rows, split, causal, want):
     p = pkg.make_params(S, H * d_h, H, 64, 2, split, causal)

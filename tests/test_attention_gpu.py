@@ -191,13 +191,24 @@ def form(pkg, H, d_h, S, q_start, q_rows, split, causal):
     return "+".join(n for n, items in (("256", plan.items_256), ("128", plan.items_128), ("tiles", plan.tiles)) if items)
 
 
-# One to 16 key stages, ragged last blocks, rows that see no key of a split, both directions of the mask.
+# One to seven key stages (more than the ring of two keeps), ragged last blocks, rows that see no key of a split, both directions of the mask.
 @pytest.mark.parametrize("d_h", [16, 32])
 @pytest.mark.parametrize("H,S,q_start,q_rows,split,causal", [
-    (160, 64, 0, 64, 1, 0), (100, 256, 0, 256, 1, 1), (152, 192, 64, 128, 1, 1), (60, 640, 320, 320, 1, 0), (40, 640, 0, 640, 1, 0),
-    (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (16, 1280, 192, 576, 2, 0), (10, 2048, 0, 2048, 1, 1)])
+    (160, 64, 0, 64, 1, 0), (100, 256, 0, 256, 1, 1), (152, 192, 64, 128, 1, 1), (80, 640, 320, 320, 1, 0), (50, 640, 0, 640, 1, 0),
+    (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (25, 1280, 192, 576, 2, 0), (160, 384, 0, 384, 1, 0), (160, 448, 192, 256, 1, 0), (75, 640, 0, 640, 1, 1),
+    (75, 896, 0, 896, 1, 1)])
 def test_single_tiles_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal):
     assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == "tiles"
+    check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
+
+
+# As few keys that go as items of the four chains.
+@pytest.mark.parametrize("d_h", [16, 32])
+@pytest.mark.parametrize("H,S,q_start,q_rows,split,causal,want", [
+    (60, 640, 320, 320, 1, 0, "256"), (40, 640, 0, 640, 1, 0, "256"), (16, 1280, 192, 576, 2, 0, "256"), (10, 2048, 0, 2048, 1, 1, "128"),
+    (148, 512, 0, 512, 1, 0, "256"), (32, 1024, 0, 1024, 1, 1, "128")])
+def test_few_keys_as_items_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal, want):
+    assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == want
     check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)
 
 
@@ -242,7 +253,7 @@ def test_a_short_last_wave(pkg, torch_cuda, d_h, H, q_start, q_rows, split, tile
 
 
 @pytest.mark.parametrize("entry,d_h", [("forward", 16), ("forward", 32), ("noalloc", 16), ("noalloc", 64), ("noalloc", 128)])
-@pytest.mark.parametrize("H,S", [(2, 512), (100, 512), (80, 1024)])
+@pytest.mark.parametrize("H,S", [(2, 512), (100, 512), (80, 1024), (160, 448)])
 def test_the_largest_weight_of_a_row_is_not_rounded(pkg, torch_cuda, entry, d_h, H, S):
     """One key in the first stage and, by 2^3 to 2^8 larger in weight, one two stages later; V is 1 for the later one
     only, so that O is its softmax weight. With the row maximum as the exponent offset that weight enters P*V as exactly

@@ -13,14 +13,14 @@ SOURCE = """
 extern "C" void plan(int q_start, int q_rows, int S, int H, int split, int causal, int d_h, int longest_first, int* out)
 {
     const efa::FaPlan p = efa::plan_items(efa::PlanShape{q_start, q_rows, S, H, split, S / split, causal, d_h, true, longest_first != 0, 148});
-    out[0] = p.items256; out[1] = p.items128; out[2] = p.tiles; out[3] = p.tile_rows;
+    out[0] = p.items256; out[1] = p.items128; out[2] = p.tiles;
 }
 """
 
 
 @pytest.fixture(scope="module")
 def plan_items(tmp_path_factory):
-    """The arithmetic of the plan, compiled for the CPU: (items of 256 rows, of 128 rows, tiles, rows that tiles go by)."""
+    """The arithmetic of the plan, compiled for the CPU: (items of 256 rows, of 128 rows, tiles)."""
     d = tmp_path_factory.mktemp("plan")
     (d / "plan.cpp").write_text(SOURCE)
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "eager-flash-attention_b200", "csrc"),
@@ -28,7 +28,7 @@ def plan_items(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "plan.so"))
 
     def run(*args):
-        out = (ctypes.c_int * 4)()
+        out = (ctypes.c_int * 3)()
         lib.plan(*args, out)
         return tuple(out)
     return run
@@ -50,24 +50,27 @@ def test_items_under_a_mask(pkg, d_h, S, H, q_start, split, halves):
     (128, 8192, 3, 0, True, True), (128, 3072, 20, 1536, False, False), (64, 768, 32, 0, True, False), (64, 4096, 8, 0, True, True), (32, 4096, 20, 2048, True, True)])
 def test_items_under_a_mask_by_the_order_of_the_launch(plan_items, d_h, S, H, q_start, longest_first, in_order):
     for first, halves in ((1, longest_first), (0, in_order)):
-        items256, items128, tiles, _ = plan_items(q_start, S - q_start, S, H, 1, 1, d_h, first)
+        items256, items128, tiles = plan_items(q_start, S - q_start, S, H, 1, 1, d_h, first)
         assert ((items256 > 0), (items128 > 0), tiles) == (not halves, halves, 0), first
 
 
 # Without a mask by waves: of 256-row items against those of tiles, two to an SM. Under one, heads that end on half an item.
-@pytest.mark.parametrize("S,H,causal,rows", [(640, 50, 0, 0), (640, 110, 0, 0), (640, 60, 0, 256), (640, 160, 0, 256), (384, 160, 0, 0), (384, 250, 0, 0), (384, 200, 0, 256),
+@pytest.mark.parametrize("S,H,causal,item_rows", [(640, 50, 0, 0), (640, 110, 0, 0), (640, 60, 0, 256), (640, 160, 0, 256), (384, 160, 0, 0), (384, 250, 0, 0), (384, 200, 0, 256),
                                              (576, 160, 0, 256), (512, 148, 0, 256), (896, 60, 1, 0), (896, 110, 1, 256), (768, 75, 1, 256)])
-def test_few_keys_by_waves(plan_items, S, H, causal, rows):
-    assert plan_items(0, S, S, H, 1, causal, 32, 1)[2:] == (H * ((S + 127) // 128), rows)
+def test_few_keys_by_waves(plan_items, S, H, causal, item_rows):
+    want = (0, 0, H * ((S + 127) // 128)) if item_rows == 0 else (H * ((S + 255) // 256), 0, 0)
+    assert plan_items(0, S, S, H, 1, causal, 32, 1) == want
 
 
 @pytest.mark.parametrize("d_h,S,H,causal,slots,step", [(16, 128, 592, 0, 2, 1), (16, 256, 200, 1, 2, 1), (32, 384, 200, 0, 4, 1), (32, 512, 128, 1, 2, 1), (32, 512, 64, 1, 4, 1), (16, 640, 75, 1, 2, 1), (16, 768, 100, 1, 4, 1),
                                                        (32, 384, 148, 0, 4, 1), (32, 384, 222, 0, 4, 1),
                                                        (16, 2048, 16, 1, 4, 2), (32, 1024, 32, 1, 4, 2), (32, 640, 160, 0, 4, 1)])
 def test_tiles_of_few_keys(pkg, d_h, S, H, causal, slots, step):
-    """Blocks of their own (two slots) up to two stages of keys, or four in uneven waves; items of 256 or 128 rows (four slots) above that."""
+    """Blocks of their own (two slots) up to two stages of keys, or five in uneven waves; items of 256 or 128 rows (four slots) above that. The plan
+    names what is launched."""
     plan = pkg.flash_attn_tc_plan(pkg.FlashParams(S, d_h, H, 1, causal, 1.0), 0, S)
-    assert plan.tiles == H * S // 128 and plan.items_256 == plan.items_128 == 0
+    tiles, items256 = H * S // 128, H * ((S + 255) // 256)
+    assert (plan.items_256, plan.items_128, plan.tiles) == ((0, 0, tiles) if slots == 2 else (items256, 0, 0) if step == 1 else (0, tiles, 0))
     assert (plan.k_slots, plan.v_slots, plan.stage_step) == (slots, slots, step)
 
 

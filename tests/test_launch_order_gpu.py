@@ -6,8 +6,8 @@ pytestmark = pytest.mark.gpu
 
 
 # One wave and several of every kernel; split keys with their merge; a short last wave in a launch of its own (13 heads of 128);
-# the kernel of small heads and few keys.
-@pytest.mark.parametrize("S,H,d_h,split", [(192, 2, 64, 1), (1024, 4, 64, 4), (4096, 13, 128, 1), (2048, 16, 128, 2), (512, 40, 32, 1)])
+# items of four chains; the kernel of small heads and few keys.
+@pytest.mark.parametrize("S,H,d_h,split", [(192, 2, 64, 1), (1024, 4, 64, 4), (4096, 13, 128, 1), (2048, 16, 128, 2), (512, 40, 32, 1), (256, 80, 32, 1)])
 @pytest.mark.parametrize("side", [False, True], ids=["default stream", "other stream"])
 def test_a_chain_of_calls_needs_no_synchronisation(pkg, torch_cuda, S, H, d_h, split, side):
     torch = torch_cuda
@@ -54,7 +54,7 @@ def test_a_chain_of_calls_needs_no_synchronisation(pkg, torch_cuda, S, H, d_h, s
         assert torch.isfinite(y).all() and torch.equal(y, want[i // 2])
 
 
-@pytest.mark.parametrize("S,H,d_h,split", [(192, 2, 64, 1), (1024, 4, 64, 4), (4096, 13, 128, 1), (512, 40, 32, 1)])
+@pytest.mark.parametrize("S,H,d_h,split", [(192, 2, 64, 1), (1024, 4, 64, 4), (4096, 13, 128, 1), (512, 40, 32, 1), (256, 80, 32, 1)])
 def test_a_captured_chain_with_joins_keeps_its_order(pkg, torch_cuda, S, H, d_h, split):
     """The same kernels in a CUDA graph, where a call also follows work of another stream (a join), on inputs that change from replay to
     replay: as the calls give one by one."""

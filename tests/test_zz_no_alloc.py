@@ -97,7 +97,7 @@ assert pkg.flash_attn_tc_noalloc_status()[0] == 0
 """
 
 
-@pytest.mark.parametrize("d_h,S", [(16, 256), (32, 512), (64, 512), (128, 512)])
+@pytest.mark.parametrize("d_h,S", [(16, 256), (32, 256), (32, 512), (64, 512), (128, 512)])
 def test_after_the_first_call_every_form_can_be_captured(torch_cuda, d_h, S):
     """Few and many rows take different forms of the kernel; the first call of a head size has prepared them all. In a
     process of its own: nothing may have been loaded before."""

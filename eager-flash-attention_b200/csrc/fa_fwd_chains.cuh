@@ -37,7 +37,7 @@ constexpr int CH_THREADS = 768;
 
 template <int D, bool OUT_F16, int WAYS>
 __global__ void __launch_bounds__(CH_THREADS, 1)
-fa_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ,
+fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV,
                      const FaArgs a, int items_x, int items_total)

@@ -1,6 +1,6 @@
 // The attention launch interface (flash_attn_tc_forward of eager-flash-attention, flash_attn_tc.cu:363-399): argument
-// checks, tensor maps, the merge of split-KV partials and the entry that allocates nothing. The kernels are in
-// fa_fwd_ws_sm100.cu (which also says which launch takes which) and fa_fwd_tile_sm100.cu.
+// checks, tensor maps, the merge of split-KV partials and the entry that allocates nothing. The kernels are in fa_fwd_ws_sm100.cu
+// (d_h 128), fa_fwd_chains.cuh (16 to 64) and fa_fwd_tile_sm100.cu (16 and 32, few keys); attention_plan.h says which launch goes as what.
 #include "fa_fwd_sm100.cuh"
 #include "fa_args.cuh"
 #include "host_util.h"

@@ -2,8 +2,9 @@
 // Stands in for flash_attn_tc_kernel (flash_attn_tc.cu:73-312 of eager-flash-attention) behind the same launch
 // interface: same tensor layouts, split-KV partial format (row max in the log2 domain) and completion counters.
 //
-// Two kernels of one name: this one for d_h = 128, where the tensor pipe and the exponentials are about even (and for d_h = 64 in the persistent
-// form), and that of four chains for d_h 16, 32 and 64 (fa_fwd_chains.cuh). Few rows (KSPLIT) use it with the differences stated there.
+// Two kernels: this one (fa_fwd_ws_kernel) for d_h = 128, where the tensor pipe and the exponentials are about even (and for d_h = 64 in the persistent
+// form), and that of four chains (fa_fwd_chains_kernel, fa_fwd_chains.cuh) for d_h 16, 32 and 64. Few rows (KSPLIT) use this one with the differences
+// stated there.
 //
 // One CTA = 256 query rows (two 128-row Q tiles) of one (head, split), 384 threads:
 //   warps 0-3   softmax of Q tile 0        (one thread per row; registers raised with setmaxnreg)
@@ -677,9 +678,9 @@ template <int D, bool OUT_F16, int WAYS>
 int configure_chains()
 {
     cudaFuncAttributes attr;
-    EFA_CUDA(cudaFuncGetAttributes(&attr, fa_fwd_ws_kernel<D, OUT_F16, WAYS>));
+    EFA_CUDA(cudaFuncGetAttributes(&attr, fa_fwd_chains_kernel<D, OUT_F16, WAYS>));
     if ((attr.numRegs + 7) / 8 * 8 * CH_THREADS < 512 * 104 + 128 * 40 + 128 * 24) { set_error("attention kernel compiled to %d registers", attr.numRegs); return 1; }
-    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_ws_kernel<D, OUT_F16, WAYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainCfg<D, WAYS>::SMEM_BYTES));
+    EFA_CUDA(cudaFuncSetAttribute(fa_fwd_chains_kernel<D, OUT_F16, WAYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainCfg<D, WAYS>::SMEM_BYTES));
     return 0;
 }
 
@@ -712,7 +713,7 @@ int launch_chains(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     const int items_x = args.H_local * args.nsplit, rows = C::TILES * WS_BM;
     const int items_y = (args.q_rows + rows - 1) / rows;
     const dim3 grid = blocks > 0 ? dim3(blocks) : dim3(items_x, items_y);
-    EFA_CUDA(launch_early(fa_fwd_ws_kernel<D, OUT_F16, WAYS>, grid, CH_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, items_x, WAYS == 4 && blocks > 0 ? blocks : items_x * items_y));
+    EFA_CUDA(launch_early(fa_fwd_chains_kernel<D, OUT_F16, WAYS>, grid, CH_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, args, items_x, WAYS == 4 && blocks > 0 ? blocks : items_x * items_y));
     return 0;
 }
 
@@ -847,7 +848,7 @@ static int touch_forms()
     if constexpr (D == 128)
         return touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, false, false>) || touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, false, true>);
     else
-        return touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, 2>) || touch_kernel(fa_fwd_ws_kernel<D, OUT_F16, 4>);
+        return touch_kernel(fa_fwd_chains_kernel<D, OUT_F16, 2>) || touch_kernel(fa_fwd_chains_kernel<D, OUT_F16, 4>);
 }
 
 int fa_ws_preload()

@@ -31,16 +31,25 @@ def _definition(text, name):
 
 
 def _early_kernels():
+    sources = _sources()
+    names = {n for text in sources.values() for n in re.findall(r"launch_early(?:_cluster)?\((?:\w+,\s*)?(\w+_kernel)\b", text)}
     found = {}
-    for path, text in _sources().items():
-        for name in re.findall(r"launch_early(?:_cluster)?\((?:\w+,\s*)?(\w+_kernel)\b", text):
-            found[name] = _definition(text, name)
+    for name in names:
+        bodies = [b for b in (_definition(text, name) for text in sources.values()) if b]
+        assert len(bodies) == 1, name                       # two kernels of one name could not be told apart
+        found[name] = bodies[0]
     return found
 
 
 def test_kernels_that_start_early_are_found():
-    assert set(_early_kernels()) == {"combine_splits_kernel", "fa_fwd_ws_kernel", "fa_fwd_tile_kernel", "proj_gemm_kernel", "proj_pair_kernel",
-                                     "proj_tile_kernel", "proj_split_kernel"}
+    assert set(_early_kernels()) == {"combine_splits_kernel", "fa_fwd_ws_kernel", "fa_fwd_chains_kernel", "fa_fwd_tile_kernel", "proj_gemm_kernel",
+                                     "proj_pair_kernel", "proj_tile_kernel", "proj_split_kernel"}
+
+
+def test_kernels_have_names_of_their_own():
+    """Profiles and launch lists tell kernels apart by name."""
+    names = [n for text in _sources().values() for n in re.findall(r"__global__\s+void\s+(?:__\w+__\s*\([^)]*\)\s*)*(\w+)\s*\(", text)]
+    assert {"fa_fwd_ws_kernel", "combine_splits_kernel"} < set(names) and len(names) == len(set(names)), sorted(names)
 
 
 def test_kernels_that_start_early_presume_no_read_only_memory():
@@ -51,5 +60,6 @@ def test_kernels_that_start_early_presume_no_read_only_memory():
 
 
 def test_helpers_that_kernels_share_presume_no_read_only_memory():
-    with open(os.path.join(CSRC, "sm100_ptx.cuh")) as f:
-        assert not re.search(r"__restrict__|__ldg\b|global\.nc\b", f.read())
+    for name in ("sm100_ptx.cuh", "fa_args.cuh", "work_order.h"):
+        with open(os.path.join(CSRC, name)) as f:
+            assert not re.search(r"__restrict__|__ldg\b|global\.nc\b", f.read())

@@ -33,9 +33,10 @@ inline FaPlan plan_items(const PlanShape& a)
     const double stages = keys / ((double)kStage * a.nsplit);                  // of an average item
     // Under a causal mask the longest item can be what a launch takes, and as 128-row items it is half of it. When the last item ends, in stages of
     // 256 rows; an item costs two of them besides, and 128 rows take 0.55 of a stage (0.67 at d_h 128). Longest first: the longest item, everything spread
-    // over the SMs, or the two that meet on an SM between two waves. In the order of the rows SMs take items in turn, and the longest comes last,
+    // over the SMs, or (d_h 128) the two that meet on an SM between two waves. In the order of the rows SMs take items in turn, and the longest comes last,
     // behind one of each wave. The times measured are 0.95 to 1.06 of that, at d_h 128 1.05 to 1.16, hence the lines. (Splits in the order of the
-    // rows fit neither; up to d_h 64 they are taken as the first, at 128 as the second.)
+    // rows fit neither; up to d_h 64 they are taken as the first, at 128 as the second. With more than two waves of 256-row items that order
+    // costs less than twice as many items: 41216 rows, three heads of 64 956 us, as 128-row items 1034.)
     // us, 256 against 128 rows, d_h 32 / 64 / 128, longest first: S=4096, 8 heads 47 / 47 / 56 against 27 / 28 / 43; S=8192, 4 heads 89 / 86 / 103
     // against 49 / 46 / 78; S=1024, 32 heads 15.6 / 17.0 / 20.1 against 12.9 / 14.0 / 20.8; S=4096, 12 heads 48 / 48 / 59 against 44 / 45 / 71;
     // S=2048, 24 heads 26.5 / 27.8 / 34.0 against 27.8 / 30.1 / 44.8; S=3072, 20 heads, rows from 1536 on, d_h 128 46 against 50; nothing at four
@@ -45,14 +46,17 @@ inline FaPlan plan_items(const PlanShape& a)
     if (a.causal) {
         const double longest = std::min<double>(a.kv_len, a.q_start + a.q_rows) / kStage, part = a.d_h < 128 ? 0.55 : 0.67, fixed = 2;
         const double shortest = a.nsplit > 1 ? 0 : (a.q_start + 128.) / kStage;
-        const bool in_turn = !a.longest_first && (a.nsplit == 1 || a.d_h == 128);
+        const bool in_turn = !a.longest_first && (a.nsplit == 1 || a.d_h == 128) && total <= 2 * sms;
         auto end = [&](long n, double cost) {
             const double most = cost * longest, wave = cost * (longest - shortest) * sms / n;      // by which items differ that are a wave apart
             const long waves = (n + sms - 1) / sms;
             if (in_turn) return waves * (most + fixed) - wave * waves * (waves - 1) / 2;
-            return std::max({most + fixed, n * (cost * stages + fixed) / sms, waves == 2 ? 2 * (most - wave + fixed) : 0});
+            return std::max({most + fixed, n * (cost * stages + fixed) / sms, a.d_h == 128 && waves == 2 ? 2 * (most - wave + fixed) : 0});
         };
-        const double line = a.d_h == 128 ? 0.88 : in_turn ? 0.985 : 0.92;
+        // In order, heads that end on 128 rows: their last 256-row item, the longest, is half empty and takes less (S=1536, rows from 384 on, 48 heads of 16
+        // 30.2 us against 31.9).
+        const bool half_ends = in_turn && total * 2 > total128;
+        const double line = (a.d_h == 128 ? 0.88 : in_turn ? 0.985 : 0.92) - (half_ends ? 0.08 : 0);
         even = longest < 1.25 * stages;
         short_ends = !even && longest >= 4 && end(total128, part) < line * end(total, 1);
     }

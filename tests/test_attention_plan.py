@@ -47,7 +47,9 @@ def test_items_under_a_mask(pkg, d_h, S, H, q_start, split, halves):
 # With completion counters the rows go in order, and the longest item is the last to start.
 @pytest.mark.parametrize("d_h,S,H,q_start,longest_first,in_order", [
     (128, 4096, 8, 0, True, False), (128, 8192, 4, 2048, True, False), (128, 2048, 12, 0, True, False), (128, 1024, 24, 0, True, False), (128, 4096, 5, 0, True, True),
-    (128, 8192, 3, 0, True, True), (128, 3072, 20, 1536, False, False), (64, 768, 32, 0, True, False), (64, 4096, 8, 0, True, True), (32, 4096, 20, 2048, True, True)])
+    (128, 8192, 3, 0, True, True), (128, 3072, 20, 1536, False, False), (64, 768, 32, 0, True, False), (64, 4096, 8, 0, True, True), (32, 4096, 20, 2048, False, True),
+    (64, 65536, 1, 0, False, True), (64, 41216, 3, 0, False, False), (16, 1536, 48, 384, False, False),
+    (64, 640, 40, 128, True, False)])
 def test_items_under_a_mask_by_the_order_of_the_launch(plan_items, d_h, S, H, q_start, longest_first, in_order):
     for first, halves in ((1, longest_first), (0, in_order)):
         items256, items128, tiles = plan_items(q_start, S - q_start, S, H, 1, 1, d_h, first)

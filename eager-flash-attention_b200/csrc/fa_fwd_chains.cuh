@@ -81,7 +81,7 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
     }
-    if (tid == 32) {
+    if (tid == 32) {                                       // reads an order table: a launch with one does not start early
         int head, split, row0;
         pick_item((int)(blockIdx.y * gridDim.x + blockIdx.x), a, items_x, items_total, ITEM_ROWS, tail, head, split, row0);
         s_head = head;

@@ -76,8 +76,9 @@ bool own_device_memory(const void* p);
 // projections 77 -> 55); a single kernel on an idle GPU has nothing ahead of it to start under and pays 0.2 to 0.3 us of host time for the
 // attribute and as much for the wait (projection 2496 x 576 x 512 16.4 -> 17.0 us from call to completion, 4160 x 512 x 4096 29.9 -> 30.4).
 // cluster > 1: the blocks along the grid's third dimension, all of them, are a cluster.
+// early = false: an ordinary launch, behind all that is ahead of it in the stream.
 template <class... P, class... A>
-cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)
+cudaError_t launch_kernel(bool early, int cluster, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -86,7 +87,7 @@ cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, u
     cfg.stream = stream;
     cudaLaunchAttribute attr[2]{};
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = (unsigned)cluster;
@@ -95,6 +96,11 @@ cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, u
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
     if (e != cudaSuccess) (void)cudaGetLastError();        // reported here: not once more by whoever asks next
     return e;
+}
+template <class... P, class... A>
+cudaError_t launch_early_cluster(int cluster, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)
+{
+    return launch_kernel(true, cluster, kernel, grid, threads, smem, stream, args...);
 }
 template <class... P, class... A>
 cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args)

@@ -32,7 +32,7 @@ def _definition(text, name):
 
 def _early_kernels():
     sources = _sources()
-    names = {n for text in sources.values() for n in re.findall(r"launch_early(?:_cluster)?\((?:\w+,\s*)?(\w+_kernel)\b", text)}
+    names = {n for text in sources.values() for n in re.findall(r"launch_(?:early|early_cluster|kernel)\((?:\w+,\s*)*(\w+_kernel)\b", text)}
     found = {}
     for name in names:
         bodies = [b for b in (_definition(text, name) for text in sources.values()) if b]
@@ -63,3 +63,18 @@ def test_helpers_that_kernels_share_presume_no_read_only_memory():
     for name in ("sm100_ptx.cuh", "fa_args.cuh", "work_order.h"):
         with open(os.path.join(CSRC, name)) as f:
             assert not re.search(r"__restrict__|__ldg\b|global\.nc\b", f.read())
+
+
+def test_an_order_table_is_not_read_while_it_may_be_written():
+    """order_tab, which pick_item reads, is device memory. A kernel that picks its item ahead of pdl_wait() is not launched early with a table."""
+    kernels = {name: body for name, body in _early_kernels().items() if re.search(r"\bpick_item\(|order_tab", body)}
+    assert set(kernels) == {"fa_fwd_ws_kernel", "fa_fwd_chains_kernel"}
+    text = "".join(_sources().values())
+    for name, body in kernels.items():
+        body = re.sub(r"auto (\w+) = \[&\]\([^)]*\)(?: -> \w+)? \{.*?\n    \};", "", body, flags=re.S)     # what they define is judged where it is called
+        ahead = re.search(r"\b(?:fetch_item|pick_item)\(", body.split("pdl_wait()", 1)[0])
+        launches = re.findall(r"launch_(early|kernel)\((?:(\w+), \d, )?" + name + "<", text)
+        assert launches
+        if ahead:
+            assert set(launches) == {("kernel", "early")}, name
+            assert text.count("const bool early = args.order_tab == nullptr;") == len(launches), name

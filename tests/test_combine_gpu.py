@@ -4,7 +4,7 @@ import pytest
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("split", [2, 3, 4, 8, 16])
+@pytest.mark.parametrize("split", [2, 3, 4, 5, 6, 8, 15, 16])
 @pytest.mark.parametrize("rows,row0,H,d_h,f16", [(64, 0, 3, 16, True), (192, 64, 5, 64, False), (2048, 0, 2, 128, True)])
 def test_merge(pkg, torch_cuda, split, rows, row0, H, d_h, f16):
     torch = torch_cuda

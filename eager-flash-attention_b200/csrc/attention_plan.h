@@ -66,11 +66,13 @@ inline FaPlan plan_items(const PlanShape& a)
     // Small heads with few keys and more than one wave of anything: the one-tile kernel. Two small blocks to an SM are faster up to two
     // stages, and above that where the 256-row items are more than one wave and end less evenly (the figures are in
     // fa_fwd_tile_sm100.cu). Without a mask that is so where the last wave of items is poorly filled (below four stages), or where they take more
-    // waves than the tiles do two to an SM: a third more up to three stages, half as many again to five. Under a mask below four stages. Over 900 shapes of
-    // one to six and a half stages the form taken is 2 % slower than the better one in the mean (0.8 % without a mask; always the one-tile kernel 13 %, never 4 %).
+    // waves than the tiles do two to an SM: a third more up to three stages, half as many again to five. Under a mask below four stages, and
+    // to six and a half by the same half more where items are of about one length or tiles more than one wave. Over 900 shapes of one to six and a half
+    // stages the form taken is 1.9 % slower than the better one in the mean (0.8 % without a mask; always the one-tile kernel 13 %, never 4 %).
     const long pairs = (total128 + 2 * sms - 1) / (2 * sms);                   // waves of tiles
-    const bool uneven = a.causal ? stages < 4
-                                 : (stages < 4 && total * 10 < waves256 * sms * 7) || (stages <= 3 ? waves256 * 3 >= pairs * 4 : stages <= 5 && waves256 * 2 >= pairs * 3);
+    const bool half_more = waves256 * 2 >= pairs * 3;
+    const bool uneven = a.causal ? stages < 4 || (stages < 6.5 && half_more && (even || pairs > 1))
+                                 : (stages < 4 && total * 10 < waves256 * sms * 7) || (stages <= 3 ? waves256 * 3 >= pairs * 4 : stages <= 5 && half_more);
     if (a.d_h < 64 && a.free_form && total128 > sms && (stages <= 2 || (waves256 > 1 && uneven))) {
         plan.items256 = 0;
         plan.tiles = (int)total128;

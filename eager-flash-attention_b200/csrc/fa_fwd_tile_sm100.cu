@@ -6,8 +6,8 @@
 // other's; the kernel of four chains has the SM to itself, but is faster per stage. The line lies at two stages: 592 items of 256 rows, d_h 16 / 32,
 // 8.8 / 9.5 us here against 15.1 / 16.1 (one stage), 23.9 / 26.4 against 24.4 / 27.2 (two), 32.1 / 36.5 against 29.9 / 34.8 (three), 48 / 53 against
 // 41 / 47 (five). Under a mask, or where a last wave of 256-row items is poorly filled, the smaller blocks also end more evenly, which
-// decides between two and five stages of more than one wave: causal, 100 heads x 512 rows 12.2 / 12.8 against 13.3 / 14.4, 75 x 640 12.6 / 13.2 against
-// 15.4 / 16.9 (148 x 512 15.0 / 15.9 against 14.1 / 15.3); without a mask 160 heads x 256
+// decides between two and six stages of more than one wave: causal, 100 heads x 512 rows 12.2 / 12.8 against 13.3 / 14.4, 75 x 640 12.6 / 13.2 against
+// 15.4 / 16.9 (148 x 512 15.0 / 15.9 against 14.1 / 15.3), 90 x rows 320 to 640 (d_h 32) 13.5 against 18.1; without a mask 160 heads x 256
 // rows x 384 keys 14.9 / 15.9 against 14.6 / 16.5, 50 x 640 12.4 / 13.2 against 16.8 / 18.4, 110 x 640 24.4 / 25.4 against 27.0 / 29.2, 160 x 384 16.0 / 17.1 against
 // 18.6 / 20.5, 250 x 384 23.3 / 24.3 against 25.7 / 28.0 (200 x 384 22.0 / 23.0 against 20.3 / 22.1, 160 x 576 37.1 / 38.9 against 33.6 / 36.2); but 64 x 512, one
 // wave, 11.0 / 11.3 against 8.9 / 9.8, four stages (100 x 768) 21.8 / 22.8 against 21.1 / 22.7, 16 x 2048 32.7 / 34.0 against 16.4 / 17.7 (as 128-row items).

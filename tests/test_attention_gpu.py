@@ -191,11 +191,12 @@ def form(pkg, H, d_h, S, q_start, q_rows, split, causal):
     return "+".join(n for n, items in (("256", plan.items_256), ("128", plan.items_128), ("tiles", plan.tiles)) if items)
 
 
-# One to five key stages (more than the ring of two keeps), ragged last blocks, rows that see no key of a split, both directions of the mask.
+# One to seven key stages (more than the ring of two keeps), ragged last blocks, rows that see no key of a split, both directions of the mask.
 @pytest.mark.parametrize("d_h", [16, 32])
 @pytest.mark.parametrize("H,S,q_start,q_rows,split,causal", [
     (160, 64, 0, 64, 1, 0), (100, 256, 0, 256, 1, 1), (152, 192, 64, 128, 1, 1), (80, 640, 320, 320, 1, 0), (50, 640, 0, 640, 1, 0),
-    (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (25, 1280, 192, 576, 2, 0), (160, 384, 0, 384, 1, 0), (160, 448, 192, 256, 1, 0), (75, 640, 0, 640, 1, 1)])
+    (80, 448, 0, 192, 1, 1), (12, 1024, 0, 1024, 4, 1), (25, 1280, 192, 576, 2, 0), (160, 384, 0, 384, 1, 0), (160, 448, 192, 256, 1, 0), (75, 640, 0, 640, 1, 1),
+    (75, 896, 0, 896, 1, 1), (90, 640, 320, 320, 1, 1), (190, 640, 512, 128, 1, 1)])
 def test_single_tiles_against_float64(pkg, torch_cuda, d_h, H, S, q_start, q_rows, split, causal):
     assert form(pkg, H, d_h, S, q_start, q_rows, split, causal) == "tiles"
     check_against_float64(pkg, torch_cuda, H, d_h, S, q_start, q_rows, split, causal)

@@ -56,10 +56,13 @@ def test_items_under_a_mask_by_the_order_of_the_launch(plan_items, d_h, S, H, q_
         assert ((items256 > 0), (items128 > 0), tiles) == (not halves, halves, 0), first
 
 
-# Without a mask by waves: of 256-row items against those of tiles, two to an SM.
+# By waves: of 256-row items against those of tiles, two to an SM; under a mask where items are of about one length or tiles more than a wave.
 @pytest.mark.parametrize("S,H,causal,item_rows", [(640, 50, 0, 0), (640, 110, 0, 0), (640, 60, 0, 256), (640, 160, 0, 256), (384, 160, 0, 0), (384, 250, 0, 0), (384, 200, 0, 256),
-                                             (576, 160, 0, 256), (512, 148, 0, 256), (896, 60, 1, 256), (768, 75, 1, 256), (640, 75, 1, 0)])
+                                             (576, 160, 0, 256), (512, 148, 0, 256), (896, 60, 1, 256), (896, 75, 1, 0), (768, 75, 1, 256), (640, 75, 1, 0)])
 def test_few_keys_by_waves(plan_items, S, H, causal, item_rows):
+    if causal:          # a window of the last rows: items of 4.25 to 6 stages
+        assert plan_items(320, 320, 640, 90, 1, 1, 32, 1) == plan_items(320, 320, 640, 90, 1, 1, 32, 0) == (0, 0, 270)
+        assert plan_items(512, 128, 640, 190, 1, 1, 16, 0) == (0, 0, 190) and plan_items(128, 640, 768, 50, 1, 1, 16, 1) == (150, 0, 0)
     want = (0, 0, H * ((S + 127) // 128)) if item_rows == 0 else (H * ((S + 255) // 256), 0, 0)
     assert plan_items(0, S, S, H, 1, causal, 32, 1) == want
 

@@ -38,9 +38,13 @@ def check(torch, out, q, k, v, q_start, q_rows, causal):
         assert bool((err <= bound).all()), (h, float((err - bound).max()))
 
 
+def launched(plan):
+    return "+".join(n for n, items in (("256", plan.items_256), ("128", plan.items_128), ("tiles", plan.tiles)) if items)
+
+
 @pytest.mark.gpu
-# One to nine blocks of 64 keys (chains without a block, ragged halves of a stage), one to four 64-row blocks, and beyond the K/V ring; few
-# heads: 128-row items on four chains, many: 256-row items on two chains per tile.
+# One to nine blocks of 64 keys (chains without a block, ragged halves of a stage), one to four 64-row blocks, and beyond the K/V ring. Two heads: 128-row
+# items on four chains. 300: 256-row items on two chains per tile; at d_h 16 and 32, but for the longest, the kernel of one tile.
 @pytest.mark.parametrize("d_h", [16, 32, 64])
 @pytest.mark.parametrize("H", [2, 300])
 @pytest.mark.parametrize("S,q_start,q_rows,split,causal", [(64, 0, 64, 1, 0), (128, 64, 64, 1, 1), (192, 0, 192, 1, 0), (320, 64, 256, 1, 1), (576, 0, 64, 1, 0),
@@ -50,9 +54,55 @@ def test_blocks_of_keys_and_rows(pkg, torch_cuda, d_h, H, S, q_start, q_rows, sp
     g = torch.Generator(device="cuda").manual_seed(S + d_h)
     q, k, v = (torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
     counters = torch.zeros(q_rows // 64, dtype=torch.int32, device="cuda")
-    out, _ = attention(pkg, torch, q, k, v, q_start, q_rows, split, causal, counters)
+    out, plan = attention(pkg, torch, q, k, v, q_start, q_rows, split, causal, counters)
+    assert launched(plan) == ("128" if H == 2 else "256" if d_h == 64 or S == 1344 else "tiles")
     check(torch, out, q, k, v, q_start, q_rows, causal)
     assert counters.tolist() == [H * split] * (q_rows // 64)
+
+
+@pytest.mark.gpu
+# Two chains per tile with as few keys, at all head sizes: chains without a block (320), 64 rows in the second tile, a split that has keys for 64 of 256 rows, ragged splits.
+@pytest.mark.parametrize("d_h", [16, 32, 64])
+@pytest.mark.parametrize("S,q_start,q_rows,split,causal", [(320, 64, 256, 1, 1), (448, 256, 192, 1, 0), (640, 320, 192, 1, 0), (1024, 320, 256, 2, 1),
+                                                           (1152, 640, 192, 2, 1)])
+def test_two_chains_per_tile_with_few_keys(pkg, torch_cuda, d_h, S, q_start, q_rows, split, causal):
+    torch = torch_cuda
+    H = 140 // split
+    g = torch.Generator(device="cuda").manual_seed(S + d_h)
+    q, k, v = (torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    for counters in (None, torch.zeros(q_rows // 64, dtype=torch.int32, device="cuda")):
+        out, plan = attention(pkg, torch, q, k, v, q_start, q_rows, split, causal, counters)
+        assert launched(plan) == "256"
+        check(torch, out, q, k, v, q_start, q_rows, causal)
+    assert counters.tolist() == [H * split] * (q_rows // 64)
+
+
+@pytest.mark.gpu
+# 128-row items, 256-row items, the kernel of one tile, and splits
+@pytest.mark.parametrize("d_h,H,S,split,want", [(16, 2, 512, 1, "128"), (32, 2, 1024, 2, "128"), (64, 2, 512, 1, "128"), (16, 74, 512, 1, "256"), (32, 148, 512, 1, "256"),
+                                                (64, 300, 512, 1, "256"), (64, 100, 1024, 2, "256"), (32, 200, 256, 1, "tiles"), (128, 2, 512, 1, "128"), (128, 150, 512, 1, "256")])
+@pytest.mark.parametrize("causal", [0, 1])
+def test_infinite_scores(pkg, torch_cuda, d_h, H, S, split, want, causal):
+    """Keys that score -inf have no weight, whichever chains have nothing else; a row that has a key scoring +inf, or none but such scoring -inf, is no number."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(S + d_h)
+    q, k, v = (torch.randn(H, S, d_h, generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    q[..., 0] = q[..., 0].abs() + 0.125
+    block = torch.arange(S, device="cuda") // 64
+    assert launched(attention(pkg, torch, q, k, v, 0, S, split, 0)[1]) == want
+    for gone in (block == 1, block % 2 == 1, block % 4 != 0, (block % 2 == 0) & (torch.arange(S, device="cuda") > 0), torch.arange(S, device="cuda") >= 3):
+        x = k.clone()
+        x[:, gone, 0] = float("-inf")
+        out, _ = attention(pkg, torch, q, x, v, 0, S, split, causal)
+        check(torch, out, q, x, v, 0, S, causal)
+    x = k.clone()
+    x[:, S // 2 + 70, 0] = float("inf")
+    out, _ = attention(pkg, torch, q, x, v, 0, S, split, causal)
+    seen = S // 2 + 70 if causal else 0
+    assert torch.isnan(out[seen:]).all() and torch.isfinite(out[:seen]).all()
+    x[..., 0] = float("-inf")
+    out, _ = attention(pkg, torch, q, x, v, 0, S, split, causal)
+    assert torch.isnan(out).all()
 
 
 @pytest.mark.gpu

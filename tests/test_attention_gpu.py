@@ -303,9 +303,10 @@ def test_merge_of_partials_by_number_of_rows(pkg, torch_cuda, rows, split, H, d_
     assert bool(((out.double() - want).abs() <= 16 * 2 ** -24 * (1 + want.abs().max())).all())
 
 
-# Launches that compute a share of the exponentials as a polynomial (d_h 128, and 128-row items of 16 and 32), and two that do not (d_h 64,
-# one wave of 128-row items and three).
-@pytest.mark.parametrize("S,H,d_h,split", [(512, 2, 128, 1), (4096, 13, 128, 1), (256, 4, 64, 1), (512, 2, 16, 1), (256, 2, 32, 2), (4096, 12, 64, 1)])
+# A share of the exponentials is a polynomial: of the four chains (d_h 16 to 64, items of 128 and 256 rows) columns 14 and 15 of every 16, at d_h 128 (both
+# kinds of items) 6 and 7 of every eight; none of the kernel of one tile (100 heads of 32, 256 keys).
+@pytest.mark.parametrize("S,H,d_h,split", [(512, 2, 128, 1), (4096, 13, 128, 1), (256, 4, 64, 1), (512, 2, 16, 1), (256, 2, 32, 2), (4096, 12, 64, 1),
+                                            (1536, 30, 32, 1), (256, 100, 32, 1)])
 def test_weights_over_the_whole_exponent_range(pkg, torch_cuda, S, H, d_h, split):
     """Scores spread over several hundred powers of two, so that most weights vanish, some of them below the smallest number;
     and a NaN in the keys reaches every row, whichever way its exponential is computed."""
@@ -320,18 +321,17 @@ def test_weights_over_the_whole_exponent_range(pkg, torch_cuda, S, H, d_h, split
         got = O.view(S, H, d_h)[:, h].double()
         # fp16 weights (2^-11 each) of values up to max |V|, fp32 scores of up to 2^9: 2^-24 * 2^9 in the exponent
         assert bool(((got - want).abs() <= (2 ** -11 + 2 ** -13) * v.abs().max()).all())
-    for key in (S - 128 + 70, 5):                              # of pairs that go the one way and the other
+    for key in (S - 128 + 78, S - 128 + 79, S - 128 + 70, 5):  # both columns of a pair that goes the one way, and two that go the other (70: at d_h up to 64)
         bad = [x.clone() for x in dev]
         bad[1][:, key, 3] = float("nan")
         O, _ = run_attention(pkg, torch, p, bad, 0, S, pkg.F32)
         assert torch.isnan(O).all()
 
 
-# A share of the exponentials as a polynomial (columns 6 and 7 of every eight): items of 256 rows at d_h 128, of 128 rows at 32 and 16; d_h 64
-# has none. One position of the key to a head and split, so that all eight columns occur.
-@pytest.mark.parametrize("S,H,d_h,poly,items128", [(4096, 8, 128, True, False), (1024, 4, 128, True, True), (1024, 4, 32, True, True),
-                                                  (1024, 4, 16, True, True), (4096, 8, 64, False, False)])
-def test_each_weight_is_as_exact_as_its_exponential(pkg, torch_cuda, S, H, d_h, poly, items128):
+# Of the columns of 16, 8 to 15, one to a head and split: those of the polynomial (14 and 15, at d_h 128 6 and 7 of every eight) and others.
+@pytest.mark.parametrize("S,H,d_h,items128", [(4096, 8, 128, False), (1024, 4, 128, True), (1024, 4, 32, True), (1024, 4, 16, True), (4096, 8, 64, False),
+                                              (4096, 8, 32, False), (4096, 8, 16, False), (1024, 4, 64, True)])
+def test_each_weight_is_as_exact_as_its_exponential(pkg, torch_cuda, S, H, d_h, items128):
     """Two keys per row and split carry weight, the maximum (weight 1) and one of 2^x, x from -1 to 0 over the rows: the fp32
     denominator shows the exponential itself, with one rounding."""
     torch = torch_cuda
@@ -350,7 +350,8 @@ def test_each_weight_is_as_exact_as_its_exponential(pkg, torch_cuda, S, H, d_h, 
     column = torch.empty(split, H, dtype=torch.int64)
     for i in range(split):
         for h in range(H):
-            column[i, h] = (2 * h + i) % 8 + 8 * ((5 * h + 3 * i) % 16)
+            # behind the maximum in the same chain: 64 keys further chains of 64 keys change, and the weight is one of their merge
+            column[i, h] = (2 * h + i) % 8 + 8 + 16 * ((5 * h + 3 * i) % (8 if d_h == 128 else 4))
             K[h, i * (S // split) + 9, 2] = 0                   # score 0, in the first stage of 128 keys
             K[h, i * (S // split) + 256 + column[i, h], :3] = torch.tensor([-1, -2.0 ** -12, 0])
     ws = [torch.full((n,), float("nan"), device="cuda") for n in (split * S * H * d_h, split * S * H, split * S * H)]
@@ -362,7 +363,8 @@ def test_each_weight_is_as_exact_as_its_exponential(pkg, torch_cuda, S, H, d_h, 
     score = -(Q[..., 0].float() + Q[..., 1].float() * 2.0 ** -12).T          # exact in fp32
     w = torch.exp2((score * 1.4426950408889634).double())                     # the argument rounded to fp32, as the kernel has it
     err = (l.double() - (1 + w)).abs()
-    by_poly = (column % 8 >= 6).to(err.device)[:, None, :] & poly
+    by_poly = (column % 16 >= 14 if d_h <= 64 else column % 8 >= 6).to(err.device)[:, None, :]
+    assert {14, 15} <= {int(c) % 16 for c in column.flatten()}
     # the error stated for either way, and the rounding of a sum between 1 and 2
     bound = torch.where(by_poly, 1.8e-7, 2.0 ** -22) * w + 2.0 ** -24
     assert bool((err <= bound).all()), float((err - bound).max())

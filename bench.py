@@ -38,8 +38,8 @@ REDUCE_BY_RANKS = {1: "nccl", 2: "pull", 4: "pull", 8: "pull"}
 
 # DRAM bytes (read + written) of one attention launch of the benchmark shape with all 32 heads on one GPU, by
 # (mode, rows taken last-first): ncu captures, one launch each. "alone": longest items first over groups of heads, as every causal launch
-# without tile counters takes them (stream mode on one rank with the library's own plan); four times a launch of eight heads.
-ATTN_TRAFFIC_32_HEADS = {("stream", False): 5.105e9, ("stream", True): 5.212e9, ("alone", True): 1.389e9}
+# without tile counters takes them (stream mode on one rank with the library's own plan).
+ATTN_TRAFFIC_32_HEADS = {("stream", False): 5.105e9, ("stream", True): 5.212e9, ("alone", True): 1.449e9}
 
 
 def measured_peaks():
@@ -440,9 +440,8 @@ def main():
                           frac_sustained=achieved / pk["tflops_sustained"], attn_kernel_ms=attn_ms,
                           algorithmic_flops=fl,
                           # dram__bytes_read.sum + dram__bytes_write.sum of this kernel's launch, from one ncu capture of
-                          # the benchmark shape on one rank (32 heads; launches without counters: of eight heads, times four); groups
-                          # of heads are independent, so a rank's traffic is that figure times H_local / 32. Shapes that were not captured
-                          # report null.
+                          # the benchmark shape on one rank (32 heads); groups of heads are independent, so a rank's traffic is that
+                          # figure times H_local / 32. Shapes that were not captured report null.
                           traffic=(ATTN_TRAFFIC_32_HEADS.get((order, descending)) * p.H_local / 32
                                    if (p.S == 32768 and p.d_h == 128 and p.causal and p.split == 1
                                        and (order, descending) in ATTN_TRAFFIC_32_HEADS) else None),

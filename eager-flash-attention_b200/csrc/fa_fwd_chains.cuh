@@ -28,7 +28,9 @@ struct ChainCfg {
     static constexpr int SWB        = D >= 64 ? 128 : D * 2;      // swizzle width = TMA box row, bytes
     static constexpr int TILE_BYTES = 128 * D * 2;
     static constexpr int TILES      = 4 / WAYS;
-    static constexpr int NS         = 4;                          // K slots, and V slots, of 128 keys
+    // K slots, and V slots, of 128 keys. Four chains on one tile of 64 take a stage in 0.7 us; with four slots the keys are asked for too late where they come from
+    // memory: 13952 rows, four heads (us, keys in the L2 / not) 238 / 285, with six 236 / 256 (the kernel of two chains 272 / 275). No more room at 256 rows, and no need.
+    static constexpr int NS         = D == 64 && WAYS == 4 ? 6 : 4;
     static constexpr int SMEM_BYTES = TILE_BYTES * (TILES + 2 * NS) + 1024;
     static constexpr int USERS      = 2 * TILES;                  // chains that read a slot: each takes 64 of its keys
     static_assert(D <= 64 && NS % 2 == 0, "a chain that takes every second stage would skip phases of a slot");

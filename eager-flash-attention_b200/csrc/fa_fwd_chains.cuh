@@ -28,12 +28,15 @@ struct ChainCfg {
     static constexpr int SWB        = D >= 64 ? 128 : D * 2;      // swizzle width = TMA box row, bytes
     static constexpr int TILE_BYTES = 128 * D * 2;
     static constexpr int TILES      = 4 / WAYS;
-    // K slots, and V slots, of 128 keys. Four chains on one tile of 64 take a stage in 0.7 us; with four slots the keys are asked for too late where they come from
-    // memory: 13952 rows, four heads (us, keys in the L2 / not) 238 / 285, with six 236 / 256 (the kernel of two chains 272 / 275). No more room at 256 rows, and no need.
-    static constexpr int NS         = D == 64 && WAYS == 4 ? 6 : 4;
-    static constexpr int SMEM_BYTES = TILE_BYTES * (TILES + 2 * NS) + 1024;
+    // K slots and V slots of 128 keys. Four chains on one tile of 64 take a stage in 0.7 us and give V back a stage of theirs after K; with four slots it is asked
+    // for too late where keys come from memory. 13952 rows, four heads, inputs in turn / behind a flush of the L2 (us): two chains 282 / 316, 4 + 4 slots 290 / 329,
+    // 6 + 4 286 / 317, 4 + 6 265 / 292, 6 + 6 256 / 283; but of launches between other kernels, 768 rows, two heads behind a fill 12.8, 12.8, 12.8, 12.8, 13.6, and one
+    // tile in eight splits with its merge 28.2, 24.7, 25.3, 24.6, 25.3. 256-row items have no room for six and lose nothing with four.
+    static constexpr int NSK        = 4;
+    static constexpr int NSV        = D == 64 && WAYS == 4 ? 6 : 4;
+    static constexpr int SMEM_BYTES = TILE_BYTES * (TILES + NSK + NSV) + 1024;
     static constexpr int USERS      = 2 * TILES;                  // chains that read a slot: each takes 64 of its keys
-    static_assert(D <= 64 && NS % 2 == 0, "a chain that takes every second stage would skip phases of a slot");
+    static_assert(D <= 64 && NSK % 2 == 0 && NSV % 2 == 0, "a chain that takes every second stage would skip phases of a slot");
 };
 constexpr int CH_THREADS = 768;
 
@@ -45,7 +48,7 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
                      const FaArgs a, int items_x, int items_total)
 {
     using C = ChainCfg<D, WAYS>;
-    constexpr int TILES = C::TILES, NS = C::NS, ITEM_ROWS = TILES * WS_BM;
+    constexpr int TILES = C::TILES, NSK = C::NSK, NSV = C::NSV, ITEM_ROWS = TILES * WS_BM;
     constexpr uint32_t SWZ = swizzle_code(C::SWB);
     constexpr uint32_t IDESC_QK = idesc_f16_f32(WS_BM, 64, 0, 0);
     constexpr uint32_t IDESC_PV = idesc_f16_f32(WS_BM, D, 0, 1);
@@ -56,11 +59,11 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = smem;                                   // TILES tiles
-    uint8_t* sK = sQ + TILES * C::TILE_BYTES;             // NS stages
-    uint8_t* sV = sK + NS * C::TILE_BYTES;                // NS stages
+    uint8_t* sK = sQ + TILES * C::TILE_BYTES;             // NSK stages
+    uint8_t* sV = sK + NSK * C::TILE_BYTES;               // NSV stages
 
     __shared__ __align__(8) uint64_t q_full[TILES];
-    __shared__ __align__(8) uint64_t k_full[NS], k_empty[NS], v_full[NS], v_empty[NS];
+    __shared__ __align__(8) uint64_t k_full[NSK], k_empty[NSK], v_full[NSV], v_empty[NSV];
     __shared__ __align__(8) uint64_t s_full[4], p_full[4], o_done[4];
     __shared__ float ends[4][3][WS_BM];                   // offset, maximum and sum of every chain's rows
     __shared__ uint32_t tmem_base_smem;
@@ -76,7 +79,8 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (tid == 0) {
         abort_word = 0;
         for (int t = 0; t < TILES; t++) { mbar_init(&q_full[t], 1); half_done[t][0] = half_done[t][1] = 0; }
-        for (int s = 0; s < NS; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], C::USERS); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], C::USERS); }
+        for (int s = 0; s < NSK; s++) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], C::USERS); }
+        for (int s = 0; s < NSV; s++) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], C::USERS); }
         for (int c = 0; c < 4; c++) { mbar_init(&s_full[c], 1); mbar_init(&p_full[c], WS_BM / 32); mbar_init(&o_done[c], 1); }
         mbar_fence_init();
         tma_prefetch_desc(&tmQ);
@@ -127,17 +131,17 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
                 if (n[t] > 0) load(sQ + t * C::TILE_BYTES, &tmQ, &q_full[t], abs0(t));
             }
             for (int j = 0; 2 * j < most; j++) {
-                const int s = j % NS, u = j / NS;
+                const int s = j % NSK, u = j / NSK, sv = j % NSV, uv = j / NSV;
                 if (u > 0 && !mbar_wait(&k_empty[s], (uint32_t)((u - 1) & 1), &abort_word, 21)) break;
                 load(sK + s * C::TILE_BYTES, &tmK, &k_full[s], kv_lo + j * WS_BN);
-                if (u > 0 && !mbar_wait(&v_empty[s], (uint32_t)((u - 1) & 1), &abort_word, 22)) break;
-                load(sV + s * C::TILE_BYTES, &tmV, &v_full[s], kv_lo + j * WS_BN);
+                if (uv > 0 && !mbar_wait(&v_empty[sv], (uint32_t)((uv - 1) & 1), &abort_word, 22)) break;
+                load(sV + sv * C::TILE_BYTES, &tmV, &v_full[sv], kv_lo + j * WS_BN);
                 int users = 0;
                 #pragma unroll
                 for (int t = 0; t < TILES; t++) users += max(0, min(2, n[t] - 2 * j));
                 for (; users < C::USERS; users++) {           // for chains that end before this stage
                     mbar_arrive(&k_empty[s]);
-                    mbar_arrive(&v_empty[s]);
+                    mbar_arrive(&v_empty[sv]);
                 }
             }
         }
@@ -166,8 +170,8 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
         auto give_back = [&](int i) -> bool {
             if (!wait(&s_full[c], i, 22)) return false;
             if (lane == 0) {
-                mbar_arrive(&k_empty[stage_of(way, i) % NS]);
-                if (i > 0) mbar_arrive(&v_empty[stage_of(way, i - 1) % NS]);
+                mbar_arrive(&k_empty[stage_of(way, i) % NSK]);
+                if (i > 0) mbar_arrive(&v_empty[stage_of(way, i - 1) % NSV]);
             }
             __syncwarp();
             return true;
@@ -176,22 +180,22 @@ fa_fwd_chains_kernel(const __grid_constant__ CUtensorMap tmQ,
         bool ok = n > 0 && wait(&q_full[tile], 0, 24);
         if (ok) {
             const int j = stage_of(way, 0);
-            ok = wait(&k_full[j % NS], j / NS, 27);
+            ok = wait(&k_full[j % NSK], j / NSK, 27);
             tc_fence_after_sync();
-            if (ok && elect_one()) issue_qk(j % NS);
+            if (ok && elect_one()) issue_qk(j % NSK);
             __syncwarp();
         }
         for (int i = 0; i < n && ok; i++) {
             const int j = stage_of(way, i), next = stage_of(way, i + 1);
             const bool more = i + 1 < n;
-            ok = give_back(i) && wait(&v_full[j % NS], j / NS, 25) && (!more || wait(&k_full[next % NS], next / NS, 28)) && wait(&p_full[c], i, 26);
+            ok = give_back(i) && wait(&v_full[j % NSV], j / NSV, 25) && (!more || wait(&k_full[next % NSK], next / NSK, 28)) && wait(&p_full[c], i, 26);
             tc_fence_after_sync();
             if (!ok) break;
             if (elect_one()) {
                 #pragma unroll
                 for (int ks = 0; ks < 4; ks++)
-                    tc_mma_ts_lh(tO, tS + ks * 8, dv_lo + (j % NS) * (C::TILE_BYTES >> 4) + ((ks * 16 * C::SWB) >> 4), dv_hi, IDESC_PV, ks > 0 || i > 0 ? 1u : 0u);
-                if (more) issue_qk(next % NS); else tc_commit(&o_done[c]);
+                    tc_mma_ts_lh(tO, tS + ks * 8, dv_lo + (j % NSV) * (C::TILE_BYTES >> 4) + ((ks * 16 * C::SWB) >> 4), dv_hi, IDESC_PV, ks > 0 || i > 0 ? 1u : 0u);
+                if (more) issue_qk(next % NSK); else tc_commit(&o_done[c]);
             }
             __syncwarp();
         }

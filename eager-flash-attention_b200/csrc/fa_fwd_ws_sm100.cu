@@ -787,7 +787,8 @@ void ring_of(FaPlan& plan, bool halves)
         plan.k_slots = halves ? WsCfg<D, true>::NSTAGE_K : WsCfg<D, false>::NSTAGE_K;
         plan.v_slots = halves ? WsCfg<D, true>::NSTAGE_V : WsCfg<D, false>::NSTAGE_V;
     } else {
-        plan.k_slots = plan.v_slots = halves ? ChainCfg<D, 4>::NS : ChainCfg<D, 2>::NS;
+        plan.k_slots = halves ? ChainCfg<D, 4>::NSK : ChainCfg<D, 2>::NSK;
+        plan.v_slots = halves ? ChainCfg<D, 4>::NSV : ChainCfg<D, 2>::NSV;
     }
     plan.stage_step = halves ? 2 : 1;
 }

@@ -20,7 +20,7 @@
 // us, two 128-key chains to an SM -> this: S=4096, 16 heads of 64 104 -> 94, causal 53.8 -> 50.9; S=16384 causal 720 -> 665; S=65536, two heads of
 // 64 2710 -> 2594 (power: 1.75 GHz); S=4032, eight heads of 32 54.3 -> 49.0; S=16384, 16 heads of 32 1326 -> 1200, four heads of 16 374 -> 323;
 // S=1024, eight heads of 64 (128-row items) 10.7 -> 9.5. One tile of 128 rows without a workspace (offset = maximum, so O is rescaled
-// more often) 28.3 -> 29.2 in eight splits, 112 -> 103 in one.
+// more often) 27.2 -> 23.1 in eight splits with the merge, 110 -> 100 in one.
 #pragma once
 
 template <int D, int WAYS>
